@@ -36,7 +36,7 @@ if not Path(NVCC).exists():
 NVCC_FLAGS = ARCH + [
     "-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
     "-Xcompiler", "-fPIC,-O3", "-I" + str(INCLUDE), "-I" + str(CSRC),
-    "-diag-suppress", "177",
+    "-diag-suppress", "177,550,1886",
 ]
 CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-Wall", "-ffp-contract=off",
              "-I" + str(INCLUDE), "-I" + str(CSRC), "-I" + str(Path(CUDA_HOME) / "include")]

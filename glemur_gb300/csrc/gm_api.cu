@@ -137,10 +137,10 @@ struct Impl : ImplBase {
     int64_t step_launches = 7;      // kernel launches in the captured step
     // TMA-fed stage kernel: tensor maps of X[0], X[1], XS[0], XS[1]
     bool use_tma = true;
-    CUtensorMap tmaps[10];      // single-case kernel (tile height stage_tma_ty<T>(pressure))
+    CUtensorMap tmaps[10];      // single-case kernel (tile height 2 NW2)
     CUtensorMap tmaps_b[10];    // batched kernel (tile height STAGE_BATCH_TY)
     dim3 grid2;
-    int TZ2 = 32;
+    int TZ2 = 32, NW2 = gmk::STAGE_NW;      // planes and row pairs of its tile
     size_t NG = 0, N = 0, NP = 0;
 
     ~Impl() override {
@@ -229,7 +229,17 @@ struct Impl : ImplBase {
             kp.cmc[m] = (double)(T)cd[m] - (double)(T)csd[m];
             kp.cmcT[m] = (T)kp.cmc[m];
         }
-        kp.inv8dxdydz = (T)(1.0 / (8.0 * (double)(T)p->dx * (double)(T)p->dy * (double)(T)p->dz));
+        for (int m = 0; m < 6; m++) {
+            const double b5 = (double)(T)bd[5][m];
+            kp.cb[m] = (T)((double)(T)cd[m] - b5);
+            kp.cbz[m] = kp.zUpdate ? kp.cb[m] : (T)-b5;
+        }
+        kp.vol8 = (T)(8.0 * (double)(T)p->dx * (double)(T)p->dy * (double)(T)p->dz);
+        const T w4[3] = {4 * kp.dy * kp.dz, 4 * kp.dx * kp.dz, 4 * kp.dx * kp.dy};   // as k_scale_b0
+        for (int l = 0; l < 3; l++) {
+            kp.w4[l] = w4[l];
+            kp.w4i[l] = (T)(1.0 / (double)w4[l]);
+        }
         NG = (size_t)(nx + 2) * (ny + 2) * (nz + 2);
         N = (size_t)kp.N;
         NP = (size_t)kp.cs * 3;
@@ -332,12 +342,11 @@ struct Impl : ImplBase {
     // starts (multiples of 32 elements), so every copy starts on a 16-byte
     // boundary.
     int init_tma(int nsm) {
-        CUDA_TRY(gmk::prepare_stage_tma<T>());
-        int rc = encode_maps(tmaps, gmk::stage_tma_ty<T>(gp.pressure));
+        CUDA_TRY(gmk::prepare_stage_tma<T>(gp.pressure));
+        choose_tile(nsm);
+        int rc = encode_maps(tmaps, 2 * NW2);
         if (!rc) rc = encode_maps(tmaps_b, gmk::STAGE_BATCH_TY);
-        if (rc) return rc;
-        choose_tz2(nsm);
-        return GM_OK;
+        return rc;
     }
 
     int encode_maps(CUtensorMap* maps, int ty) {
@@ -370,24 +379,42 @@ struct Impl : ImplBase {
         return GM_OK;
     }
 
-    // z chunking of the single-case TMA kernel: minimise the iterations of the
-    // busiest SM, ceil(tiles / SMs) x (TZ + 2) (the kernel is issue-bound, so
-    // an SM's time follows the work of all the tiles it runs)
-    void choose_tz2(int nsm) {
-        const int nx = kp.nx, ny = kp.ny, nz = kp.nz;
-        const int ty = gmk::stage_tma_ty<T>(gp.pressure);
-        const long long ncol = (long long)((nx + gmk::TX - 1) / gmk::TX) * ((ny + ty - 1) / ty);
+    // Tile height and z chunking of the single-case TMA kernel.  Cost of a choice
+    // in microseconds of a stage, from an iteration's time with m CTAs on an SM
+    // (measured on the FP32 frictional stages, 32x32x32 to 256x256x512): one wave
+    // of CTAs takes its tz + 3 iterations; a little more than one costs nearly two
+    // (128x128x256: 264 CTAs 74 us, 308 97, 352 101, 528 79); many waves keep the
+    // rate of full SMs and end in a part of one.  The taller tile moves 495
+    // points/us and SM against 403, the lower one fills the SMs on small grids
+    // (64x64x128: 94 against 102 us a step; 96x96x192: 250 against 225).
+    double tile_cost(int nw, int tz, int nsm) const {
+        static const double t6[2] = {1.25, 1.55}, t2[4] = {0.85, 0.95, 1.1, 1.27};
+        const int ctas = nw == gmk::STAGE_NW ? 2 : 4;
+        const double* t = nw == gmk::STAGE_NW ? t6 : t2;
+        const long long tiles = tile_columns(nw) * ((kp.nz + tz - 1) / tz), slots = (long long)ctas * nsm;
+        const long long m = (tiles + nsm - 1) / nsm;
+        if (tiles <= slots) return t[m - 1] * (m == ctas ? 1.06 : 1.0) * (tz + 3);   // full SMs end together, late
+        const double w = (double)tiles / slots;
+        return t[ctas - 1] * (tz + 3) * (w <= 2 ? 1.75 + 0.3 * (w - 1) : w + 0.15);
+    }
+    long long tile_columns(int nw) const {
+        return (long long)((kp.nx + gmk::TX - 1) / gmk::TX) * ((kp.ny + 2 * nw - 1) / (2 * nw));
+    }
+    void set_tile(int tz) {
+        TZ2 = tz;
+        grid2 = dim3((unsigned)((kp.nx + gmk::TX - 1) / gmk::TX), (unsigned)((kp.ny + 2 * NW2 - 1) / (2 * NW2)),
+                     (unsigned)((kp.nz + tz - 1) / tz));
+    }
+    void choose_tile(int nsm) {
         double best = 1e300;
-        for (int nzc = 1; nzc <= nz; nzc++) {
-            const int tz = (nz + nzc - 1) / nzc;
-            if (tz < 4 && nz >= 4) break;
-            const long long tiles = ncol * ((nz + tz - 1) / tz);
-            const long long per_sm = (tiles + nsm - 1) / nsm;
-            const double cost = (double)per_sm * (tz + 2);   // tz + 2 iterations per tile
-            if (cost < best * 0.999) { best = cost; TZ2 = tz; }
-        }
-        grid2 = dim3((unsigned)((nx + gmk::TX - 1) / gmk::TX), (unsigned)((ny + ty - 1) / ty),
-                     (unsigned)((nz + TZ2 - 1) / TZ2));
+        int tz_best = kp.nz;
+        for (int nw : {gmk::STAGE_NW, gmk::STAGE_NW_SMALL})
+            for (int nzc = 1; nzc <= kp.nz; nzc++) {
+                const int tz = (kp.nz + nzc - 1) / nzc;
+                const double cost = tile_cost(nw, tz, nsm);
+                if (cost < best * 0.999) { best = cost; tz_best = tz; NW2 = nw; }
+            }
+        set_tile(tz_best);
     }
 
     StageArgs<T> args(int n) {
@@ -462,7 +489,7 @@ struct Impl : ImplBase {
             memcpy(A.tm, tmaps, sizeof tmaps);
             A.a = args(n);
             A.a.TZ = TZ2;
-            CUDA_TRY(gmk::launch_stage_tma<T>(A, gp.pressure, grid2, stream));
+            CUDA_TRY(gmk::launch_stage_tma<T>(A, gp.pressure, NW2, grid2, stream));
         } else {
             if (kp.jxbAver || kp.jOct || kp.jQuint || kp.jTri) {
                 // the averaged Lorentz force reads J and B of this stage at every
@@ -532,7 +559,7 @@ struct Impl : ImplBase {
 
     // Autotuner of the TMA stage kernel's z-chunk depth TZ2 (the tile shape in
     // z: planes a CTA marches through, each chunk paying two halo planes).
-    // Candidates: the eight best depths by the cost model of choose_tz2 and
+    // Candidates: the eight best depths by the cost model of choose_tile and
     // the current one.  Each is timed with CUDA events on the handle's stream over
     // `trials` rounds of stages 0..4 on the uploaded state (those stages write
     // only the stage buffers, not the step-start grid), after one untimed
@@ -548,17 +575,14 @@ struct Impl : ImplBase {
         int dev = 0, nsm = 152;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        const int nx = kp.nx, ny = kp.ny, nz = kp.nz, ty = gmk::stage_tma_ty<T>(gp.pressure);
-        const long long ncol = (long long)((nx + gmk::TX - 1) / gmk::TX) * ((ny + ty - 1) / ty);
+        const int nz = kp.nz;
         std::vector<std::pair<double, int>> cand;
         int last = -1;
         for (int nzc = 1; nzc <= nz; nzc++) {
             const int tz = (nz + nzc - 1) / nzc;
-            if (tz < 4 && nz >= 4) break;
             if (tz == last) continue;
             last = tz;
-            const long long tiles = ncol * ((nz + tz - 1) / tz);
-            cand.emplace_back((double)((tiles + nsm - 1) / nsm) * (tz + 2), tz);
+            cand.emplace_back(tile_cost(NW2, tz, nsm), tz);
         }
         std::sort(cand.begin(), cand.end());
         std::vector<int> tzs;
@@ -571,8 +595,7 @@ struct Impl : ImplBase {
         int best_tz = TZ2;
         int rc = GM_OK;
         for (int tz : tzs) {
-            TZ2 = tz;
-            grid2 = dim3(grid2.x, grid2.y, (unsigned)((nz + tz - 1) / tz));
+            set_tile(tz);
             for (int r = 0; r <= trials && rc == GM_OK; r++) {
                 if (r == 1 && cudaEventRecord(e0, stream) != cudaSuccess) rc = GM_ECUDA;
                 for (int n = 0; n < 5 && rc == GM_OK; n++) rc = stage(n);
@@ -588,8 +611,7 @@ struct Impl : ImplBase {
         }
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        TZ2 = best_tz;
-        grid2 = dim3(grid2.x, grid2.y, (unsigned)((nz + best_tz - 1) / best_tz));
+        set_tile(best_tz);
         if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
         if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
         if (rc != GM_OK) return rc;
@@ -610,8 +632,7 @@ struct Impl : ImplBase {
     int set_tile_z(int tz) override {
         if (!use_tma) return gm::fail(GM_EPARAM, "gm_set_tile_z: the run does not use the TMA stage kernel");
         if (tz < 1 || tz > kp.nz) return gm::fail(GM_EPARAM, "gm_set_tile_z: depth must be 1..nz");
-        TZ2 = tz;
-        grid2 = dim3(grid2.x, grid2.y, (unsigned)((kp.nz + tz - 1) / tz));
+        set_tile(tz);
         if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
         if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
         return GM_OK;

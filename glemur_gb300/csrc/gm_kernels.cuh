@@ -81,7 +81,9 @@ struct KP {
     T c[6], cst[6];          // 5th- and 4th-order weights
     double cmc[6];           // c - c* in double (error norm of errMode 1)
     T cmcT[6];               // c - c* in the run precision
-    T inv8dxdydz;            // 1 / (8 dx dy dz): det(a, b, c) -> Delta
+    T cb[6], cbz[6];         // c - b5 (cbz: along z, -b5 without zUpdate): x_new from x_5
+    T vol8;                  // 8 dx dy dz: 1/det(a, b, c) -> 1/Delta
+    T w4[3], w4i[3];         // scale of B0s (4 dy dz, 4 dx dz, 4 dx dy) and its reciprocal
     double ar, az, phi1;     // analytic-field parameters (distance-to-analytic diagnostic)
     int shear;               // initShearA or initShearB != 0: addDist on the line-tied z ghost planes
     int initDistCode;        // 0: initShearX, 1: centerShift (src/readNamelist.f90)
@@ -177,49 +179,51 @@ template <typename T>
 cudaError_t launch_eps_star(const KP<T>& p, const T* B, const T* J, const T* X, T* scratch, double* out,
                             cudaStream_t s);
 
-// TMA-fed stage kernel (gm_stage_tma.cuh): 32 x 8 tiles, operand planes
-// streamed by cp.async.bulk.tensor.  tm[0..3] are the tensor maps of X[0],
-// X[1], XS[0], XS[1] and tm[4] of B0s (box 36 x 12 x 1 x 3 over (px, py, pz,
-// component)); tm[5..9] those of k_0..k_4 (box 32 x 8 x 1 x 3 over
-// (nx, ny, nz, component) with row pitch kpx).
+// TMA-fed stage kernel (gm_stage_tma.cuh): 32 x 2 nw tiles (nw = STAGE_NW or STAGE_NW_SMALL),
+// operand planes streamed by cp.async.bulk.tensor.  tm[0..3] are the tensor
+// maps of X[0], X[1], XS[0], XS[1] and tm[4] of B0s (box 36 x (2 nw + 4) x 1 x 3
+// over (px, py, pz, component)); tm[5..9] those of k_0..k_4 (box 32 x 2 nw x 1 x
+// 3 over (nx, ny, nz, component) with row pitch kpx).
 template <typename T>
 struct StageArgsTMA {
     CUtensorMap tm[10];
     StageArgs<T> a;
 };
-template <typename T>
-size_t stage_tma_smem_bytes(int pressure, int n);
-template <typename T>
-cudaError_t prepare_stage_tma();
-template <typename T>
-int stage_tma_occupancy(int pressure);
-template <typename T>
-cudaError_t launch_stage_tma(const StageArgsTMA<T>& A, int pressure, dim3 grid, cudaStream_t s);
-// Row groups of the single-case FP32 pressure stage kernel's tile (32 x 8
-// STAGE_ROWS columns) and the tile heights of the single-case and batched
-// launches.
-#ifndef GM_STAGE_ROWS
-#define GM_STAGE_ROWS 2
-#endif
-constexpr int STAGE_ROWS = GM_STAGE_ROWS;
-constexpr int STAGE_BATCH_TY = 8;
-// Two row groups pay where a point has much work (the pressure gradient:
-// 30.6 against 28.9 G cell-RK-stages/s on 256x256x512); without it the third
-// CTA per SM that one row group allows is worth more (36.3 against 34.7 G on
-// the 128x128x256 braid).  FP64 keeps one: two would not fit two CTAs'
-// shared memory per SM.
+// The launchers with the pressure flag as a template parameter are instantiated
+// one translation unit each (gm_stage_f32.cu, ...), which compile in parallel.
 template <typename T, bool PRESS>
-constexpr int stage_rows() { return (sizeof(T) == 4 && PRESS) ? STAGE_ROWS : 1; }
+cudaError_t prepare_stage_tma_p();
+template <typename T, bool PRESS>
+cudaError_t launch_stage_tma_p(const StageArgsTMA<T>& A, int nw, dim3 grid, cudaStream_t s);
+template <typename T, bool PRESS>
+int stage_tma_batch_occupancy_p();
+template <typename T, bool PRESS>
+cudaError_t launch_stage_tma_batch_p(const StageArgsTMA<T>* cases, const int4* work, int nwork, int* counter, int n,
+                                     int nblocks, cudaStream_t s);
 template <typename T>
-inline int stage_tma_ty(int pressure) { return 8 * (pressure ? stage_rows<T, true>() : stage_rows<T, false>()); }
+cudaError_t prepare_stage_tma(int pressure) {
+    return pressure ? prepare_stage_tma_p<T, true>() : prepare_stage_tma_p<T, false>();
+}
+template <typename T>
+cudaError_t launch_stage_tma(const StageArgsTMA<T>& A, int pressure, int nw, dim3 grid, cudaStream_t s) {
+    return pressure ? launch_stage_tma_p<T, true>(A, nw, grid, s) : launch_stage_tma_p<T, false>(A, nw, grid, s);
+}
+// Row pairs of the tiles: single case (two forms) and batched launches.
+constexpr int STAGE_NW = 6, STAGE_NW_SMALL = 2;
+constexpr int STAGE_BATCH_NW = STAGE_NW, STAGE_BATCH_TY = 2 * STAGE_BATCH_NW;
 // Batched stage launch: `work` holds (case, bx, by, bz) items over the
 // device array `cases`; `counter` is this stage's work counter (zero on
 // entry).  `nblocks` CTAs, persistent.
 template <typename T>
 cudaError_t launch_stage_tma_batch(const StageArgsTMA<T>* cases, const int4* work, int nwork, int* counter, int n,
-                                   int pressure, int nblocks, cudaStream_t s);
+                                   int pressure, int nblocks, cudaStream_t s) {
+    return pressure ? launch_stage_tma_batch_p<T, true>(cases, work, nwork, counter, n, nblocks, s)
+                    : launch_stage_tma_batch_p<T, false>(cases, work, nwork, counter, n, nblocks, s);
+}
 template <typename T>
-int stage_tma_batch_occupancy(int pressure);
+int stage_tma_batch_occupancy(int pressure) {
+    return pressure ? stage_tma_batch_occupancy_p<T, true>() : stage_tma_batch_occupancy_p<T, false>();
+}
 // The controllers of all cases of a batch (and the re-arm of the counters).
 template <typename T>
 cudaError_t launch_control_batch(const StageArgsTMA<T>* cases, int ncases, int* counters, cudaStream_t s);

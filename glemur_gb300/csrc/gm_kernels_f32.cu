@@ -1,8 +1,7 @@
-// gm_kernels_f32.cu -- FP32-storage instantiation of the relaxation kernels.
+// gm_kernels_f32.cu -- FP32-storage instantiation of the relaxation kernels
+// (the TMA-fed stage kernels: gm_stage_f32.cu and gm_stage_f32_press.cu).
 #include "gm_kernels_impl.cuh"
-#include "gm_stage_tma.cuh"
 
 namespace gmk {
 GMK_INSTANTIATE(float)
-GMK_INSTANTIATE_TMA(float)
 }

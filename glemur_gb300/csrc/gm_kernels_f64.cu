@@ -1,8 +1,7 @@
-// gm_kernels_f64.cu -- FP64 instantiation of the relaxation kernels.
+// gm_kernels_f64.cu -- FP64-storage instantiation of the relaxation kernels
+// (the TMA-fed stage kernels: gm_stage_f64.cu and gm_stage_f64_press.cu).
 #include "gm_kernels_impl.cuh"
-#include "gm_stage_tma.cuh"
 
 namespace gmk {
 GMK_INSTANTIATE(double)
-GMK_INSTANTIATE_TMA(double)
 }

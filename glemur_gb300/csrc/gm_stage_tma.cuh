@@ -1,50 +1,56 @@
-// gm_stage_tma.cuh -- the RK stage kernel with TMA-fed plane rings.
+// gm_stage_tma.cuh -- the RK stage kernel: TMA-fed plane rings, two points per
+// thread.
 //
-// Same arithmetic as k_stage (gm_kernels_impl.cuh); different data movement:
-//   * tiles are 32 x 8 columns (compile time), one warp per tile row;
-//   * one thread streams, plane by plane, every operand of the stage with
+//   * A tile is 32 x 2 NW columns (NW warps); a warp covers two rows of 16
+//     x-neighbouring pairs, and a thread's arithmetic runs on its pair
+//     (gm_vec2.cuh: packed FP32 instructions, 64-bit shared-memory accesses).
+//   * One thread streams, plane by plane, every operand of the stage with
 //     cp.async.bulk.tensor into shared-memory rings: the grid positions
 //     (tile + 2-point halo, all three components as one 4-D box), the scaled
 //     field B0s (same box) and the increments k_0..k_{n-1} over the tile;
-//     completion is tracked by one mbarrier per ring slot;
+//     completion is tracked by one mbarrier per ring slot.
 //   * J for plane k is formed in the same iteration as B of plane k+1, so an
-//     iteration needs a single __syncthreads;
-//   * every shared-memory access is a constant offset from a per-plane base.
+//     iteration needs a single __syncthreads; the march is unrolled by two, so
+//     that the diagonals a, b, c of two planes alternate between two register
+//     sets instead of being copied.
 // Waits on the mbarriers are bounded: after kWaitLimit polls the CTA records
 // GM_ST_TIMEOUT, drains the copies it has in flight (again bounded) and
 // returns.
+//
+// What bounds it.  FP32: the algorithmic traffic of a stage is 12 + 3 n reals
+// per point (21 + 3 in stage 5).  The form with one point per thread and
+// scalar instructions took 450 to 650 thread instructions per point at 57 %
+// issue activity: issue-bound, 0.44 of the measured HBM bandwidth.  FP64: the
+// FP64 pipe (one warp instruction per 15 clocks and SM on a GB300), so what
+// counts there is the number of FP64 operations per point.
 #pragma once
 
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "gm_kernels_impl.cuh"
+#include "gm_vec2.cuh"
 
 namespace gmk {
 
-constexpr int TY2 = 8;                   // warps per CTA (one tile row each, per row group)
-constexpr int HX2 = TX + 4;              // position-plane row: the tile + 2-point halo
-constexpr int BX2 = TX + 2;              // B-plane row: the tile + face halo
-// resident CTAs per SM the stage kernel is compiled for (register budget)
-#ifndef GM_STAGE_MINB
-#define GM_STAGE_MINB 3
-#endif
+constexpr int HX2 = TX + 4;              // row pitch of position, B0s and B planes: the tile + 2-point halo
 constexpr unsigned kWaitLimit = 1u << 22;
 
-// Tile of R row groups: 32 x 8R columns, each thread owning the points of
-// rows ty, ty + 8, ..., ty + 8 (R - 1) of its column.
-template <int R>
+// Tile of NW warps: 32 x 2 NW columns.
+template <int NW>
 struct TileShape {
-    static constexpr int TYR = TY2 * R;                  // tile rows
+    static constexpr int TYR = 2 * NW;                   // tile rows
     static constexpr int HYR = TYR + 4, BYR = TYR + 2;   // position / B plane rows
     static constexpr int PLANE_C = HYR * HX2;            // elements of one component of a position plane
     static constexpr int PLANE_X = 3 * PLANE_C;
+    static constexpr int BPLANE_C = BYR * HX2;           // of a B plane
 };
 
-// Stride of a position-plane slot in elements: the plane rounded up so every
-// slot (a TMA destination) starts on a 128-byte boundary.
-template <typename T, int R>
-constexpr int slot_elems() {
-    return (int)(((TileShape<R>::PLANE_X * sizeof(T) + 127) / 128) * 128 / sizeof(T));
+// elements rounded up so that a slot (a TMA destination) starts on 128 bytes
+template <typename T>
+constexpr int slot_round(int elems) {
+    return (int)(((elems * sizeof(T) + 127) / 128) * 128 / sizeof(T));
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -70,10 +76,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 
 // bounded wait; returns false when the limit ran out
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
+static __device__ __noinline__ bool mbar_wait_loop(uint64_t* bar, uint32_t parity) {
     for (unsigned it = 0; it < kWaitLimit; it++)
         if (mbar_try_wait(bar, parity)) return true;
     return false;
+}
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
+    return mbar_try_wait(bar, parity) || mbar_wait_loop(bar, parity);
 }
 
 __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2,
@@ -85,154 +94,431 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, u
         : "memory");
 }
 
-
-// Reciprocal for the stage kernel: FP32 uses the hardware approximation plus
-// one Newton step (within ~1 ulp; FP32 parity is judged at 1e-5), FP64 the
-// correctly rounded one.
-__device__ __forceinline__ float rcp_stage(float x) {
+// Reciprocal for the stage kernel, by Newton's iteration r <- r + r (1 - x r)
+// from the hardware's approximation: one step in FP32 (within ~1 ulp; FP32
+// parity is judged at 1e-5), two in FP64 (the approximation has about 20 bits;
+// the last step's residual is exact to an FMA, so the result is the rounded
+// reciprocal but for rare ties).
+__device__ __forceinline__ float rcp_approx(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return fmaf(fmaf(-x, r, 1.0f), r, r);
+    return r;
 }
-__device__ __forceinline__ double rcp_stage(double x) { return __drcp_rn(x); }
+__device__ __forceinline__ double rcp_approx(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    return r;
+}
+__device__ __forceinline__ F2 rcp_approx(F2 x) { return mk2(rcp_approx(lo(x)), rcp_approx(hi(x))); }
+__device__ __forceinline__ D2 rcp_approx(D2 x) { return mk2(rcp_approx(lo(x)), rcp_approx(hi(x))); }
+template <typename T, typename V>
+__device__ __forceinline__ V rcp_stage(V x) {
+    V r = rcp_approx(x);
+    const V one = splat<V>((T)1), nx = vneg(x);
+#pragma unroll
+    for (int it = 0; it < (sizeof(T) == 4 ? 1 : 2); it++) r = vfma(vfma(nx, r, one), r, r);
+    return r;
+}
 
-// det(a, b, c) of the columns of A.  In FP32 the determinant of a strongly
-// sheared cell (|det| small against the bound |a|_1 |b|_1 |c|_1 of the six
-// Sarrus products) is recomputed in double from the same entries.
-template <typename T>
-__device__ __forceinline__ T det_cols(const T A[3][3]) {
-    T d = det3(A);
-    if (sizeof(T) == 4) {
-        const T m = (fabs(A[0][0]) + fabs(A[1][0]) + fabs(A[2][0])) * (fabs(A[0][1]) + fabs(A[1][1]) + fabs(A[2][1])) *
-                    (fabs(A[0][2]) + fabs(A[1][2]) + fabs(A[2][2]));
-        if (fabs(d) < (T)0.03125 * m) {
-            double jd[3][3];
-            for (int r = 0; r < 3; r++)
-                for (int c = 0; c < 3; c++) jd[r][c] = (double)A[r][c];
-            d = (T)det3<double>(jd);
-        }
-    }
+// FP32: the determinant d of the columns of A, recomputed in double from the
+// same entries when the cell is strongly sheared: |d| small against the bound
+// |a|_1 |b|_1 |c|_1 of the six Sarrus products.
+__device__ __forceinline__ float det_sheared(float d, float a0, float a1, float a2, float b0, float b1, float b2,
+                                             float c0, float c1, float c2) {
+    const float m = (fabsf(a0) + fabsf(a1) + fabsf(a2)) * (fabsf(b0) + fabsf(b1) + fabsf(b2)) *
+                    (fabsf(c0) + fabsf(c1) + fabsf(c2));
+    if (!(fabsf(d) < 0.03125f * m)) return d;
+    const double jd[3][3] = {{a0, b0, c0}, {a1, b1, c1}, {a2, b2, c2}};
+    return (float)det3<double>(jd);
+}
+// The cheap test in front of it: |v|_1 <= sqrt(3) |v|_2, so a cell with
+// d^2 > (0.03125 sqrt(27))^2 |a|^2 |b|^2 |c|^2 cannot be one; everything else
+// (an underflow or a NaN of the squares too) takes the test above.
+constexpr float kShear2 = 0.0266f;
+template <typename V>
+__device__ __forceinline__ V norm2(const V A[3][3], int c) {
+    return vfma(A[2][c], A[2][c], vfma(A[1][c], A[1][c], vmul(A[0][c], A[0][c])));
+}
+// (out of line: the double determinant would double the plane loop's code)
+static __device__ __noinline__ F2 det_sheared2(F2 d, F2 a0, F2 a1, F2 a2, F2 b0, F2 b1, F2 b2, F2 c0, F2 c1, F2 c2) {
+    const float x = det_sheared(lo(d), lo(a0), lo(a1), lo(a2), lo(b0), lo(b1), lo(b2), lo(c0), lo(c1), lo(c2));
+    const float y = det_sheared(hi(d), hi(a0), hi(a1), hi(a2), hi(b0), hi(b1), hi(b2), hi(c0), hi(c1), hi(c2));
+    return mk2(x, y);
+}
+__device__ __forceinline__ float det_guard(float d, const float A[3][3], bool act) {
+    const float t = vmul(vmul(norm2(A, 0), norm2(A, 1)), vmul(norm2(A, 2), kShear2));
+    if (!(vmul(d, d) > t) && act)
+        d = det_sheared(d, A[0][0], A[1][0], A[2][0], A[0][1], A[1][1], A[2][1], A[0][2], A[1][2], A[2][2]);
     return d;
 }
+__device__ __forceinline__ F2 det_guard(F2 d, const F2 A[3][3], bool act) {
+    const F2 t = vmul(vmul(norm2(A, 0), norm2(A, 1)), vmul(norm2(A, 2), splat<F2>(kShear2))), q = vmul(d, d);
+    if (!(lo(q) > lo(t) && hi(q) > hi(t)) && act)
+        d = det_sheared2(d, A[0][0], A[1][0], A[2][0], A[0][1], A[1][1], A[2][1], A[0][2], A[1][2], A[2][2]);
+    return d;
+}
+__device__ __forceinline__ double det_guard(double d, const double[3][3], bool) { return d; }
+__device__ __forceinline__ D2 det_guard(D2 d, const D2[3][3], bool) { return d; }
 
-// B at a non-face point from the position planes (constant offsets), in the
-// form B = (s_x a + s_y b + s_z c) / det(a, b, c) with the unscaled central
-// differences a = x(+x) - x(-x), b, c and the pre-scaled field
-// s = (4 dy dz B0x, 4 dx dz B0y, 4 dx dy B0z): since jac = [a/2dx, b/2dy,
-// c/2dz], this is jac.B0 / det(jac) of B_JacB0 (rungeKutta.cu:79-99) with
-// the constant factors folded.  x and s come from shared-memory planes at the
-// same offset o; PC is the component stride of a plane.  Returns the columns
-// a, b, c in Am[l][0..2] and 1/det(a, b, c) in *rdet (Delta = 1 / (8 dx dy dz
-// rdet)).
-template <typename T, int PC>
-__device__ __forceinline__ void b_point(const T* __restrict__ xm, const T* __restrict__ x0, const T* __restrict__ xp,
-                                        int o, const T* __restrict__ b0s, T Bv[3], T Am[3][3], T* rdet) {
-    const T s0 = b0s[o], s1 = b0s[o + PC], s2 = b0s[o + 2 * PC];
+// B = (s_x a + s_y b + s_z c) / det(a, b, c) with the unscaled central
+// differences a = x(+x) - x(-x), b, c (the columns of A) and the pre-scaled
+// field s = (4 dy dz B0x, 4 dx dz B0y, 4 dx dy B0z): since jac = [a/2dx, b/2dy,
+// c/2dz], this is jac.B0 / det(jac) of B_JacB0 (rungeKutta.cu:79-99) with the
+// constant factors folded.  *r = 1/det(a, b, c) (Delta = 1 / (8 dx dy dz r)).
+// Without `act` the result is not used (and B may come out inexact).
+template <typename T, typename V>
+__device__ __forceinline__ void b_from(const V A[3][3], const V s[3], V B[3], V* r, bool act) {
+    const V b[3] = {A[0][1], A[1][1], A[2][1]}, c[3] = {A[0][2], A[1][2], A[2][2]};
+    V n[3];
+    vcross(b, c, n);
+    V d = vfma(A[0][0], n[0], vfma(A[1][0], n[1], vmul(A[2][0], n[2])));
+    if (sizeof(T) == 4) d = det_guard(d, A, act);
+    const V q = rcp_stage<T>(d);
+    const V s0 = vmul(s[0], q), s1 = vmul(s[1], q), s2 = vmul(s[2], q);
+#pragma unroll
+    for (int l = 0; l < 3; l++) B[l] = vfma(A[l][0], s0, vfma(A[l][1], s1, vmul(A[l][2], s2)));
+    *r = q;
+}
+
+// The columns of A at a pair / a point whose shared-memory addresses in the
+// planes k-1, k, k+1 are xm, x0, xp; C is the component stride in bytes.
+template <typename T, int C>
+__device__ __forceinline__ void diffs(uint32_t xm, uint32_t x0, uint32_t xp, typename PairOf<T>::type A[3][3]) {
+    constexpr int E = sizeof(T), R = HX2 * E;
 #pragma unroll
     for (int l = 0; l < 3; l++) {
-        const int q = o + l * PC;
-        Am[l][0] = x0[q + 1] - x0[q - 1];
-        Am[l][1] = x0[q + HX2] - x0[q - HX2];
-        Am[l][2] = xp[q] - xm[q];
+        const int q = l * C;
+        const auto c = Sh<T>::ld2(x0 + q);
+        A[l][0] = mk2(vsub(hi(c), Sh<T>::ld(x0 + q - E)), vsub(Sh<T>::ld(x0 + q + 2 * E), lo(c)));
+        A[l][1] = vsub(Sh<T>::ld2(x0 + q + R), Sh<T>::ld2(x0 + q - R));
+        A[l][2] = vsub(Sh<T>::ld2(xp + q), Sh<T>::ld2(xm + q));
     }
-    const T r = rcp_stage(det_cols(Am));
+}
+template <typename T, int C>
+__device__ __forceinline__ void diffs1(uint32_t xm, uint32_t x0, uint32_t xp, T A[3][3]) {
+    constexpr int E = sizeof(T), R = HX2 * E;
 #pragma unroll
-    for (int l = 0; l < 3; l++) Bv[l] = (Am[l][0] * s0 + Am[l][1] * s1 + Am[l][2] * s2) * r;
-    *rdet = r;
+    for (int l = 0; l < 3; l++) {
+        const int q = l * C;
+        A[l][0] = vsub(Sh<T>::ld(x0 + q + E), Sh<T>::ld(x0 + q - E));
+        A[l][1] = vsub(Sh<T>::ld(x0 + q + R), Sh<T>::ld(x0 + q - R));
+        A[l][2] = vsub(Sh<T>::ld(xp + q), Sh<T>::ld(xm + q));
+    }
 }
 
-// One B point in a shared-memory B plane: three components and a pad, so a
-// neighbour is one 128-bit load (two for double).
-__device__ __forceinline__ void st_b(float* d, const float v[3]) {
-    *reinterpret_cast<float4*>(d) = make_float4(v[0], v[1], v[2], 0.f);
+template <typename T>
+struct Vec3 { T x, y, z; };
+
+// B on the ghost plane of a line-tied face with normal axis AX, at the point
+// (i, j, k) with addresses xm, x0, xp in the planes k-1, k, k+1 and b0 in the
+// B0s plane: updateBbound, src/boundaries.cu:39-446.  The ghost plane continues
+// by one spacing outwards, and in-plane neighbours at the edges of the
+// reference's 16-wide launch blocks are the own position shifted by the spacing
+// (boundaries.cu:72-109, 212-237, 340-365); the differences come out in the
+// scaling of b_from, and B.n = B0.n is s.n over its scale w (one corrected
+// step, so the quotient is B0.n but for rare last bits).  Everything is read
+// from the shared-memory planes: the form that read B0 from global memory
+// stalled every plane of a line-tied run (110 us a stage on 97x75x133, 35 %
+// issue).
+template <int AX, int C, typename T>
+__device__ __forceinline__ Vec3<T> b_face_s(const KP<T>& p, uint32_t xm, uint32_t x0, uint32_t xp, uint32_t b0, int i,
+                                            int j, int k) {
+    constexpr int E = sizeof(T), R = HX2 * E;
+    const int idx[3] = {i, j, k};
+    const int n3[3] = {p.nx, p.ny, p.nz};
+    const T d3[3] = {p.dx, p.dy, p.dz};
+    const bool side = idx[AX] >= 0;
+    T A[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        if (a == AX) {
+            const uint32_t xi = AX == 2 ? (side ? xm : xp) : x0 + (side ? -1 : 1) * (AX == 0 ? E : R);
+#pragma unroll
+            for (int l = 0; l < 3; l++) {
+                T xo = Sh<T>::ld(x0 + l * C);
+                if (l == AX) xo = side ? vadd(xo, d3[AX]) : vsub(xo, d3[AX]);
+                if (AX == 2 && l < 2 && p.shear)
+                    xo = p.shearTab[10 * ((long long)side * p.nx * p.ny + (long long)j * p.nx + i) + l];
+                const T xn = Sh<T>::ld(xi + l * C);
+                A[l][a] = side ? vsub(xo, xn) : vsub(xn, xo);
+            }
+        } else {
+            const int u = idx[a];
+            const bool eL = u % 16 == 0, eR = u % 16 == 15 || u == n3[a] - 1;
+            const uint32_t xl = eL ? x0 : (a == 2 ? xm : x0 - (a == 1 ? R : E));
+            const uint32_t xr = eR ? x0 : (a == 2 ? xp : x0 + (a == 1 ? R : E));
+#pragma unroll
+            for (int l = 0; l < 3; l++) {
+                T vl = Sh<T>::ld(xl + l * C);
+                T vr = Sh<T>::ld(xr + l * C);
+                if (l == a) {
+                    if (eL) vl = vsub(vl, d3[a]);
+                    if (eR) vr = vadd(vr, d3[a]);
+                }
+                if (AX == 2 && l < 2 && p.shear) {
+                    // an initially distorted grid: the neighbours extrapolated at the
+                    // block edges carry the distortion (k_shear_table)
+                    const T* tb = p.shearTab + 10 * ((long long)side * p.nx * p.ny + (long long)j * p.nx + i);
+                    if (eL) vl = tb[2 + 4 * a + l];
+                    if (eR) vr = tb[4 + 4 * a + l];
+                }
+                A[l][a] = vsub(vr, vl);
+            }
+        }
+    }
+    const T s[3] = {Sh<T>::ld(b0), Sh<T>::ld(b0 + C), Sh<T>::ld(b0 + 2 * C)};
+    T r, B[3];
+    b_from<T, T>(A, s, B, &r, true);
+    const T q = vmul(s[AX], p.w4i[AX]);
+    B[AX] = vfma(vfma(-q, p.w4[AX], s[AX]), p.w4i[AX], q);
+    return Vec3<T>{B[0], B[1], B[2]};
 }
-__device__ __forceinline__ void st_b(double* d, const double v[3]) {
-    reinterpret_cast<double2*>(d)[0] = make_double2(v[0], v[1]);
-    reinterpret_cast<double2*>(d)[1] = make_double2(v[2], 0.0);
-}
-__device__ __forceinline__ void ld_b(const float* d, float v[3]) {
-    const float4 q = *reinterpret_cast<const float4*>(d);
-    v[0] = q.x; v[1] = q.y; v[2] = q.z;
-}
-__device__ __forceinline__ void ld_b(const double* d, double v[3]) {
-    const double2 q0 = reinterpret_cast<const double2*>(d)[0], q1 = reinterpret_cast<const double2*>(d)[1];
-    v[0] = q0.x; v[1] = q0.y; v[2] = q1.x;
+// the line-tied z ghost planes, two of a run (out of line, as det_sheared2)
+template <int C, typename T>
+__device__ __noinline__ Vec3<T> b_face_z(const KP<T>& p, uint32_t xm, uint32_t x0, uint32_t xp, uint32_t b0, int i,
+                                         int j, int k) {
+    return b_face_s<2, C>(p, xm, x0, xp, b0, i, j, k);
 }
 
 // Shared memory of the stage kernels, all in the dynamic buffer (the base is
 // rounded up to 128 bytes at run time; the launch asks for 128 bytes of
 // slack):
 //   XR position-plane slots (the tile + 2-point halo, three components),
-//   2 slots of B0s planes (same box),
-//   2 slots of k-planes (the n arrays k_0..k_{n-1} over the tile; 1 slot in
-//   the late stages, so that the CTAs per SM the kernel is built for fit),
-//   2 B planes (float4 per point: B and a pad),
-//   XR + 4 mbarriers, warp maxima, the abort flag and the work-item slot.
+//   BR slots of B0s planes (same box),
+//   KS slots of k-planes (the n arrays k_0..k_{n-1} over the tile),
+//   3 B planes (the tile + face halo, in the pitch of the position planes),
+//   the mbarriers, warp maxima, the abort flags and the work-item slot.
 // Every slot is a multiple of 128 bytes, the alignment TMA destinations need.
-template <typename T, bool PRESS, int NS, int R>
+// CTAs per SM the kernel is built for, of NW + 2 warps: FP32 16 warps an SM (up
+// to 128 registers a thread; from 17 warps on the limit is 96), FP64 8; the
+// shared memory follows.
+constexpr int STAGE_HALO_WARPS = 2;
+template <int NW>
+constexpr int stage_threads() { return 32 * (NW + STAGE_HALO_WARPS); }
+template <typename T, int NW>
+constexpr int stage_ctas() { return (sizeof(T) == 4 ? 16 : 8) / (NW + STAGE_HALO_WARPS); }
+
+template <typename T, bool PRESS, int NS, int NW>
 struct StageSmem {
-    static constexpr int XR = PRESS ? 5 : 4;                      // position ring (one plane of prefetch)
-    static constexpr int SLOT = slot_elems<T, R>();
+    using S = TileShape<NW>;
+    static constexpr int SLOT = slot_round<T>(S::PLANE_X);
+    static constexpr int BSLOT = slot_round<T>(3 * S::BPLANE_C);
     static constexpr int NK = NS;                                 // k arrays read by stage NS
-    static constexpr int KBOX = 3 * TileShape<R>::TYR * TX;       // elements of one k-array plane
+    static constexpr int KBOX = 3 * S::TYR * TX;                  // elements of one k-array plane
     static constexpr int KSLOT = NK * KBOX;
-    // k-plane slots: two (the next plane streams in while this one is read),
-    // or one where two would not leave room for the CTAs per SM the kernel is
-    // built for (its plane is then loaded during the B phase of the same
-    // iteration, behind a second barrier)
-    static constexpr int KS = R == 1 ? ((PRESS && NS == 5) ? 1 : 2) : ((NS >= 4 || (PRESS && NS >= 3)) ? 1 : 2);
-    static constexpr int PLANE_B = 4 * TileShape<R>::BYR * BX2;
+    static constexpr int XMIN = PRESS ? 4 : 3;                    // position planes an iteration reads
+    static constexpr size_t bytes(int xr, int br, int ks) {
+        return sizeof(T) * ((size_t)(xr + br) * SLOT + 3 * (size_t)BSLOT + (size_t)ks * KSLOT) + 128 + 8 * (xr + br + ks) +
+               8 * NW + 64;
+    }
+    static constexpr bool fits(int xr, int br, int ks) {
+        return (bytes(xr, br, ks) + 1024) * stage_ctas<T, NW>() <= 228 * 1024;
+    }
+    // Position and B0s planes are loaded XR - XMIN and BR - 1 iterations ahead, two
+    // where the CTAs per SM the kernel is built for still fit (an iteration is about
+    // the latency of a copy: one ahead left 2.8 to 3.7 of 9.5 cycles per instruction
+    // in waiting for it), else one.  k planes have two slots, or one where two would
+    // not fit (the plane is then loaded during the B phase of its own iteration).
+    static constexpr int KS = fits(XMIN + 1, 2, 2) ? 2 : 1;
+    static constexpr int XR = fits(XMIN + 2, 2, KS) ? XMIN + 2 : XMIN + 1;
+    static constexpr int BR = fits(XR, 3, KS) ? 3 : 2;
     static constexpr size_t OFF_B0 = sizeof(T) * (size_t)XR * SLOT;
-    static constexpr size_t OFF_K = OFF_B0 + sizeof(T) * 2 * (size_t)SLOT;
+    static constexpr size_t OFF_K = OFF_B0 + sizeof(T) * (size_t)BR * SLOT;
     static constexpr size_t OFF_B = OFF_K + sizeof(T) * KS * (size_t)KSLOT;
-    static constexpr size_t OFF_BAR = OFF_B + sizeof(T) * 2 * (size_t)PLANE_B;
-    static constexpr int NBAR = XR + 2 + KS;                     // x slots, 2 B0s slots, k slots
+    static constexpr size_t OFF_BAR = OFF_B + sizeof(T) * 3 * (size_t)BSLOT;
+    static constexpr int NBAR = XR + BR + KS;                    // x slots, B0s slots, k slots
     static constexpr size_t OFF_WMAX = OFF_BAR + 8 * NBAR;
-    static constexpr size_t OFF_CTL = OFF_WMAX + 16 * TY2;
-    static constexpr size_t BYTES = 128 + OFF_CTL + 64;
+    static constexpr size_t OFF_CTL = OFF_WMAX + 8 * NW;
+    static constexpr size_t BYTES = bytes(XR, BR, KS);
+    static_assert(BYTES <= 227 * 1024, "stage tile does not fit the shared memory");
 };
 
-// Copy bookkeeping of a CTA, kept in shared memory and touched by the
-// producer thread only (abort and the work item are read by all threads after
-// a barrier).
+// What a CTA keeps in shared memory besides the planes.
 struct StageCtl {
-    uint32_t ph;                 // next completion parity of each mbarrier
-    int x_iss, x_done;           // position planes issued / completed
-    int b_iss, b_done;           // B0s planes
-    int k_iss, k_done;           // k planes
-    int abort;                   // a bounded wait ran out
+    uint32_t ph;                 // completion parity of each mbarrier, carried from tile to tile
+    // A bounded wait ran out: set in iteration kk's entry (kk & 1), which every
+    // warp reads behind the next barrier, so that all leave in the same iteration.
+    int abort[2];
     int work;                    // batched launch: the current work item
 };
 
-// Kind of a B-region point, fixed for the whole z march of a thread.
-enum { BK_SKIP = 0, BK_INNER = 1, BK_FACE_X = 2, BK_FACE_Y = 3 };
+// Offsets (elements) from a stored position to its periodic images along x and
+// y, 0 where there is none: ghost layers 1 and 2 hold the images of the two
+// inner layers of the opposite face, shifted by -/+ (L + d) as setGridPeriFace
+// writes them (boundaries.cu:546-549, 561-564, 576-579).
+__device__ __forceinline__ int image_step(int peri, int i, int n) { return !peri ? 0 : i < 2 ? n : i >= n - 2 ? -n : 0; }
 
-// One RK stage over the 32 x 8R x TZ block (bx, by, bz) of one case.
+template <typename T, typename V>
+__device__ __forceinline__ V image_shift(V v, int step, T L, T d) {
+    return step > 0 ? vadd(vadd(v, splat<V>(L)), splat<V>(d)) : vsub(vsub(v, splat<V>(L)), splat<V>(d));
+}
+
+template <typename T, typename V>
+__device__ __forceinline__ void st_xyz(T* q, long long cs, V a, V b, V c) {
+    stv(q, a);
+    stv(q + cs, b);
+    stv(q + 2 * cs, c);
+}
+
+// The periodic images, beyond those along x alone, of the position v stored at
+// q (ix, iy, iz: image_step).
+template <typename T, typename V>
+__device__ __forceinline__ void store_images_yz(const KP<T>& p, T* q, const V v[3], int ix, int iy, int iz) {
+    const long long cs = p.cs, oy = (long long)iy * p.px;
+    const V vx = image_shift<T>(v[0], ix, p.Lx, p.dx), vy = image_shift<T>(v[1], iy, p.Ly, p.dy);
+    if (iy) st_xyz(q + oy, cs, v[0], vy, v[2]);
+    if (ix && iy) st_xyz(q + ix + oy, cs, vx, vy, v[2]);
+    if (iz) {
+        T* qz = q + (long long)iz * p.px * p.py;
+        const V vz = image_shift<T>(v[2], iz, p.Lz, p.dz);
+        st_xyz(qz, cs, v[0], v[1], vz);
+        if (ix) st_xyz(qz + ix, cs, vx, v[1], vz);
+        if (iy) st_xyz(qz + oy, cs, v[0], vy, vz);
+        if (ix && iy) st_xyz(qz + ix + oy, cs, vx, vy, vz);
+    }
+}
+template <typename T, typename V>
+__device__ __noinline__ void store_images_call(const KP<T>& p, T* q, V a, V b, V c, int ix, int iy, int iz) {
+    const V v[3] = {a, b, c};
+    store_images_yz<T, V>(p, q, v, ix, iy, iz);
+}
+// Every image of one point, in any grid: a direction of three points, whose
+// middle point has two images, takes the loop over all shifts (store_pos).
+template <typename T>
+__device__ __noinline__ void store_point_images(const KP<T>& p, T* X, int i, int j, int k, T a, T b, T c) {
+    const T v[3] = {a, b, c};
+    store_pos<T>(p, X, i, j, k, v);
+}
+// The start grid's own images, refreshed by stage 5 of the first attempted step
+// (a retry reads them; until then they are those the caller supplied).
+template <typename T>
+__device__ __noinline__ void refresh_images(const KP<T>& p, T* X0, int i, int j, int k, bool pairs, bool two, int ix,
+                                            int iy, int iz) {
+    using V = typename PairOf<T>::type;
+    T* q = X0 + gidx(p.px, p.py, i, j, k);
+    if (pairs) {
+        const V v[3] = {ldv2(q), ldv2(q + p.cs), ldv2(q + 2 * p.cs)};
+        if (ix) st_xyz(q + ix, p.cs, image_shift<T>(v[0], ix, p.Lx, p.dx), v[1], v[2]);
+        store_images_yz<T, V>(p, q, v, ix, iy, iz);
+        return;
+    }
+    for (int h = 0; h < (two ? 2 : 1); h++) {
+        const T u[3] = {q[h], q[h + p.cs], q[h + 2 * p.cs]};
+        store_pos<T>(p, X0, i + h, j, k, u);
+    }
+}
+
+// The pressure gradient at a pair on plane k from the planes k-1, k, k+1 (grad_p's
+// formula): with the columns of A and r = 1/det A, jac^-1 = 2 d A^-1 and the
+// second differences over d d, every spacing but that of p0's derivative
+// cancels: grad(1/Delta) Delta = -4 sum_l S_l (A^-1)_l with S_l = sum_{a,b}
+// delta_b delta_l x_a (A^-1)_{ba}.  The second differences are differences of
+// differences of neighbours, which are exact or nearly so.
+template <typename T, int C>
+__device__ __forceinline__ void grad_p2(const KP<T>& p, uint32_t xm, uint32_t x0, uint32_t xp,
+                                        const typename PairOf<T>::type A[3][3], typename PairOf<T>::type r,
+                                        const typename PairOf<T>::type pe[3], typename PairOf<T>::type g[3]) {
+    using V = typename PairOf<T>::type;
+    using M = Sh<T>;
+    constexpr int E = sizeof(T), R = HX2 * E;
+    const V quarter = splat<V>((T)0.25);
+    const V a[3] = {A[0][0], A[1][0], A[2][0]}, b[3] = {A[0][1], A[1][1], A[2][1]}, c[3] = {A[0][2], A[1][2], A[2][2]};
+    V Ai[3][3];   // rows of A^-1
+    vcross(b, c, Ai[0]);
+    vcross(c, a, Ai[1]);
+    vcross(a, b, Ai[2]);
+#pragma unroll
+    for (int e = 0; e < 9; e++) Ai[e / 3][e % 3] = vmul(Ai[e / 3][e % 3], r);
+    V S[3];
+#pragma unroll
+    for (int l = 0; l < 3; l++) {
+        const int q = l * C;
+        const V xc = M::ld2(x0 + q);
+        const V ex = mk2(M::ld(x0 + q - E), lo(xc)), fx = mk2(hi(xc), M::ld(x0 + q + 2 * E));
+        const V yp = M::ld2(x0 + q + R), ym = M::ld2(x0 + q - R), zp = M::ld2(xp + q), zm = M::ld2(xm + q);
+        const V dxx = vsub(vsub(fx, xc), vsub(xc, ex));
+        const V dyy = vsub(vsub(yp, xc), vsub(xc, ym));
+        const V dzz = vsub(vsub(zp, xc), vsub(xc, zm));
+        // differences along y and z at x - 1 .. x + 2, then along x
+        const V dy = vsub(yp, ym), dz = vsub(zp, zm);
+        const T dyl = vsub(M::ld(x0 + q + R - E), M::ld(x0 + q - R - E));
+        const T dyr = vsub(M::ld(x0 + q + R + 2 * E), M::ld(x0 + q - R + 2 * E));
+        const T dzl = vsub(M::ld(xp + q - E), M::ld(xm + q - E)), dzr = vsub(M::ld(xp + q + 2 * E), M::ld(xm + q + 2 * E));
+        const V dxy = vmul(mk2(vsub(hi(dy), dyl), vsub(dyr, lo(dy))), quarter);
+        const V dxz = vmul(mk2(vsub(hi(dz), dzl), vsub(dzr, lo(dz))), quarter);
+        const V dyz = vmul(vsub(vsub(M::ld2(xp + q + R), M::ld2(xm + q + R)), vsub(M::ld2(xp + q - R), M::ld2(xm + q - R))),
+                           quarter);
+        const V i0 = Ai[0][l], i1 = Ai[1][l], i2 = Ai[2][l];
+        if (l == 0) {
+            S[0] = vfma(dxx, i0, vfma(dxy, i1, vmul(dxz, i2)));
+            S[1] = vfma(dxy, i0, vfma(dyy, i1, vmul(dyz, i2)));
+            S[2] = vfma(dxz, i0, vfma(dyz, i1, vmul(dzz, i2)));
+        } else {
+            S[0] = vfma(dxx, i0, vfma(dxy, i1, vfma(dxz, i2, S[0])));
+            S[1] = vfma(dxy, i0, vfma(dyy, i1, vfma(dyz, i2, S[1])));
+            S[2] = vfma(dxz, i0, vfma(dyz, i1, vfma(dzz, i2, S[2])));
+        }
+    }
+    // 1/Delta = r 8 dx dy dz
+    const V det1 = vmul(r, splat<V>(p.vol8));
+    const V w = vmul(pe[0], splat<V>((T)-4));
+#pragma unroll
+    for (int l = 0; l < 3; l++) {
+        V t = vmul(w, vfma(S[0], Ai[0][l], vfma(S[1], Ai[1][l], vmul(S[2], Ai[2][l]))));
+        t = vfma(pe[1], Ai[0][l], vfma(pe[2], Ai[1][l], t));
+        g[l] = vmul(t, det1);
+    }
+}
+
+__device__ __forceinline__ bool finite_bits(float x) { return (__float_as_uint(x) & 0x7f800000u) != 0x7f800000u; }
+__device__ __forceinline__ bool finite_bits(double x) { return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u; }
+
+// Running maximum of non-negative values; NaN never wins (maths.cu:144-153).
+// In FP64 on the bits (non-negative doubles order as integers): a comparison
+// of doubles would cost a slot of the FP64 pipe.
+__device__ __forceinline__ void max_nn(float& m, float x) { m = fmaxf(m, fabsf(x)); }
+__device__ __forceinline__ void max_nn(double& m, double x) {
+    const long long b = __double_as_longlong(x) & 0x7fffffffffffffffll;
+    if (b > __double_as_longlong(m) && b <= 0x7ff0000000000000ll) m = __longlong_as_double(b);
+}
+
+// One RK stage over the 32 x 2 NW x TZ block (bx, by, bz) of one case.
 // Iteration kk of the z march computes B on plane kb = kk - 1 (the tile and
 // its face halo) and then J, k_n and the stage position on plane kc = kk - 2.
-// Each thread keeps, for each of its R points of the plane, B at kc - 1, kc,
-// kc + 1 and the
-// diagonals a, b, c and 1/det of plane kc in registers, so J needs only the
-// four in-plane neighbours' B from shared memory, written in the previous
-// iteration.  Operands arrive by TMA one iteration ahead: position plane
+// NW warps own the tile's pairs: the diagonals a, b, c and 1/det of plane kc
+// stay in their registers from the iteration that computed its B, and B of the
+// planes kc - 1 and kc is read back from shared memory (three planes), written
+// in the two previous iterations.  Two more warps compute B on the face halo,
+// one of them issues and awaits the copies; as some of the NW warps' extra work
+// it held up every iteration's barrier (3.2 of 10.6 cycles per instruction).  Halo
+// points stand where the domain ends in a partial tile, so a pair is always
+// inner points.  Operands arrive by TMA one iteration ahead: position plane
 // kk + 1 (into the slot of plane kk + 1 - XR: the B phase last read it in the
 // previous iteration, and so did the pressure gradient, which reads planes
 // kc - 1 .. kc + 1, with its fifth slot), the B0s plane of the next B phase
-// and the k planes of the next J phase.  `base` is the 128-byte aligned shared buffer
-// with initialised mbarriers; the mbarrier parities in its StageCtl carry
-// over to the next tile.  Returns false
-// after a bounded wait ran out or an alignment check failed (the status word
-// says which).
-template <typename T, bool PRESS, int NS, int R>
+// and the k planes of the next J phase.  `base` is the 128-byte aligned shared
+// buffer with initialised mbarriers; the mbarrier parities in its StageCtl
+// carry over to the next tile.  Returns false after a bounded wait ran out or
+// an alignment check failed (the status word says which).
+//
+// Stage 5 does not store x_6 = x_5 - sum b_5m k_m, the start of a rejected
+// step's retry (rungeKutta.cu:216-227): it is x_0 up to rounding, and X[cur]
+// still holds x_0.  With the cancellation-free error norm x_6 is not formed
+// either: x_new = x_5 + sum_m (c_m - b_5m) k_m.
+template <typename T, bool PRESS, int NS, int NW>
 __device__ __forceinline__ bool stage_tile(const StageArgsTMA<T>& A, int bx, int by, int bz, unsigned char* base) {
-    using L = StageSmem<T, PRESS, NS, R>;
-    using S = TileShape<R>;
+    using V = typename PairOf<T>::type;
+    using L = StageSmem<T, PRESS, NS, NW>;
+    using S = TileShape<NW>;
+    using M = Sh<T>;
     constexpr bool LAST = NS == 5;
     constexpr int n = NS;
-    constexpr int XR = L::XR;
-    constexpr int SLOT = L::SLOT;
-    constexpr int PLANE_B = L::PLANE_B;
-    constexpr int TYR = S::TYR, BYR = S::BYR, PC = S::PLANE_C;
+    constexpr int XR = L::XR, BR = L::BR, KS = L::KS;
+    constexpr int XD = XR - L::XMIN, BD = BR - 1;        // iterations the copies run ahead
+    constexpr int TYR = S::TYR;
+    // strides in bytes: element, row, components of the planes, slots
+    constexpr int E = sizeof(T), R = HX2 * E, C = S::PLANE_C * E, BC = S::BPLANE_C * E, KC = TX * TYR * E;
+    constexpr int XSLOT = L::SLOT * E, BSLOT = L::BSLOT * E, KSLOT = L::KSLOT * E;
 
     const StageArgs<T>& a = A.a;
     const KP<T>& p = a.p;
@@ -241,266 +527,237 @@ __device__ __forceinline__ bool stage_tile(const StageArgsTMA<T>& A, int bx, int
     // failed its alignment check: nothing to compute
     if (st->done || (st->status & (GM_ST_TIMEOUT | GM_ST_ALIGN))) return true;
 
-    T* xs = reinterpret_cast<T*>(base);                                   // XR position slots
-    T* b0r = reinterpret_cast<T*>(base + L::OFF_B0);                       // 2 B0s slots
-    T* kr = reinterpret_cast<T*>(base + L::OFF_K);                         // k slots
-    T* bs = reinterpret_cast<T*>(base + L::OFF_B);                         // 2 B planes
     uint64_t* bars = reinterpret_cast<uint64_t*>(base + L::OFF_BAR);       // x | B0s | k
     T* s_wmax = reinterpret_cast<T*>(base + L::OFF_WMAX);
     StageCtl* ctl = reinterpret_cast<StageCtl*>(base + L::OFF_CTL);
-    int* s_abort = &ctl->abort;
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-    // the producer (copy issue and waits) is lane 0 of the last warp, which
-    // computes no face-halo B points
-    const bool producer = tid == (TY2 - 1) * TX;
+    volatile int* s_abort = ctl->abort;
+    auto barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(stage_threads<NW>()) : "memory"); };
+    uint32_t sb, tid;      // (volatile: kept, not recomputed)
+    asm volatile("mov.u32 %0, %1;" : "=r"(sb) : "r"(smem_u32(base)));
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+    const int lane = tid & 31, warp = tid >> 5;
     const int i0 = bx * TX, j0 = by * TYR, k0 = bz * a.TZ;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const int kend = min(k0 + a.TZ, nz);
     const int cur = st->cur;
-    const int mapi = (n == 0) ? cur : 2 + ((n - 1) & 1);
-    const CUtensorMap* tmap = &A.tm[mapi];
-    const CUtensorMap* tmb0 = &A.tm[4];
-    const T dtT = (T)st->dt;
-    const int KC = (int)p.kcs;
-    const int cs = (int)p.cs;
-    const int pxy = p.px * p.py;
     const bool zPeri = p.zPeri != 0;
-    constexpr uint32_t kPlaneBytes = S::PLANE_X * sizeof(T);
-    constexpr uint32_t kKBytes = (uint32_t)(L::KSLOT * sizeof(T));
 
     // self-check of the alignment TMA needs: destination slots on 128 bytes,
     // mbarriers on 8 bytes, tensor maps on 64 bytes, box start on 16 bytes; on
     // failure record a status bit and issue no copy
-    if ((smem_u32(xs) & 127u) || (smem_u32(b0r) & 127u) || (smem_u32(kr) & 127u) || (smem_u32(bs) & 15u) ||
-        (smem_u32(bars) & 7u) || (reinterpret_cast<uintptr_t>(&A.tm[0]) & 63u) || ((i0 * (int)sizeof(T)) & 15)) {
-        if (producer) atomicOr(&st->status, (unsigned)GM_ST_ALIGN);
+    if ((sb & 127u) || ((XSLOT | KSLOT | (int)L::OFF_B0 | (int)L::OFF_K) & 127) || (smem_u32(bars) & 7u) ||
+        (reinterpret_cast<uintptr_t>(&A.tm[0]) & 63u) || ((i0 * E) & 15)) {
+        if (tid == 0) atomicOr(&st->status, (unsigned)GM_ST_ALIGN);
         return false;
     }
-
-    // ---- per-thread descriptors, fixed for the whole z march ----------------
-    // the thread's own points: column i0 + tx, rows ty + 8 r (r < R)
-    const int ic = i0 + tx;
-    int jc[R], ox1[R], ob1[R], tyx[R], kind1[R], gxy1[R], lin0[R];
-    bool own[R], img_xy[R];
-    T exy[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-        const int tyr = ty + TY2 * r;
-        jc[r] = j0 + tyr;
-        own[r] = ic < nx && jc[r] < ny;
-        ox1[r] = (tyr + 2) * HX2 + (tx + 2);           // in a position / B0s plane
-        ob1[r] = 4 * ((tyr + 1) * BX2 + (tx + 1));     // in a B plane
-        tyx[r] = tyr * TX + tx;                        // in a k plane
-        // in a partial tile the ghost column i = nx or row j = ny is a tile point
-        kind1[r] = BK_SKIP;
-        const bool xo1 = ic >= nx, yo1 = jc[r] >= ny;
-        if (ic <= nx && jc[r] <= ny && !(xo1 && yo1)) {
-            if (xo1 && !p.xPeri) kind1[r] = BK_FACE_X;
-            else if (yo1 && !p.yPeri) kind1[r] = BK_FACE_Y;
-            else kind1[r] = BK_INNER;
-        }
-        exy[r] = own[r] ? p.ex[ic] * p.ey[jc[r]] : (T)0;
-        gxy1[r] = (ic + 2) + p.px * (jc[r] + 2);      // padded offset without the plane term
-        lin0[r] = ic + p.kpx * jc[r];                 // k_m index of the own column
-        img_xy[r] = (p.xPeri && (ic < 2 || ic >= nx - 2)) || (p.yPeri && (jc[r] < 2 || jc[r] >= ny - 2));
-    }
-    // one face-halo point for warps 0-2: the rows above and below the tile
-    // (warps 0 and 1) and its left and right columns (warp 2, 2 TYR <= 32 points)
-    int jj2 = 0, ii2 = 0, kind2 = BK_SKIP;
-    if (ty == 0) { jj2 = 0; ii2 = tx + 1; }
-    else if (ty == 1) { jj2 = BYR - 1; ii2 = tx + 1; }
-    else if (ty == 2 && tx < 2 * TYR) { jj2 = (tx % TYR) + 1; ii2 = tx < TYR ? 0 : BX2 - 1; }
-    else ii2 = -1;
-    const int i2 = i0 - 1 + ii2, j2 = j0 - 1 + jj2;
-    if (ii2 >= 0 && i2 <= nx && j2 <= ny) {
-        const bool xo2 = (i2 < 0 || i2 >= nx);
-        const bool yo2 = (j2 < 0 || j2 >= ny);
-        if (xo2 && yo2) kind2 = BK_SKIP;
-        else if (xo2 && !p.xPeri) kind2 = BK_FACE_X;
-        else if (yo2 && !p.yPeri) kind2 = BK_FACE_Y;
-        else kind2 = BK_INNER;
-    }
-    const int ox2 = (jj2 + 1) * HX2 + (ii2 + 1);
-    const int ob2 = 4 * (jj2 * BX2 + ii2);
-    const int kplane = p.kpx * ny;
-    const T* __restrict__ ezp = p.ez;
-
+    const uint32_t ph0 = ctl->ph;      // rewritten at the end, behind a barrier
+    // ring slot of a position plane
     auto xslot = [&](int plane) { return (plane + 20) % XR; };
-    // thread 0: wait for the copy tracked by mbarrier b, then flip its parity
-    auto wait_bar = [&](int b) {
-        const bool ok = mbar_wait_bounded(&bars[b], (ctl->ph >> b) & 1u);
-        ctl->ph ^= 1u << b;
-        return ok;
-    };
-    auto issue_x = [&](int q) {
-        uint64_t* b = &bars[xslot(q)];
-        mbar_expect_tx(b, kPlaneBytes);
-        tma_load_4d(xs + xslot(q) * SLOT, tmap, b, i0, j0, q + 2, 0);
-    };
-    auto issue_b0 = [&](int q) {
-        uint64_t* b = &bars[XR + (q & 1)];
-        mbar_expect_tx(b, kPlaneBytes);
-        tma_load_4d(b0r + (q & 1) * SLOT, tmb0, b, i0, j0, q + 2, 0);
-    };
-    constexpr int KS = L::KS;
-    auto kbar = [&](int q) { return XR + 2 + (KS == 2 ? (q & 1) : 0); };
-    auto kslot = [&](int q) { return kr + (KS == 2 ? (q & 1) : 0) * L::KSLOT; };
-    auto issue_k = [&](int q) {
-        uint64_t* b = &bars[kbar(q)];
-        mbar_expect_tx(b, kKBytes);
-#pragma unroll
-        for (int m = 0; m < n; m++)
-            tma_load_4d(kslot(q) + m * L::KBOX, &A.tm[5 + m], b, i0, j0, q, 0);
-    };
-    // ring positions relative to plane kk, from one modulo per iteration
-    auto xring = [&](int m, int back) { int s = m - back; s += s < 0 ? XR : 0; return xs + s * SLOT; };
-    // the face formula at x / y face points (no initial-distortion terms: those
-    // concern the z faces only) and at the z ghost planes
-    auto face_b = [&](int face, int i, int j, int kb, T Bv[3]) {
-        Tile<T, 4, XR, 20> tl;
-        tl.xs = xs;
-        tl.i0 = i0; tl.j0 = j0; tl.HX = HX2; tl.HY = S::HYR;
-        tl.slot = SLOT;
-        T D;
-        b_face<T, false>(p, tl, a.B0, face, i, j, kb, Bv, &D);
-    };
-    auto face_bz = [&](int i, int j, int kb, T Bv[3]) {
-        Tile<T, 4, XR, 20> tl;
-        tl.xs = xs;
-        tl.i0 = i0; tl.j0 = j0; tl.HX = HX2; tl.HY = S::HYR;
-        tl.slot = SLOT;
-        T D;
-        b_face<T, true>(p, tl, a.B0, 2, i, j, kb, Bv, &D);
-    };
-
-    // copies issued / completed so far (the producer): position planes
-    // k0-2 .. kend+1, B0s planes k0-1 .. kend, k planes k0 .. kend-1
-    if (producer) {
-        // failure-detection test (a.stall): the first position planes are
-        // withheld, so the bounded waits for them run out
-        if (!a.stall)
-            for (int q = k0 - 2; q <= min(k0 + 1, kend + 1); q++) issue_x(q);
-        ctl->x_iss = min(k0 + 1, kend + 1);
-        ctl->x_done = k0 - 3;
-        issue_b0(k0 - 1);
-        ctl->b_iss = k0 - 1;
-        ctl->b_done = k0 - 2;
-        ctl->k_iss = k0 - 1;
-        ctl->k_done = k0 - 1;
-    }
-
+    auto bslot = [&](int plane) { return (plane + 6) % BR; };
+    auto kbar = [&](int q) { return XR + BR + (KS == 2 ? (q & 1) : 0); };
     T dmax = 0;
     bool bad = false;
-    // own columns: B at kc-1, kc, kc+1 and a, b, c, 1/det at kc
-    T Bm[R][3], Bz[R][3], Bp[R][3], Ac[R][3][3], An[R][3][3], Rc[R], Rn[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-#pragma unroll
-        for (int l = 0; l < 3; l++) {
-            Bm[r][l] = 0; Bz[r][l] = 0; Bp[r][l] = 0;
-            Ac[r][l][0] = 0; Ac[r][l][1] = 0; Ac[r][l][2] = 0;
-            An[r][l][0] = 0; An[r][l][1] = 0; An[r][l][2] = 0;
-        }
-        Rc[r] = 0; Rn[r] = 0;
-    }
+    int kstop = kend + 2;              // the iteration that was left early
 
-    for (int kk = k0; kk <= kend + 1; kk++) {
-        // (1) the producer waits for position plane kk, the B0s plane of
-        // kb = kk-1 and the k planes of kc = kk-2
+    if (warp >= NW) {
+        // ---- the halo warps: NW the rows, NW + 1 the columns and the copies -------
+        const bool producer = tid == 32 * (NW + 1), rows = warp == NW;
+        const CUtensorMap* tmap = &A.tm[(n == 0) ? cur : 2 + ((n - 1) & 1)];
+        uint32_t ph = ph0;
+        auto wait_bar = [&](int b) {
+            const bool ok = mbar_wait_bounded(&bars[b], (ph >> b) & 1u);
+            ph ^= 1u << b;
+            return ok;
+        };
+        auto issue_x = [&](int q) {
+            uint64_t* b = &bars[xslot(q)];
+            mbar_expect_tx(b, S::PLANE_X * E);
+            tma_load_4d(base + xslot(q) * XSLOT, tmap, b, i0, j0, q + 2, 0);
+        };
+        auto issue_b0 = [&](int q) {
+            uint64_t* b = &bars[XR + bslot(q)];
+            mbar_expect_tx(b, S::PLANE_X * E);
+            tma_load_4d(base + L::OFF_B0 + bslot(q) * XSLOT, &A.tm[4], b, i0, j0, q + 2, 0);
+        };
+        auto issue_k = [&](int q) {
+            uint64_t* b = &bars[kbar(q)];
+            mbar_expect_tx(b, KSLOT);
+#pragma unroll
+            for (int m = 0; m < n; m++)
+                tma_load_4d(base + L::OFF_K + (KS == 2 ? (q & 1) : 0) * KSLOT + m * (L::KBOX * E), &A.tm[5 + m], b, i0, j0,
+                            q, 0);
+        };
+        // rows: lanes 0-15 the row below the tile, 16-31 the row above it, one
+        // pair each; columns: one point per lane, left then right
+        const int ic = i0 + 2 * (lane & 15);
+        const int iend = min(i0 + TX, nx), jend = min(j0 + TYR, ny);
+        const bool hup = lane >= 16, hright = lane >= TYR;
+        const int jR = hup ? jend : j0 - 1;
+        const bool doR = rows && ic < nx, faceR = !p.yPeri && (hup ? jend == ny : j0 == 0);
+        const int iC = hright ? iend : i0 - 1, jC = j0 + (lane % TYR);
+        const bool doC = !rows && jC < ny && lane < 2 * TYR, faceC = !p.xPeri && (hright ? iend == nx : i0 == 0);
+        const uint32_t aR = sb + ((jR - j0 + 2) * HX2 + (ic - i0 + 2)) * E;
+        const uint32_t aC = sb + ((jC - j0 + 2) * HX2 + (iC - i0 + 2)) * E;
+        // failure-detection test (a.stall): the first position planes are
+        // withheld, so the bounded waits for them run out
         if (producer) {
-            const int need = min(kk, kend + 1);
-            bool ok = true;
-            while (ok && ctl->x_done < need) { ok = wait_bar(xslot(ctl->x_done + 1)); ctl->x_done++; }
-            while (ok && ctl->b_done < kk - 1) { ok = wait_bar(XR + ((ctl->b_done + 1) & 1)); ctl->b_done++; }
-            if (n > 0 && KS == 2)
-                while (ok && ctl->k_done < kk - 2) { ok = wait_bar(kbar(ctl->k_done + 1)); ctl->k_done++; }
-            if (!ok) {
-                *s_abort = 1;
-                atomicOr(&st->status, (unsigned)GM_ST_TIMEOUT);
-            }
+            if (!a.stall)
+                for (int q = k0 - 2; q <= min(k0 + XD, kend + 1); q++) issue_x(q);
+            for (int q = k0 - 1; q <= min(k0 - 2 + BD, kend); q++) issue_b0(q);
         }
-        __syncthreads();
-        if (*s_abort) break;
-        // (2) refills, into slots whose last reader was the previous iteration
-        // (every thread is past this iteration's barrier)
-        if (producer) {
-            const int qx = kk + 1;
-            if (qx <= kend + 1 && qx > ctl->x_iss) { issue_x(qx); ctl->x_iss = qx; }
-            if (kk <= kend && kk > ctl->b_iss) { issue_b0(kk); ctl->b_iss = kk; }
-            // k planes: the next J phase's (two slots), or this one's (one slot:
-            // the previous J phase, its last reader, is behind the barrier)
-            const int qk = KS == 2 ? kk - 1 : kk - 2;
-            if (n > 0 && qk >= k0 && qk < kend && qk > ctl->k_iss) { issue_k(qk); ctl->k_iss = qk; }
-        }
-        const int mx = (kk + 20) % XR;      // ring slot of position plane kk
-        // (3) B on plane kb = kk - 1 into B plane kb & 1
-        const int kb = kk - 1;
-        T Bv[R][3];
-        {
-            T* bdst = bs + (kb & 1) * PLANE_B;
-            const T* xm = xring(mx, 2);
-            const T* x0 = xring(mx, 1);
-            const T* xq = xring(mx, 0);
-            const T* s0 = b0r + (kb & 1) * SLOT;
-            const bool zo = (kb < 0 || kb >= nz);
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                Bv[r][0] = 0; Bv[r][1] = 0; Bv[r][2] = 0;
-                if (!zo) {
-                    if (kind1[r] != BK_SKIP) {
-                        if (kind1[r] == BK_INNER) b_point<T, PC>(xm, x0, xq, ox1[r], s0, Bv[r], An[r], &Rn[r]);
-                        else face_b(kind1[r] == BK_FACE_X ? 0 : 1, ic, jc[r], kb, Bv[r]);
-                        st_b(bdst + ob1[r], Bv[r]);
-                    }
-                } else if (!zPeri) {
-                    // line-tied ghost plane: only the own columns are needed
-                    if (own[r]) face_bz(ic, jc[r], kb, Bv[r]);
-                } else {
-                    // periodic image plane: only the own columns are needed
-                    if (own[r]) b_point<T, PC>(xm, x0, xq, ox1[r], s0, Bv[r], An[r], &Rn[r]);
-                }
-            }
-            if (!zo && kind2 != BK_SKIP) {
-                T Bh[3], Ah[3][3], Rh;
-                if (kind2 == BK_INNER) b_point<T, PC>(xm, x0, xq, ox2, s0, Bh, Ah, &Rh);
-                else face_b(kind2 == BK_FACE_X ? 0 : 1, i2, j2, kb, Bh);
-                st_b(bdst + ob2, Bh);
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < R; r++)
-#pragma unroll
-            for (int l = 0; l < 3; l++) { Bm[r][l] = Bz[r][l]; Bz[r][l] = Bp[r][l]; Bp[r][l] = Bv[r][l]; }
-        // (4) J, k_n and the stage position on plane kc = kk - 2
-        const int kc = kk - 2;
-        if (KS == 1 && kc >= k0) {
-            // one k slot: the producer waits for this plane's k copies (issued
-            // at the top of this iteration), then a barrier publishes them
+        uint32_t o2 = xslot(k0 - 2) * XSLOT, o1 = xslot(k0 - 1) * XSLOT, o0 = xslot(k0) * XSLOT;
+        uint32_t q2 = 0, q1 = BSLOT, q0 = 2 * BSLOT;
+        for (int kk = k0; kk <= kend + 1; kk++) {
+            // position plane kk and the B0s plane of kb = kk-1 have arrived
             if (producer) {
                 bool ok = true;
-                while (ok && ctl->k_done < kc) { ok = wait_bar(kbar(ctl->k_done + 1)); ctl->k_done++; }
+                for (int q = kk == k0 ? k0 - 2 : kk; q <= kk; q++) ok = wait_bar(xslot(q)) && ok;
+                ok = wait_bar(XR + bslot(kk - 1)) && ok;
                 if (!ok) {
-                    *s_abort = 1;
+                    s_abort[(kk - 1) & 1] = 1;
                     atomicOr(&st->status, (unsigned)GM_ST_TIMEOUT);
                 }
             }
-            __syncthreads();
-            if (*s_abort) break;
-        }
-        if (kc >= k0) {
-            const T* bc = bs + (kc & 1) * PLANE_B;
-            const T* x0 = xring(mx, 2);   // position plane kc
-            const T ezk = __ldg(&ezp[kc]);
-            const bool zimg = zPeri && (kc < 2 || kc >= nz - 2);
+            barrier();
+            if (s_abort[(kk - 1) & 1]) {
+                kstop = kk;
+                break;
+            }
+            // refills, into slots whose last reader was the previous iteration
+            // (every thread is past this iteration's barrier)
+            if (producer) {
+                if (kk > k0 && kk + XD <= kend + 1) issue_x(kk + XD);
+                if (kk - 1 + BD <= kend) issue_b0(kk - 1 + BD);
+                // k planes: the next J phase's (two slots), or this one's (one slot:
+                // the previous J phase, its last reader, is behind the barrier)
+                const int qk = KS == 2 ? kk - 1 : kk - 2;
+                if (n > 0 && qk >= k0 && qk < kend) issue_k(qk);
+            }
+            const int kb = kk - 1;
+            if (kb >= k0 && kb < kend) {
+                __syncwarp();
+                const uint32_t ob0 = L::OFF_B0 + bslot(kb) * XSLOT, obd = L::OFF_B + q0 - R;
+                if (doR) {
+                    const uint32_t s0 = aR + ob0, d0 = aR + obd;
+                    V Bh[3];
+                    if (!faceR) {
+                        V Ah[3][3], rh;
+                        diffs<T, C>(aR + o2, aR + o1, aR + o0, Ah);
+                        const V s[3] = {M::ld2(s0), M::ld2(s0 + C), M::ld2(s0 + 2 * C)};
+                        b_from<T>(Ah, s, Bh, &rh, true);
+                    } else {
+                        const Vec3<T> u = b_face_s<1, C>(p, aR + o2, aR + o1, aR + o0, s0, ic, jR, kb);
+                        const Vec3<T> v = b_face_s<1, C>(p, aR + o2 + E, aR + o1 + E, aR + o0 + E, s0 + E, ic + 1, jR, kb);
+                        Bh[0] = mk2(u.x, v.x); Bh[1] = mk2(u.y, v.y); Bh[2] = mk2(u.z, v.z);
+                    }
 #pragma unroll
-            for (int r = 0; r < R; r++) {
-                if (!own[r]) continue;
-                // in-plane neighbours' B: -x, +x, -y, +y
-                T bxm[3], bxp[3], bym[3], byp[3];
-                ld_b(bc + ob1[r] - 4, bxm);
-                ld_b(bc + ob1[r] + 4, bxp);
-                ld_b(bc + ob1[r] - 4 * BX2, bym);
-                ld_b(bc + ob1[r] + 4 * BX2, byp);
+                    for (int l = 0; l < 3; l++) M::st2(d0 + l * BC, Bh[l]);
+                }
+                if (doC) {
+                    const uint32_t s0 = aC + ob0, d0 = aC + obd;
+                    T Bh[3];
+                    if (!faceC) {
+                        T Ah[3][3], rh;
+                        diffs1<T, C>(aC + o2, aC + o1, aC + o0, Ah);
+                        const T s[3] = {M::ld(s0), M::ld(s0 + C), M::ld(s0 + 2 * C)};
+                        b_from<T>(Ah, s, Bh, &rh, true);
+                    } else {
+                        const Vec3<T> u = b_face_s<0, C>(p, aC + o2, aC + o1, aC + o0, s0, iC, jC, kb);
+                        Bh[0] = u.x; Bh[1] = u.y; Bh[2] = u.z;
+                    }
+#pragma unroll
+                    for (int l = 0; l < 3; l++) M::st(d0 + l * BC, Bh[l]);
+                }
+                __syncwarp();
+            }
+            o2 = o1; o1 = o0;
+            o0 = o0 == (XR - 1) * XSLOT ? 0 : o0 + XSLOT;
+            const uint32_t qt = q2;
+            q2 = q1; q1 = q0; q0 = qt;
+        }
+        // the k planes are awaited by the warps that read them; their parities
+        // follow from the tile's planes
+        if (producer) {
+            if (n > 0)
+                for (int q = k0; q < kend; q++) ph ^= 1u << kbar(q);
+            ctl->ph = ph;
+        }
+    } else {
+        // ---- a pair of the tile: columns ic, ic + 1 of row jc -------------------
+        const int ic = i0 + 2 * (lane & 15), jr = 2 * warp + (lane >> 4), jc = j0 + jr;
+        const bool own = ic < nx && jc < ny, own2 = own && ic + 1 < nx;
+        const uint32_t ax = sb + ((jr + 2) * HX2 + (ic - i0 + 2)) * E;          // in a position / B0s plane
+        const uint32_t ab = ax + (uint32_t)L::OFF_B - R;                        // in a B plane (one halo row fewer)
+        const uint32_t ak = sb + (uint32_t)L::OFF_K + (jr * TX + (ic - i0)) * E;
+        const T dtT = (T)st->dt;
+        V exy = splat<V>((T)0);
+        if (own) exy = mk2(vmul(vmul(p.ex[ic], p.ey[jc]), dtT), own2 ? vmul(vmul(p.ex[ic + 1], p.ey[jc]), dtT) : (T)0);
+        const int iy = image_step(p.yPeri, jc, ny), ix = image_step(p.xPeri, ic, nx);
+        // both points of a pair have the same images when nx is even; an odd nx,
+        // or a direction of three points (two images), takes the general store
+        const bool pairs = !(nx & 1) && !(p.xPeri && nx < 4) && !(p.yPeri && ny < 4) && !(zPeri && nz < 4);
+        const bool xyimage = (iy | ix | image_step(p.xPeri, ic + 1, nx)) != 0;
+        const bool first = LAST && st->nAttempted == 0;
+        V pe[3];
+        if (PRESS) {
+            // p0 and its derivatives along x, y (times 2 dx, 2 dy) at the pair
+            T e[3][2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const T X = p.dx * (T)(ic + h) + p.Ox, Y = p.dy * (T)jc + p.Oy;
+                const T ex = p.p0Amp != (T)0 ? p.p0Amp * exp(-(X * X + Y * Y) * p.inv_p0W2) : (T)0;
+                const T be2 = -2 * p.beta * ex * p.inv_p0W2;
+                e[0][h] = p.beta * ((T)1 + ex);
+                e[1][h] = be2 * X * (2 * p.dx);
+                e[2][h] = be2 * Y * (2 * p.dy);
+            }
+#pragma unroll
+            for (int q = 0; q < 3; q++) pe[q] = mk2(e[q][0], e[q][1]);
+        }
+        // addresses of the pair in the position planes kk - 3 .. kk and in the B
+        // planes kb - 2 .. kb, stepped with kk
+        uint32_t x3 = ax + xslot(k0 - 3) * XSLOT, x2 = ax + xslot(k0 - 2) * XSLOT, x1 = ax + xslot(k0 - 1) * XSLOT,
+                 x0 = ax + xslot(k0) * XSLOT;
+        uint32_t b2 = ab, b1 = ab + BSLOT, b0 = ab + 2 * BSLOT;
+        uint32_t kph = ph0 >> (XR + BR);         // parity of the k slots
+        uint32_t s0 = ax + (uint32_t)L::OFF_B0 + bslot(k0 - 1) * XSLOT;      // in the B0s plane kb
+        // the outputs: the plane's base (the same for all threads) and the pair's
+        // offset in the plane, in bytes
+        T* const Xb = LAST ? a.X[cur ^ 1] : a.XS[n & 1];
+        char* xo = reinterpret_cast<char*>(Xb + (long long)p.px * p.py * (k0 + 2));
+        char* ko = LAST ? nullptr : reinterpret_cast<char*>(a.K[n] + (long long)p.kpx * ny * k0);
+        const uint32_t gx = (uint32_t)(ic + 2 + p.px * (jc + 2)) * E, gk = (uint32_t)(ic + p.kpx * jc) * E;
+        const long long cs = p.cs * E, kcs = p.kcs * E;
+
+        // One iteration; Ac, Rc: the diagonals of plane kc, An, Rn: those of plane kb.
+        auto iteration = [&](int kk, const V (&Ac)[3][3], const V& Rc, V (&An)[3][3], V& Rn) -> bool {
+            const int kb = kk - 1, kc = kk - 2;
+            const T ezk = __ldg(&p.ez[max(kc, 0)]);
+            barrier();
+            if (s_abort[(kk - 1) & 1]) return false;
+            // B on plane kb
+            V Bp[3];
+            {
+                if (!zPeri && (unsigned)kb >= (unsigned)nz) {
+                    // line-tied ghost plane
+                    Vec3<T> u = {0, 0, 0}, v = {0, 0, 0};
+                    if (own) u = b_face_z<C, T>(p, x2, x1, x0, s0, ic, jc, kb);
+                    if (own2) v = b_face_z<C, T>(p, x2 + E, x1 + E, x0 + E, s0 + E, ic + 1, jc, kb);
+                    Bp[0] = mk2(u.x, v.x); Bp[1] = mk2(u.y, v.y); Bp[2] = mk2(u.z, v.z);
+                } else {
+                    diffs<T, C>(x2, x1, x0, An);
+                    const V s[3] = {M::ld2(s0), M::ld2(s0 + C), M::ld2(s0 + 2 * C)};
+                    b_from<T>(An, s, Bp, &Rn, own);
+                }
+#pragma unroll
+                for (int l = 0; l < 3; l++) M::st2_if(own2, b0 + l * BC, Bp[l]);
+                if ((nx & 1) && own && !own2) {
+#pragma unroll
+                    for (int l = 0; l < 3; l++) M::st(b0 + l * BC, lo(Bp[l]));
+                }
+            }
+            // J, k_n and the stage position on plane kc
+            if (kc >= k0) {
                 // Stokes current (current.cu:290-406).  The circulation around a
                 // quadrilateral P1..P4, sum (B_a + B_b).(x_b - x_a) over its edges,
                 // regroups exactly into sum B_a.(x_{a+1} - x_{a-1}); for the quads
@@ -512,158 +769,201 @@ __device__ __forceinline__ bool stage_tile(const StageArgsTMA<T>& A, int bx, int
                 // (1/4) sum of consecutive edge cross products = (1/2) d1 x d2),
                 // and the matrix with those rows has the inverse
                 // 2 [a b c] P / det(a, b, c), so J = (a I1 + b I2 + c I0) / det.
-                T I0 = 0, I1 = 0, I2 = 0;
+                V I0, I1, I2, Bz[3];
 #pragma unroll
                 for (int l = 0; l < 3; l++) {
-                    const T dx = bxp[l] - bxm[l], dy = byp[l] - bym[l], dz = Bp[r][l] - Bm[r][l];
-                    I0 += Ac[r][l][1] * dx - Ac[r][l][0] * dy;
-                    I1 += Ac[r][l][2] * dy - Ac[r][l][1] * dz;
-                    I2 += Ac[r][l][0] * dz - Ac[r][l][2] * dx;
+                    Bz[l] = M::ld2(b1 + l * BC);
+                    const V dx = mk2(vsub(hi(Bz[l]), M::ld(b1 + l * BC - E)), vsub(M::ld(b1 + l * BC + 2 * E), lo(Bz[l])));
+                    const V dy = vsub(M::ld2(b1 + l * BC + R), M::ld2(b1 + l * BC - R));
+                    const V dz = vsub(Bp[l], M::ld2(b2 + l * BC));
+                    if (l == 0) {
+                        I0 = vfms(Ac[l][1], dx, vmul(Ac[l][0], dy));
+                        I1 = vfms(Ac[l][2], dy, vmul(Ac[l][1], dz));
+                        I2 = vfms(Ac[l][0], dz, vmul(Ac[l][2], dx));
+                    } else {
+                        I0 = vfma(Ac[l][1], dx, vfma(vneg(Ac[l][0]), dy, I0));
+                        I1 = vfma(Ac[l][2], dy, vfma(vneg(Ac[l][1]), dz, I1));
+                        I2 = vfma(Ac[l][0], dz, vfma(vneg(Ac[l][2]), dx, I2));
+                    }
                 }
-                T Jv[3];
+                V Jv[3], kn[3];
 #pragma unroll
-                for (int l = 0; l < 3; l++) Jv[l] = (Ac[r][l][0] * I1 + Ac[r][l][1] * I2 + Ac[r][l][2] * I0) * Rc[r];
-                const int lin = lin0[r] + kplane * kc;
-                T kn[3];
-                cross3(Jv, Bz[r], kn);
-                const T f = dtT * (exy[r] * ezk);
+                for (int l = 0; l < 3; l++) Jv[l] = vfma(Ac[l][0], I1, vfma(Ac[l][1], I2, vmul(Ac[l][2], I0)));
+                vcross(Jv, Bz, kn);
+                const V f = vmul(vmul(exy, splat<V>(ezk)), Rc);
 #pragma unroll
-                for (int l = 0; l < 3; l++) kn[l] *= f;
+                for (int l = 0; l < 3; l++) kn[l] = vmul(kn[l], f);
                 if (PRESS) {
-                    Tile<T, 4, XR, 20> tl;
-                    tl.xs = xs;
-                    tl.i0 = i0; tl.j0 = j0; tl.HX = HX2; tl.HY = S::HYR;
-                    tl.slot = SLOT;
-                    T gp[3];
-                    const T D = rcp_stage(Rc[r]) * p.inv8dxdydz;     // Delta = det(a, b, c) / (8 dx dy dz)
-                    grad_p<T>(p, tl, ic, jc[r], kc, D, gp);
+                    V gp[3];
+                    grad_p2<T, C>(p, x3, x2, x1, Ac, Rc, pe, gp);
 #pragma unroll
-                    for (int l = 0; l < 3; l++) kn[l] += -dtT * gp[l];
+                    for (int l = 0; l < 3; l++) kn[l] = vfma(splat<V>(-dtT), gp[l], kn[l]);
                 }
-                T xa[3];
+                V xa[3];
 #pragma unroll
-                for (int l = 0; l < 3; l++) xa[l] = x0[ox1[r] + l * PC];
-                const bool images = img_xy[r] || zimg;
-                const int g = gxy1[r] + pxy * (kc + 2);
-                const T* kp = kslot(kc) + tyx[r];    // k_m component l at kp[(3m + l) * TX * TYR]
+                for (int l = 0; l < 3; l++) xa[l] = M::ld2(x2 + l * C);
+                uint32_t kp = ak;                    // k_m component l at kp + (3 m + l) KC
+                if (n > 0) {
+                    const int ks = KS == 2 ? (kc & 1) : 0;
+                    kp += ks * KSLOT;
+                    if (!mbar_wait_bounded(&bars[XR + BR + ks], (kph >> ks) & 1u)) {
+                        s_abort[kk & 1] = 1;
+                        atomicOr(&st->status, (unsigned)GM_ST_TIMEOUT);
+                    }
+                    kph ^= 1u << ks;
+                }
                 if (!LAST) {
                     // x_{n+1} = x_n + sum_{m<=n} (b[n+1][m] - b[n][m]) k_m (rungeKutta.cu:216-227)
 #pragma unroll
                     for (int m = 0; m < n; m++) {
-                        const T w = p.db[n][m];
+                        const V w = splat<V>(p.db[n][m]);
 #pragma unroll
-                        for (int l = 0; l < 3; l++) xa[l] += w * kp[(3 * m + l) * TX * TYR];
+                        for (int l = 0; l < 3; l++) xa[l] = vfma(w, M::ld2(kp + (3 * m + l) * KC), xa[l]);
                     }
-                    const T w = p.db[n][n];
+                    const V w = splat<V>(p.db[n][n]);
 #pragma unroll
-                    for (int l = 0; l < 3; l++) xa[l] += w * kn[l];
-                    T* Kn = a.K[n];
-                    Kn[lin] = kn[0];
-                    Kn[KC + lin] = kn[1];
-                    Kn[2 * KC + lin] = kn[2];
-                    T* Xo = a.XS[n & 1];
-                    if (images) {
-                        store_pos<T>(p, Xo, ic, jc[r], kc, xa);
-                    } else {
-                        Xo[g] = xa[0];
-                        Xo[cs + g] = xa[1];
-                        Xo[2 * cs + g] = xa[2];
+                    for (int l = 0; l < 3; l++) xa[l] = vfma(w, kn[l], xa[l]);
+                    if (own2) {
+#pragma unroll
+                        for (int l = 0; l < 3; l++) stv(reinterpret_cast<T*>(ko + l * kcs + gk), kn[l]);
+                    }
+                    if ((nx & 1) && own && !own2) {
+#pragma unroll
+                        for (int l = 0; l < 3; l++) *reinterpret_cast<T*>(ko + l * kcs + gk) = lo(kn[l]);
                     }
                 } else {
-                    // stage 5: x_6, x_new, x* and the error norm (rungeKutta.cu:251-339)
-                    T km[6][3];
+                    // stage 5: x_new and the error norm |x_new - x*| or |sum (c - c*) k|
+                    V e[3];
+                    if (p.errMode == 0) {
+                        // the reference's sums in their order (x_6 and its last term, which
+                        // is zero, apart; c_1 = c_4 = c*_1 = 0): a first step's error norm is
+                        // rounding, and its dt follows from it
+                        V xst[3];
 #pragma unroll
-                    for (int m = 0; m < 5; m++)
+                        for (int m = 0; m < 5; m++)
 #pragma unroll
-                        for (int l = 0; l < 3; l++) km[m][l] = kp[(3 * m + l) * TX * TYR];
+                            for (int l = 0; l < 3; l++)
+                                xa[l] = vfma(splat<V>(p.db[5][m]), M::ld2(kp + (3 * m + l) * KC), xa[l]);
 #pragma unroll
-                    for (int l = 0; l < 3; l++) km[5][l] = kn[l];
+                        for (int l = 0; l < 3; l++) xst[l] = xa[l];
 #pragma unroll
-                    for (int m = 0; m < 6; m++)
+                        for (int m = 0; m < 6; m++) {
+                            if (m == 1) continue;
 #pragma unroll
-                        for (int l = 0; l < 3; l++) xa[l] += p.db[5][m] * km[m][l];
-                    T xnew[3];
-#pragma unroll
-                    for (int l = 0; l < 3; l++) {
-                        xnew[l] = xa[l];
-                        T xst = xa[l];
-                        T dl = 0;
-                        if (l < 2 || p.zUpdate) {
-                            if (p.errMode == 0) {
-#pragma unroll
-                                for (int m = 0; m < 6; m++) {
-                                    xnew[l] += p.c[m] * km[m][l];
-                                    xst += p.cst[m] * km[m][l];
-                                }
-                                dl = fabs(xnew[l] - xst);
-                            } else {
-                                // sum (c - c*) k: no cancellation against x
-                                T e = 0;
-#pragma unroll
-                                for (int m = 0; m < 6; m++) {
-                                    xnew[l] += p.c[m] * km[m][l];
-                                    e += p.cmcT[m] * km[m][l];
-                                }
-                                dl = fabs(e);
+                            for (int l = 0; l < 3; l++) {
+                                if (l == 2 && !p.zUpdate) continue;
+                                const V km = m < 5 ? M::ld2(kp + (3 * m + l) * KC) : kn[l];
+                                if (m != 4) xa[l] = vfma(splat<V>(p.c[m]), km, xa[l]);
+                                xst[l] = vfma(splat<V>(p.cst[m]), km, xst[l]);
                             }
                         }
-                        if (dl > dmax) dmax = dl;     // NaN never wins (maths.cu:144-153)
-                        if (!isfinite(dl) || !isfinite(xnew[l])) bad = true;   // NaN/Inf anywhere in k_0..k_5
-                    }
-                    if (images) {
-                        store_pos<T>(p, a.X[cur], ic, jc[r], kc, xa);
-                        store_pos<T>(p, a.X[cur ^ 1], ic, jc[r], kc, xnew);
+#pragma unroll
+                        for (int l = 0; l < 3; l++) e[l] = vsub(xa[l], xst[l]);
                     } else {
-                        T* X6 = a.X[cur];
-                        T* Xn = a.X[cur ^ 1];
-                        X6[g] = xa[0]; X6[cs + g] = xa[1]; X6[2 * cs + g] = xa[2];
-                        Xn[g] = xnew[0]; Xn[cs + g] = xnew[1]; Xn[2 * cs + g] = xnew[2];
+                        // sum (c - c*) k: no cancellation against x
+                        e[0] = e[1] = e[2] = splat<V>((T)0);
+#pragma unroll
+                        for (int m = 0; m < 6; m++) {
+                            const V wc = splat<V>(p.cb[m]), wz = splat<V>(p.cbz[m]), we = splat<V>(p.cmcT[m]);
+#pragma unroll
+                            for (int l = 0; l < 3; l++) {
+                                const V km = m < 5 ? M::ld2(kp + (3 * m + l) * KC) : kn[l];
+                                xa[l] = vfma(l == 2 ? wz : wc, km, xa[l]);
+                                e[l] = vfma(we, km, e[l]);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int l = 0; l < 3; l++) {
+                        const T y1 = lo(xa[l]), y2 = hi(xa[l]), e1 = lo(e[l]), e2 = hi(e[l]);
+                        if (own && (l < 2 || p.zUpdate)) max_nn(dmax, e1);
+                        if (own2 && (l < 2 || p.zUpdate)) max_nn(dmax, e2);
+                        // NaN/Inf anywhere in k_0..k_5
+                        bad |= own && (!finite_bits(y1) || !finite_bits(e1));
+                        bad |= own2 && (!finite_bits(y2) || !finite_bits(e2));
                     }
                 }
-            }
-        }
-        // the diagonals of plane kb become those of the next iteration's kc
+                const int iz = image_step(p.zPeri, kc, nz);
+                if (pairs) {
+                    if (own2) {
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-#pragma unroll
-            for (int l = 0; l < 3; l++) {
-                Ac[r][l][0] = An[r][l][0]; Ac[r][l][1] = An[r][l][1]; Ac[r][l][2] = An[r][l][2];
+                        for (int l = 0; l < 3; l++) stv(reinterpret_cast<T*>(xo + l * cs + gx), xa[l]);
+                    }
+                    if (own2 && (ix | iy | iz)) {
+                        T* q = reinterpret_cast<T*>(xo + gx);
+                        if (ix) st_xyz(q + ix, p.cs, image_shift<T>(xa[0], ix, p.Lx, p.dx), xa[1], xa[2]);
+                        if (iy | iz) store_images_call<T, V>(p, q, xa[0], xa[1], xa[2], ix, iy, iz);
+                    }
+                } else {
+                    T* q = reinterpret_cast<T*>(xo + gx);
+                    if (own) st_xyz(q, p.cs, lo(xa[0]), lo(xa[1]), lo(xa[2]));
+                    if (own2) st_xyz(q + 1, p.cs, hi(xa[0]), hi(xa[1]), hi(xa[2]));
+                    if (own && (xyimage || iz)) {
+                        store_point_images<T>(p, Xb, ic, jc, kc, lo(xa[0]), lo(xa[1]), lo(xa[2]));
+                        if (own2) store_point_images<T>(p, Xb, ic + 1, jc, kc, hi(xa[0]), hi(xa[1]), hi(xa[2]));
+                    }
+                }
+                if (LAST && first && own && (xyimage || iz)) refresh_images<T>(p, a.X[cur], ic, jc, kc, pairs, own2, ix, iy, iz);
+                xo += (long long)p.px * p.py * E;
+                if (!LAST) ko += (long long)p.kpx * ny * E;
             }
-            Rc[r] = Rn[r];
+            // step the rings
+            x3 = x2; x2 = x1; x1 = x0;
+            x0 = x0 == ax + (XR - 1) * XSLOT ? ax : x0 + XSLOT;
+            const uint32_t bt = b2;
+            b2 = b1; b1 = b0; b0 = bt;
+            s0 = s0 == ax + (uint32_t)L::OFF_B0 + (BR - 1) * XSLOT ? ax + (uint32_t)L::OFF_B0 : s0 + XSLOT;
+            return true;
+        };
+
+        const V zero = splat<V>((T)0);
+        V A0[3][3], A1[3][3], R0 = zero, R1 = zero;
+#pragma unroll
+        for (int e = 0; e < 9; e++) { A0[e / 3][e % 3] = zero; A1[e / 3][e % 3] = zero; }
+#pragma unroll 1
+        for (int kk = k0; kk <= kend + 1; kk += 2) {
+            if (!iteration(kk, A0, R0, A1, R1)) break;
+            if (kk + 1 > kend + 1) break;
+            if (!iteration(kk + 1, A1, R1, A0, R0)) break;
         }
-    }
-    // drain copies still in flight (after an abort), bounded
-    if (producer && *s_abort) {
-        for (int q = ctl->x_done + 1; q <= ctl->x_iss; q++) wait_bar(xslot(q));
-        for (int q = ctl->b_done + 1; q <= ctl->b_iss; q++) wait_bar(XR + (q & 1));
-        if (n > 0)
-            for (int q = ctl->k_done + 1; q <= ctl->k_iss; q++) wait_bar(kbar(q));
     }
     if (bad) atomicOr(&st->status, (unsigned)GM_ST_NAN);
     if (LAST) {
-        for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-        if (tx == 0) s_wmax[ty] = dmax;
-        __syncthreads();
-        if (tid == 0) {
-            T m = 0;
-            for (int w = 0; w < TY2; w++) m = fmax(m, s_wmax[w]);
-            if (m > 0) atomicMax(&st->maxDeltaBits, (unsigned long long)__double_as_longlong((double)m));
-        }
+        for (int o = 16; o > 0; o >>= 1) max_nn(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+        if (lane == 0 && warp < NW) s_wmax[warp] = dmax;
     }
-    return *s_abort == 0;
+    __syncthreads();       // the warp maxima; ctl for the next tile
+    const bool left = s_abort[0] || s_abort[1];
+    if (left && tid == 32 * (NW + 1)) {
+        // left early: the copies that may still be in flight (bounded waits); those
+        // of an iteration's start have been waited for.  A slot's parity follows
+        // from the tile's earlier planes in it.
+        auto drain = [&](int b, int uses) { mbar_wait_bounded(&bars[b], ((ph0 >> b) + uses) & 1u); };
+        for (int q = kstop + 1; q <= min(max(kstop - 1, k0) + XD, kend + 1); q++) drain(xslot(q), (q - (k0 - 2)) / XR);
+        for (int q = kstop; q <= min(kstop - 2 + BD, kend); q++) drain(XR + bslot(q), (q - (k0 - 1)) / BR);
+        if (n > 0)
+            for (int q = max(k0, kstop - 3); q <= min(kstop - (KS == 2 ? 2 : 3), kend - 1); q++)
+                drain(kbar(q), KS == 2 ? (q - k0) / 2 : q - k0);
+    }
+    if (LAST && tid == 0) {
+        T m = 0;
+        for (int w = 0; w < NW; w++) max_nn(m, s_wmax[w]);
+        if (m > 0) atomicMax(&st->maxDeltaBits, (unsigned long long)__double_as_longlong((double)m));
+    }
+    return !left;
 }
 
 // Shared-memory set-up common to the stage kernels: the 128-byte aligned
 // base, the mbarriers and the abort flag.
-template <typename T, bool PRESS, int NS, int R>
+template <typename T, bool PRESS, int NS, int NW>
 __device__ __forceinline__ unsigned char* stage_smem_setup(unsigned char* smraw) {
-    using L = StageSmem<T, PRESS, NS, R>;
+    using L = StageSmem<T, PRESS, NS, NW>;
     unsigned char* base = smraw + ((128u - (smem_u32(smraw) & 127u)) & 127u);
     uint64_t* bars = reinterpret_cast<uint64_t*>(base + L::OFF_BAR);
     StageCtl* ctl = reinterpret_cast<StageCtl*>(base + L::OFF_CTL);
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
+    if (threadIdx.x == 0) {
         ctl->ph = 0;
-        ctl->abort = 0;
+        ctl->abort[0] = ctl->abort[1] = 0;
         for (int s = 0; s < L::NBAR; s++) mbar_init(&bars[s], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -671,160 +971,108 @@ __device__ __forceinline__ unsigned char* stage_smem_setup(unsigned char* smraw)
     return base;
 }
 
-// One RK stage of one case: one CTA per 32 x 8R x TZ block, R =
-// stage_rows<T, PRESS>() (minimum CTAs per SM: 3 for one FP32 row group, 2 for
-// two, 2 in FP64).
-template <typename T, bool PRESS, int NS>
-__global__ void __launch_bounds__(TX * TY2, sizeof(T) == 4 ? (stage_rows<T, PRESS>() == 1 ? GM_STAGE_MINB : 2) : 2)
+// One RK stage of one case: one CTA per 32 x 2 NW x TZ block.
+template <typename T, bool PRESS, int NS, int NW>
+__global__ void __launch_bounds__(stage_threads<NW>(), stage_ctas<T, NW>())
     k_stage_tma(const __grid_constant__ StageArgsTMA<T> A) {
     extern __shared__ __align__(128) unsigned char smraw[];
     if (A.a.st->done || (A.a.st->status & (GM_ST_TIMEOUT | GM_ST_ALIGN))) return;
-    constexpr int R = stage_rows<T, PRESS>();
-    unsigned char* base = stage_smem_setup<T, PRESS, NS, R>(smraw);
-    stage_tile<T, PRESS, NS, R>(A, blockIdx.x, blockIdx.y, blockIdx.z, base);
+    unsigned char* base = stage_smem_setup<T, PRESS, NS, NW>(smraw);
+    stage_tile<T, PRESS, NS, NW>(A, blockIdx.x, blockIdx.y, blockIdx.z, base);
 }
 
 // One RK stage of many cases: a persistent launch whose CTAs take work items
 // (case, tile) from a counter until none is left; cases whose controller has
 // stopped are skipped.  The counter is reset by the batched controller.
 template <typename T, bool PRESS, int NS>
-__global__ void __launch_bounds__(TX * TY2, 2)
+__global__ void __launch_bounds__(stage_threads<STAGE_BATCH_NW>(), stage_ctas<T, STAGE_BATCH_NW>())
     k_stage_tma_batch(const StageArgsTMA<T>* __restrict__ cases, const int4* __restrict__ work, int nwork,
                       int* __restrict__ counter) {
-    using L = StageSmem<T, PRESS, NS, 1>;
+    constexpr int NW = STAGE_BATCH_NW;
+    using L = StageSmem<T, PRESS, NS, NW>;
     extern __shared__ __align__(128) unsigned char smraw[];
-    unsigned char* base = stage_smem_setup<T, PRESS, NS, 1>(smraw);
+    unsigned char* base = stage_smem_setup<T, PRESS, NS, NW>(smraw);
     int* s_w = &reinterpret_cast<StageCtl*>(base + L::OFF_CTL)->work;
     for (;;) {
-        if (threadIdx.x == 0 && threadIdx.y == 0) *s_w = atomicAdd(counter, 1);
+        if (threadIdx.x == 0) *s_w = atomicAdd(counter, 1);
         __syncthreads();
         const int w = *s_w;
         __syncthreads();   // s_w is rewritten only after every thread has read it
         if (w >= nwork) break;
         const int4 it = work[w];
-        if (!stage_tile<T, PRESS, NS, 1>(cases[it.x], it.y, it.z, it.w, base)) break;
+        if (!stage_tile<T, PRESS, NS, NW>(cases[it.x], it.y, it.z, it.w, base)) break;
         __syncthreads();   // the next tile's copies overwrite slots this one read
     }
 }
 
-template <typename T, int R>
-size_t stage_tma_smem_bytes_r(int pressure, int n) {
+// f(integral constant NS) for a run-time stage index
+template <typename F>
+static auto stage_dispatch(int n, F f) {
     switch (n) {
-        case 0: return pressure ? StageSmem<T, true, 0, R>::BYTES : StageSmem<T, false, 0, R>::BYTES;
-        case 1: return pressure ? StageSmem<T, true, 1, R>::BYTES : StageSmem<T, false, 1, R>::BYTES;
-        case 2: return pressure ? StageSmem<T, true, 2, R>::BYTES : StageSmem<T, false, 2, R>::BYTES;
-        case 3: return pressure ? StageSmem<T, true, 3, R>::BYTES : StageSmem<T, false, 3, R>::BYTES;
-        case 4: return pressure ? StageSmem<T, true, 4, R>::BYTES : StageSmem<T, false, 4, R>::BYTES;
-        default: return pressure ? StageSmem<T, true, 5, R>::BYTES : StageSmem<T, false, 5, R>::BYTES;
+        case 0: return f(std::integral_constant<int, 0>());
+        case 1: return f(std::integral_constant<int, 1>());
+        case 2: return f(std::integral_constant<int, 2>());
+        case 3: return f(std::integral_constant<int, 3>());
+        case 4: return f(std::integral_constant<int, 4>());
+        default: return f(std::integral_constant<int, 5>());
     }
 }
 
-// dynamic shared memory of the single-case stage kernel
-template <typename T>
-size_t stage_tma_smem_bytes(int pressure, int n) {
-    return pressure ? stage_tma_smem_bytes_r<T, stage_rows<T, true>()>(1, n)
-                    : stage_tma_smem_bytes_r<T, stage_rows<T, false>()>(0, n);
-}
-
-template <typename T, bool PRESS, int NS>
-static cudaError_t prep_one() {
-    return cudaFuncSetAttribute(k_stage_tma<T, PRESS, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-}
-
-template <typename T, bool PRESS, int NS>
-static cudaError_t prep_batch() {
-    return cudaFuncSetAttribute(k_stage_tma_batch<T, PRESS, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                200 * 1024);
-}
-
-template <typename T>
-cudaError_t prepare_stage_tma() {
-    cudaError_t e;
-    if ((e = prep_one<T, false, 0>()) || (e = prep_one<T, false, 1>()) || (e = prep_one<T, false, 2>()) ||
-        (e = prep_one<T, false, 3>()) || (e = prep_one<T, false, 4>()) || (e = prep_one<T, false, 5>()) ||
-        (e = prep_one<T, true, 0>()) || (e = prep_one<T, true, 1>()) || (e = prep_one<T, true, 2>()) ||
-        (e = prep_one<T, true, 3>()) || (e = prep_one<T, true, 4>()) || (e = prep_one<T, true, 5>()))
-        return e;
-    if ((e = prep_batch<T, false, 0>()) || (e = prep_batch<T, false, 1>()) || (e = prep_batch<T, false, 2>()) ||
-        (e = prep_batch<T, false, 3>()) || (e = prep_batch<T, false, 4>()) || (e = prep_batch<T, false, 5>()) ||
-        (e = prep_batch<T, true, 0>()) || (e = prep_batch<T, true, 1>()) || (e = prep_batch<T, true, 2>()) ||
-        (e = prep_batch<T, true, 3>()) || (e = prep_batch<T, true, 4>()) || (e = prep_batch<T, true, 5>()))
-        return e;
+template <typename T, bool PRESS>
+cudaError_t prepare_stage_tma_p() {
+    const int lim = 227 * 1024;
+    for (int n = 0; n < 6; n++) {
+        const cudaError_t e = stage_dispatch(n, [&](auto N) {
+            cudaError_t r = cudaFuncSetAttribute(k_stage_tma<T, PRESS, N.value, STAGE_NW>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+            if (r == cudaSuccess)
+                r = cudaFuncSetAttribute(k_stage_tma<T, PRESS, N.value, STAGE_NW_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+            if (r == cudaSuccess)
+                r = cudaFuncSetAttribute(k_stage_tma_batch<T, PRESS, N.value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         lim);
+            return r;
+        });
+        if (e != cudaSuccess) return e;
+    }
     return cudaSuccess;
 }
 
-template <typename T>
-int stage_tma_batch_occupancy(int pressure) {
+template <typename T, bool PRESS>
+int stage_tma_batch_occupancy_p() {
     int nb = 0;
-    const size_t sm = stage_tma_smem_bytes_r<T, 1>(pressure, 5);
-    cudaError_t e = pressure
-        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_stage_tma_batch<T, true, 5>, TX * TY2, sm)
-        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_stage_tma_batch<T, false, 5>, TX * TY2, sm);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &nb, k_stage_tma_batch<T, PRESS, 5>, stage_threads<STAGE_BATCH_NW>(), StageSmem<T, PRESS, 5, STAGE_BATCH_NW>::BYTES);
     return e == cudaSuccess && nb > 0 ? nb : 1;
 }
 
-template <typename T>
-cudaError_t launch_stage_tma_batch(const StageArgsTMA<T>* cases, const int4* work, int nwork, int* counter, int n,
-                                   int pressure, int nblocks, cudaStream_t s) {
-    const dim3 block(TX, TY2, 1);
-    const size_t sm = stage_tma_smem_bytes_r<T, 1>(pressure, n);
-#define GMK_LAUNCH_B(PR)                                                                                        \
-    switch (n) {                                                                                                \
-        case 0: k_stage_tma_batch<T, PR, 0><<<nblocks, block, sm, s>>>(cases, work, nwork, counter); break;      \
-        case 1: k_stage_tma_batch<T, PR, 1><<<nblocks, block, sm, s>>>(cases, work, nwork, counter); break;      \
-        case 2: k_stage_tma_batch<T, PR, 2><<<nblocks, block, sm, s>>>(cases, work, nwork, counter); break;      \
-        case 3: k_stage_tma_batch<T, PR, 3><<<nblocks, block, sm, s>>>(cases, work, nwork, counter); break;      \
-        case 4: k_stage_tma_batch<T, PR, 4><<<nblocks, block, sm, s>>>(cases, work, nwork, counter); break;      \
-        default: k_stage_tma_batch<T, PR, 5><<<nblocks, block, sm, s>>>(cases, work, nwork, counter); break;     \
-    }
-    if (pressure) {
-        GMK_LAUNCH_B(true)
-    } else {
-        GMK_LAUNCH_B(false)
-    }
-#undef GMK_LAUNCH_B
-    return cudaGetLastError();
+template <typename T, bool PRESS>
+cudaError_t launch_stage_tma_batch_p(const StageArgsTMA<T>* cases, const int4* work, int nwork, int* counter, int n,
+                                     int nblocks, cudaStream_t s) {
+    return stage_dispatch(n, [&](auto N) {
+        constexpr size_t sm = StageSmem<T, PRESS, N.value, STAGE_BATCH_NW>::BYTES;
+        k_stage_tma_batch<T, PRESS, N.value><<<nblocks, stage_threads<STAGE_BATCH_NW>(), sm, s>>>(cases, work, nwork, counter);
+        return cudaGetLastError();
+    });
 }
 
-template <typename T>
-int stage_tma_occupancy(int pressure) {
-    int nb = 0;
-    const size_t sm = stage_tma_smem_bytes<T>(pressure, 5);
-    cudaError_t e = pressure
-        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_stage_tma<T, true, 5>, TX * TY2, sm)
-        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_stage_tma<T, false, 5>, TX * TY2, sm);
-    return e == cudaSuccess && nb > 0 ? nb : 1;
+template <typename T, bool PRESS>
+cudaError_t launch_stage_tma_p(const StageArgsTMA<T>& A, int nw, dim3 grid, cudaStream_t s) {
+    return stage_dispatch(A.a.n, [&](auto N) {
+        if (nw == STAGE_NW)
+            k_stage_tma<T, PRESS, N.value, STAGE_NW>
+                <<<grid, stage_threads<STAGE_NW>(), StageSmem<T, PRESS, N.value, STAGE_NW>::BYTES, s>>>(A);
+        else
+            k_stage_tma<T, PRESS, N.value, STAGE_NW_SMALL>
+                <<<grid, stage_threads<STAGE_NW_SMALL>(), StageSmem<T, PRESS, N.value, STAGE_NW_SMALL>::BYTES, s>>>(A);
+        return cudaGetLastError();
+    });
 }
 
-template <typename T>
-cudaError_t launch_stage_tma(const StageArgsTMA<T>& A, int pressure, dim3 grid, cudaStream_t s) {
-    const dim3 block(TX, TY2, 1);
-    const size_t sm = stage_tma_smem_bytes<T>(pressure, A.a.n);
-#define GMK_LAUNCH_N(PR)                                                              \
-    switch (A.a.n) {                                                                  \
-        case 0: k_stage_tma<T, PR, 0><<<grid, block, sm, s>>>(A); break;              \
-        case 1: k_stage_tma<T, PR, 1><<<grid, block, sm, s>>>(A); break;              \
-        case 2: k_stage_tma<T, PR, 2><<<grid, block, sm, s>>>(A); break;              \
-        case 3: k_stage_tma<T, PR, 3><<<grid, block, sm, s>>>(A); break;              \
-        case 4: k_stage_tma<T, PR, 4><<<grid, block, sm, s>>>(A); break;              \
-        default: k_stage_tma<T, PR, 5><<<grid, block, sm, s>>>(A); break;             \
-    }
-    if (pressure) {
-        GMK_LAUNCH_N(true)
-    } else {
-        GMK_LAUNCH_N(false)
-    }
-#undef GMK_LAUNCH_N
-    return cudaGetLastError();
-}
-
-#define GMK_INSTANTIATE_TMA(T)                                                                \
-    template size_t stage_tma_smem_bytes<T>(int, int);                                             \
-    template cudaError_t prepare_stage_tma<T>();                                              \
-    template int stage_tma_occupancy<T>(int);                                                 \
-    template cudaError_t launch_stage_tma<T>(const StageArgsTMA<T>&, int, dim3, cudaStream_t);                 \
-    template int stage_tma_batch_occupancy<T>(int);                                                           \
-    template cudaError_t launch_stage_tma_batch<T>(const StageArgsTMA<T>*, const int4*, int, int*, int, int, int, \
-                                                   cudaStream_t);
+#define GMK_INSTANTIATE_TMA(T, PRESS)                                                                          \
+    template cudaError_t prepare_stage_tma_p<T, PRESS>();                                                      \
+    template cudaError_t launch_stage_tma_p<T, PRESS>(const StageArgsTMA<T>&, int, dim3, cudaStream_t);        \
+    template int stage_tma_batch_occupancy_p<T, PRESS>();                                                      \
+    template cudaError_t launch_stage_tma_batch_p<T, PRESS>(const StageArgsTMA<T>*, const int4*, int, int*, int, int, \
+                                                            cudaStream_t);
 
 }  // namespace gmk
