@@ -113,6 +113,7 @@ struct Impl : ImplBase {
     T* KU[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     T* B0 = nullptr;
     T* B0s = nullptr;           // B0 scaled for the algebraic B formula
+    T* BF = nullptr;            // field kernels: B and 1/det, padded (3 components and a scalar)
     T* shear_tab = nullptr;     // initially distorted grid: the z ghost planes' corrected positions
     T* outB = nullptr;
     T* outJ = nullptr;
@@ -137,6 +138,8 @@ struct Impl : ImplBase {
     int64_t step_launches = 7;      // kernel launches in the captured step
     // TMA-fed stage kernel: tensor maps of X[0], X[1], XS[0], XS[1]
     bool use_tma = true;
+    bool use_fields = false;    // single-case stages by the field kernels
+    bool batched = false;       // a case of a batch: its stages are the batch's
     CUtensorMap tmaps[10];      // single-case kernel (tile height 2 NW2)
     CUtensorMap tmaps_b[10];    // batched kernel (tile height STAGE_BATCH_TY)
     dim3 grid2;
@@ -148,7 +151,7 @@ struct Impl : ImplBase {
         if (graph) cudaGraphDestroy(graph);
         void* ptrs[] = {X[0], X[1], XS[0], XS[1], K[0], K[1], K[2], K[3], K[4], B0, B0s, outB, outJ,
                         outD, stage_buf, eps, eps_col, st, log, part, red, U[0], U[1], US[0], US[1],
-                        KU[0], KU[1], KU[2], KU[3], KU[4], shear_tab};
+                        KU[0], KU[1], KU[2], KU[3], KU[4], shear_tab, BF};
         for (void* q : ptrs)
             if (q) cudaFree(q);
         if (h_st) cudaFreeHost(h_st);
@@ -234,6 +237,7 @@ struct Impl : ImplBase {
             kp.cb[m] = (T)((double)(T)cd[m] - b5);
             kp.cbz[m] = kp.zUpdate ? kp.cb[m] : (T)-b5;
         }
+        kp.inv8 = (T)(1.0 / (8.0 * (double)(T)p->dx * (double)(T)p->dy * (double)(T)p->dz));
         kp.vol8 = (T)(8.0 * (double)(T)p->dx * (double)(T)p->dy * (double)(T)p->dz);
         const T w4[3] = {4 * kp.dy * kp.dz, 4 * kp.dx * kp.dz, 4 * kp.dx * kp.dy};   // as k_scale_b0
         for (int l = 0; l < 3; l++) {
@@ -329,7 +333,19 @@ struct Impl : ImplBase {
         if (use_tma) {
             if ((rc = init_tma(nsm))) return rc;
         }
-        if ((rc = alloc((void**)&part, (size_t)nparts * gmk::R_COUNT * sizeof(double)))) return rc;
+        // Stages by the field kernels (gm_fields.cuh): FP64 frictional Stokes runs,
+        // the inertial equation and the currents with a kernel of their own.  Where
+        // their B field does not fit the device's memory, the tile kernels stay.
+        const bool stokes = strncmp(p->jMethod, "Stokes ", 7) == 0;
+        use_fields = p->stageKernel == 0 && !batched && !kp.jClassic && !kp.jxbAver &&
+                     (sizeof(T) == 8 || !stokes || kp.inertia);
+        if (use_fields && stokes && cudaMalloc((void**)&BF, 4 * (size_t)kp.cs * sizeof(T)) != cudaSuccess) {
+            cudaGetLastError();
+            BF = nullptr;
+            use_fields = false;
+        }
+        const int np = std::max(nparts, gmk::diag_blocks<T>(kp.N));
+        if ((rc = alloc((void**)&part, (size_t)np * gmk::R_COUNT * sizeof(double)))) return rc;
         if ((rc = alloc((void**)&red, (gmk::R_COUNT + 1) * sizeof(double)))) return rc;   // + eps*
         CUDA_TRY(cudaStreamSynchronize(stream));
         return GM_OK;
@@ -429,6 +445,8 @@ struct Impl : ImplBase {
         for (int m = 0; m < 5; m++) a.KU[m] = KU[m];
         a.B0 = B0;
         a.B0s = B0s;
+        a.BF = BF;
+        a.RF = BF ? BF + 3 * kp.cs : nullptr;
         a.st = st;
         a.log = log;
         a.n = n;
@@ -484,7 +502,20 @@ struct Impl : ImplBase {
     int stage(int n) override {
         if (!uploaded) return gm::fail(GM_ENOTREADY, "gm_stage before gm_upload");
         if (n < 0 || n > 5) return gm::fail(GM_EPARAM, "stage index must be 0..5");
-        if (use_tma) {
+        if (use_fields && !stall_on) {
+            const StageArgs<T> a = args(n);
+            const bool own = kp.jOct || kp.jQuint || kp.jTri;
+            CUDA_TRY(gmk::launch_b_field<T>(a, own, 0, stream));
+            if (own) {
+                // these currents read B at the edge neighbours too, with the
+                // reference's ghost values (current() before kk(), main.cu:272-281)
+                CUDA_TRY(gmk::launch_export_ghosts<T>(kp, outB, outD, stream));
+                CUDA_TRY(gmk::launch_j_own<T>(a, 0, stream));
+                launches += 1 + kp.xPeri + kp.yPeri + kp.zPeri;
+            }
+            CUDA_TRY(gmk::launch_stage_field<T>(a, gp.pressure, own, stream));
+            launches++;
+        } else if (use_tma) {
             gmk::StageArgsTMA<T> A;
             memcpy(A.tm, tmaps, sizeof tmaps);
             A.a = args(n);
@@ -502,7 +533,7 @@ struct Impl : ImplBase {
                 CUDA_TRY(gmk::launch_export_ghosts<T>(kp, outB, outD, stream));
                 launches += 1 + kp.xPeri + kp.yPeri + kp.zPeri;
                 if (kp.jOct || kp.jQuint || kp.jTri) {
-                    CUDA_TRY(kp.jOct ? gmk::launch_j_oct<T>(args(n), stream) : gmk::launch_j_quint<T>(args(n), stream));
+                    CUDA_TRY(gmk::launch_j_own<T>(args(n), 0, stream));
                     launches++;
                 }
             }
@@ -764,25 +795,38 @@ struct Impl : ImplBase {
         if (!uploaded) return gm::fail(GM_ENOTREADY, "gm_refresh before gm_upload");
         int rc = read_state();
         if (rc) return rc;
-        StageArgs<T> a = args(0);
-        if (kp.jOct || kp.jQuint || kp.jTri) {
-            // the octilateral and quintilateral currents need the exported B
-            // with its ghosts first; the diagnostic pass then reads J from it
-            StageArgs<T> aj = args(0);
-            aj.jpass = 1;
-            CUDA_TRY(gmk::launch_stage<T>(aj, gmk::MODE_DIAG, gp.pressure, grid, block, smem_diag, stream));
-            CUDA_TRY(gmk::launch_export_ghosts<T>(kp, outB, outD, stream));
-            CUDA_TRY(kp.jOct ? gmk::launch_j_oct<T>(aj, stream) : gmk::launch_j_quint<T>(aj, stream));
-            launches += 2 + kp.xPeri + kp.yPeri + kp.zPeri;
-        }
-        CUDA_TRY(gmk::launch_stage<T>(a, gmk::MODE_DIAG, gp.pressure, grid, block, smem_diag, stream));
-        CUDA_TRY(gmk::launch_finalize<T>(part, nparts, red, stream));
+        if ((rc = enqueue_diag())) return rc;
+        // the exported arrays' periodic faces (setPeriFace)
         CUDA_TRY(gmk::launch_export_ghosts<T>(kp, outB, outD, stream));
+        launches += kp.xPeri + kp.yPeri + kp.zPeri;
         CUDA_TRY(gmk::launch_eps_star<T>(kp, outB, outJ, X[h_st->cur], eps_col, red + gmk::R_COUNT, stream));
-        launches += 3 + kp.xPeri + kp.yPeri + kp.zPeri;
+        launches += 2;
         CUDA_TRY(cudaMemcpyAsync(h_red, red, (gmk::R_COUNT + 1) * sizeof(double), cudaMemcpyDeviceToHost, stream));
         CUDA_TRY(cudaStreamSynchronize(stream));
         reduction_from_host(r);
+        return GM_OK;
+    }
+
+    // B, Delta and J at the current grid into the exported arrays, and the
+    // reductions into `red`.
+    int enqueue_diag() {
+        StageArgs<T> a = args(0);
+        if (kp.jClassic) {      // its J needs Delta at the neighbours: the tile kernel
+            CUDA_TRY(gmk::launch_stage<T>(a, gmk::MODE_DIAG, gp.pressure, grid, block, smem_diag, stream));
+            CUDA_TRY(gmk::launch_finalize<T>(part, nparts, red, stream));
+            launches += 2;
+            return GM_OK;
+        }
+        const bool own = kp.jOct || kp.jQuint || kp.jTri;
+        CUDA_TRY(gmk::launch_b_field<T>(a, 1, 1, stream));
+        if (own) {
+            CUDA_TRY(gmk::launch_export_ghosts<T>(kp, outB, outD, stream));
+            CUDA_TRY(gmk::launch_j_own<T>(a, 1, stream));
+            launches += 1 + kp.xPeri + kp.yPeri + kp.zPeri;
+        }
+        CUDA_TRY(gmk::launch_diag_field<T>(a, own, stream));
+        CUDA_TRY(gmk::launch_finalize<T>(part, gmk::diag_blocks<T>(kp.N), red, stream));
+        launches += 3;
         return GM_OK;
     }
 
@@ -792,10 +836,8 @@ struct Impl : ImplBase {
     // After the stream has synchronised, h_st holds the state and
     // reduction_from_host the reductions (no exported ghosts or epsilon*).
     int enqueue_check() {
-        StageArgs<T> a = args(0);
-        CUDA_TRY(gmk::launch_stage<T>(a, gmk::MODE_DIAG, gp.pressure, grid, block, smem_diag, stream));
-        CUDA_TRY(gmk::launch_finalize<T>(part, nparts, red, stream));
-        launches += 2;
+        const int rc = enqueue_diag();
+        if (rc) return rc;
         CUDA_TRY(cudaMemcpyAsync(h_red, red, (gmk::R_COUNT + 1) * sizeof(double), cudaMemcpyDeviceToHost, stream));
         CUDA_TRY(cudaMemcpyAsync(h_st, st, sizeof(DevState), cudaMemcpyDeviceToHost, stream));
         return GM_OK;
@@ -970,6 +1012,7 @@ struct Batch : BatchBase {
             if (strncmp(p.jMethod, "Stokes ", 7) != 0 || p.inertia || p.jxbAver)
                 return gm::fail(GM_EPARAM, "gm_batch_create: batched cases use the frictional equation and the Stokes current");
             cs.emplace_back(new Impl<T>());
+            cs.back()->batched = true;
             if ((rc = cs.back()->init(&p))) return rc;
             cs.back()->stream = stream;
             memcpy(h[c].tm, cs.back()->tmaps_b, sizeof h[c].tm);

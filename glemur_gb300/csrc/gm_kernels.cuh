@@ -82,7 +82,7 @@ struct KP {
     double cmc[6];           // c - c* in double (error norm of errMode 1)
     T cmcT[6];               // c - c* in the run precision
     T cb[6], cbz[6];         // c - b5 (cbz: along z, -b5 without zUpdate): x_new from x_5
-    T vol8;                  // 8 dx dy dz: 1/det(a, b, c) -> 1/Delta
+    T vol8, inv8;            // 8 dx dy dz: 1/det(a, b, c) -> 1/Delta; its reciprocal: det -> Delta
     T w4[3], w4i[3];         // scale of B0s (4 dy dz, 4 dx dz, 4 dx dy) and its reciprocal
     double ar, az, phi1;     // analytic-field parameters (distance-to-analytic diagnostic)
     int shear;               // initShearA or initShearB != 0: addDist on the line-tied z ghost planes
@@ -119,6 +119,8 @@ struct StageArgs {
     T* KU[5];                // inertia: velocity increments k_u,0..k_u,4
     const T* B0;
     const T* B0s;            // B0 scaled by (4 dy dz, 4 dx dz, 4 dx dy), padded layout
+    T* BF;                   // field kernels: B, padded layout
+    T* RF;                   // field kernels: 1/det(a, b, c) (or Delta), padded scalar
     DevState* st;
     double* log;             // per attempt: maxDelta, dt after the update, accepted
     int n;                   // stage index 0..5
@@ -134,10 +136,19 @@ struct StageArgs {
 };
 
 // Host-side launchers (explicitly instantiated for float and double).
+// field kernels (gm_fields.cuh)
 template <typename T>
-cudaError_t launch_j_oct(const StageArgs<T>& a, cudaStream_t s);
+cudaError_t launch_b_field(const StageArgs<T>& a, int out, int always, cudaStream_t s);
 template <typename T>
-cudaError_t launch_j_quint(const StageArgs<T>& a, cudaStream_t s);
+cudaError_t launch_diag_field(const StageArgs<T>& a, int jout, cudaStream_t s);
+constexpr int kMaxDiagBlocks = 152 * 8;
+template <typename T>
+int diag_blocks(long long N);
+template <typename T>
+cudaError_t launch_stage_field(const StageArgs<T>& a, int pressure, int jout, cudaStream_t s);
+// the octilateral, quintilateral or triangular current (p.jOct, p.jQuint, p.jTri)
+template <typename T>
+cudaError_t launch_j_own(const StageArgs<T>& a, int always, cudaStream_t s);
 template <typename T>
 cudaError_t launch_stage(const StageArgs<T>& a, int mode, int pressure, dim3 grid, dim3 block, size_t smem,
                          cudaStream_t s);

@@ -884,34 +884,22 @@ __global__ void k_control_batch(const StageArgsTMA<T>* __restrict__ cases, int n
     if (c < ncases) control_one<T>(cases[c].a.p, cases[c].a.st, cases[c].a.log);
 }
 
-// Fixed-order reduction of the CTA partials.
+// Fixed-order reduction of the CTA partials, one warp per quantity; clears the
+// place of epsilon*.
 template <typename T>
-__global__ void k_finalize(const double* __restrict__ part, int nparts, double* out) {
-    __shared__ double red[R_COUNT][256];
-    const int tid = threadIdx.x;
-    for (int r = 0; r < R_COUNT; r++) {
-        double acc = r <= R_LAST_SUM ? 0.0 : (r <= R_LAST_MAX ? 0.0 : DBL_MAX);
-        if (r == R_MIN_CONVEX) acc = 1.0;
-        for (int q = tid; q < nparts; q += blockDim.x) {
-            const double v = part[(long long)q * R_COUNT + r];
-            if (r <= R_LAST_SUM) acc += v;
-            else if (r <= R_LAST_MAX) acc = fmax(acc, v);
-            else acc = fmin(acc, v);
-        }
-        red[r][tid] = acc;
+__global__ void __launch_bounds__(32 * R_COUNT) k_finalize(const double* __restrict__ part, int nparts, double* out) {
+    const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double acc = r <= R_LAST_MAX ? 0.0 : r == R_MIN_CONVEX ? 1.0 : DBL_MAX;
+    for (int q = lane; q < nparts; q += 32) {
+        const double v = part[(long long)q * R_COUNT + r];
+        acc = r <= R_LAST_SUM ? acc + v : r <= R_LAST_MAX ? fmax(acc, v) : fmin(acc, v);
     }
-    __syncthreads();
-    if (tid < R_COUNT) {
-        const int r = tid;
-        double acc = red[r][0];
-        for (int q = 1; q < (int)blockDim.x; q++) {
-            const double v = red[r][q];
-            if (r <= R_LAST_SUM) acc += v;
-            else if (r <= R_LAST_MAX) acc = fmax(acc, v);
-            else acc = fmin(acc, v);
-        }
-        out[r] = acc;
+    for (int o = 16; o > 0; o >>= 1) {
+        const double v = __shfl_xor_sync(0xffffffffu, acc, o);
+        acc = r <= R_LAST_SUM ? acc + v : r <= R_LAST_MAX ? fmax(acc, v) : fmin(acc, v);
     }
+    if (lane == 0) out[r] = acc;
+    if (threadIdx.x == 0) out[R_COUNT] = 0.0;
 }
 
 template <typename T>
@@ -1028,262 +1016,6 @@ __global__ void k_pack_k(const KP<T> p, const T* __restrict__ k, T* __restrict__
     }
 }
 
-// Octilateral Stokes current (JStokes4th, src/current.cu:413-736) at every
-// inner point, from the positions (padded SoA) and the ghosted B of the
-// reference layout (as the J pass exports it, ghost edges included).  For
-// each plane through the point, axes (u, v) = (x, y), (y, z), (z, x): the
-// circulation of B around the eight neighbours (-1,-1) (0,-1) (1,-1) (1,0)
-// (1,1) (0,1) (-1,1) (-1,0) and the area vector (1/2) of the corner cross
-// products plus (1/4) of the inner diamond's; then the 3x3 solve.
-template <typename T>
-__global__ void k_j_oct(const __grid_constant__ StageArgs<T> a) {
-    const KP<T>& p = a.p;
-    // the stage's input grid (the step start for stage 0, chosen on the device)
-    const T* __restrict__ X = a.n == 0 ? a.X[a.st->cur] : a.XS[(a.n - 1) & 1];
-    const T* __restrict__ B = a.outB;
-    T* __restrict__ J = a.outJ;
-    const int ax[3][2] = {{0, 1}, {1, 2}, {2, 0}};
-    const int ring[9][2] = {{0, 0}, {1, 0}, {2, 0}, {2, 1}, {2, 2}, {1, 2}, {0, 2}, {0, 1}, {0, 0}};
-    const int dia[5][2] = {{0, 1}, {1, 0}, {2, 1}, {1, 2}, {0, 1}};
-    const long long nx2 = p.nx + 2, ny2 = p.ny + 2;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < p.N; q += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(q % p.nx), j = (int)((q / p.nx) % p.ny), k = (int)(q / ((long long)p.nx * p.ny));
-        auto xat = [&](const int o[3], int l) { return X[l * p.cs + gidx(p.px, p.py, i + o[0], j + o[1], k + o[2])]; };
-        auto bat = [&](const int o[3], int l) {
-            return B[3 * ((i + 1 + o[0]) + nx2 * ((j + 1 + o[1]) + ny2 * (long long)(k + 1 + o[2]))) + l];
-        };
-        T NA[3][3], II[3];
-#pragma unroll
-        for (int pl = 0; pl < 3; pl++) {
-            T xr[9][3], br[9][3], dx[8][3], dd[4][3], c[4][3];
-#pragma unroll
-            for (int e = 0; e < 8; e++) {
-                int o[3] = {0, 0, 0};
-                o[ax[pl][0]] = ring[e][0] - 1;
-                o[ax[pl][1]] = ring[e][1] - 1;
-#pragma unroll
-                for (int l = 0; l < 3; l++) { xr[e][l] = xat(o, l); br[e][l] = bat(o, l); }
-            }
-#pragma unroll
-            for (int l = 0; l < 3; l++) { xr[8][l] = xr[0][l]; br[8][l] = br[0][l]; }
-            T I = 0;
-#pragma unroll
-            for (int l = 0; l < 3; l++) {
-#pragma unroll
-                for (int e = 0; e < 8; e++) dx[e][l] = xr[e + 1][l] - xr[e][l];
-                I += (br[1][l] + br[0][l]) / 2 * dx[0][l] + (br[2][l] + br[1][l]) / 2 * dx[1][l] +
-                     (br[3][l] + br[2][l]) / 2 * dx[2][l] + (br[4][l] + br[3][l]) / 2 * dx[3][l] +
-                     (br[5][l] + br[4][l]) / 2 * dx[4][l] + (br[6][l] + br[5][l]) / 2 * dx[5][l] +
-                     (br[7][l] + br[6][l]) / 2 * dx[6][l] + (br[8][l] + br[7][l]) / 2 * dx[7][l];
-            }
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                int o0[3] = {0, 0, 0}, o1[3] = {0, 0, 0};
-                o0[ax[pl][0]] = dia[e][0] - 1; o0[ax[pl][1]] = dia[e][1] - 1;
-                o1[ax[pl][0]] = dia[e + 1][0] - 1; o1[ax[pl][1]] = dia[e + 1][1] - 1;
-#pragma unroll
-                for (int l = 0; l < 3; l++) dd[e][l] = xat(o1, l) - xat(o0, l);
-            }
-            II[pl] = I;
-            cross3(dx[1], dx[2], c[0]);
-            cross3(dx[3], dx[4], c[1]);
-            cross3(dx[5], dx[6], c[2]);
-            cross3(dx[7], dx[0], c[3]);
-#pragma unroll
-            for (int l = 0; l < 3; l++) NA[pl][l] = (c[0][l] + c[1][l] + c[2][l] + c[3][l]) / 2;
-            cross3(dd[0], dd[1], c[0]);
-            cross3(dd[1], dd[2], c[1]);
-            cross3(dd[2], dd[3], c[2]);
-            cross3(dd[3], dd[0], c[3]);
-#pragma unroll
-            for (int l = 0; l < 3; l++) NA[pl][l] += (c[0][l] + c[1][l] + c[2][l] + c[3][l]) / 4;
-        }
-        const T det = NA[0][0] * NA[1][1] * NA[2][2] + NA[0][1] * NA[1][2] * NA[2][0] + NA[0][2] * NA[1][0] * NA[2][1] -
-                      NA[0][0] * NA[1][2] * NA[2][1] - NA[0][1] * NA[1][0] * NA[2][2] - NA[0][2] * NA[1][1] * NA[2][0];
-        T N1[3][3];
-        N1[0][0] = (NA[1][1] * NA[2][2] - NA[1][2] * NA[2][1]) / det;
-        N1[0][1] = (NA[0][2] * NA[2][1] - NA[0][1] * NA[2][2]) / det;
-        N1[0][2] = (NA[0][1] * NA[1][2] - NA[0][2] * NA[1][1]) / det;
-        N1[1][0] = (NA[1][2] * NA[2][0] - NA[1][0] * NA[2][2]) / det;
-        N1[1][1] = (NA[0][0] * NA[2][2] - NA[0][2] * NA[2][0]) / det;
-        N1[1][2] = (NA[0][2] * NA[1][0] - NA[0][0] * NA[1][2]) / det;
-        N1[2][0] = (NA[1][0] * NA[2][1] - NA[1][1] * NA[2][0]) / det;
-        N1[2][1] = (NA[0][1] * NA[2][0] - NA[0][0] * NA[2][1]) / det;
-        N1[2][2] = (NA[0][0] * NA[1][1] - NA[0][1] * NA[1][0]) / det;
-#pragma unroll
-        for (int l = 0; l < 3; l++) {
-            T Jl = 0;
-#pragma unroll
-            for (int m = 0; m < 3; m++) Jl += N1[l][m] * II[m];
-            J[3 * q + l] = Jl;
-        }
-    }
-}
-
-// Quintilateral Stokes current (JStokesQuint, src/current.cu:737-1199) at
-// every inner point, from the positions and the exported ghosted B, as
-// k_j_oct.  Per plane, axes (u, v, w) = (x, y, z), (y, z, x), (z, x, y) and
-// P(a, b) the neighbour at in-plane offsets (a - 1, b - 1): the diamond through
-// the face neighbours, with a corner triangle's two outer edges in place of one
-// diamond edge where the orientation tests pick one.  The tests are the
-// reference's as written: each later test reads the edge vectors the previous
-// one stored, the third compares with 4 instead of 0, the first triangle's
-// edges take the B averages of the other edge, and in the (y, z, x) and
-// (z, x, y) planes the fourth triangle's second edge runs from P(1, 2), not
-// P(0, 2), to P(0, 1) (src/current.cu:995-996, 1104-1105).
-// With p.jTri, the triangular Stokes current (JStokesTri, src/current.cu:
-// 1202-1681): the same tests, but a plane where they pick a triangle takes that
-// triangle alone (its two outer edges and the reversed diamond edge) as the
-// contour and half the outer edges' cross product as the area vector.  The
-// reference adds that to an area vector it never set (src/current.cu:1420-
-// 1424), and its compiled kernel returns NaN in J wherever a plane takes a
-// triangle; the unset start is NaN here too, so the stage's NaN check stops
-// the step there.
-template <typename T>
-__device__ __forceinline__ T quiet_nan() {
-    if constexpr (sizeof(T) == 8) return __longlong_as_double(0x7ff8000000000000ll);
-    else return __int_as_float(0x7fc00000);
-}
-
-template <typename T>
-__global__ void k_j_quint(const __grid_constant__ StageArgs<T> a) {
-    const KP<T>& p = a.p;
-    const T* __restrict__ X = a.n == 0 ? a.X[a.st->cur] : a.XS[(a.n - 1) & 1];
-    const T* __restrict__ Bg = a.outB;
-    T* __restrict__ J = a.outJ;
-    const int ax[3][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}};
-    const long long nx2 = p.nx + 2, ny2 = p.ny + 2;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < p.N; q += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(q % p.nx), j = (int)((q / p.nx) % p.ny), k = (int)(q / ((long long)p.nx * p.ny));
-        T NA[3][3], II[3];
-#pragma unroll
-        for (int pl = 0; pl < 3; pl++) {
-            T x[3][3][3], b[3][3][3], xwp[3], xwm[3];
-#pragma unroll
-            for (int aa = 0; aa < 3; aa++)
-#pragma unroll
-                for (int bb = 0; bb < 3; bb++) {
-                    int o[3] = {0, 0, 0};
-                    o[ax[pl][0]] = aa - 1; o[ax[pl][1]] = bb - 1;
-                    const long long g = gidx(p.px, p.py, i + o[0], j + o[1], k + o[2]);
-                    const long long gb = (i + 1 + o[0]) + nx2 * ((j + 1 + o[1]) + ny2 * (long long)(k + 1 + o[2]));
-#pragma unroll
-                    for (int l = 0; l < 3; l++) { x[aa][bb][l] = X[l * p.cs + g]; b[aa][bb][l] = Bg[3 * gb + l]; }
-                }
-            {
-                int o[3] = {0, 0, 0};
-                o[ax[pl][2]] = 1;
-                const long long gp = gidx(p.px, p.py, i + o[0], j + o[1], k + o[2]);
-                const long long gm = gidx(p.px, p.py, i - o[0], j - o[1], k - o[2]);
-#pragma unroll
-                for (int l = 0; l < 3; l++) { xwp[l] = X[l * p.cs + gp]; xwm[l] = X[l * p.cs + gm]; }
-            }
-            T dx1[3], dx2[3], dx3[3], dx4[3], dx5[3], dx6[3], c[3];
-            int tri = 0;
-#pragma unroll
-            for (int l = 0; l < 3; l++) {
-                dx1[l] = x[1][0][l] - x[1][1][l];
-                dx2[l] = x[2][1][l] - x[1][1][l];
-                dx3[l] = x[1][2][l] - x[1][1][l];
-                dx4[l] = x[0][1][l] - x[1][1][l];
-                dx5[l] = xwp[l] - x[1][1][l];
-                dx6[l] = xwm[l] - x[1][1][l];
-            }
-            auto dot = [](const T* u, const T* v) { return u[0] * v[0] + u[1] * v[1] + u[2] * v[2]; };
-            cross3(dx1, dx2, c);
-            if (dot(c, dx5) < 0 || dot(c, dx6) > 0) {
-#pragma unroll
-                for (int l = 0; l < 3; l++) { dx5[l] = x[2][0][l] - x[1][0][l]; dx6[l] = x[2][1][l] - x[2][0][l]; }
-                tri = 2;
-            }
-            if (tri != 0) {
-                cross3(dx2, dx3, c);
-                if (dot(c, dx5) < 0 || dot(c, dx6) > 0) {
-#pragma unroll
-                    for (int l = 0; l < 3; l++) { dx5[l] = x[2][2][l] - x[2][1][l]; dx6[l] = x[1][2][l] - x[2][2][l]; }
-                    tri = 3;
-                }
-            }
-            if (tri != 0) {
-                cross3(dx3, dx4, c);
-                if (dot(c, dx5) < 0 || dot(c, dx6) > 4) {
-#pragma unroll
-                    for (int l = 0; l < 3; l++) { dx5[l] = x[0][2][l] - x[1][2][l]; dx6[l] = x[0][1][l] - (pl == 0 ? x[0][2][l] : x[1][2][l]); }
-                    tri = 4;
-                }
-            }
-            cross3(dx4, dx1, c);
-            if (tri != 0) {
-                if (dot(c, dx5) < 0 || dot(c, dx6) > 0) {
-#pragma unroll
-                    for (int l = 0; l < 3; l++) { dx5[l] = x[1][0][l] - x[0][0][l]; dx6[l] = x[0][0][l] - x[0][1][l]; }
-                    tri = 1;
-                }
-            }
-            T I = 0;
-#pragma unroll
-            for (int l = 0; l < 3; l++) {
-                dx1[l] = x[1][0][l] - x[0][1][l];
-                dx2[l] = x[2][1][l] - x[1][0][l];
-                dx3[l] = x[1][2][l] - x[2][1][l];
-                dx4[l] = x[0][1][l] - x[1][2][l];
-                if (p.jTri && tri != 0) {
-                    // the triangle's closing edge: the diamond edge reversed
-                    if (tri == 1) I -= (b[1][0][l] + b[0][1][l]) / 2 * dx1[l];
-                    if (tri == 2) I -= (b[2][1][l] + b[1][0][l]) / 2 * dx2[l];
-                    if (tri == 3) I -= (b[1][2][l] + b[2][1][l]) / 2 * dx3[l];
-                    if (tri == 4) I -= (b[0][1][l] + b[1][2][l]) / 2 * dx4[l];
-                } else {
-                    if (tri != 1) I += (b[1][0][l] + b[0][1][l]) / 2 * dx1[l];
-                    if (tri != 2) I += (b[2][1][l] + b[1][0][l]) / 2 * dx2[l];
-                    if (tri != 3) I += (b[1][2][l] + b[2][1][l]) / 2 * dx3[l];
-                    if (tri != 4) I += (b[0][1][l] + b[1][2][l]) / 2 * dx4[l];
-                }
-                if (tri == 1) I += (b[0][1][l] + b[0][0][l]) / 2 * dx5[l] + (b[1][0][l] + b[0][0][l]) / 2 * dx6[l];
-                if (tri == 2) I += (b[1][0][l] + b[2][0][l]) / 2 * dx5[l] + (b[2][1][l] + b[2][0][l]) / 2 * dx6[l];
-                if (tri == 3) I += (b[2][1][l] + b[2][2][l]) / 2 * dx5[l] + (b[1][2][l] + b[2][2][l]) / 2 * dx6[l];
-                if (tri == 4) I += (b[1][2][l] + b[0][2][l]) / 2 * dx5[l] + (b[0][1][l] + b[0][2][l]) / 2 * dx6[l];
-            }
-            T c12[3], c23[3], c34[3], c41[3], c56[3] = {0, 0, 0};
-            cross3(dx1, dx2, c12);
-            cross3(dx2, dx3, c23);
-            cross3(dx3, dx4, c34);
-            cross3(dx4, dx1, c41);
-            if (tri > 0) cross3(dx5, dx6, c56);
-            II[pl] = I;
-#pragma unroll
-            for (int l = 0; l < 3; l++) {
-                if (p.jTri && tri > 0) {
-                    NA[pl][l] = quiet_nan<T>() + c56[l] / 2;
-                } else {
-                    NA[pl][l] = (c12[l] + c23[l] + c34[l] + c41[l]) / 4;
-                    if (tri > 0) NA[pl][l] += c56[l] / 2;
-                }
-            }
-        }
-        const T det = NA[0][0] * NA[1][1] * NA[2][2] + NA[0][1] * NA[1][2] * NA[2][0] + NA[0][2] * NA[1][0] * NA[2][1] -
-                      NA[0][0] * NA[1][2] * NA[2][1] - NA[0][1] * NA[1][0] * NA[2][2] - NA[0][2] * NA[1][1] * NA[2][0];
-        const T det1 = (T)1 / det;
-        T N1[3][3];
-        N1[0][0] = (NA[1][1] * NA[2][2] - NA[1][2] * NA[2][1]) * det1;
-        N1[0][1] = (NA[0][2] * NA[2][1] - NA[0][1] * NA[2][2]) * det1;
-        N1[0][2] = (NA[0][1] * NA[1][2] - NA[0][2] * NA[1][1]) * det1;
-        N1[1][0] = (NA[1][2] * NA[2][0] - NA[1][0] * NA[2][2]) * det1;
-        N1[1][1] = (NA[0][0] * NA[2][2] - NA[0][2] * NA[2][0]) * det1;
-        N1[1][2] = (NA[0][2] * NA[1][0] - NA[0][0] * NA[1][2]) * det1;
-        N1[2][0] = (NA[1][0] * NA[2][1] - NA[1][1] * NA[2][0]) * det1;
-        N1[2][1] = (NA[0][1] * NA[2][0] - NA[0][0] * NA[2][1]) * det1;
-        N1[2][2] = (NA[0][0] * NA[1][1] - NA[0][1] * NA[1][0]) * det1;
-#pragma unroll
-        for (int l = 0; l < 3; l++) {
-            T Jl = 0;
-#pragma unroll
-            for (int m = 0; m < 3; m++) Jl += N1[l][m] * II[m];
-            J[3 * q + l] = Jl;
-        }
-    }
-}
-
 // Two k-layout arrays (x and velocity increments) into the reference's
 // six-value kk record per inner point.
 template <typename T>
@@ -1387,38 +1119,41 @@ __global__ void k_grid_fields(const KP<T> p, const T* __restrict__ X, T* __restr
 // eps* (maths.cu:203-290 with diagnostics.cu:32-47): along the central column
 // i = nx/2, j = ny/2, a_k = J.B/B^2 and z_k = x_z; eps* is the largest
 // sqrt(2) |(a_n - a_p)/(z_n - z_p)| over the pairs with z_n != z_p, in REAL;
-// NaN values never win (maths.cu:144-153).  One CTA.
+// NaN values never win (maths.cu:144-153).  The column first, then the pairs
+// over many CTAs (in one they took 79 us of a 128x128x256 refresh, waiting for
+// their divisions); the factor is applied to the largest quotient, which
+// rounding leaves the largest.  *out is zero on entry (k_finalize).
 template <typename T>
-__global__ void k_eps_star(const KP<T> p, const T* __restrict__ B, const T* __restrict__ J, const T* __restrict__ X,
-                           T* __restrict__ sc, double* __restrict__ out) {
+__global__ void k_eps_column(const KP<T> p, const T* __restrict__ B, const T* __restrict__ J, const T* __restrict__ X,
+                             T* __restrict__ sc) {
     const int i = p.nx / 2, j = p.ny / 2, nz = p.nz;
-    T* a = sc;
-    T* z = sc + nz;
-    for (int k = threadIdx.x; k < nz; k += blockDim.x) {
-        const long long g = (long long)(i + 1) + (long long)(p.nx + 2) * ((j + 1) + (long long)(p.ny + 2) * (k + 1));
-        const long long l = (long long)i + (long long)p.nx * (j + (long long)p.ny * k);
-        const T b0 = B[3 * g], b1 = B[3 * g + 1], b2 = B[3 * g + 2];
-        const T j0 = J[3 * l], j1 = J[3 * l + 1], j2 = J[3 * l + 2];
-        a[k] = (j0 * b0 + j1 * b1 + j2 * b2) / (b0 * b0 + b1 * b1 + b2 * b2);
-        z[k] = X[2 * p.cs + (i + 2) + (long long)p.px * ((j + 2) + (long long)p.py * (k + 2))];
-    }
-    __syncthreads();
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nz) return;
+    const long long g = (long long)(i + 1) + (long long)(p.nx + 2) * ((j + 1) + (long long)(p.ny + 2) * (k + 1));
+    const long long l = (long long)i + (long long)p.nx * (j + (long long)p.ny * k);
+    const T b0 = B[3 * g], b1 = B[3 * g + 1], b2 = B[3 * g + 2];
+    const T j0 = J[3 * l], j1 = J[3 * l + 1], j2 = J[3 * l + 2];
+    sc[k] = (j0 * b0 + j1 * b1 + j2 * b2) / (b0 * b0 + b1 * b1 + b2 * b2);
+    sc[nz + k] = X[2 * p.cs + (i + 2) + (long long)p.px * ((j + 2) + (long long)p.py * (k + 2))];
+}
+template <typename T>
+__global__ void k_eps_star(const T* __restrict__ sc, int nz, double* __restrict__ out) {
+    const T* a = sc;
+    const T* z = sc + nz;
     T m = 0;    // every value is >= 0, and the pairs n == p give 0
-    for (int q = threadIdx.x; q < nz * nz; q += blockDim.x) {
-        const int pp = q / nz, n = q % nz;
-        if (z[n] != z[pp]) {
-            const T v = (T)(1.414213562373095 * (double)fabs((a[n] - a[pp]) / (z[n] - z[pp])));
-            if (v > m) m = v;
-        }
+    for (int pp = blockIdx.x; pp < nz; pp += gridDim.x)
+        for (int n = pp + 1 + threadIdx.x; n < nz; n += blockDim.x)
+            if (z[n] != z[pp]) {
+                const T v = fabs((a[n] - a[pp]) / (z[n] - z[pp]));
+                if (v > m) m = v;
+            }
+    for (int o = 16; o > 0; o >>= 1) {
+        const T v = __shfl_xor_sync(0xffffffffu, m, o);
+        if (v > m) m = v;
     }
-    __shared__ double red[256];
-    red[threadIdx.x] = (double)m;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + w]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *out = red[0];
+    if ((threadIdx.x & 31) == 0 && m > 0)
+        atomicMax(reinterpret_cast<unsigned long long*>(out),
+                  (unsigned long long)__double_as_longlong((double)(T)(1.414213562373095 * (double)m)));
 }
 
 // ---- host launchers ---------------------------------------------------------
@@ -1491,7 +1226,7 @@ cudaError_t launch_control_batch(const StageArgsTMA<T>* cases, int ncases, int* 
 
 template <typename T>
 cudaError_t launch_finalize(const double* part, int nparts, double* out, cudaStream_t s) {
-    k_finalize<T><<<1, 256, 0, s>>>(part, nparts, out);
+    k_finalize<T><<<1, 32 * R_COUNT, 0, s>>>(part, nparts, out);
     return cudaGetLastError();
 }
 
@@ -1537,18 +1272,6 @@ cudaError_t launch_pack_k(const KP<T>& p, const T* k, T* aos, cudaStream_t s) {
 }
 
 template <typename T>
-cudaError_t launch_j_oct(const StageArgs<T>& a, cudaStream_t s) {
-    k_j_oct<T><<<nblk(a.p.N), 128, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t launch_j_quint(const StageArgs<T>& a, cudaStream_t s) {
-    k_j_quint<T><<<nblk(a.p.N), 128, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
-template <typename T>
 cudaError_t launch_pack_k6(const KP<T>& p, const T* kx, const T* ku, T* aos, cudaStream_t s) {
     k_pack_k6<T><<<nblk(p.N), 256, 0, s>>>(p, kx, ku, aos);
     return cudaGetLastError();
@@ -1578,7 +1301,8 @@ cudaError_t launch_grid_fields(const KP<T>& p, const T* X, T* cellVol, T* convex
 template <typename T>
 cudaError_t launch_eps_star(const KP<T>& p, const T* B, const T* J, const T* X, T* scratch, double* out,
                             cudaStream_t s) {
-    k_eps_star<T><<<1, 256, 0, s>>>(p, B, J, X, scratch, out);
+    k_eps_column<T><<<(p.nz + 127) / 128, 128, 0, s>>>(p, B, J, X, scratch);
+    k_eps_star<T><<<p.nz < 304 ? p.nz : 304, 128, 0, s>>>(scratch, p.nz, out);
     return cudaGetLastError();
 }
 
@@ -1597,8 +1321,6 @@ cudaError_t launch_eps_star(const KP<T>& p, const T* B, const T* J, const T* X, 
     template cudaError_t launch_shear_table<T>(const KP<T>&, const T*, T*, cudaStream_t);                         \
     template cudaError_t launch_pack_k<T>(const KP<T>&, const T*, T*, cudaStream_t);                              \
     template cudaError_t launch_pack_k6<T>(const KP<T>&, const T*, const T*, T*, cudaStream_t);                  \
-    template cudaError_t launch_j_oct<T>(const StageArgs<T>&, cudaStream_t);                                    \
-    template cudaError_t launch_j_quint<T>(const StageArgs<T>&, cudaStream_t);                                  \
     template cudaError_t launch_unpack_k<T>(const KP<T>&, const T*, T*, cudaStream_t);                          \
     template cudaError_t launch_export_ghosts<T>(const KP<T>&, T*, T*, cudaStream_t);                            \
     template cudaError_t launch_grid_fields<T>(const KP<T>&, const T*, T*, T*, T*, cudaStream_t);                 \

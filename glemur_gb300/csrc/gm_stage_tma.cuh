@@ -30,7 +30,7 @@
 #include <type_traits>
 
 #include "gm_kernels_impl.cuh"
-#include "gm_vec2.cuh"
+#include "gm_point.cuh"
 
 namespace gmk {
 
@@ -94,92 +94,6 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, u
         : "memory");
 }
 
-// Reciprocal for the stage kernel, by Newton's iteration r <- r + r (1 - x r)
-// from the hardware's approximation: one step in FP32 (within ~1 ulp; FP32
-// parity is judged at 1e-5), two in FP64 (the approximation has about 20 bits;
-// the last step's residual is exact to an FMA, so the result is the rounded
-// reciprocal but for rare ties).
-__device__ __forceinline__ float rcp_approx(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ double rcp_approx(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    return r;
-}
-__device__ __forceinline__ F2 rcp_approx(F2 x) { return mk2(rcp_approx(lo(x)), rcp_approx(hi(x))); }
-__device__ __forceinline__ D2 rcp_approx(D2 x) { return mk2(rcp_approx(lo(x)), rcp_approx(hi(x))); }
-template <typename T, typename V>
-__device__ __forceinline__ V rcp_stage(V x) {
-    V r = rcp_approx(x);
-    const V one = splat<V>((T)1), nx = vneg(x);
-#pragma unroll
-    for (int it = 0; it < (sizeof(T) == 4 ? 1 : 2); it++) r = vfma(vfma(nx, r, one), r, r);
-    return r;
-}
-
-// FP32: the determinant d of the columns of A, recomputed in double from the
-// same entries when the cell is strongly sheared: |d| small against the bound
-// |a|_1 |b|_1 |c|_1 of the six Sarrus products.
-__device__ __forceinline__ float det_sheared(float d, float a0, float a1, float a2, float b0, float b1, float b2,
-                                             float c0, float c1, float c2) {
-    const float m = (fabsf(a0) + fabsf(a1) + fabsf(a2)) * (fabsf(b0) + fabsf(b1) + fabsf(b2)) *
-                    (fabsf(c0) + fabsf(c1) + fabsf(c2));
-    if (!(fabsf(d) < 0.03125f * m)) return d;
-    const double jd[3][3] = {{a0, b0, c0}, {a1, b1, c1}, {a2, b2, c2}};
-    return (float)det3<double>(jd);
-}
-// The cheap test in front of it: |v|_1 <= sqrt(3) |v|_2, so a cell with
-// d^2 > (0.03125 sqrt(27))^2 |a|^2 |b|^2 |c|^2 cannot be one; everything else
-// (an underflow or a NaN of the squares too) takes the test above.
-constexpr float kShear2 = 0.0266f;
-template <typename V>
-__device__ __forceinline__ V norm2(const V A[3][3], int c) {
-    return vfma(A[2][c], A[2][c], vfma(A[1][c], A[1][c], vmul(A[0][c], A[0][c])));
-}
-// (out of line: the double determinant would double the plane loop's code)
-static __device__ __noinline__ F2 det_sheared2(F2 d, F2 a0, F2 a1, F2 a2, F2 b0, F2 b1, F2 b2, F2 c0, F2 c1, F2 c2) {
-    const float x = det_sheared(lo(d), lo(a0), lo(a1), lo(a2), lo(b0), lo(b1), lo(b2), lo(c0), lo(c1), lo(c2));
-    const float y = det_sheared(hi(d), hi(a0), hi(a1), hi(a2), hi(b0), hi(b1), hi(b2), hi(c0), hi(c1), hi(c2));
-    return mk2(x, y);
-}
-__device__ __forceinline__ float det_guard(float d, const float A[3][3], bool act) {
-    const float t = vmul(vmul(norm2(A, 0), norm2(A, 1)), vmul(norm2(A, 2), kShear2));
-    if (!(vmul(d, d) > t) && act)
-        d = det_sheared(d, A[0][0], A[1][0], A[2][0], A[0][1], A[1][1], A[2][1], A[0][2], A[1][2], A[2][2]);
-    return d;
-}
-__device__ __forceinline__ F2 det_guard(F2 d, const F2 A[3][3], bool act) {
-    const F2 t = vmul(vmul(norm2(A, 0), norm2(A, 1)), vmul(norm2(A, 2), splat<F2>(kShear2))), q = vmul(d, d);
-    if (!(lo(q) > lo(t) && hi(q) > hi(t)) && act)
-        d = det_sheared2(d, A[0][0], A[1][0], A[2][0], A[0][1], A[1][1], A[2][1], A[0][2], A[1][2], A[2][2]);
-    return d;
-}
-__device__ __forceinline__ double det_guard(double d, const double[3][3], bool) { return d; }
-__device__ __forceinline__ D2 det_guard(D2 d, const D2[3][3], bool) { return d; }
-
-// B = (s_x a + s_y b + s_z c) / det(a, b, c) with the unscaled central
-// differences a = x(+x) - x(-x), b, c (the columns of A) and the pre-scaled
-// field s = (4 dy dz B0x, 4 dx dz B0y, 4 dx dy B0z): since jac = [a/2dx, b/2dy,
-// c/2dz], this is jac.B0 / det(jac) of B_JacB0 (rungeKutta.cu:79-99) with the
-// constant factors folded.  *r = 1/det(a, b, c) (Delta = 1 / (8 dx dy dz r)).
-// Without `act` the result is not used (and B may come out inexact).
-template <typename T, typename V>
-__device__ __forceinline__ void b_from(const V A[3][3], const V s[3], V B[3], V* r, bool act) {
-    const V b[3] = {A[0][1], A[1][1], A[2][1]}, c[3] = {A[0][2], A[1][2], A[2][2]};
-    V n[3];
-    vcross(b, c, n);
-    V d = vfma(A[0][0], n[0], vfma(A[1][0], n[1], vmul(A[2][0], n[2])));
-    if (sizeof(T) == 4) d = det_guard(d, A, act);
-    const V q = rcp_stage<T>(d);
-    const V s0 = vmul(s[0], q), s1 = vmul(s[1], q), s2 = vmul(s[2], q);
-#pragma unroll
-    for (int l = 0; l < 3; l++) B[l] = vfma(A[l][0], s0, vfma(A[l][1], s1, vmul(A[l][2], s2)));
-    *r = q;
-}
-
 // The columns of A at a pair / a point whose shared-memory addresses in the
 // planes k-1, k, k+1 are xm, x0, xp; C is the component stride in bytes.
 template <typename T, int C>
@@ -206,72 +120,23 @@ __device__ __forceinline__ void diffs1(uint32_t xm, uint32_t x0, uint32_t xp, T 
     }
 }
 
-template <typename T>
-struct Vec3 { T x, y, z; };
-
-// B on the ghost plane of a line-tied face with normal axis AX, at the point
-// (i, j, k) with addresses xm, x0, xp in the planes k-1, k, k+1 and b0 in the
-// B0s plane: updateBbound, src/boundaries.cu:39-446.  The ghost plane continues
-// by one spacing outwards, and in-plane neighbours at the edges of the
-// reference's 16-wide launch blocks are the own position shifted by the spacing
-// (boundaries.cu:72-109, 212-237, 340-365); the differences come out in the
-// scaling of b_from, and B.n = B0.n is s.n over its scale w (one corrected
-// step, so the quotient is B0.n but for rare last bits).  Everything is read
-// from the shared-memory planes: the form that read B0 from global memory
-// stalled every plane of a line-tied run (110 us a stage on 97x75x133, 35 %
-// issue).
+// Positions around a point by its shared-memory addresses in the planes k-1, k,
+// k+1 and in the B0s plane.  The face formula reads nothing else: the form that
+// read B0 from global memory stalled every plane of a line-tied run (110 us a
+// stage on 97x75x133, 35 % issue).
+template <typename T, int C>
+struct SharedX {
+    uint32_t xm, x0, xp, b0;
+    __device__ __forceinline__ T operator()(int l, int di, int dj, int dk) const {
+        return Sh<T>::ld((dk < 0 ? xm : dk > 0 ? xp : x0) + (uint32_t)(l * C + (dj * HX2 + di) * (int)sizeof(T)));
+    }
+    __device__ __forceinline__ T s(int l) const { return Sh<T>::ld(b0 + l * C); }
+};
 template <int AX, int C, typename T>
 __device__ __forceinline__ Vec3<T> b_face_s(const KP<T>& p, uint32_t xm, uint32_t x0, uint32_t xp, uint32_t b0, int i,
                                             int j, int k) {
-    constexpr int E = sizeof(T), R = HX2 * E;
-    const int idx[3] = {i, j, k};
-    const int n3[3] = {p.nx, p.ny, p.nz};
-    const T d3[3] = {p.dx, p.dy, p.dz};
-    const bool side = idx[AX] >= 0;
-    T A[3][3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        if (a == AX) {
-            const uint32_t xi = AX == 2 ? (side ? xm : xp) : x0 + (side ? -1 : 1) * (AX == 0 ? E : R);
-#pragma unroll
-            for (int l = 0; l < 3; l++) {
-                T xo = Sh<T>::ld(x0 + l * C);
-                if (l == AX) xo = side ? vadd(xo, d3[AX]) : vsub(xo, d3[AX]);
-                if (AX == 2 && l < 2 && p.shear)
-                    xo = p.shearTab[10 * ((long long)side * p.nx * p.ny + (long long)j * p.nx + i) + l];
-                const T xn = Sh<T>::ld(xi + l * C);
-                A[l][a] = side ? vsub(xo, xn) : vsub(xn, xo);
-            }
-        } else {
-            const int u = idx[a];
-            const bool eL = u % 16 == 0, eR = u % 16 == 15 || u == n3[a] - 1;
-            const uint32_t xl = eL ? x0 : (a == 2 ? xm : x0 - (a == 1 ? R : E));
-            const uint32_t xr = eR ? x0 : (a == 2 ? xp : x0 + (a == 1 ? R : E));
-#pragma unroll
-            for (int l = 0; l < 3; l++) {
-                T vl = Sh<T>::ld(xl + l * C);
-                T vr = Sh<T>::ld(xr + l * C);
-                if (l == a) {
-                    if (eL) vl = vsub(vl, d3[a]);
-                    if (eR) vr = vadd(vr, d3[a]);
-                }
-                if (AX == 2 && l < 2 && p.shear) {
-                    // an initially distorted grid: the neighbours extrapolated at the
-                    // block edges carry the distortion (k_shear_table)
-                    const T* tb = p.shearTab + 10 * ((long long)side * p.nx * p.ny + (long long)j * p.nx + i);
-                    if (eL) vl = tb[2 + 4 * a + l];
-                    if (eR) vr = tb[4 + 4 * a + l];
-                }
-                A[l][a] = vsub(vr, vl);
-            }
-        }
-    }
-    const T s[3] = {Sh<T>::ld(b0), Sh<T>::ld(b0 + C), Sh<T>::ld(b0 + 2 * C)};
-    T r, B[3];
-    b_from<T, T>(A, s, B, &r, true);
-    const T q = vmul(s[AX], p.w4i[AX]);
-    B[AX] = vfma(vfma(-q, p.w4[AX], s[AX]), p.w4i[AX], q);
-    return Vec3<T>{B[0], B[1], B[2]};
+    T r, d;
+    return b_face_v<AX>(p, SharedX<T, C>{xm, x0, xp, b0}, i, j, k, &r, &d);
 }
 // the line-tied z ghost planes, two of a run (out of line, as det_sheared2)
 template <int C, typename T>
@@ -342,53 +207,6 @@ struct StageCtl {
     int work;                    // batched launch: the current work item
 };
 
-// Offsets (elements) from a stored position to its periodic images along x and
-// y, 0 where there is none: ghost layers 1 and 2 hold the images of the two
-// inner layers of the opposite face, shifted by -/+ (L + d) as setGridPeriFace
-// writes them (boundaries.cu:546-549, 561-564, 576-579).
-__device__ __forceinline__ int image_step(int peri, int i, int n) { return !peri ? 0 : i < 2 ? n : i >= n - 2 ? -n : 0; }
-
-template <typename T, typename V>
-__device__ __forceinline__ V image_shift(V v, int step, T L, T d) {
-    return step > 0 ? vadd(vadd(v, splat<V>(L)), splat<V>(d)) : vsub(vsub(v, splat<V>(L)), splat<V>(d));
-}
-
-template <typename T, typename V>
-__device__ __forceinline__ void st_xyz(T* q, long long cs, V a, V b, V c) {
-    stv(q, a);
-    stv(q + cs, b);
-    stv(q + 2 * cs, c);
-}
-
-// The periodic images, beyond those along x alone, of the position v stored at
-// q (ix, iy, iz: image_step).
-template <typename T, typename V>
-__device__ __forceinline__ void store_images_yz(const KP<T>& p, T* q, const V v[3], int ix, int iy, int iz) {
-    const long long cs = p.cs, oy = (long long)iy * p.px;
-    const V vx = image_shift<T>(v[0], ix, p.Lx, p.dx), vy = image_shift<T>(v[1], iy, p.Ly, p.dy);
-    if (iy) st_xyz(q + oy, cs, v[0], vy, v[2]);
-    if (ix && iy) st_xyz(q + ix + oy, cs, vx, vy, v[2]);
-    if (iz) {
-        T* qz = q + (long long)iz * p.px * p.py;
-        const V vz = image_shift<T>(v[2], iz, p.Lz, p.dz);
-        st_xyz(qz, cs, v[0], v[1], vz);
-        if (ix) st_xyz(qz + ix, cs, vx, v[1], vz);
-        if (iy) st_xyz(qz + oy, cs, v[0], vy, vz);
-        if (ix && iy) st_xyz(qz + ix + oy, cs, vx, vy, vz);
-    }
-}
-template <typename T, typename V>
-__device__ __noinline__ void store_images_call(const KP<T>& p, T* q, V a, V b, V c, int ix, int iy, int iz) {
-    const V v[3] = {a, b, c};
-    store_images_yz<T, V>(p, q, v, ix, iy, iz);
-}
-// Every image of one point, in any grid: a direction of three points, whose
-// middle point has two images, takes the loop over all shifts (store_pos).
-template <typename T>
-__device__ __noinline__ void store_point_images(const KP<T>& p, T* X, int i, int j, int k, T a, T b, T c) {
-    const T v[3] = {a, b, c};
-    store_pos<T>(p, X, i, j, k, v);
-}
 // The start grid's own images, refreshed by stage 5 of the first attempted step
 // (a retry reads them; until then they are those the caller supplied).
 template <typename T>
@@ -468,18 +286,6 @@ __device__ __forceinline__ void grad_p2(const KP<T>& p, uint32_t xm, uint32_t x0
         t = vfma(pe[1], Ai[0][l], vfma(pe[2], Ai[1][l], t));
         g[l] = vmul(t, det1);
     }
-}
-
-__device__ __forceinline__ bool finite_bits(float x) { return (__float_as_uint(x) & 0x7f800000u) != 0x7f800000u; }
-__device__ __forceinline__ bool finite_bits(double x) { return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u; }
-
-// Running maximum of non-negative values; NaN never wins (maths.cu:144-153).
-// In FP64 on the bits (non-negative doubles order as integers): a comparison
-// of doubles would cost a slot of the FP64 pipe.
-__device__ __forceinline__ void max_nn(float& m, float x) { m = fmaxf(m, fabsf(x)); }
-__device__ __forceinline__ void max_nn(double& m, double x) {
-    const long long b = __double_as_longlong(x) & 0x7fffffffffffffffll;
-    if (b > __double_as_longlong(m) && b <= 0x7ff0000000000000ll) m = __longlong_as_double(b);
 }
 
 // One RK stage over the 32 x 2 NW x TZ block (bx, by, bz) of one case.
@@ -700,19 +506,11 @@ __device__ __forceinline__ bool stage_tile(const StageArgsTMA<T>& A, int bx, int
         const bool first = LAST && st->nAttempted == 0;
         V pe[3];
         if (PRESS) {
-            // p0 and its derivatives along x, y (times 2 dx, 2 dy) at the pair
-            T e[3][2];
+            T e[2][3];
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const T X = p.dx * (T)(ic + h) + p.Ox, Y = p.dy * (T)jc + p.Oy;
-                const T ex = p.p0Amp != (T)0 ? p.p0Amp * exp(-(X * X + Y * Y) * p.inv_p0W2) : (T)0;
-                const T be2 = -2 * p.beta * ex * p.inv_p0W2;
-                e[0][h] = p.beta * ((T)1 + ex);
-                e[1][h] = be2 * X * (2 * p.dx);
-                e[2][h] = be2 * Y * (2 * p.dy);
-            }
+            for (int h = 0; h < 2; h++) p0_at(p, ic + h, jc, e[h]);
 #pragma unroll
-            for (int q = 0; q < 3; q++) pe[q] = mk2(e[q][0], e[q][1]);
+            for (int q = 0; q < 3; q++) pe[q] = mk2(e[0][q], e[1][q]);
         }
         // addresses of the pair in the position planes kk - 3 .. kk and in the B
         // planes kb - 2 .. kb, stepped with kk

@@ -1,0 +1,196 @@
+"""The stage and field kernels at the edges of their tiles and dispatch: the
+tall and the low tile, the two elementwise passes and the general tile kernel
+compute the same points, so they are compared with each other over sizes,
+boundaries and options, and the diagnostics with numpy in 64 bits."""
+import numpy as np
+import pytest
+
+import cases  # noqa: F401  (tests/golden on the path)
+import make_folded
+from conftest import ROOT, inner, relerr
+from glemur_gb300 import BatchRelaxation, Relaxation, _abi, configs
+
+pytestmark = pytest.mark.gpu
+
+# partial and whole tiles of 32 x 12 and 32 x 4 columns, odd sizes (the last
+# pair of a row is half a pair), three points in a direction, one plane a tile
+SHAPES = [(3, 3, 3), (4, 5, 6), (33, 13, 9), (32, 12, 24), (31, 11, 7), (34, 25, 40), (65, 4, 5), (7, 66, 10)]
+PERI = [(1, 1, 0), (0, 0, 0), (1, 0, 1), (0, 1, 0)]
+
+
+def case(shape, peri, precision, pressure=False, inertia=False, method="Stokes", seed=0, amplitude=0.1):
+    """A braid on a randomly moved grid (periodic ghosts as images)."""
+    p = configs.random_braid(11 + seed, shape=shape, precision=precision)
+    p.xPeri, p.yPeri, p.zPeri = peri
+    if pressure:
+        p.pressure, p.beta, p.p0Amp, p.p0Width = 1, p.rnd(0.1), p.rnd(0.5), p.rnd(2.0)
+    p.inertia = int(inertia)
+    p.set_str("jMethod", method)
+    p = configs.derive(p)
+    B0, xb = configs.init_state(p)
+    sp = np.array([p.dx, p.dy, p.dz])
+    rng = np.random.default_rng(seed)
+    x = xb.astype(np.float64)
+    x[1:-1, 1:-1, 1:-1] += rng.uniform(-amplitude, amplitude, size=x[1:-1, 1:-1, 1:-1].shape) * sp
+    L = (p.Lx + p.dx, p.Ly + p.dy, p.Lz + p.dz)
+    for axis, on in ((2, peri[0]), (1, peri[1]), (0, peri[2])):
+        if on:
+            lo = np.take(x, -2, axis).copy()
+            lo[..., 2 - axis] -= L[2 - axis]
+            hi = np.take(x, 1, axis).copy()
+            hi[..., 2 - axis] += L[2 - axis]
+            ix = [slice(None)] * 4
+            ix[axis] = 0
+            x[tuple(ix)] = lo
+            ix[axis] = -1
+            x[tuple(ix)] = hi
+    return p, x.astype(p.real_dtype()), B0
+
+
+def stages(p, x, B0, kernel):
+    q = p.copy()
+    q.stageKernel = kernel
+    g = Relaxation(q)
+    g.upload(x, B0, 0.0, 1e-3)
+    if p.inertia:
+        g.upload_u(0.01 * np.random.default_rng(5).normal(size=g.I + (3,)))
+    out = {}
+    for n in range(6):
+        g.stage(n)
+        if n < 5:
+            out[f"k{n}"] = g.k(n)
+            out[f"x{n}"] = g.x(n)
+    out["xnew"] = g.x(6)
+    if p.inertia:
+        out["unew"] = g.u(6)
+    g.control()
+    s = g.state()
+    g.close()
+    return out, s
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("peri", PERI)
+@pytest.mark.parametrize("shape", SHAPES)
+def test_stage_matches_the_general_kernel(shape, peri, precision):
+    """Every stage's increments and grids, ghosts included: FP64 to rounding,
+    FP32 within the 1e-5 per stage of the parity tests."""
+    a, sa = stages(*case(shape, peri, precision), 0)
+    b, sb = stages(*case(shape, peri, precision), 1)
+    tol = 1e-12 if precision == 64 else 1e-5
+    for name in a:
+        assert relerr(a[name], b[name]) < tol, name
+    assert sa["status"] == sb["status"] and sa["timeIndex"] == sb["timeIndex"]
+
+
+@pytest.mark.parametrize("precision,form", [(p, f) for p in (32, 64) for f in
+                                            ("pressure", "inertia", "inertia_pressure", "Stokes4th", "StokesQuint")])
+@pytest.mark.parametrize("shape,peri", [((33, 13, 9), (1, 1, 0)), ((20, 24, 17), (0, 0, 0)), ((3, 40, 12), (0, 1, 1))])
+def test_options_match_the_general_kernel(shape, peri, precision, form):
+    """As above with the pressure gradient (second differences of the positions:
+    1e-3 in FP32, as in the large case's parity test), the velocity equation and
+    the currents with a kernel of their own."""
+    kw = dict(pressure="pressure" in form, inertia="inertia" in form, method=form if form.startswith("Stokes") else "Stokes")
+    a, _ = stages(*case(shape, peri, precision, **kw), 0)
+    b, _ = stages(*case(shape, peri, precision, **kw), 1)
+    tol = 1e-12 if precision == 64 else (1e-3 if kw["pressure"] else 1e-5)
+    if precision == 64 and kw["pressure"]:
+        tol = 1e-10            # the same noise at FP64 rounding
+    for name in a:
+        assert relerr(a[name], b[name]) < tol, name
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+def test_batched_and_single_runs_agree_bit_for_bit_on_odd_sizes(precision):
+    """The batch's tall tile against the single case's low tile (FP32) and
+    elementwise passes (FP64)."""
+    cs = [case(s, p, precision, seed=i) for i, (s, p) in enumerate([((33, 13, 9), (1, 1, 0)), ((34, 25, 40), (0, 0, 0)),
+                                                                   ((5, 66, 10), (0, 1, 1)), ((64, 24, 12), (1, 1, 0))])]
+    b = BatchRelaxation([p for p, _, _ in cs])
+    for i, (p, x, B0) in enumerate(cs):
+        b.upload(i, x, B0, 0.0, 1e-3)
+    b.steps_async(4)
+    for i, (p, x, B0) in enumerate(cs):
+        g = Relaxation(p)
+        g.upload(x, B0, 0.0, 1e-3)
+        g.steps_async(4)
+        assert g.state() == b.state(i)
+        assert np.array_equal(g.grid(), b.download(i)["xb"])
+        g.close()
+    b.close()
+
+
+def test_sheared_cells_keep_their_precision_in_fp32():
+    """Random displacements of 0.45 spacings: many determinants cancel and are
+    recomputed in double.  Against the FP64 increments of the same grid the
+    pair kernel is no further off than the general one (up to rounding)."""
+    p, x, B0 = case((40, 30, 21), (1, 1, 0), 32, amplitude=0.45)
+    q = p.copy()
+    q.precision, q.errMode = 64, 1
+    ref, _ = stages(q, x.astype(np.float64), B0.astype(np.float64), 1)
+    new, _ = stages(p, x, B0, 0)
+    old, _ = stages(p, x, B0, 1)
+    err = lambda a: float(np.median(np.abs(a["k0"] - ref["k0"]) / (np.abs(ref["k0"]) + 1e-12)))  # noqa: E731
+    assert err(new) <= 1.5 * err(old) + 1e-7
+    norm = lambda a: float(np.linalg.norm((a["k0"] - ref["k0"]).ravel()) / np.linalg.norm(ref["k0"].ravel()))  # noqa: E731
+    assert norm(new) <= 1.5 * norm(old) + 1e-6
+
+
+@pytest.mark.parametrize("method", make_folded.METHODS)
+def test_currents_on_the_folded_grid_match_the_fixture(method):
+    """J of every current on the folded grid against the values stored from the
+    reference's kernels (corner triangles, NaN points included)."""
+    z = np.load(ROOT / "tests" / "golden" / "folded_currents.npz")
+    p, _, _ = make_folded.folded_case(method)
+    g = Relaxation(p)
+    g.upload(z["x"], z["B0"])
+    g.refresh()
+    f = g.download()
+    Jr = z[f"J_{method}"]
+    assert np.array_equal(np.isnan(f["J"]), np.isnan(Jr))
+    assert relerr(np.nan_to_num(f["J"]), np.nan_to_num(Jr)) < 1e-10
+    assert relerr(inner(f["B"]), z["B"]) < 1e-12
+    g.close()
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("shape,peri,scale", [((33, 20, 17), (1, 1, 0), 1.0), ((12, 12, 12), (0, 0, 0), 1.0),
+                                              ((24, 16, 20), (1, 1, 1), 1e-13), ((24, 16, 20), (1, 1, 0), 0.0)])
+def test_reductions_match_numpy_in_64_bits(shape, peri, scale, precision):
+    """The sums and maxima of gm_refresh against numpy on the downloaded B, J and
+    Delta; with scaled blobs J is far below the range of the FP32 pairs, or
+    zero.  Sums of up to 11,000 non-negative terms: 1e-12."""
+    p, x, B0 = case(shape, peri, precision)
+    B0[..., :2] *= scale
+    if scale < 1:                     # no grid noise: J comes from B0 alone
+        _, x = configs.init_state(p)
+    g = Relaxation(p)
+    g.upload(x, B0)
+    r = g.refresh()
+    f = g.download()
+    B, J, D = inner(f["B"]).astype(np.float64), f["J"].astype(np.float64), f["detJac"].astype(np.float64)
+    jn, bn = np.linalg.norm(J, axis=-1), np.linalg.norm(B, axis=-1)
+    cn = np.linalg.norm(np.cross(J, B), axis=-1)
+    w = np.ones(D[1:-1, 1:-1, 1:-1].shape)
+    for a in range(3):
+        for e in (0, -1):
+            ix = [slice(None)] * 3
+            ix[a] = e
+            w[tuple(ix)] *= 0.5
+    both = jn * bn
+    pw = np.divide(cn, both, out=np.zeros_like(cn), where=both > 0)
+    b2 = (inner(f["B"]) ** 2).sum(-1, dtype=p.real_dtype()).astype(np.float64)
+    want = dict(BMax=bn.max(), JMax=jn.max(), residual=cn.sum() / both.sum() if both.sum() > 0 else 0.0, residualPw=pw.mean(),
+                errB_1ez=np.sqrt(((B - [0, 0, 1]) ** 2).sum(-1).mean()))
+    for k, v in want.items():
+        assert abs(r[k] - v) <= 1e-12 * max(abs(v), 1e-300) + 1e-30, (k, r[k], v)
+    assert abs(r["B2"] / ((b2 * inner(D) * w).sum() * p.dx * p.dy * p.dz) - 1) < (1e-12 if precision == 64 else 1e-6)
+    faces = [D[1:-1, 1:-1, 1:-1]]
+    for a, on in ((2, peri[0]), (1, peri[1]), (0, peri[2])):
+        if not on:
+            ix = [slice(1, -1)] * 3
+            for e in (0, -1):
+                ix[a] = e
+                faces.append(D[tuple(ix)])
+    assert r["minDetJac"] == min(v.min() for v in faces)
+    g.close()
