@@ -88,6 +88,7 @@ struct ConvArgs {
     int Kc, Np;                              // padded input channels (multiple of 16), padded outputs
     int Nt;                                  // output channels per CTA (multiple of 16; blockIdx.y picks the slice)
     int Kch;                                 // input channels per pipeline step (multiple of 16)
+    int vec;                                 // out and mask rows start on 16 bytes: 8 channels an access
     int* status;
     int stall;                               // failure-detection test: wait on an mbarrier nothing arrives on
 };
@@ -112,6 +113,39 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Sixteen accumulators of voxel v, output channels c .. c + 15: bias, ReLU,
+// mask, BF16; 8 channels a store (and mask load) where the views allow it.
+__device__ __forceinline__ void conv_store16(const ConvArgs& a, long long v, int c, const float acc[16]) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int c8 = c + 8 * h;
+        if (c8 >= a.co) break;
+        if (a.vec && c8 + 8 <= a.co) {
+            uint4 m = make_uint4(0, 0, 0, 0);
+            if (a.mask) m = *reinterpret_cast<const uint4*>(a.mask + v * a.ldm + c8);
+            const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(&m);
+            __nv_bfloat16 o[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                float y = acc[8 * h + q] + (a.bias ? __ldg(a.bias + c8 + q) : 0.f);
+                if (a.relu) y = fmaxf(y, 0.f);
+                if (a.mask && !(__bfloat162float(mb[q]) > 0.f)) y = 0.f;
+                o[q] = __float2bfloat16_rn(y);
+            }
+            *reinterpret_cast<uint4*>(a.out + v * a.ldo + c8) = *reinterpret_cast<const uint4*>(o);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                if (c8 + q >= a.co) break;
+                float y = acc[8 * h + q] + (a.bias ? a.bias[c8 + q] : 0.f);
+                if (a.relu) y = fmaxf(y, 0.f);
+                if (a.mask && !(__bfloat162float(a.mask[v * a.ldm + c8 + q]) > 0.f)) y = 0.f;
+                a.out[v * a.ldo + c8 + q] = __float2bfloat16_rn(y);
+            }
+        }
+    }
+}
 
 // One CTA: 128 consecutive voxels x one slice of Nt output channels
 // (blockIdx.y; all Np when they fit), accumulated over the 27 taps.  The
@@ -246,18 +280,7 @@ __global__ void __launch_bounds__(128) k_conv(const ConvArgs a) {
         for (int c0 = 0; c0 < Np; c0 += 16) {
             float acc[16];
             tmem_ld16(tbase + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, acc);
-            if (valid) {
-                const long long vv = v;
-#pragma unroll
-                for (int q = 0; q < 16; q++) {
-                    const int c = n0 + c0 + q;
-                    if (c >= a.co) break;
-                    float y = acc[q] + (a.bias ? a.bias[c] : 0.f);
-                    if (a.relu) y = fmaxf(y, 0.f);
-                    if (a.mask && !(__bfloat162float(a.mask[vv * a.ldm + c]) > 0.f)) y = 0.f;
-                    a.out[vv * a.ldo + c] = __float2bfloat16_rn(y);
-                }
-            }
+            if (valid) conv_store16(a, v, n0 + c0, acc);
         }
     } else if (tid == 0) {
         atomicExch(a.status, 1);
@@ -265,6 +288,161 @@ __global__ void __launch_bounds__(128) k_conv(const ConvArgs a) {
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_free(tbase, ncols);
+}
+
+// ---- convolution on resident input tiles ---------------------------------------
+
+// The same convolution with the input tile copied once: a CTA takes 8 x 16
+// voxels of kz output planes, copies the kz + 2 input planes of its tile with
+// their halo (10 x 18 voxels) into shared memory, and all 27 taps read them
+// there.  In the K-major no-swizzle layout a row of a core matrix is the 16
+// bytes of 8 channels of one voxel; with the planes stored as [8-channel
+// group][y][x][16 bytes], 8 rows along x are 128 contiguous bytes, 8-row groups
+// (the next y) are one halo row apart (the descriptor's stride-dimension offset,
+// 160 bytes) and the two core matrices of a K = 16 step one group apart (its
+// leading-dimension offset), so a tap is nothing but another start address.
+// k_conv above copies a tap's 128 x K operand for every tap, 27 times the tile,
+// and spent its time issuing those copies (24 -> 24 channels at 64x64x128: 375
+// us, 3 % tensor activity).  The weights of a tap are streamed through kConvStages
+// stages and used for kz planes.  Each accumulator takes taps and channels in
+// k_conv's order, so the results are the same to the bit.
+constexpr int kTileX = 8, kTileY = 16, kHaloX = kTileX + 2, kSlots = kHaloX * (kTileY + 2);
+constexpr int kGroupBytes = kSlots * 16;       // one plane of 8 channels
+
+struct ConvTileArgs {
+    ConvArgs a;
+    int kz;                                    // output planes per CTA
+    int tx, ty;                                // tiles along x, y
+    int cstride;                               // accumulator columns per plane
+    int ncols;                                 // tensor-memory columns (a power of two)
+};
+
+__global__ void __launch_bounds__(128) k_conv_tile(const ConvTileArgs b) {
+    extern __shared__ __align__(128) unsigned char sm[];
+    constexpr int S = kConvStages;
+    const ConvArgs& a = b.a;
+    const int Kc = a.Kc, nkg = Kc >> 3, kz = b.kz;
+    const int n0 = blockIdx.y * a.Nt, Np = min(a.Nt, a.Np - n0);
+    const int planeBytes = nkg * kGroupBytes, bBytes = a.Nt * Kc * 2;
+    unsigned char* stA = sm;                              // kz + 2 planes
+    unsigned char* stB = sm + (kz + 2) * planeBytes;      // S stages of weights
+    uint64_t* bars = reinterpret_cast<uint64_t*>(stB + S * bBytes);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + S + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int x0 = (blockIdx.x % b.tx) * kTileX, y0 = (blockIdx.x / b.tx % b.ty) * kTileY;
+    const int z0 = blockIdx.x / (b.tx * b.ty) * kz;
+    if (tid == 0)
+        for (int q = 0; q <= S; q++) mbar_init_tc(&bars[q]);
+    if (warp == 0) tmem_alloc(tslot, b.ncols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tbase = *tslot;
+    const uint32_t id = idesc_bf16(128, Np);
+
+    auto issue_b = [&](int t) {
+        const __nv_bfloat16* Wt = a.W + ((size_t)t * a.Np + n0) * Kc;
+        unsigned char* d = stB + (t % S) * bBytes;
+        for (int e = tid; e < Np * nkg; e += 128) {
+            const int r = e / nkg, g = e - r * nkg;
+            cp_async16(d + (g * a.Nt + r) * 16, Wt + (size_t)r * Kc + g * 8, true);
+        }
+    };
+
+    uint32_t ph[S];
+    bool pend[S];                    // a commit on bars[s] not yet waited for
+    for (int q = 0; q < S; q++) { ph[q] = 0; pend[q] = false; }
+    // failure-detection test: a bounded wait that runs out before any MMA
+    bool ok = a.stall ? mbar_wait_tc(&bars[S], 0, 1u << 10) : true;
+    if (__syncthreads_and(ok)) {
+        // the input planes, zero where the padding is
+        for (int s = tid; s < kSlots; s += 128) {
+            const int sy = s / kHaloX, sx = s - sy * kHaloX;
+            int i = x0 + sx - 1, j = y0 + sy - 1;
+            // wrapped halo points of the domain; points beyond it (partial tiles) are zero
+            const bool in = (i >= 0 || a.xper) && (j >= 0 || a.yper) && (i < a.nx || (a.xper && i == a.nx)) &&
+                            (j < a.ny || (a.yper && j == a.ny));
+            i = wrap(i, a.nx);
+            j = wrap(j, a.ny);
+            for (int pz = 0; pz < kz + 2; pz++) {
+                const int k = z0 + pz - 1;
+                const bool ok8 = in && k >= 0 && k < a.nz;
+                const __nv_bfloat16* src = a.in1 + (ok8 ? ((long long)i + (long long)a.nx * (j + (long long)a.ny * k)) * a.ld1 : 0);
+                unsigned char* d = stA + pz * planeBytes + s * 16;
+                for (int g = 0; g < nkg; g++) {
+                    const bool on = ok8 && 8 * g < a.c1;
+                    cp_async16(d + g * kGroupBytes, on ? src + 8 * g : a.in1, on);
+                }
+            }
+        }
+        for (int q = 0; q < S - 1; q++) {
+            issue_b(q);
+            cp_async_commit();
+        }
+        for (int t = 0; t < 27; t++) {
+            // refill the stage of tap t + S - 1: the MMAs of tap t - 1 read it
+            const int tn = t + S - 1;
+            if (tn < 27) {
+                const int sn = tn % S;
+                if (pend[sn]) {
+                    if (!mbar_wait_tc(&bars[sn], ph[sn])) ok = false;
+                    ph[sn] ^= 1;
+                    pend[sn] = false;
+                }
+            }
+            // after a wait ran out no thread copies into a stage and no MMA is issued
+            if (!__syncthreads_and(ok)) {
+                ok = false;
+                break;
+            }
+            if (tn < 27) issue_b(tn);
+            cp_async_commit();
+            cp_async_wait<S - 1>();                  // the planes and tap t's weights have landed
+            fence_async_smem();
+            tc_fence_before();
+            __syncthreads();
+            tc_fence_after();
+            const int s = t % S;
+            if (tid == 0) {
+                const int dk = t / 9, dj = t / 3 % 3, di = t % 3;
+                const uint32_t as = sm_addr(stA) + (dj * kHaloX + di) * 16, bs = sm_addr(stB + s * bBytes);
+                for (int z = 0; z < kz; z++)
+                    for (int kk = 0; kk < nkg / 2; kk++) {
+                        const uint64_t ad = smem_desc(as + (z + dk) * planeBytes + kk * 2 * kGroupBytes, kGroupBytes, kHaloX * 16);
+                        const uint64_t bd = smem_desc(bs + kk * 2 * a.Nt * 16, a.Nt * 16, 128);
+                        mma_bf16(tbase + z * b.cstride, ad, bd, id, t > 0 || kk > 0);
+                    }
+                mma_commit(&bars[s]);
+            }
+            pend[s] = true;
+        }
+    }
+    cp_async_wait_all();
+    for (int q = 0; q < S; q++)
+        if (pend[q]) {
+            if (!mbar_wait_tc(&bars[q], ph[q])) ok = false;
+            ph[q] ^= 1;
+        }
+    ok = __syncthreads_and(ok);
+    tc_fence_after();
+    if (ok) {
+        // row 32 warp + lane of the accumulator is the voxel (row % 8, row / 8)
+        const int i = x0 + (lane & 7), j = y0 + 4 * warp + (lane >> 3);
+        for (int z = 0; z < kz; z++) {
+            const bool valid = i < a.nx && j < a.ny && z0 + z < a.nz;
+            const long long v = (long long)i + (long long)a.nx * (j + (long long)a.ny * (z0 + z));
+            for (int c0 = 0; c0 < Np; c0 += 16) {
+                float acc[16];
+                tmem_ld16(tbase + ((uint32_t)(32 * warp) << 16) + (uint32_t)(z * b.cstride + c0), acc);
+                if (valid) conv_store16(a, v, n0 + c0, acc);
+            }
+        }
+    } else if (tid == 0) {
+        atomicExch(a.status, 1);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_free(tbase, b.ncols);
 }
 
 // ---- convolution: weight gradient --------------------------------------------
@@ -767,6 +945,43 @@ __global__ void k_wg_grid(const float* __restrict__ d, const T* __restrict__ xid
     }
 }
 
+// Shape of k_conv_tile's launch, false where the tile does not fit (more than 96
+// input channels: the operands of a tap and chunk are streamed by k_conv).  kz
+// and the output slice: the most planes of the widest slice that still leave
+// about three CTAs for two SMs; two CTAs per SM (their copies and epilogues
+// overlap) if they fit, else one.
+static bool choose_conv_tile(const ConvArgs& a, ConvTileArgs* b, size_t* smem) {
+    if (a.Kc > 96) return false;
+    int dev = 0, nsm = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    b->a = a;
+    b->tx = (a.nx + kTileX - 1) / kTileX;
+    b->ty = (a.ny + kTileY - 1) / kTileY;
+    const long long cols = (long long)b->tx * b->ty;
+    for (int two = 1; two >= 0; two--)
+        for (int split = 1; split <= 4; split++) {
+            const int Nt = ((a.Np + split - 1) / split + 15) / 16 * 16;
+            for (int kz : {4, 2, 1}) {
+                const int cs = (Nt + 31) / 32 * 32;
+                int nc = 32;
+                while (nc < cs * kz) nc <<= 1;
+                const size_t sm = (size_t)(kz + 2) * (a.Kc / 8) * kGroupBytes + (size_t)kConvStages * Nt * a.Kc * 2 + 64;
+                if (nc > (two ? 256 : 512) || sm > (size_t)(two ? 112 : 226) * 1024) continue;
+                const long long ctas = cols * ((a.nz + kz - 1) / kz) * ((a.Np + Nt - 1) / Nt);
+                if (kz > 1 && ctas < 3ll * nsm / 2) continue;
+                if (split > 1 && kz == 1 && ctas > 4ll * nsm && !two) continue;
+                b->a.Nt = Nt;
+                b->kz = kz;
+                b->cstride = cs;
+                b->ncols = nc;
+                *smem = sm;
+                return true;
+            }
+        }
+    return false;
+}
+
 static unsigned nb(long long n) {
     long long b = (n + 255) / 256;
     return (unsigned)(b < 1 ? 1 : (b > 152 * 16 ? 152 * 16 : b));
@@ -836,6 +1051,18 @@ int gm_nn_conv(const void* in1, int ld1, int c1, const void* in2, int ld2, int c
     a.mask = (const __nv_bfloat16*)mask; a.ldm = ldm; a.relu = relu;
     a.nx = nx; a.ny = ny; a.nz = nz; a.xper = xper; a.yper = yper; a.Kc = Kc; a.Np = Np; a.Nt = Nt; a.Kch = Kch; a.status = status;
     a.stall = g_nn_stall;
+    auto aligned = [](const void* q, int ld) { return q == nullptr || (!(reinterpret_cast<uintptr_t>(q) & 15) && ld % 8 == 0); };
+    a.vec = aligned(out, ldo) && aligned(mask, ldm);
+    gmnn::ConvTileArgs b;
+    size_t tile_smem;
+    if (!in2 && gmnn::choose_conv_tile(a, &b, &tile_smem)) {
+        cudaError_t e = cudaFuncSetAttribute(gmnn::k_conv_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (e != cudaSuccess) return gm::fail(GM_ECUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+        const dim3 grid((unsigned)(b.tx * b.ty * ((nz + b.kz - 1) / b.kz)), (unsigned)((Np + b.a.Nt - 1) / b.a.Nt));
+        gmnn::k_conv_tile<<<grid, 128, tile_smem, (cudaStream_t)stream>>>(b);
+        e = cudaGetLastError();
+        return e == cudaSuccess ? GM_OK : gm::fail(GM_ECUDA, std::string("k_conv_tile: ") + cudaGetErrorString(e));
+    }
     const size_t smem = conv_smem(Nt);
     cudaError_t e = cudaFuncSetAttribute(gmnn::k_conv, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return gm::fail(GM_ECUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));

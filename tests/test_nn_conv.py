@@ -1,0 +1,84 @@
+"""The convolution kernels over the edges of their tiles: partial 8 x 16 tiles,
+grids below a tile, every padding, input channels beyond the view, output
+channels that are no multiple of 8 or 16 and more than one slice, narrow and
+wide inputs.  The reference is the same sum in FP64 on the BF16 operands."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+# nx, ny, nz, xper, yper, c1 (view), Kc, co, Np, relu, mask
+CASES = [
+    (8, 16, 4, 1, 1, 16, 16, 16, 16, 1, 0),       # one tile
+    (4, 4, 2, 1, 1, 8, 16, 3, 16, 0, 0),          # below a tile, head
+    (5, 3, 1, 0, 1, 24, 32, 24, 32, 1, 1),        # one plane, ragged
+    (9, 17, 7, 1, 0, 24, 32, 20, 32, 0, 0),       # one point over a tile
+    (23, 37, 11, 0, 0, 72, 80, 24, 32, 1, 0),     # wide input, bounded
+    (16, 33, 5, 1, 1, 48, 48, 192, 192, 1, 1),    # several slices
+    (24, 16, 19, 1, 1, 32, 32, 72, 80, 0, 1),     # 80 columns
+    (10, 18, 6, 1, 1, 96, 96, 96, 96, 1, 0),
+    (17, 9, 5, 0, 1, 192, 192, 192, 192, 1, 1),   # wide on both sides
+    (9, 20, 6, 1, 0, 240, 240, 48, 48, 0, 0),
+    (8, 8, 4, 1, 1, 104, 112, 45, 48, 1, 0),
+    (12, 6, 3, 1, 1, 200, 256, 256, 256, 1, 0),   # the largest channel counts
+    (64, 48, 40, 1, 1, 24, 32, 24, 32, 1, 1),     # several items a CTA
+]
+
+
+def _reference(x, W, b, xper, yper):
+    """sum over taps in FP64; x [nx, ny, nz, c], W [27, co, c]"""
+    nx, ny, nz, c = x.shape
+    xp = np.zeros((nx + 2, ny + 2, nz + 2, c))
+    xp[1:-1, 1:-1, 1:-1] = x
+    if xper:
+        xp[0], xp[-1] = xp[-2], xp[1]
+    if yper:
+        xp[:, 0], xp[:, -1] = xp[:, -2], xp[:, 1]
+    y = np.zeros((nx, ny, nz, W.shape[1]))
+    s = np.zeros_like(y)
+    for t in range(27):
+        dk, dj, di = t // 9, t // 3 % 3, t % 3
+        v = xp[di:di + nx, dj:dj + ny, dk:dk + nz]
+        y += v @ W[t].T
+        s += np.abs(v) @ np.abs(W[t]).T
+    return y + b, s + np.abs(b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "x".join(map(str, c)))
+def test_conv(case):
+    import torch
+    from glemur_gb300 import _abi
+    nx, ny, nz, xper, yper, c1, Kc, co, Np, relu, mask = case
+    rng = np.random.default_rng(1)
+    bf = lambda a: torch.tensor(a, dtype=torch.float32, device="cuda").to(torch.bfloat16)  # noqa: E731
+    V = nx * ny * nz
+    x = bf(rng.normal(size=(V, c1)))
+    W = bf(np.pad(rng.normal(size=(27, co, c1)) / np.sqrt(27 * c1), ((0, 0), (0, Np - co), (0, Kc - c1))))
+    b = torch.tensor(np.pad(rng.normal(size=co), (0, Np - co)), dtype=torch.float32, device="cuda")
+    lo = (co + 7) // 8 * 8 + 8
+    y = torch.full((V, lo), 7.0, dtype=torch.bfloat16, device="cuda")
+    m = bf(rng.normal(size=(V, lo)))
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    torch.cuda.synchronize()
+    lib = _abi.load()
+    _abi.check(lib.gm_nn_conv(P(x), c1, c1, None, 0, 0, P(W), C.cast(b.data_ptr(), C.POINTER(C.c_float)), P(y), lo, co,
+                              P(m) if mask else None, lo if mask else 0, relu, nx, ny, nz, xper, yper, Kc, Np, P(st),
+                              None), "gm_nn_conv")
+    torch.cuda.synchronize()
+    assert int(st[0]) == 0
+    xs = x.double().cpu().numpy().reshape(nz, ny, nx, c1).transpose(2, 1, 0, 3)
+    ref, size = _reference(xs, W.double().cpu().numpy()[:, :co, :c1], b.double().cpu().numpy()[:co], xper, yper)
+    if relu:
+        ref = np.maximum(ref, 0)
+    if mask:
+        ms = m.double().cpu().numpy()[:, :co].reshape(nz, ny, nx, co).transpose(2, 1, 0, 3)
+        ref = np.where(ms > 0, ref, 0)
+    got = y.double().cpu().numpy()
+    g = got[:, :co].reshape(nz, ny, nx, co).transpose(2, 1, 0, 3)
+    # FP32 sums of 27 Kc products (each addition off by at most an ulp of the sum
+    # of magnitudes) and one rounding to BF16 (2^-9 relative)
+    tol = size * (27 * Kc * 2.0 ** -23) + np.abs(ref) * 2.0 ** -8
+    assert np.all(np.abs(g - ref) <= tol), np.max(np.abs(g - ref) / tol)
+    assert np.all(got[:, co:] == 7.0)          # nothing beyond the output's channels
