@@ -9,6 +9,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 
 #include "glemur.h"
@@ -108,6 +109,9 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool vali
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sm_addr(dst)), "l"(src),
                  "r"(valid ? 16 : 0)
                  : "memory");
+}
+__device__ __forceinline__ void cp_async16s(uint32_t dst, const void* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -290,158 +294,462 @@ __global__ void __launch_bounds__(128) k_conv(const ConvArgs a) {
     if (warp == 0) tmem_free(tbase, ncols);
 }
 
-// ---- convolution on resident input tiles ---------------------------------------
+// ---- convolution on resident input planes ---------------------------------------
 
-// The same convolution with the input tile copied once: a CTA takes 8 x 16
-// voxels of kz output planes, copies the kz + 2 input planes of its tile with
-// their halo (10 x 18 voxels) into shared memory, and all 27 taps read them
-// there.  In the K-major no-swizzle layout a row of a core matrix is the 16
-// bytes of 8 channels of one voxel; with the planes stored as [8-channel
-// group][y][x][16 bytes], 8 rows along x are 128 contiguous bytes, 8-row groups
-// (the next y) are one halo row apart (the descriptor's stride-dimension offset,
-// 160 bytes) and the two core matrices of a K = 16 step one group apart (its
-// leading-dimension offset), so a tap is nothing but another start address.
-// k_conv above copies a tap's 128 x K operand for every tap, 27 times the tile,
-// and spent its time issuing those copies (24 -> 24 channels at 64x64x128: 375
-// us, 3 % tensor activity).  The weights of a tap are streamed through kConvStages
-// stages and used for kz planes.  Each accumulator takes taps and channels in
-// k_conv's order, so the results are the same to the bit.
+// The same convolution with every input plane copied once, the weights resident
+// and each MMA used for three taps.  A CTA takes items of 8 x 16 voxels and kz
+// output planes and marches along z; an input plane of the tile with its halo
+// (10 x 18 voxels) is copied into shared memory and all taps read it there.  In
+// the K-major no-swizzle layout a row of a core matrix is the 16 bytes of 8
+// channels of one voxel; with a plane stored as [8-channel group][y][x][16
+// bytes], 8 rows along x are 128 contiguous bytes, 8-row groups (the next y) are
+// one halo row apart (the descriptor's stride-dimension offset, 160 bytes) and
+// the two core matrices of a K = 16 step one group apart (its leading-dimension
+// offset), so an in-plane tap is nothing but another start address.  The three
+// taps along z of an in-plane tap use the same 128 x 16 operand for the output
+// planes p - 2, p - 1 and p: their weights are stacked along N and the
+// accumulators of consecutive output planes lie in consecutive columns.  (An MMA
+// takes 46 clocks up to N = 48, 57 at N = 96, N / 2 from N = 128 on.)
+//
+// Warps 0-3 read finished accumulators and store, warps 4-7 copy planes, one
+// thread of warp 12 issues the MMAs; they meet in mbarriers only.  With the copies, MMAs and
+// stores of a step in one program order every step was a chain of about 9000
+// clocks around 2000 clocks of MMAs.
+//
+// The weights of the CTA's output channels (all 27 taps) are copied once.
 constexpr int kTileX = 8, kTileY = 16, kHaloX = kTileX + 2, kSlots = kHaloX * (kTileY + 2);
+constexpr int kMaxPlanes = 3, kMaxKz = 32;
+constexpr int kPlaneThreads = 416, kCopyThreads = 128;
+
+// Copies.  The layout scatters the 16-byte groups of a voxel or weight row over shared
+// memory.  Asynchronous copies (cp.async) do that at 16 bytes a clock and SM whatever
+// the order of lanes, but need few warps and no registers: the planes go that way, a
+// warp taking 16 slots x 2 groups (32 bytes of a voxel) an instruction.  Loads into
+// registers and stores are faster if many warps share the latency and neither side
+// has conflicts: the weights go that way, the groups of a row in gl neighbouring
+// lanes and the groups' stride in shared memory padded so that 8 such lanes write all
+// 32 banks.
 constexpr int kGroupBytes = kSlots * 16;       // one plane of 8 channels
 
-struct ConvTileArgs {
-    ConvArgs a;
-    int kz;                                    // output planes per CTA
-    int tx, ty;                                // tiles along x, y
-    int cstride;                               // accumulator columns per plane
-    int ncols;                                 // tensor-memory columns (a power of two)
+struct ConvLanes {
+    int ng, gl, sl;            // groups; lanes per row; rows per load of a warp
+    __host__ __device__ explicit ConvLanes(int channels)
+        : ng(channels >> 3), gl(ng >= 6 ? 8 : ng), sl(32 / gl) {}
+    __host__ __device__ int row_stride(int rows) const { return rows * 16 + 128 / gl; }      // of a group (rows a multiple of 8)
 };
 
-__global__ void __launch_bounds__(128) k_conv_tile(const ConvTileArgs b) {
-    extern __shared__ __align__(128) unsigned char sm[];
-    constexpr int S = kConvStages;
-    const ConvArgs& a = b.a;
-    const int Kc = a.Kc, nkg = Kc >> 3, kz = b.kz;
-    const int n0 = blockIdx.y * a.Nt, Np = min(a.Nt, a.Np - n0);
-    const int planeBytes = nkg * kGroupBytes, bBytes = a.Nt * Kc * 2;
-    unsigned char* stA = sm;                              // kz + 2 planes
-    unsigned char* stB = sm + (kz + 2) * planeBytes;      // S stages of weights
-    uint64_t* bars = reinterpret_cast<uint64_t*>(stB + S * bBytes);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + S + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int x0 = (blockIdx.x % b.tx) * kTileX, y0 = (blockIdx.x / b.tx % b.ty) * kTileY;
-    const int z0 = blockIdx.x / (b.tx * b.ty) * kz;
-    if (tid == 0)
-        for (int q = 0; q <= S; q++) mbar_init_tc(&bars[q]);
-    if (warp == 0) tmem_alloc(tslot, b.ncols);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tbase = *tslot;
-    const uint32_t id = idesc_bf16(128, Np);
+struct ConvPlace { int x0, y0, z0, kz; };
 
-    auto issue_b = [&](int t) {
-        const __nv_bfloat16* Wt = a.W + ((size_t)t * a.Np + n0) * Kc;
-        unsigned char* d = stB + (t % S) * bBytes;
-        for (int e = tid; e < Np * nkg; e += 128) {
-            const int r = e / nkg, g = e - r * nkg;
-            cp_async16(d + (g * a.Nt + r) * 16, Wt + (size_t)r * Kc + g * 8, true);
+__device__ __forceinline__ ConvPlace conv_place(int item, int tx, int ty, int kz, int nz) {
+    ConvPlace q;
+    q.x0 = item % tx * kTileX;
+    q.y0 = item / tx % ty * kTileY;
+    q.z0 = item / (tx * ty) * kz;
+    q.kz = min(kz, nz - q.z0);
+    return q;
+}
+
+// rows x L.ng groups of weights to shared memory at dst (group stride gs) by four
+// warps, eight 16-byte loads of a thread in flight; src(r) is row r, or null for
+// zeros.  The first loads go out before acquire() waits for the buffer; false when
+// its wait ran out.
+template <class Src, class Acquire>
+__device__ __forceinline__ bool conv_copy_rows(const ConvLanes& L, int rows, uint32_t dst, int gs, int wq, int lane,
+                                               Src src, Acquire acquire) {
+    const int g0 = lane & (L.gl - 1), dr = 4 * L.sl;
+    int r = wq * L.sl + lane / L.gl, g = g0;
+    bool first = true;
+    do {
+        uint4 v[8];
+        uint32_t d[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            v[q] = make_uint4(0, 0, 0, 0);
+            d[q] = 0;
+            if (r < rows) {
+                if (g < L.ng) {
+                    d[q] = dst + g * gs + r * 16;
+                    const __nv_bfloat16* p = src(r);
+                    if (p) v[q] = __ldg(reinterpret_cast<const uint4*>(p + 8 * g));
+                }
+                g += L.gl;
+                if (g - g0 >= L.ng) { g = g0; r += dr; }
+            }
         }
-    };
+        if (first) {
+            first = false;
+            if (!acquire()) return false;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+            if (d[q])
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(d[q]), "r"(v[q].x), "r"(v[q].y), "r"(v[q].z),
+                             "r"(v[q].w)
+                             : "memory");
+    } while (r < rows);
+    fence_async_smem();
+    return true;
+}
 
-    uint32_t ph[S];
-    bool pend[S];                    // a commit on bars[s] not yet waited for
-    for (int q = 0; q < S; q++) { ph[q] = 0; pend[q] = false; }
-    // failure-detection test: a bounded wait that runs out before any MMA
-    bool ok = a.stall ? mbar_wait_tc(&bars[S], 0, 1u << 10) : true;
-    if (__syncthreads_and(ok)) {
-        // the input planes, zero where the padding is
-        for (int s = tid; s < kSlots; s += 128) {
-            const int sy = s / kHaloX, sx = s - sy * kHaloX;
-            int i = x0 + sx - 1, j = y0 + sy - 1;
-            // wrapped halo points of the domain; points beyond it (partial tiles) are zero
-            const bool in = (i >= 0 || a.xper) && (j >= 0 || a.yper) && (i < a.nx || (a.xper && i == a.nx)) &&
+// The four warps that copy the planes of a CTA's items, in turn into NA buffers.  A
+// plane's full barrier is arrived on once its copies have landed, when the next plane
+// has been issued or before a wait (others may need the plane before that wait can
+// end).  False when a wait ran out.
+__device__ __forceinline__ bool conv_copy_planes(const ConvArgs& a, int tx, int ty, int items, int kz, int NA,
+                                                 uint32_t stA, uint64_t* full, uint64_t* empty, int wq, int lane) {
+    const int ng = a.Kc >> 3, gh = lane >> 4, planeBytes = ng * kGroupBytes;
+    uint64_t* pending = nullptr;
+    uint32_t n = 0;                                    // planes so far
+    int buf = 0;
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+        const ConvPlace w = conv_place(item, tx, ty, kz, a.nz);
+        // the voxels within a plane of this thread's slots 16 (wq + 4 q) + lane % 16:
+        // halo points wrap, -1 for what is zero (beyond the domain)
+        int vx[3];
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const int s = 16 * (wq + 4 * q) + (lane & 15), sy = s / kHaloX;
+            const int i = w.x0 + s - sy * kHaloX - 1, j = w.y0 + sy - 1;
+            const bool in = s < kSlots && (i >= 0 || a.xper) && (j >= 0 || a.yper) && (i < a.nx || (a.xper && i == a.nx)) &&
                             (j < a.ny || (a.yper && j == a.ny));
-            i = wrap(i, a.nx);
-            j = wrap(j, a.ny);
-            for (int pz = 0; pz < kz + 2; pz++) {
-                const int k = z0 + pz - 1;
-                const bool ok8 = in && k >= 0 && k < a.nz;
-                const __nv_bfloat16* src = a.in1 + (ok8 ? ((long long)i + (long long)a.nx * (j + (long long)a.ny * k)) * a.ld1 : 0);
-                unsigned char* d = stA + pz * planeBytes + s * 16;
-                for (int g = 0; g < nkg; g++) {
-                    const bool on = ok8 && 8 * g < a.c1;
-                    cp_async16(d + g * kGroupBytes, on ? src + 8 * g : a.in1, on);
+            vx[q] = in ? wrap(i, a.nx) + a.nx * wrap(j, a.ny) : -1;
+        }
+        for (int p = 0; p < w.kz + 2; p++, n++) {
+            if (n >= (uint32_t)NA && !mbar_test_tc(&empty[buf], n / NA - 1 & 1)) {
+                if (pending) {
+                    cp_async_wait<0>();
+                    fence_async_smem();
+                    mbar_arrive_tc(pending);
+                    pending = nullptr;
+                }
+                if (!mbar_wait_tc(&empty[buf], n / NA - 1 & 1)) return false;
+            }
+            const int k = w.z0 + p - 1;
+            const bool zin = k >= 0 && k < a.nz;
+            const __nv_bfloat16* src = a.in1 + (long long)a.nx * a.ny * (zin ? k : 0) * a.ld1 + 8 * gh;
+            const uint32_t dst = stA + buf * planeBytes + gh * kGroupBytes;
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const int s = 16 * (wq + 4 * q) + (lane & 15);
+                if (s >= kSlots) continue;
+                const bool in = zin && vx[q] >= 0;
+                const __nv_bfloat16* v = src + (long long)max(vx[q], 0) * a.ld1;
+                for (int g = 0; g < ng; g += 2) {
+                    const bool on = in && 8 * (g + gh) < a.c1;
+                    cp_async16s(dst + g * kGroupBytes + s * 16, on ? v + 8 * g : a.in1, on);
                 }
             }
-        }
-        for (int q = 0; q < S - 1; q++) {
-            issue_b(q);
             cp_async_commit();
-        }
-        for (int t = 0; t < 27; t++) {
-            // refill the stage of tap t + S - 1: the MMAs of tap t - 1 read it
-            const int tn = t + S - 1;
-            if (tn < 27) {
-                const int sn = tn % S;
-                if (pend[sn]) {
-                    if (!mbar_wait_tc(&bars[sn], ph[sn])) ok = false;
-                    ph[sn] ^= 1;
-                    pend[sn] = false;
-                }
+            if (pending) {
+                cp_async_wait<1>();
+                fence_async_smem();
+                mbar_arrive_tc(pending);
             }
-            // after a wait ran out no thread copies into a stage and no MMA is issued
-            if (!__syncthreads_and(ok)) {
-                ok = false;
-                break;
-            }
-            if (tn < 27) issue_b(tn);
-            cp_async_commit();
-            cp_async_wait<S - 1>();                  // the planes and tap t's weights have landed
-            fence_async_smem();
-            tc_fence_before();
-            __syncthreads();
-            tc_fence_after();
-            const int s = t % S;
-            if (tid == 0) {
-                const int dk = t / 9, dj = t / 3 % 3, di = t % 3;
-                const uint32_t as = sm_addr(stA) + (dj * kHaloX + di) * 16, bs = sm_addr(stB + s * bBytes);
-                for (int z = 0; z < kz; z++)
-                    for (int kk = 0; kk < nkg / 2; kk++) {
-                        const uint64_t ad = smem_desc(as + (z + dk) * planeBytes + kk * 2 * kGroupBytes, kGroupBytes, kHaloX * 16);
-                        const uint64_t bd = smem_desc(bs + kk * 2 * a.Nt * 16, a.Nt * 16, 128);
-                        mma_bf16(tbase + z * b.cstride, ad, bd, id, t > 0 || kk > 0);
-                    }
-                mma_commit(&bars[s]);
-            }
-            pend[s] = true;
+            pending = &full[buf];
+            buf = buf + 1 == NA ? 0 : buf + 1;
         }
     }
-    cp_async_wait_all();
-    for (int q = 0; q < S; q++)
-        if (pend[q]) {
-            if (!mbar_wait_tc(&bars[q], ph[q])) ok = false;
-            ph[q] ^= 1;
-        }
-    ok = __syncthreads_and(ok);
-    tc_fence_after();
-    if (ok) {
-        // row 32 warp + lane of the accumulator is the voxel (row % 8, row / 8)
-        const int i = x0 + (lane & 7), j = y0 + 4 * warp + (lane >> 3);
-        for (int z = 0; z < kz; z++) {
-            const bool valid = i < a.nx && j < a.ny && z0 + z < a.nz;
-            const long long v = (long long)i + (long long)a.nx * (j + (long long)a.ny * (z0 + z));
-            for (int c0 = 0; c0 < Np; c0 += 16) {
-                float acc[16];
-                tmem_ld16(tbase + ((uint32_t)(32 * warp) << 16) + (uint32_t)(z * b.cstride + c0), acc);
-                if (valid) conv_store16(a, v, n0 + c0, acc);
-            }
-        }
-    } else if (tid == 0) {
-        atomicExch(a.status, 1);
+    cp_async_wait<0>();
+    if (pending) {
+        fence_async_smem();
+        mbar_arrive_tc(pending);
     }
+    return true;
+}
+
+struct ConvPlaneArgs {
+    ConvArgs a;                                // a.Nt: output channels per CTA
+    int kz;                                    // output planes per item
+    int tx, ty, items;                         // tiles along x, y; items (tiles x chunks along z)
+    int ncols;                                 // tensor-memory columns, at least kz Nt
+    int planes;                                // input planes in shared memory (2 .. kMaxPlanes)
+};
+
+// The mbarriers and shared scalars of a CTA, in front of its operands.
+struct ConvPlaneShared {
+    uint64_t full[kMaxPlanes], empty[kMaxPlanes];      // input planes: copied; read by the MMAs
+    uint64_t wfull[9];                                 // the weights of an in-plane tap
+    uint64_t afull[kMaxKz], aempty[kMaxKz];            // accumulators: complete; read
+    uint64_t done, never;                              // all MMAs; nothing arrives on the last
+    uint32_t tslot;
+};
+constexpr int kPlaneShared = (sizeof(ConvPlaneShared) + 127) / 128 * 128;
+
+__global__ void __launch_bounds__(kPlaneThreads) k_conv_planes(const ConvPlaneArgs b) {
+    extern __shared__ __align__(128) unsigned char sm[];
+    ConvPlaneShared& sh = *reinterpret_cast<ConvPlaneShared*>(sm);
+    const ConvArgs& a = b.a;
+    const int Nt = a.Nt, n0 = blockIdx.y * Nt, Kc = a.Kc, NA = b.planes;
+    const ConvLanes L(Kc);
+    const int gs = kGroupBytes, rs = L.row_stride(3 * Nt), planeBytes = L.ng * gs, tapBytes = L.ng * rs;
+    unsigned char* stB = sm + kPlaneShared;                    // 9 in-plane taps
+    unsigned char* stA = stB + 9 * tapBytes;                   // NA planes
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int q = 0; q < NA; q++) { mbar_init_tc(&sh.full[q], kCopyThreads); mbar_init_tc(&sh.empty[q]); }
+        for (int q = 0; q < 9; q++) mbar_init_tc(&sh.wfull[q], kCopyThreads);
+        for (int q = 0; q < b.kz; q++) { mbar_init_tc(&sh.afull[q]); mbar_init_tc(&sh.aempty[q], 4); }
+        mbar_init_tc(&sh.done);
+        mbar_init_tc(&sh.never);
+    }
+    if (warp == 0) tmem_alloc(&sh.tslot, b.ncols);
     tc_fence_before();
     __syncthreads();
+    tc_fence_after();
+    const uint32_t tbase = sh.tslot;
+
+    auto place = [&](int item) { return conv_place(item, b.tx, b.ty, b.kz, a.nz); };
+    // failure-detection test: a bounded wait that runs out before any copy or MMA
+    bool ok = a.stall ? mbar_wait_tc(&sh.never, 0, 1u << 10) : true;
+    if (__syncthreads_and(ok)) {
+        // the weights, before they have else to do, by warps 0-3 and 8-11: in-plane tap
+        // u = 3 dj + di as rows [dk = +1 | 0 | -1] x Nt; rows beyond the channels are zero
+        if (warp < 4 || (warp >= 8 && warp < 12))
+            for (int u = warp >> 3; u < 9; u += 2) {
+                conv_copy_rows(L, 3 * Nt, sm_addr(stB + u * tapBytes), rs, warp & 3, lane, [&](int r) {
+                    const int dk = r >= 2 * Nt ? 2 : r >= Nt ? 1 : 0, o = n0 + r - dk * Nt;
+                    return o < a.Np ? a.W + ((size_t)((2 - dk) * 9 + u) * a.Np + o) * Kc : nullptr;
+                }, [] { return true; });
+                mbar_arrive_tc(&sh.wfull[u]);
+            }
+        if (warp < 4) {
+            // epilogue: output o of the item is the accumulator in columns o Nt ..
+            uint32_t use = 0;
+            for (int item = blockIdx.x; item < b.items && ok; item += gridDim.x, use ^= 1) {
+                const ConvPlace w = place(item);
+                const int i = w.x0 + (lane & 7), j = w.y0 + 4 * warp + (lane >> 3);
+                const bool valid = i < a.nx && j < a.ny;
+                const long long v = (long long)i + (long long)a.nx * (j + (long long)a.ny * w.z0);
+                for (int o = 0; o < w.kz; o++) {
+                    ok = __all_sync(~0u, mbar_wait_tc(&sh.afull[o], use));
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t col = tbase + ((uint32_t)(32 * warp) << 16) + (uint32_t)(o * Nt);
+                    for (int c0 = 0; c0 < Nt; c0 += 16) {
+                        float acc[16];
+                        tmem_ld16(col + c0, acc);
+                        if (c0 + 16 >= Nt) {
+                            // the last read: the columns are free
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_tc(&sh.aempty[o]);
+                        }
+                        if (valid) conv_store16(a, v + (long long)a.nx * a.ny * o, n0 + c0, acc);
+                    }
+                }
+            }
+        } else if (warp < 8) {
+            ok = conv_copy_planes(a, b.tx, b.ty, b.items, b.kz, NA, sm_addr(stA), sh.full, sh.empty, warp & 3, lane);
+        } else if (warp == 12 && elect_one()) {
+            // MMAs.  The per-MMA arithmetic is adding to the low words of the
+            // descriptors: what this thread does between two MMAs, the tensor core waits for
+            uint32_t n = 0, use = 0;
+            int buf = 0;
+            const int ks = Kc / 16;
+            const uint32_t ak = 2 * gs >> 4, bk = 2 * rs >> 4;
+            const uint64_t bd0 = smem_desc(sm_addr(stB), rs, 128);
+            for (int item = blockIdx.x; item < b.items && ok; item += gridDim.x, use ^= 1) {
+                const ConvPlace w = place(item);
+                for (int p = 0; p < w.kz + 2; p++, n++) {
+                    const int lo = max(p - 2, 0), hi = min(p, w.kz - 1);
+                    const bool fresh = p < w.kz;               // output p is new
+                    if (fresh && item != (int)blockIdx.x) ok = mbar_wait_tc(&sh.aempty[p], use ^ 1);
+                    ok = ok && mbar_wait_tc(&sh.full[buf], n / NA & 1);
+                    const uint32_t d = tbase + lo * Nt, id = idesc_bf16(128, (hi - lo + 1) * Nt);
+                    const uint64_t ad0 = smem_desc(sm_addr(stA + buf * planeBytes), gs, kHaloX * 16);
+                    const uint64_t bdp = bd0 + (lo - p + 2) * Nt;
+#pragma unroll
+                    for (int u = 0; u < 9; u++) {
+                        if (n == 0) ok = ok && mbar_wait_tc(&sh.wfull[u], 0);
+                        if (!ok) break;
+                        if (u == 0 || n == 0) tc_fence_after();
+                        uint64_t ad = ad0 + u / 3 * kHaloX + u % 3, bd = bdp + (uint32_t)(u * (tapBytes >> 4));
+                        int kk = 0;
+                        if (fresh && u == 0) {
+                            // the first product of output p does not accumulate
+                            if (p > lo) mma_bf16(d, ad, bd, idesc_bf16(128, (p - lo) * Nt), true);
+                            mma_bf16(tbase + p * Nt, ad, bd + (p - lo) * Nt, idesc_bf16(128, Nt), false);
+                            ad += ak;
+                            bd += bk;
+                            kk = 1;
+                        }
+                        for (; kk < ks; kk++) {
+                            mma_bf16(d, ad, bd, id, true);
+                            ad += ak;
+                            bd += bk;
+                        }
+                    }
+                    if (!ok) break;
+                    mma_commit(&sh.empty[buf]);
+                    if (p >= 2) mma_commit(&sh.afull[p - 2]);
+                    buf = buf + 1 == NA ? 0 : buf + 1;
+                }
+            }
+            // every MMA has completed before the tensor memory is freed
+            mma_commit(&sh.done);
+            if (!mbar_wait_tc(&sh.done, 0)) ok = false;
+        }
+    }
+    tc_fence_before();
+    ok = __syncthreads_and(ok);
+    if (!ok && tid == 0) atomicExch(a.status, 1);
+    if (warp == 0) tmem_free(tbase, b.ncols);
+}
+
+// ---- convolution with many input channels -------------------------------------------
+
+// The same with the weights streamed, for layers whose weights do not fit the
+// shared memory: for each tap (along z first, k_conv's order) and chunk of
+// input channels a stage of Nt x kch weights, used for the kz output planes of
+// the item; the planes in a ring of at least kz + 1 buffers with all channels.
+// Warps 0-3 store, 4-7 copy planes, the next copy weights (the latency of
+// their loads is what bounds a group), one thread of the last issues the MMAs.
+constexpr int kWideGroups = 4, kWideThreads = 32 * (4 + 4 + 4 * kWideGroups + 1), kWideStages = 8, kWideKz = 4;
+
+struct ConvWideArgs {
+    ConvArgs a;                                // a.Nt: output channels per CTA
+    int kz;                                    // output planes per item, at most kWideKz
+    int tx, ty, items;
+    int ncols, sets;                           // tensor-memory columns; accumulator sets (1 or 2) of kz Nt
+    int planes;                                // plane buffers (kz + 1 ..)
+    int kch, stages;                           // input channels per stage (divides Kc), stages
+};
+
+struct ConvWideShared {
+    uint64_t full[kWideKz + 2], empty[kWideKz + 2];
+    uint64_t wfull[kWideStages], wempty[kWideStages];
+    uint64_t afull[2], aempty[2];
+    uint64_t done, never;
+    uint32_t tslot;
+};
+constexpr int kWideShared = (sizeof(ConvWideShared) + 127) / 128 * 128;
+
+__global__ void __launch_bounds__(kWideThreads) k_conv_wide(const ConvWideArgs b) {
+    extern __shared__ __align__(128) unsigned char sm[];
+    ConvWideShared& sh = *reinterpret_cast<ConvWideShared*>(sm);
+    const ConvArgs& a = b.a;
+    const int Nt = a.Nt, n0 = blockIdx.y * Nt, Kc = a.Kc, NA = b.planes, S = b.stages, KCH = b.kch, nch = Kc / KCH;
+    const ConvLanes L(Kc), LW(KCH);
+    const int gs = kGroupBytes, rs = LW.row_stride(Nt), planeBytes = L.ng * gs, stepBytes = LW.ng * rs;
+    unsigned char* stB = sm + kWideShared;
+    unsigned char* stA = stB + S * stepBytes;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int q = 0; q < NA; q++) { mbar_init_tc(&sh.full[q], kCopyThreads); mbar_init_tc(&sh.empty[q]); }
+        for (int q = 0; q < S; q++) { mbar_init_tc(&sh.wfull[q], kCopyThreads); mbar_init_tc(&sh.wempty[q]); }
+        for (int q = 0; q < 2; q++) { mbar_init_tc(&sh.afull[q]); mbar_init_tc(&sh.aempty[q], 4); }
+        mbar_init_tc(&sh.done);
+        mbar_init_tc(&sh.never);
+    }
+    if (warp == 0) tmem_alloc(&sh.tslot, b.ncols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tbase = sh.tslot;
+    auto place = [&](int item) { return conv_place(item, b.tx, b.ty, b.kz, a.nz); };
+    bool ok = a.stall ? mbar_wait_tc(&sh.never, 0, 1u << 10) : true;
+    if (__syncthreads_and(ok)) {
+        if (warp < 4) {
+            uint32_t m = 0;                            // items so far
+            for (int item = blockIdx.x; item < b.items; item += gridDim.x, m++) {
+                const ConvPlace w = place(item);
+                const int set = m % b.sets;
+                ok = __all_sync(~0u, mbar_wait_tc(&sh.afull[set], m / b.sets & 1));
+                if (!ok) break;
+                tc_fence_after();
+                const int i = w.x0 + (lane & 7), j = w.y0 + 4 * warp + (lane >> 3);
+                const bool valid = i < a.nx && j < a.ny;
+                const long long v = (long long)i + (long long)a.nx * (j + (long long)a.ny * w.z0);
+                const uint32_t col = tbase + ((uint32_t)(32 * warp) << 16) + (uint32_t)(set * b.kz * Nt);
+                for (int o = 0; o < w.kz; o++)
+                    for (int c0 = 0; c0 < Nt; c0 += 16) {
+                        float acc[16];
+                        tmem_ld16(col + o * Nt + c0, acc);
+                        if (o == w.kz - 1 && c0 + 16 >= Nt) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_tc(&sh.aempty[set]);
+                        }
+                        if (valid) conv_store16(a, v + (long long)a.nx * a.ny * o, n0 + c0, acc);
+                    }
+            }
+        } else if (warp < 8) {
+            ok = conv_copy_planes(a, b.tx, b.ty, b.items, b.kz, NA, sm_addr(stA), sh.full, sh.empty, warp & 3, lane);
+        } else if (warp < 8 + 4 * kWideGroups) {
+            // weights: groups of four warps, a stage in turn
+            const int grp = (warp >> 2) - 2, wq = warp & 3;
+            int tap = 0, c = 0, st = 0;
+            uint32_t turn = 0, round = 0;              // stages so far, rounds of the ring
+            for (int item = blockIdx.x; item < b.items && ok; item += gridDim.x)
+                for (int q = 0; q < 27 * nch && ok; q++, turn++) {
+                    if (turn % kWideGroups == (uint32_t)grp) {
+                        const __nv_bfloat16* W = a.W + ((size_t)tap * a.Np + n0) * Kc + c * KCH;
+                        ok = conv_copy_rows(LW, Nt, sm_addr(stB + st * stepBytes), rs, wq, lane,
+                                       [&](int r) { return n0 + r < a.Np ? W + (size_t)r * Kc : nullptr; },
+                                       [&] { return round == 0 || mbar_wait_tc(&sh.wempty[st], round - 1 & 1); });
+                        if (ok) mbar_arrive_tc(&sh.wfull[st]);
+                    }
+                    if (++st == S) { st = 0; round++; }
+                    if (++c == nch) { c = 0; if (++tap == 27) tap = 0; }
+                }
+        } else if (elect_one()) {
+            uint32_t n = 0, m = 0;                     // planes, items so far
+            uint32_t wq = 0;                           // parity of the current round of stages
+            int sq = 0;                                // stage
+            const int ks = KCH / 16;
+            const uint32_t id = idesc_bf16(128, Nt);
+            const uint64_t ad00 = smem_desc(sm_addr(stA), gs, kHaloX * 16), bd00 = smem_desc(sm_addr(stB), rs, 128);
+            const uint32_t ak = 2 * gs >> 4, bk = 2 * rs >> 4;
+            for (int item = blockIdx.x; item < b.items && ok; item += gridDim.x, m++) {
+                const ConvPlace w = place(item);
+                const int set = m % b.sets;
+                if (m >= (uint32_t)b.sets) ok = mbar_wait_tc(&sh.aempty[set], m / b.sets - 1 & 1);
+                const uint32_t d0 = tbase + set * b.kz * Nt;
+                int b0 = n % NA;                       // buffer of plane dk
+                for (int dk = 0; dk < 3 && ok; dk++) {
+                    // planes dk .. dk + kz - 1; those not yet waited for
+                    for (int p = dk == 0 ? 0 : w.kz - 1 + dk; p < w.kz + dk; p++)
+                        ok = ok && mbar_wait_tc(&sh.full[(n + p) % NA], (n + p) / NA & 1);
+                    const uint32_t pstep = planeBytes >> 4;
+                    for (int u = 0; u < 9 && ok; u++) {
+                        const uint32_t tapoff = u / 3 * kHaloX + u % 3;
+                        for (int c = 0; c < nch; c++) {
+                            ok = mbar_wait_tc(&sh.wfull[sq], wq);
+                            if (!ok) break;
+                            tc_fence_after();
+                            const uint64_t bdc = bd00 + (uint32_t)(sq * (stepBytes >> 4));
+                            const uint32_t aoff = tapoff + c * (KCH / 8) * (gs >> 4);
+                            const bool first = dk == 0 && u == 0 && c == 0;
+                            uint32_t aplane = b0 * pstep;
+                            for (int z = 0; z < w.kz; z++) {
+                                uint64_t ad = ad00 + aplane + aoff, bd = bdc;
+                                const uint32_t d = d0 + z * Nt;
+                                for (int kk = 0; kk < ks; kk++) {
+                                    mma_bf16(d, ad, bd, id, !first || kk > 0);
+                                    ad += ak;
+                                    bd += bk;
+                                }
+                                aplane = aplane == (NA - 1) * pstep ? 0 : aplane + pstep;
+                            }
+                            mma_commit(&sh.wempty[sq]);
+                            if (++sq == S) { sq = 0; wq ^= 1; }
+                        }
+                    }
+                    if (!ok) break;
+                    b0 = b0 + 1 == NA ? 0 : b0 + 1;
+                    for (int p = dk; p < (dk == 2 ? w.kz + 2 : dk + 1); p++) mma_commit(&sh.empty[(n + p) % NA]);
+                }
+                if (!ok) break;
+                mma_commit(&sh.afull[set]);
+                n += w.kz + 2;
+            }
+            mma_commit(&sh.done);
+            if (!mbar_wait_tc(&sh.done, 0)) ok = false;
+        }
+    }
+    tc_fence_before();
+    ok = __syncthreads_and(ok);
+    if (!ok && tid == 0) atomicExch(a.status, 1);
     if (warp == 0) tmem_free(tbase, b.ncols);
 }
 
@@ -945,41 +1253,91 @@ __global__ void k_wg_grid(const float* __restrict__ d, const T* __restrict__ xid
     }
 }
 
-// Shape of k_conv_tile's launch, false where the tile does not fit (more than 96
-// input channels: the operands of a tap and chunk are streamed by k_conv).  kz
-// and the output slice: the most planes of the widest slice that still leave
-// about three CTAs for two SMs; two CTAs per SM (their copies and epilogues
-// overlap) if they fit, else one.
-static bool choose_conv_tile(const ConvArgs& a, ConvTileArgs* b, size_t* smem) {
-    if (a.Kc > 96) return false;
+// The launch of a convolution of one view: k_conv_planes with resident weights or
+// k_conv_wide with streamed ones, the candidates (output slices, planes per item)
+// compared by an estimate in clocks.  An MMA with N columns takes
+// max(46, 32 + N / 4, N / 2) clocks; CTAs on an SM share the tensor core; resident
+// weights arrive at about 40 bytes a clock and SM, a stage of streamed ones takes 600
+// clocks more, and an item of k_conv_wide starts 4000 clocks late; a plane's barriers take about 700 clocks of one CTA that another
+// hides; starting and draining a CTA takes 5000.  Against all shapes that fit, the
+// choice was the fastest or within 10 % of it (64x64x128: 24 -> 24 channels 38 us,
+// 72 -> 24 75 us, 24 -> 72 81 us; 32x32x64: 240 -> 48 160 us with streamed weights,
+// the only form that fits; 16x16x32: 48 -> 192 19 us, 24 streamed).
+struct ConvPlan {
+    bool wide;
+    int Nt, kz, occ, planes, ncols, sets, kch, stages;
+    long long items;
+    dim3 grid;
+    size_t smem;
+};
+
+static bool choose_conv(const ConvArgs& a, ConvPlan* best) {
     int dev = 0, nsm = 152;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    b->a = a;
-    b->tx = (a.nx + kTileX - 1) / kTileX;
-    b->ty = (a.ny + kTileY - 1) / kTileY;
-    const long long cols = (long long)b->tx * b->ty;
-    for (int two = 1; two >= 0; two--)
-        for (int split = 1; split <= 4; split++) {
-            const int Nt = ((a.Np + split - 1) / split + 15) / 16 * 16;
-            for (int kz : {4, 2, 1}) {
-                const int cs = (Nt + 31) / 32 * 32;
-                int nc = 32;
-                while (nc < cs * kz) nc <<= 1;
-                const size_t sm = (size_t)(kz + 2) * (a.Kc / 8) * kGroupBytes + (size_t)kConvStages * Nt * a.Kc * 2 + 64;
-                if (nc > (two ? 256 : 512) || sm > (size_t)(two ? 112 : 226) * 1024) continue;
-                const long long ctas = cols * ((a.nz + kz - 1) / kz) * ((a.Np + Nt - 1) / Nt);
-                if (kz > 1 && ctas < 3ll * nsm / 2) continue;
-                if (split > 1 && kz == 1 && ctas > 4ll * nsm && !two) continue;
-                b->a.Nt = Nt;
-                b->kz = kz;
-                b->cstride = cs;
-                b->ncols = nc;
-                *smem = sm;
-                return true;
+    const long long cols = (long long)((a.nx + kTileX - 1) / kTileX) * ((a.ny + kTileY - 1) / kTileY);
+    const ConvLanes L(a.Kc);
+    const size_t limit = 227 * 1024, plane = (size_t)L.ng * kGroupBytes;
+    double tbest = 0;
+    auto mma = [](double N) { return std::max(46.0, std::max(32 + N / 4, N / 2)); };
+    int last = 0;
+    for (int Nt = 16; Nt <= 256 && Nt <= a.Np; Nt += 16) {
+        const int slices = (a.Np + Nt - 1) / Nt;
+        if (slices == last) continue;          // no fewer slices than the width before
+        last = slices;
+        const double ksteps = a.Kc / 16;
+        ConvPlan c;
+        c.Nt = Nt;
+        if (Nt <= 80) {
+            c.wide = false;
+            c.planes = 3;
+            c.smem = kPlaneShared + (size_t)9 * L.ng * L.row_stride(3 * Nt) + 3 * plane;
+            if (c.smem > limit) { c.planes = 2; c.smem -= plane; }
+            for (int kz = 1; c.smem <= limit && kz <= kMaxKz && kz <= a.nz && kz * Nt <= 512; kz++) {
+                c.kz = kz;
+                c.ncols = 32;
+                while (c.ncols < kz * Nt) c.ncols <<= 1;
+                c.occ = std::min((int)(228 * 1024 / (c.smem + 1024)), std::min(512 / c.ncols, 4));
+                c.items = cols * ((a.nz + kz - 1) / kz);
+                const long long gx = std::max(1ll, std::min(c.items, (long long)nsm * c.occ / slices));
+                c.grid = dim3((unsigned)gx, (unsigned)slices);
+                const double on = (double)((gx * slices + nsm - 1) / nsm);        // CTAs on an SM
+                const double per = 9 * ksteps * mma(3.0 * Nt * kz / (kz + 2));
+                const double t = (double)((c.items + gx - 1) / gx) * (kz + 2) * std::max(on * per, per + (c.planes > 2 ? 700 : 1500)) +
+                                 27.0 * Nt * a.Kc * 2 / 40 * on + 5000;
+                if (c.items < (1ll << 31) && (tbest == 0 || t < tbest)) { tbest = t; *best = c; }
             }
         }
-    return false;
+        c.wide = true;
+        c.occ = 1;
+        for (int kz = 1; kz <= kWideKz && kz <= a.nz && kz * Nt <= 512; kz++) {
+            c.kz = kz;
+            c.planes = kz + 1;
+            c.kch = a.Kc;
+            auto step = [&]() { return (size_t)(c.kch / 8) * ConvLanes(c.kch).row_stride(Nt); };
+            auto room = [&](int stages) { return kWideShared + c.planes * plane + stages * step() <= limit; };
+            // the widest chunk of at most 16 KB of which six stages fit
+            int nch = 1;
+            for (; nch <= a.Kc / 16; nch++) {
+                if (a.Kc / 16 % nch) continue;
+                c.kch = a.Kc / nch;
+                if (Nt * c.kch * 2 <= 16384 && room(6)) break;
+            }
+            if (nch > a.Kc / 16) continue;
+            c.stages = room(8) ? 8 : 6;
+            c.sets = 2 * kz * Nt <= 512 ? 2 : 1;
+            c.ncols = 32;
+            while (c.ncols < c.sets * kz * Nt) c.ncols <<= 1;
+            c.items = cols * ((a.nz + kz - 1) / kz);
+            const long long gx = std::max(1ll, std::min(c.items, (long long)nsm / slices));
+            c.grid = dim3((unsigned)gx, (unsigned)slices);
+            c.smem = kWideShared + c.planes * plane + c.stages * step();
+            const double item = 27.0 * nch * std::max(ksteps / nch * kz * mma(Nt), 600 + Nt * c.kch * 2 / 40.0);
+            const double t = (double)((c.items + gx - 1) / gx) * (item + 4000) + 8000;
+            if (c.items < (1ll << 31) && (tbest == 0 || t < tbest)) { tbest = t; *best = c; }
+        }
+    }
+    return tbest > 0;
 }
 
 static unsigned nb(long long n) {
@@ -1053,15 +1411,21 @@ int gm_nn_conv(const void* in1, int ld1, int c1, const void* in2, int ld2, int c
     a.stall = g_nn_stall;
     auto aligned = [](const void* q, int ld) { return q == nullptr || (!(reinterpret_cast<uintptr_t>(q) & 15) && ld % 8 == 0); };
     a.vec = aligned(out, ldo) && aligned(mask, ldm);
-    gmnn::ConvTileArgs b;
-    size_t tile_smem;
-    if (!in2 && gmnn::choose_conv_tile(a, &b, &tile_smem)) {
-        cudaError_t e = cudaFuncSetAttribute(gmnn::k_conv_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    gmnn::ConvPlan c;
+    if (!in2 && gmnn::choose_conv(a, &c)) {
+        a.Nt = c.Nt;
+        const int tx = (nx + gmnn::kTileX - 1) / gmnn::kTileX, ty = (ny + gmnn::kTileY - 1) / gmnn::kTileY;
+        cudaError_t e = c.wide ? cudaFuncSetAttribute(gmnn::k_conv_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)
+                               : cudaFuncSetAttribute(gmnn::k_conv_planes, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return gm::fail(GM_ECUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-        const dim3 grid((unsigned)(b.tx * b.ty * ((nz + b.kz - 1) / b.kz)), (unsigned)((Np + b.a.Nt - 1) / b.a.Nt));
-        gmnn::k_conv_tile<<<grid, 128, tile_smem, (cudaStream_t)stream>>>(b);
+        if (c.wide)
+            gmnn::k_conv_wide<<<c.grid, gmnn::kWideThreads, c.smem, (cudaStream_t)stream>>>(
+                gmnn::ConvWideArgs{a, c.kz, tx, ty, (int)c.items, c.ncols, c.sets, c.planes, c.kch, c.stages});
+        else
+            gmnn::k_conv_planes<<<c.grid, gmnn::kPlaneThreads, c.smem, (cudaStream_t)stream>>>(
+                gmnn::ConvPlaneArgs{a, c.kz, tx, ty, (int)c.items, c.ncols, c.planes});
         e = cudaGetLastError();
-        return e == cudaSuccess ? GM_OK : gm::fail(GM_ECUDA, std::string("k_conv_tile: ") + cudaGetErrorString(e));
+        return e == cudaSuccess ? GM_OK : gm::fail(GM_ECUDA, std::string("convolution launch: ") + cudaGetErrorString(e));
     }
     const size_t smem = conv_smem(Nt);
     cudaError_t e = cudaFuncSetAttribute(gmnn::k_conv, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);

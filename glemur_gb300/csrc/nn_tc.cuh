@@ -44,9 +44,27 @@ __device__ __forceinline__ uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-__device__ __forceinline__ void mbar_init_tc(uint64_t* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sm_addr(bar)) : "memory");
+__device__ __forceinline__ void mbar_init_tc(uint64_t* bar, uint32_t count = 1) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sm_addr(bar)), "r"(count) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive_tc(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sm_addr(bar)) : "memory");
+}
+
+// Whether the phase has completed, without waiting (try_wait may suspend the
+// thread, and others may wait for what it has yet to announce).
+__device__ __forceinline__ bool mbar_test_tc(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(sm_addr(bar)), "r"(parity)
+        : "memory");
+    return ok;
 }
 
 __device__ __forceinline__ bool mbar_wait_tc(uint64_t* bar, uint32_t parity, unsigned limit = kTcWaitLimit) {
@@ -73,6 +91,20 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
 
 __device__ __forceinline__ void tmem_free(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+
+// One lane of a converged warp.  A branch on elect.sync is known to leave one lane,
+// so the operands of the MMAs in it are computed in uniform registers; in a branch
+// on the lane number every operand word is moved there first (measured in a loop of
+// MMAs of 57 clocks: 95 to 310 clocks each).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(p));
+    return p != 0;
 }
 
 // D (+)= A . B^T for one K = 16 slice, issued by a single thread.
