@@ -755,218 +755,240 @@ __global__ void __launch_bounds__(kWideThreads) k_conv_wide(const ConvWideArgs b
 
 // ---- convolution: weight gradient --------------------------------------------
 
-// dW[t][o][i] = sum_v dout[v][o] in[v + off(t)][i] as one GEMM per voxel chunk
-// with the 27 taps stacked along M: row m = t Cp + i (Cp = ci rounded up to 8),
-// column n = output channel o (N = co rounded up to 16), K = voxels.  Both
-// operands are read as they lie in the channels-last buffers: 16 bytes are 8
-// channels of one voxel, which is one row of a core matrix of the MN-major
-// operand layout, so a copy goes straight from global to shared memory
-// (cp.async) with no transpose.
+// dW[t][o][i] = sum_v dout[v][o] in[v + off(t)][i]: a GEMM over the voxels (K) with
+// both operands MN-major, read as they lie: 16 bytes are 8 channels of one voxel,
+// one row of a core matrix, and 8 voxels along x are a core matrix.  A CTA takes
+// blocks of 8 x 16 voxels and kb planes, a slice of at most 3 groups of 8 input
+// channels and a slice of at most 48 output channels.  The kb + 2 input planes of a
+// block with their halo lie in shared memory one after the other as [8-channel
+// group][y][x][16 bytes], so the groups of three consecutive planes are one run of
+// equal strides: the three taps along z are stacked along M (3 planes x 3 groups x 8 = 72
+// of 128 rows; the rows beyond read what follows and are dropped), and the nine
+// in-plane taps are nine start addresses with an accumulator each (9 x 48 columns).
+// An MMA takes 16 voxels (two rows along x: the K-direction offset is a halo row, 160
+// bytes) against as many of the upstream gradient, [8-channel group][voxel][16 bytes].
+// Accumulators stay in tensor memory over a chain of blocks and are then added to dW.
+// (The tensor core's sums are truncated: the error grows with the products in a
+// chain, 3e-6 of the gradient at 3500 voxels.)  Slices of 5 groups (120 rows) take
+// fewer MMAs, but the copies bound them, as their planes leave room for two a block
+// (72 -> 24 channels at 64x64x128: 195 us).
 //
-// MN-major, no swizzle: a step of kWgKV voxels of an operand with R rows (M or
-// N) is kWgKV / 16 slices of 16 voxels, one per MMA (K = 16); slice s holds
-// R / 8 x 2 core matrices of 128 bytes (8 voxels x 8 channels), core (rb, h) at
-// s R 32 + rb 256 + h 128 bytes.  So neighbouring core matrices along the rows
-// are 256 bytes apart (the descriptor's stride-dimension offset) and along K
-// 128 bytes apart (its leading-dimension offset).  Read with the two offsets
-// exchanged, every address would still fall inside the slice.
-constexpr int kWgKV = 64;
-constexpr int kWgStages = 4;
-
-__device__ __forceinline__ uint32_t mn_off(int rb, int w, int R) {
-    return (uint32_t)((w >> 4) * R * 32 + rb * 256 + (w & 15) * 16);
-}
+// With the 27 taps' rows copied one by one (27 times the input through cp.async, 16
+// bytes a clock) this took 2700 of the 4200 us of a training step.
+//
+// Warps 0-3 add the accumulators of a finished chain to dW, warps 4-7 copy planes,
+// 8-11 the upstream gradient, one thread of warp 12 issues the MMAs; an accumulator's
+// next chain starts when it has been read.
+constexpr int kWgKb = 6, kWgGroups = 3, kWgN = 48, kWgThreads = 416;
+constexpr int kDoutGroup = 128 * 16;           // one plane of 8 output channels
 
 struct WgradArgs {
     const __nv_bfloat16* dout; int ldd, co;  // upstream gradient (channels up to co rounded to 8 readable)
-    const __nv_bfloat16* in1; int ld1, c1;   // forward input views
-    const __nv_bfloat16* in2; int ld2, c2;
+    const __nv_bfloat16* in1; int ld1, c1;   // forward input views (channels up to ci rounded to 8 read)
+    const __nv_bfloat16* in2; int ld2;
     float* dW;                               // [27][co][ci] FP32, accumulated with atomics
-    int ci, Cp;                              // input channels of the weights; rows per tap (ci rounded to 8)
-    int N;                                   // MMA columns: co rounded up to 16
+    int ci;
     int nx, ny, nz, xper, yper;
-    int vchunk;                              // voxels per CTA (multiple of kWgKV)
+    int tx, ty, kb, blocks;                  // tiles along x, y; planes per block; blocks (tiles x chunks along z)
+    int cs, cslices, N;                      // input groups per slice, slices; output channels per slice (MMA columns)
+    int ncols;                               // tensor-memory columns, at least 9 N
+    int chain;                               // blocks per chain
     int* status;
     int stall;                               // failure-detection test: wait on an mbarrier nothing arrives on
 };
 
-// grid = (voxel chunks, row tiles of 128 stacked (tap, channel) rows).  The
-// operands of a step (kWgKV voxels: the tile's rows of the input at their taps'
-// offsets, and the upstream gradient) are copied kWgStages steps ahead while
-// one thread issues the MMAs of the current step; a stage is refilled once the
-// MMAs that read it have committed.
-__global__ void __launch_bounds__(128) k_conv_wgrad(const WgradArgs a) {
-    extern __shared__ __align__(128) unsigned char sm[];
-    constexpr int S = kWgStages, KV = kWgKV;
-    const int N = a.N;
-    const int aBytes = 128 * KV * 2, bBytes = N * KV * 2;
-    unsigned char* stA = sm;                          // S stages of A, then S stages of B
-    unsigned char* stB = sm + S * aBytes;
-    // mbarriers: one per stage (MMA commits) and one that nothing arrives on
-    // (the failure-detection test waits on it)
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + S * (aBytes + bBytes));
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + S + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = 128 * blockIdx.y;                  // first stacked row of this CTA
-    const int V = a.nx * a.ny * a.nz;                 // < 2^31 (checked by the host)
-    const int v0 = blockIdx.x * a.vchunk;
-    const int nv = min(V - v0, a.vchunk);             // voxels of this chunk
-    const int T = (nv + KV - 1) / KV;                 // steps
-    const int w = tid & (KV - 1);                     // this thread's voxel within a step
-    const int cpb = a.Cp >> 3;                        // 8-channel groups per tap
-    // this thread's 8 row blocks of A (rb = tid / 64 + 2 r): the tap's offset
-    // packed as (di + 1) | (dj + 1) << 2 | (dk + 1) << 4 (-1: a row beyond the
-    // 27 taps or the input's channels, zero-filled), and the source view from
-    // the block's first channel, with its channel stride
-    int tapo[8], ldr[8];
-    const __nv_bfloat16* srcr[8];
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-        const int g = (m0 >> 3) + (tid >> 6) + 2 * r;
-        const int t = g / cpb, c = (g - t * cpb) * 8;
-        tapo[r] = t < 27 ? (t % 3) | (((t / 3) % 3) << 2) | ((t / 9) << 4) : -1;
-        srcr[r] = a.in1;
-        ldr[r] = 0;
-        if (c < a.c1) { srcr[r] = a.in1 + c; ldr[r] = a.ld1; }
-        else if (c - a.c1 < a.c2) { srcr[r] = a.in2 + (c - a.c1); ldr[r] = a.ld2; }
-        else tapo[r] = -1;
-    }
-    // the coordinates of this thread's voxel v0 + kWgKV q + w of the next step
-    // to issue, advanced by kWgKV = si + nx (sj + ny sk) voxels per step
-    int vi, vj, vk;
-    {
-        const int v = v0 + w;
-        vi = v % a.nx;
-        vj = (v / a.nx) % a.ny;
-        vk = v / (a.nx * a.ny);
-    }
-    const int si = KV % a.nx, sj = (KV / a.nx) % a.ny, sk = KV / (a.nx * a.ny);
-    uint32_t ncols = 32;
-    while ((int)ncols < N) ncols <<= 1;
-    if (tid == 0)
-        for (int q = 0; q <= S; q++) mbar_init_tc(&bars[q]);
-    if (warp == 0) tmem_alloc(tslot, ncols);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tbase = *tslot;
-    // A and B both MN-major (transpose bits 15 and 16)
-    const uint32_t id = idesc_bf16(128, N) | (1u << 15) | (1u << 16);
+struct WgradShared {
+    uint64_t full[2], empty[2];              // the two block buffers: copied; read by the MMAs
+    uint64_t afull, aempty[9];               // the chain's MMAs; an in-plane tap's accumulator read
+    uint64_t done, never;
+    uint32_t tslot;
+};
+constexpr int kWgShared = 256;
+static_assert(sizeof(WgradShared) <= kWgShared);
 
-    // the copies of step q into stage q % S (called for q = 0, 1, 2, ... in turn)
-    auto issue = [&](int q) {
-        const int st = q % S;
-        const int vl = q * KV + w;
-        const bool vin = vl < nv;
-        const int v = v0 + vl;
-        unsigned char* dA = stA + st * aBytes;
-#pragma unroll
-        for (int r = 0; r < 8; r++) {
-            const int to = tapo[r];
-            int ii = vi + (to & 3) - 1, jj = vj + ((to >> 2) & 3) - 1;
-            const int kk = vk + (to >> 4) - 1;
-            const bool ok = vin && to >= 0 && kk >= 0 && kk < a.nz && (a.xper || (ii >= 0 && ii < a.nx)) &&
-                            (a.yper || (jj >= 0 && jj < a.ny));
-            ii = wrap(ii, a.nx);
-            jj = wrap(jj, a.ny);
-            const int u = ok ? ii + a.nx * (jj + a.ny * kk) : 0;
-            cp_async16(dA + mn_off((tid >> 6) + 2 * r, w, 128), ok ? srcr[r] + (size_t)u * ldr[r] : a.in1, ok);
-        }
-        unsigned char* dB = stB + st * bBytes;
-        for (int nb = tid >> 6; nb < N / 8; nb += 2) {
-            const bool ok = vin && nb * 8 < a.co;
-            cp_async16(dB + mn_off(nb, w, N), ok ? a.dout + (size_t)v * a.ldd + nb * 8 : a.dout, ok);
-        }
-        // the next step's voxel
-        vi += si;
-        const int cx = vi >= a.nx;
-        vi -= cx ? a.nx : 0;
-        vj += sj + cx;
-        const int cy = vj >= a.ny;
-        vj -= cy ? a.ny : 0;
-        vk += sk + cy;
-    };
-
-    uint32_t ph[S];
-    bool pend[S];                    // a commit on bars[s] not yet waited for
-    for (int q = 0; q < S; q++) { ph[q] = 0; pend[q] = false; }
-    // failure-detection test: a bounded wait that runs out before any MMA
-    bool ok = a.stall ? mbar_wait_tc(&bars[S], 0, 1u << 10) : true;
-    if (__syncthreads_and(ok)) {
-        for (int q = 0; q < S - 1; q++) {
-            if (q < T) issue(q);
-            cp_async_commit();
-        }
-        for (int q = 0; q < T; q++) {
-            // refill the stage of step q + S - 1: the MMAs of step q - 1 read it
-            const int qn = q + S - 1;
-            if (qn < T) {
-                const int sn = qn % S;
-                if (pend[sn]) {
-                    if (!mbar_wait_tc(&bars[sn], ph[sn])) ok = false;
-                    ph[sn] ^= 1;
-                    pend[sn] = false;
-                }
-            }
-            // after a wait ran out no thread copies into a stage and no MMA is issued
-            if (!__syncthreads_and(ok)) {
-                ok = false;
-                break;
-            }
-            if (qn < T) issue(qn);
-            cp_async_commit();
-            cp_async_wait<S - 1>();                  // step q's copies have landed
-            fence_async_smem();
-            tc_fence_before();
-            __syncthreads();
-            tc_fence_after();
-            const int s = q % S;
-            if (tid == 0) {
-                for (int kk = 0; kk < KV / 16; kk++) {
-                    const uint64_t ad = smem_desc(sm_addr(stA + s * aBytes) + kk * 128 * 32, 128, 256);
-                    const uint64_t bd = smem_desc(sm_addr(stB + s * bBytes) + kk * N * 32, 128, 256);
-                    mma_bf16(tbase, ad, bd, id, q > 0 || kk > 0);
-                }
-                mma_commit(&bars[s]);
-            }
-            pend[s] = true;
-        }
-    }
-    // the copies still in flight, and the commits not yet waited for: bounded
-    // waits before the accumulator is read or freed
-    cp_async_wait_all();
-    for (int q = 0; q < S; q++)
-        if (pend[q]) {
-            if (!mbar_wait_tc(&bars[q], ph[q])) ok = false;
-            ph[q] ^= 1;
-        }
-    ok = __syncthreads_and(ok);
-    tc_fence_after();
-    // this thread's row: tap t, input channel ich
-    const int g = m0 + 32 * warp + lane;
-    const int t = g / a.Cp, ich = g - t * a.Cp;
-    const bool mine = t < 27 && ich < a.ci;
-    if (ok && T > 0) {
-        for (int c0 = 0; c0 < N; c0 += 16) {
-            float acc[16];
-            tmem_ld16(tbase + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, acc);
-            if (mine) {
-#pragma unroll
-                for (int q = 0; q < 16; q++) {
-                    const int o = c0 + q;
-                    if (o < a.co) atomicAdd(&a.dW[((size_t)t * a.co + o) * a.ci + ich], acc[q]);
-                }
-            }
-        }
-    } else if (!ok && tid == 0) {
-        atomicExch(a.status, 1);
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) tmem_free(tbase, ncols);
+// Bytes of a block buffer: the planes, and the upstream gradient's.  (The MMAs read 16
+// groups from the last three planes' start; what is beyond them lies in the rest of
+// the shared memory, which wgrad_smem leaves room for.)
+__host__ __device__ inline int wg_block_bytes(int cs, int kb, int N) {
+    return (kb + 2) * cs * kGroupBytes + kb * (N / 8) * kDoutGroup;
+}
+inline size_t wgrad_smem(int cs, int kb, int N) {
+    const size_t past = (size_t)(kb - 1) * cs * kGroupBytes + 16 * kGroupBytes;      // end of the last MMA's rows
+    const size_t one = wg_block_bytes(cs, kb, N);
+    return kWgShared + one + std::max(one, past);
 }
 
-// ---- elementwise and resampling kernels ---------------------------------------
+__global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const WgradArgs a) {
+    extern __shared__ __align__(128) unsigned char sm[];
+    WgradShared& sh = *reinterpret_cast<WgradShared*>(sm);
+    const int cs = a.cs, N = a.N, kb = a.kb, blockBytes = wg_block_bytes(cs, kb, N), planeBytes = cs * kGroupBytes;
+    const int slice = blockIdx.y % a.cslices, o0 = blockIdx.y / a.cslices * N;
+    const int c0 = slice * cs * 8;                             // first input channel of the slice
+    const uint32_t st = sm_addr(sm) + kWgShared;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int q = 0; q < 2; q++) { mbar_init_tc(&sh.full[q], 256); mbar_init_tc(&sh.empty[q]); }
+        mbar_init_tc(&sh.afull);
+        for (int u = 0; u < 9; u++) mbar_init_tc(&sh.aempty[u], 4);
+        mbar_init_tc(&sh.done);
+        mbar_init_tc(&sh.never);
+    }
+    if (warp == 0) tmem_alloc(&sh.tslot, a.ncols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tbase = sh.tslot;
+    // failure-detection test: a bounded wait that runs out before any copy or MMA
+    bool ok = a.stall ? mbar_wait_tc(&sh.never, 0, 1u << 10) : true;
+    if (__syncthreads_and(ok)) {
+        if (warp < 4) {
+            // row 32 warp + lane: stacked group row / 8 = dk cs + group, channel row % 8
+            const int row = 32 * warp + lane, sg = row >> 3, dk = sg / cs, ich = c0 + (sg - dk * cs) * 8 + (row & 7);
+            const bool mine = dk < 3 && ich < a.ci;
+            const int mine_blocks = (a.blocks - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+            for (int c = 0; c * a.chain < mine_blocks; c++) {
+                ok = __all_sync(~0u, mbar_wait_tc(&sh.afull, c & 1));
+                if (!ok) break;
+                tc_fence_after();
+                for (int u = 0; u < 9; u++) {
+                    for (int n0 = 0; n0 < N; n0 += 16) {
+                        float acc[16];
+                        tmem_ld16(tbase + ((uint32_t)(32 * warp) << 16) + (uint32_t)(u * N + n0), acc);
+                        if (n0 + 16 >= N) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_tc(&sh.aempty[u]);
+                        }
+                        if (!mine) continue;
+                        float* w = a.dW + ((size_t)(dk * 9 + u) * a.co + o0 + n0) * a.ci + ich;
+#pragma unroll
+                        for (int q = 0; q < 16; q++)
+                            if (o0 + n0 + q < a.co) atomicAdd(w + (size_t)q * a.ci, acc[q]);
+                    }
+                    __syncwarp();
+                }
+            }
+        } else if (warp < 12) {
+            const int wq = warp & 3, gh = lane >> 4;
+            uint64_t* pending = nullptr;
+            auto flush = [&]() {
+                if (!pending) return;
+                cp_async_wait<0>();
+                fence_async_smem();
+                mbar_arrive_tc(pending);
+                pending = nullptr;
+            };
+            uint32_t n = 0;
+            for (int blk = blockIdx.x; blk < a.blocks && ok; blk += gridDim.x, n++) {
+                const ConvPlace w = conv_place(blk, a.tx, a.ty, kb, a.nz);
+                const int buf = n & 1;
+                if (n >= 2 && !mbar_test_tc(&sh.empty[buf], (n >> 1) - 1 & 1)) {
+                    flush();
+                    ok = mbar_wait_tc(&sh.empty[buf], (n >> 1) - 1 & 1);
+                    if (!ok) break;
+                }
+                const uint32_t dst = st + buf * blockBytes;
+                if (warp < 8) {
+                    // the planes z0 - 1 .. z0 + kz: slots 16 (wq + 4 q) + lane % 16, two groups a copy
+#pragma unroll
+                    for (int q = 0; q < 3; q++) {
+                        const int s = 16 * (wq + 4 * q) + (lane & 15), sy = s / kHaloX;
+                        if (s >= kSlots) continue;
+                        int i = w.x0 + s - sy * kHaloX - 1, j = w.y0 + sy - 1;
+                        const bool in = (i >= 0 || a.xper) && (j >= 0 || a.yper) && (i < a.nx || (a.xper && i == a.nx)) &&
+                                        (j < a.ny || (a.yper && j == a.ny));
+                        i = wrap(i, a.nx);
+                        j = wrap(j, a.ny);
+                        for (int p = 0; p < w.kz + 2; p++) {
+                            const int k = w.z0 + p - 1;
+                            const bool on = in && k >= 0 && k < a.nz;
+                            const long long v = on ? (long long)i + (long long)a.nx * (j + (long long)a.ny * k) : 0;
+                            for (int g = gh; g < cs; g += 2) {
+                                const int c = c0 + 8 * g;
+                                const __nv_bfloat16* src = c < a.c1 ? a.in1 + v * a.ld1 + c : a.in2 + v * a.ld2 + (c - a.c1);
+                                cp_async16s(dst + p * planeBytes + g * kGroupBytes + s * 16, on && c < a.ci ? src : a.in1, on && c < a.ci);
+                            }
+                        }
+                    }
+                } else {
+                    // the upstream gradient: voxels 16 (wq + 4 q) + lane % 16
+                    const uint32_t dd = dst + (kb + 2) * planeBytes;
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {
+                        const int s = 16 * (wq + 4 * q) + (lane & 15), i = w.x0 + (s & 7), j = w.y0 + (s >> 3);
+                        const bool in = i < a.nx && j < a.ny;
+                        for (int p = 0; p < w.kz; p++) {
+                            const long long v = in ? (long long)i + (long long)a.nx * (j + (long long)a.ny * (w.z0 + p)) : 0;
+                            for (int g = gh; g < N / 8; g += 2) {
+                                const bool on = in && o0 + 8 * g < a.co;
+                                cp_async16s(dd + (p * (N / 8) + g) * kDoutGroup + s * 16, on ? a.dout + v * a.ldd + o0 + 8 * g : a.dout, on);
+                            }
+                        }
+                    }
+                }
+                cp_async_commit();
+                if (pending) {
+                    cp_async_wait<1>();
+                    fence_async_smem();
+                    mbar_arrive_tc(pending);
+                }
+                pending = &sh.full[buf];
+            }
+            flush();
+            cp_async_wait_all();
+        } else if (elect_one()) {
+            // A and B both MN-major (transpose bits 15 and 16)
+            const uint32_t id = idesc_bf16(128, N) | (1u << 15) | (1u << 16);
+            const uint64_t ad00 = smem_desc(st, kHaloX * 16, kGroupBytes);
+            const uint64_t bd00 = smem_desc(st + (kb + 2) * planeBytes, 128, kDoutGroup);
+            const uint32_t bplane = (N / 8) * (kDoutGroup >> 4);
+            uint32_t n = 0, chains = 0;                // blocks, finished chains so far
+            int link = 0;                              // blocks of the current chain
+            for (int blk = blockIdx.x; blk < a.blocks && ok; blk += gridDim.x, n++) {
+                const int buf = n & 1, kz = min(kb, a.nz - blk / (a.tx * a.ty) * kb);
+                ok = mbar_wait_tc(&sh.full[buf], n >> 1 & 1);
+                if (!ok) break;
+                tc_fence_after();
+                uint64_t ad0 = ad00 + (uint32_t)(buf * (blockBytes >> 4)), bd0 = bd00 + (uint32_t)(buf * (blockBytes >> 4));
+                const bool head = link == 0;                   // the chain's first products do not accumulate
+                for (int p = 0; p < kz && ok; p++) {
+                    const bool more = !head || p > 0;
+#pragma unroll
+                    for (int u = 0; u < 9; u++) {
+                        if (!more && n > 0) {
+                            ok = ok && mbar_wait_tc(&sh.aempty[u], chains - 1 & 1);
+                            if (!ok) break;
+                            tc_fence_after();
+                        }
+                        uint64_t ad = ad0 + u / 3 * kHaloX + u % 3, bd = bd0;
+#pragma unroll
+                        for (int kk = 0; kk < 8; kk++) {
+                            mma_bf16(tbase + u * N, ad, bd, id, more || kk > 0);
+                            ad += 2 * kHaloX;
+                            bd += 16;
+                        }
+                    }
+                    ad0 += planeBytes >> 4;
+                    bd0 += bplane;
+                }
+                if (!ok) break;
+                mma_commit(&sh.empty[buf]);
+                if (++link == a.chain || blk + (int)gridDim.x >= a.blocks) {
+                    mma_commit(&sh.afull);
+                    link = 0;
+                    chains++;
+                }
+            }
+            // every MMA has completed before the accumulators are read or freed
+            mma_commit(&sh.done);
+            if (!mbar_wait_tc(&sh.done, 0)) ok = false;
+        }
+    }
+    tc_fence_before();
+    ok = __syncthreads_and(ok);
+    if (!ok && tid == 0) atomicExch(a.status, 1);
+    if (warp == 0) tmem_free(tbase, a.ncols);
+}
 
 // Sum over voxels of an upstream gradient per channel (bias gradient).
 __global__ void k_bias_grad(const __nv_bfloat16* __restrict__ d, int ld, int c, long long V, float* __restrict__ db) {
@@ -1442,7 +1464,7 @@ int gm_nn_conv_wgrad(const void* dout, int ldd, int co, const void* in1, int ld1
                      void* stream) {
     if (!dout || !in1 || !dW || !status) return gm::fail(GM_EPARAM, "gm_nn_conv_wgrad: null argument");
     const long long V = (long long)nx * ny * nz;
-    if (ci > c1 + (in2 ? c2 : 0) || ci < 1 || co > 256 || co < 1 || vchunk < 0 || vchunk % gmnn::kWgKV || c1 % 8 ||
+    if (ci > c1 + (in2 ? c2 : 0) || ci < 1 || co > 256 || co < 1 || vchunk < 0 || vchunk % 64 || c1 % 8 ||
         nx < 1 || ny < 1 || nz < 1 || V >= (1ll << 31))
         return gm::fail(GM_EPARAM, "gm_nn_conv_wgrad: channel counts, grid or chunk out of range");
     int rc;
@@ -1451,30 +1473,54 @@ int gm_nn_conv_wgrad(const void* dout, int ldd, int co, const void* in1, int ld1
         return rc;
     WgradArgs a;
     a.dout = (const __nv_bfloat16*)dout; a.ldd = ldd; a.co = co;
-    a.in1 = (const __nv_bfloat16*)in1; a.ld1 = ld1; a.c1 = c1;
-    a.in2 = (const __nv_bfloat16*)in2; a.ld2 = ld2; a.c2 = in2 ? c2 : 0;
-    a.dW = dW; a.ci = ci; a.Cp = (ci + 7) / 8 * 8; a.N = (co + 15) / 16 * 16;
+    a.in1 = (const __nv_bfloat16*)in1; a.ld1 = ld1; a.c1 = in2 ? c1 : (ci + 7) / 8 * 8;
+    a.in2 = (const __nv_bfloat16*)(in2 ? in2 : in1); a.ld2 = in2 ? ld2 : ld1;
+    a.dW = dW; a.ci = ci;
     a.nx = nx; a.ny = ny; a.nz = nz; a.xper = xper; a.yper = yper;
+    a.tx = (nx + gmnn::kTileX - 1) / gmnn::kTileX;
+    a.ty = (ny + gmnn::kTileY - 1) / gmnn::kTileY;
     a.status = status;
     a.stall = g_nn_stall;
-    const int tiles = (27 * a.Cp + 127) / 128;
-    if (vchunk == 0) {
-        // about four CTAs per SM over the grid, at least 8 steps each: fewer,
-        // longer CTAs cost fewer accumulator flushes (atomics)
-        int dev = 0, nsm = 152;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        const long long chunks = (4LL * nsm + tiles - 1) / tiles;
-        long long vc = (V + chunks - 1) / chunks;
-        vc = (vc + gmnn::kWgKV - 1) / gmnn::kWgKV * gmnn::kWgKV;
-        vchunk = (int)(vc < 8 * gmnn::kWgKV ? 8 * gmnn::kWgKV : vc);
+    // even slices of at most kWgGroups input groups and kWgN output channels
+    const int ng = (ci + 7) / 8, nslices = (co + gmnn::kWgN - 1) / gmnn::kWgN;
+    a.cslices = (ng + gmnn::kWgGroups - 1) / gmnn::kWgGroups;
+    a.cs = (ng + a.cslices - 1) / a.cslices;
+    a.N = ((co + nslices - 1) / nslices + 15) / 16 * 16;
+    a.ncols = 32;
+    while (a.ncols < 9 * a.N) a.ncols <<= 1;
+    int dev = 0, nsm = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    // planes per block and CTAs along the blocks: one wave; a plane's MMAs take 3300
+    // clocks, a block about 1000 more, its copies 1 clock per 7.5 bytes; vchunk asks for at least that many voxels a CTA.
+    // Chains of lim voxels are those of four CTAs per SM with 128 of the stacked (tap,
+    // channel) rows each; a chain is no longer (the truncation error no larger), and where
+    // the voxels are many no more than 3000 voxels shorter, so that the error is the same
+    // to 1e-5 of the gradient.
+    const long long lim = std::max(512ll, V * ((27 * ng * 8 + 127) / 128) / (4 * nsm));
+    const long long slices = (long long)a.cslices * nslices;
+    double tbest = 0;
+    long long gx = 1;
+    for (int kb = 1; kb <= gmnn::kWgKb && kb <= nz; kb++) {
+        if (gmnn::wgrad_smem(a.cs, kb, a.N) > 227 * 1024) break;
+        const long long blocks = (long long)a.tx * a.ty * ((nz + kb - 1) / kb);
+        long long g = std::max(1ll, std::min(blocks, nsm / slices));
+        if (lim > 3512) g = std::min(g, (V + lim - 3001) / (lim - 3000));
+        if (vchunk > 0) g = std::min(g, (V + vchunk - 1) / vchunk);
+        const double load = gmnn::wg_block_bytes(a.cs, kb, a.N) / 7.5;
+        const double t = load + (double)((blocks + g - 1) / g) * (std::max(3300.0 * kb, load) + 1000);
+        if (tbest == 0 || t < tbest) {
+            tbest = t;
+            gx = g;
+            a.kb = kb;
+            a.blocks = (int)blocks;
+        }
     }
-    a.vchunk = vchunk;
-    const size_t smem = (size_t)gmnn::kWgStages * (128 + a.N) * gmnn::kWgKV * 2 + 8 * (gmnn::kWgStages + 1) + 16;
-    cudaError_t e = cudaFuncSetAttribute(gmnn::k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    a.chain = (int)std::max(1ll, lim / (128 * a.kb));
+    const size_t smem = gmnn::wgrad_smem(a.cs, a.kb, a.N);
+    cudaError_t e = cudaFuncSetAttribute(gmnn::k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return gm::fail(GM_ECUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-    const dim3 grid((unsigned)((V + vchunk - 1) / vchunk), (unsigned)tiles);
-    gmnn::k_conv_wgrad<<<grid, 128, smem, (cudaStream_t)stream>>>(a);
+    gmnn::k_conv_wgrad<<<dim3((unsigned)gx, (unsigned)slices), gmnn::kWgThreads, smem, (cudaStream_t)stream>>>(a);
     e = cudaGetLastError();
     return e == cudaSuccess ? GM_OK : gm::fail(GM_ECUDA, std::string("k_conv_wgrad: ") + cudaGetErrorString(e));
 }

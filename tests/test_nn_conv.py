@@ -82,3 +82,50 @@ def test_conv(case):
     tol = size * (27 * Kc * 2.0 ** -23) + np.abs(ref) * 2.0 ** -8
     assert np.all(np.abs(g - ref) <= tol), np.max(np.abs(g - ref) / tol)
     assert np.all(got[:, co:] == 7.0)          # nothing beyond the output's channels
+
+
+# nx, ny, nz, xper, yper, ci, co, chunk: ragged tiles, blocks of fewer planes at the
+# end, several slices of input and output channels, several blocks a CTA
+WGRAD_CASES = [
+    (17, 33, 9, 1, 1, 20, 20, 0),
+    (9, 16, 5, 0, 1, 44, 100, 0),
+    (24, 31, 7, 1, 0, 96, 49, 4096),
+    (32, 32, 33, 1, 1, 3, 24, 16384),
+    (7, 5, 1, 0, 0, 120, 16, 0),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", WGRAD_CASES, ids=lambda c: "x".join(map(str, c)))
+def test_conv_wgrad(case):
+    import torch
+    from glemur_gb300 import _abi
+    nx, ny, nz, xper, yper, ci, co, chunk = case
+    rng = np.random.default_rng(2)
+    V, ldi, ldo = nx * ny * nz, (ci + 7) // 8 * 8 + 8, (co + 7) // 8 * 8
+    bf = lambda a: torch.tensor(a, dtype=torch.float32, device="cuda").to(torch.bfloat16)  # noqa: E731
+    x, d = bf(rng.normal(size=(V, ldi))), bf(rng.normal(size=(V, ldo)))
+    dW = torch.zeros(27, co, ci, device="cuda")
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    torch.cuda.synchronize()
+    lib = _abi.load()
+    _abi.check(lib.gm_nn_conv_wgrad(P(d), ldo, co, P(x), ldi, ldi, None, 0, 0, C.cast(dW.data_ptr(), C.POINTER(C.c_float)),
+                                    ci, nx, ny, nz, xper, yper, chunk, P(st), None), "gm_nn_conv_wgrad")
+    torch.cuda.synchronize()
+    assert int(st[0]) == 0
+    xs = x.double().cpu().numpy()[:, :ci].reshape(nz, ny, nx, ci).transpose(2, 1, 0, 3)
+    ds = d.double().cpu().numpy()[:, :co].reshape(nz, ny, nx, co).transpose(2, 1, 0, 3).reshape(V, co)
+    xp = np.zeros((nx + 2, ny + 2, nz + 2, ci))
+    xp[1:-1, 1:-1, 1:-1] = xs
+    if xper:
+        xp[0], xp[-1] = xp[-2], xp[1]
+    if yper:
+        xp[:, 0], xp[:, -1] = xp[:, -2], xp[:, 1]
+    got = dW.double().cpu().numpy()
+    for t in range(27):
+        dk, dj, di = t // 9, t // 3 % 3, t % 3
+        v = xp[di:di + nx, dj:dj + ny, dk:dk + nz].reshape(V, ci)
+        ref, size = ds.T @ v, np.abs(ds).T @ np.abs(v)
+        # an FP32 sum of V exact products: each addition off by at most an ulp of the sum of magnitudes
+        assert np.all(np.abs(got[t] - ref) <= size * V * 2.0 ** -23), t
