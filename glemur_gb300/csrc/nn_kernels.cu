@@ -990,46 +990,113 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const WgradArgs a) {
     if (warp == 0) tmem_free(tbase, a.ncols);
 }
 
-// Sum over voxels of an upstream gradient per channel (bias gradient).
-__global__ void k_bias_grad(const __nv_bfloat16* __restrict__ d, int ld, int c, long long V, float* __restrict__ db) {
-    __shared__ float red[256];
-    const int ch = blockIdx.y;
-    float s = 0.f;
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x)
-        s += __bfloat162float(d[v * ld + ch]);
-    red[threadIdx.x] = s;
+// The passes below move each value once: they take W channels of a voxel at a time,
+// 8 (16 bytes) where the views start on 16 bytes with strides and channel counts that
+// are multiples of 8, else 1.  One channel a thread, with a division for each, they
+// took 480 us of a training step at 64x64x128, 8 take 260.
+template <int W>
+struct Chan;
+template <>
+struct Chan<1> {
+    __nv_bfloat16 v[1];
+    __device__ static Chan load(const __nv_bfloat16* p) { return Chan{{*p}}; }
+    __device__ void store(__nv_bfloat16* p) const { *p = v[0]; }
+};
+template <>
+struct alignas(16) Chan<8> {
+    __nv_bfloat16 v[8];
+    __device__ static Chan load(const __nv_bfloat16* p) {
+        Chan r;
+        *reinterpret_cast<uint4*>(r.v) = *reinterpret_cast<const uint4*>(p);
+        return r;
+    }
+    __device__ void store(__nv_bfloat16* p) const { *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(v); }
+};
+static bool by8(const void* p, int ld, int c) { return !(reinterpret_cast<uintptr_t>(p) & 15) && ld % 8 == 0 && c % 8 == 0; }
+
+// Sum over voxels of an upstream gradient per channel (bias gradient).  A thread
+// keeps its W channels (n = kBiasThreads W / c voxels a block at a time); blockIdx.y
+// picks the channels where c / W exceeds a block.  Few large blocks: what 300 blocks of
+// 256 threads took (16 us) were additions to the same addresses.
+constexpr int kBiasThreads = 1024;
+template <int W>
+__global__ void __launch_bounds__(kBiasThreads) k_bias_grad(const __nv_bfloat16* __restrict__ d, int ld, int c, long long V, float* __restrict__ db) {
+    __shared__ float red[kBiasThreads][W + 1];
+    const int groups = min(c / W - kBiasThreads * (int)blockIdx.y, kBiasThreads), n = kBiasThreads / groups;
+    const int r = (int)threadIdx.x / groups, c0 = (kBiasThreads * blockIdx.y + threadIdx.x % groups) * W;
+    float s[W] = {};
+    if (r < n)
+#pragma unroll 4
+        for (long long v = (long long)blockIdx.x * n + r; v < V; v += (long long)gridDim.x * n) {
+            const Chan<W> x = Chan<W>::load(d + v * ld + c0);
+#pragma unroll
+            for (int q = 0; q < W; q++) s[q] += __bfloat162float(x.v[q]);
+        }
+#pragma unroll
+    for (int q = 0; q < W; q++) red[threadIdx.x][q] = s[q];
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+    for (int m = n; m > 1;) {
+        const int h = (m + 1) / 2;
+        if (r + h < m)
+#pragma unroll
+            for (int q = 0; q < W; q++) red[threadIdx.x][q] += red[threadIdx.x + h * groups][q];
+        m = h;
         __syncthreads();
     }
-    if (threadIdx.x == 0) atomicAdd(&db[ch], red[0]);
+    if (r == 0)
+#pragma unroll
+        for (int q = 0; q < W; q++) atomicAdd(&db[c0 + q], red[threadIdx.x][q]);
 }
+
+// The 8 children of the coarse voxel of index q / groups, and its W channels
+// (q % groups) W.  Ix is unsigned where the indexes fit 31 bits.
+template <class Ix>
+struct Children {
+    int ch;
+    long long vc, vf[8];
+    __device__ Children(Ix q, int groups, int W, int nx, int ny) {
+        const Ix v = q / (Ix)groups, cx = nx / 2, cy = ny / 2;
+        ch = (int)(q - v * groups) * W;
+        vc = v;
+        const Ix t = v / cx, i = v - t * cx, k = t / cy, j = t - k * cy;
+#pragma unroll
+        for (int d = 0; d < 8; d++)
+            vf[d] = (long long)(2 * i + (d & 1)) + (long long)nx * ((long long)(2 * j + ((d >> 1) & 1)) + (long long)ny * (long long)(2 * k + (d >> 2)));
+    }
+};
 
 // 2x2x2 average pooling (forward) and its adjoint (backward: each child gets
 // 1/8 of the parent's gradient).  Fine grid (nx, ny, nz), coarse (nx/2, ...).
+template <int W, class Ix>
 __global__ void k_pool(const __nv_bfloat16* __restrict__ in, int ldi, __nv_bfloat16* __restrict__ out, int ldo, int c,
                        int nx, int ny, int nz, int backward, int accumulate) {
-    const int cx = nx / 2, cy = ny / 2, cz = nz / 2;
-    const long long Vc = (long long)cx * cy * cz;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < Vc * c; q += (long long)gridDim.x * blockDim.x) {
-        const int ch = (int)(q % c);
-        const long long vc = q / c;
-        const int i = (int)(vc % cx), j = (int)((vc / cx) % cy), k = (int)(vc / ((long long)cx * cy));
+    const Ix n = (Ix)((long long)(nx / 2) * (ny / 2) * (nz / 2) * (c / W));
+    for (Ix q = (Ix)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (Ix)gridDim.x * blockDim.x) {
+        const Children<Ix> f(q, c / W, W, nx, ny);
         if (!backward) {
-            float s = 0.f;
+            float s[W] = {};
+#pragma unroll
             for (int d = 0; d < 8; d++) {
-                const long long vf = (2 * i + (d & 1)) + (long long)nx * ((2 * j + ((d >> 1) & 1)) + (long long)ny * (2 * k + (d >> 2)));
-                s += __bfloat162float(in[vf * ldi + ch]);
+                const Chan<W> x = Chan<W>::load(in + f.vf[d] * ldi + f.ch);
+#pragma unroll
+                for (int w = 0; w < W; w++) s[w] += __bfloat162float(x.v[w]);
             }
-            out[vc * ldo + ch] = __float2bfloat16_rn(0.125f * s);
+            Chan<W> y;
+#pragma unroll
+            for (int w = 0; w < W; w++) y.v[w] = __float2bfloat16_rn(0.125f * s[w]);
+            y.store(out + f.vc * ldo + f.ch);
         } else {
             // in = coarse gradient, out = fine gradient
-            const float g = 0.125f * __bfloat162float(in[vc * ldi + ch]);
+            const Chan<W> g = Chan<W>::load(in + f.vc * ldi + f.ch);
+#pragma unroll
             for (int d = 0; d < 8; d++) {
-                const long long vf = (2 * i + (d & 1)) + (long long)nx * ((2 * j + ((d >> 1) & 1)) + (long long)ny * (2 * k + (d >> 2)));
-                const float o = accumulate ? __bfloat162float(out[vf * ldo + ch]) : 0.f;
-                out[vf * ldo + ch] = __float2bfloat16_rn(o + g);
+                __nv_bfloat16* o = out + f.vf[d] * ldo + f.ch;
+                Chan<W> y{};
+                if (accumulate) y = Chan<W>::load(o);
+#pragma unroll
+                for (int w = 0; w < W; w++)
+                    y.v[w] = __float2bfloat16_rn((accumulate ? __bfloat162float(y.v[w]) : 0.f) + 0.125f * __bfloat162float(g.v[w]));
+                y.store(o);
             }
         }
     }
@@ -1037,39 +1104,46 @@ __global__ void k_pool(const __nv_bfloat16* __restrict__ in, int ldi, __nv_bfloa
 
 // Nearest-neighbour 2x upsampling (forward) and its adjoint (backward: the sum
 // of the 8 children).  Coarse grid (nx/2, ...), fine (nx, ny, nz).
+template <int W, class Ix>
 __global__ void k_upsample(const __nv_bfloat16* __restrict__ in, int ldi, __nv_bfloat16* __restrict__ out, int ldo,
                            int c, int nx, int ny, int nz, int backward) {
-    const int cx = nx / 2, cy = ny / 2, cz = nz / 2;
-    const long long Vc = (long long)cx * cy * cz;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < Vc * c; q += (long long)gridDim.x * blockDim.x) {
-        const int ch = (int)(q % c);
-        const long long vc = q / c;
-        const int i = (int)(vc % cx), j = (int)((vc / cx) % cy), k = (int)(vc / ((long long)cx * cy));
+    const Ix n = (Ix)((long long)(nx / 2) * (ny / 2) * (nz / 2) * (c / W));
+    for (Ix q = (Ix)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (Ix)gridDim.x * blockDim.x) {
+        const Children<Ix> f(q, c / W, W, nx, ny);
         if (!backward) {
-            const __nv_bfloat16 x = in[vc * ldi + ch];
-            for (int d = 0; d < 8; d++) {
-                const long long vf = (2 * i + (d & 1)) + (long long)nx * ((2 * j + ((d >> 1) & 1)) + (long long)ny * (2 * k + (d >> 2)));
-                out[vf * ldo + ch] = x;
-            }
+            const Chan<W> x = Chan<W>::load(in + f.vc * ldi + f.ch);
+#pragma unroll
+            for (int d = 0; d < 8; d++) x.store(out + f.vf[d] * ldo + f.ch);
         } else {
             // in = fine gradient, out = coarse gradient
-            float s = 0.f;
+            float s[W] = {};
+#pragma unroll
             for (int d = 0; d < 8; d++) {
-                const long long vf = (2 * i + (d & 1)) + (long long)nx * ((2 * j + ((d >> 1) & 1)) + (long long)ny * (2 * k + (d >> 2)));
-                s += __bfloat162float(in[vf * ldi + ch]);
+                const Chan<W> x = Chan<W>::load(in + f.vf[d] * ldi + f.ch);
+#pragma unroll
+                for (int w = 0; w < W; w++) s[w] += __bfloat162float(x.v[w]);
             }
-            out[vc * ldo + ch] = __float2bfloat16_rn(s);
+            Chan<W> y;
+#pragma unroll
+            for (int w = 0; w < W; w++) y.v[w] = __float2bfloat16_rn(s[w]);
+            y.store(out + f.vc * ldo + f.ch);
         }
     }
 }
 
 // d *= (y > 0): the gradient through a ReLU from its output.
+template <int W, class Ix>
 __global__ void k_relu_bwd(__nv_bfloat16* __restrict__ d, int ldd, const __nv_bfloat16* __restrict__ y, int ldy, int c,
                            long long V) {
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < V * c; q += (long long)gridDim.x * blockDim.x) {
-        const long long v = q / c;
-        const int ch = (int)(q % c);
-        if (!(__bfloat162float(y[v * ldy + ch]) > 0.f)) d[v * ldd + ch] = __float2bfloat16_rn(0.f);
+    const Ix groups = c / W, n = (Ix)(V * (c / W));
+    for (Ix q = (Ix)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (Ix)gridDim.x * blockDim.x) {
+        const Ix v = q / groups, ch = (q - v * groups) * W;
+        const Chan<W> x = Chan<W>::load(y + (long long)v * ldy + ch);
+        Chan<W> g = Chan<W>::load(d + (long long)v * ldd + ch);
+#pragma unroll
+        for (int w = 0; w < W; w++)
+            if (!(__bfloat162float(x.v[w]) > 0.f)) g.v[w] = __float2bfloat16_rn(0.f);
+        g.store(d + (long long)v * ldd + ch);
     }
 }
 
@@ -1526,8 +1600,11 @@ int gm_nn_conv_wgrad(const void* dout, int ldd, int co, const void* in1, int ld1
 }
 
 int gm_nn_bias_grad(const void* d, int ld, int c, long long V, float* db, void* stream) {
-    gmnn::k_bias_grad<<<dim3(gmnn::nb(V) > 64 ? 64 : gmnn::nb(V), c), 256, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)d, ld, c, V, db);
+    const bool w8 = gmnn::by8(d, ld, c);
+    const int groups = w8 ? c / 8 : c, n = gmnn::kBiasThreads / std::max(1, std::min(groups, gmnn::kBiasThreads));
+    const dim3 grid((unsigned)std::max(1ll, std::min((V + 4 * n - 1) / (4 * n), 152ll)), (unsigned)((groups + gmnn::kBiasThreads - 1) / gmnn::kBiasThreads));
+    auto kern = w8 ? gmnn::k_bias_grad<8> : gmnn::k_bias_grad<1>;
+    kern<<<grid, gmnn::kBiasThreads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)d, ld, c, V, db);
     return cudaGetLastError() == cudaSuccess ? GM_OK : gm::fail(GM_ECUDA, "k_bias_grad");
 }
 
@@ -1535,8 +1612,10 @@ int gm_nn_pool(const void* in, int ldi, void* out, int ldo, int c, int nx, int n
                int accumulate, void* stream) {
     if (nx % 2 || ny % 2 || nz % 2) return gm::fail(GM_EPARAM, "gm_nn_pool: grid sizes must be even");
     const long long n = (long long)(nx / 2) * (ny / 2) * (nz / 2) * c;
-    gmnn::k_pool<<<gmnn::nb(n), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, ldi, (__nv_bfloat16*)out,
-                                                                 ldo, c, nx, ny, nz, backward, accumulate);
+    const bool w8 = gmnn::by8(in, ldi, c) && gmnn::by8(out, ldo, c) && n / 8 < (1ll << 31);
+    auto kern = w8 ? gmnn::k_pool<8, unsigned> : n < (1ll << 31) ? gmnn::k_pool<1, unsigned> : gmnn::k_pool<1, long long>;
+    kern<<<gmnn::nb(w8 ? n / 8 : n), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, ldi, (__nv_bfloat16*)out, ldo, c,
+                                                                     nx, ny, nz, backward, accumulate);
     return cudaGetLastError() == cudaSuccess ? GM_OK : gm::fail(GM_ECUDA, "k_pool");
 }
 
@@ -1544,8 +1623,10 @@ int gm_nn_upsample(const void* in, int ldi, void* out, int ldo, int c, int nx, i
                    void* stream) {
     if (nx % 2 || ny % 2 || nz % 2) return gm::fail(GM_EPARAM, "gm_nn_upsample: grid sizes must be even");
     const long long n = (long long)(nx / 2) * (ny / 2) * (nz / 2) * c;
-    gmnn::k_upsample<<<gmnn::nb(n), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, ldi,
-                                                                     (__nv_bfloat16*)out, ldo, c, nx, ny, nz, backward);
+    const bool w8 = gmnn::by8(in, ldi, c) && gmnn::by8(out, ldo, c) && n / 8 < (1ll << 31);
+    auto kern = w8 ? gmnn::k_upsample<8, unsigned> : n < (1ll << 31) ? gmnn::k_upsample<1, unsigned> : gmnn::k_upsample<1, long long>;
+    kern<<<gmnn::nb(w8 ? n / 8 : n), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, ldi, (__nv_bfloat16*)out, ldo, c,
+                                                                     nx, ny, nz, backward);
     return cudaGetLastError() == cudaSuccess ? GM_OK : gm::fail(GM_ECUDA, "k_upsample");
 }
 
@@ -1604,8 +1685,9 @@ int gm_nn_zero(void* p, size_t bytes, void* stream) {
 }
 
 int gm_nn_relu_bwd(void* d, int ldd, const void* y, int ldy, int c, long long V, void* stream) {
-    gmnn::k_relu_bwd<<<gmnn::nb(V * c), 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)d, ldd,
-                                                                         (const __nv_bfloat16*)y, ldy, c, V);
+    const bool w8 = gmnn::by8(d, ldd, c) && gmnn::by8(y, ldy, c) && V * (c / 8) < (1ll << 31);
+    auto kern = w8 ? gmnn::k_relu_bwd<8, unsigned> : V * c < (1ll << 31) ? gmnn::k_relu_bwd<1, unsigned> : gmnn::k_relu_bwd<1, long long>;
+    kern<<<gmnn::nb(w8 ? V * (c / 8) : V * c), 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)d, ldd, (const __nv_bfloat16*)y, ldy, c, V);
     return cudaGetLastError() == cudaSuccess ? GM_OK : gm::fail(GM_ECUDA, "k_relu_bwd");
 }
 

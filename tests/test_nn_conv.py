@@ -129,3 +129,57 @@ def test_conv_wgrad(case):
         ref, size = ds.T @ v, np.abs(ds).T @ np.abs(v)
         # an FP32 sum of V exact products: each addition off by at most an ulp of the sum of magnitudes
         assert np.all(np.abs(got[t] - ref) <= size * V * 2.0 ** -23), t
+
+
+# channels, channel stride: 16-byte rows of whole groups of 8, and what falls short of that
+PASSES = [(24, 24), (48, 72), (3, 8), (20, 24), (8, 9), (264, 264), (1030, 1030)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("c,ld", PASSES)
+def test_elementwise_passes(c, ld):
+    """Pooling, upsampling, ReLU and bias gradients: one rounding to BF16 of FP32 sums of at most 9
+    terms, and an FP32 sum over the voxels."""
+    import torch
+    from glemur_gb300 import _abi
+    lib = _abi.load()
+    nx, ny, nz = 6, 10, 4
+    V, Vc = nx * ny * nz, nx * ny * nz // 8
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda n: torch.randn(n, ld, device="cuda", generator=g).to(torch.bfloat16)  # noqa: E731
+    P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    fine, coarse, y = r(V), r(Vc), r(V)
+
+    def blocks(t):           # [Vc, 8, ld]
+        return t.view(nz // 2, 2, ny // 2, 2, nx // 2, 2, ld).permute(0, 2, 4, 1, 3, 5, 6).reshape(Vc, 8, ld)
+
+    def same(got, want, before):
+        tol = want.abs() * 2.0 ** -8 + 1e-6
+        assert bool(((got[..., :c].double() - want[..., :c]).abs() <= tol[..., :c]).all())
+        assert torch.equal(got[..., c:], before[..., c:])
+
+    def run(name, *a):
+        _abi.check(getattr(lib, name)(*a, None), name)
+        torch.cuda.synchronize()
+
+    torch.cuda.synchronize()
+    o = coarse.clone()
+    run("gm_nn_pool", P(fine), ld, P(o), ld, c, nx, ny, nz, 0, 0)
+    same(o, blocks(fine).double().mean(1), coarse)
+    for acc in (0, 1):
+        o = fine.clone()
+        run("gm_nn_pool", P(coarse), ld, P(o), ld, c, nx, ny, nz, 1, acc)
+        same(blocks(o), acc * blocks(fine).double() + coarse.double()[:, None] / 8, blocks(fine))
+    o = fine.clone()
+    run("gm_nn_upsample", P(coarse), ld, P(o), ld, c, nx, ny, nz, 0)
+    same(blocks(o), coarse.double()[:, None].expand(-1, 8, -1), blocks(fine))
+    o = coarse.clone()
+    run("gm_nn_upsample", P(fine), ld, P(o), ld, c, nx, ny, nz, 1)
+    same(o, blocks(fine).double().sum(1), coarse)
+    o = fine.clone()
+    run("gm_nn_relu_bwd", P(o), ld, P(y), ld, c, V)
+    same(o, torch.where(y > 0, fine, torch.zeros_like(fine)).double(), fine)
+    db = torch.ones(c + 1, device="cuda")
+    run("gm_nn_bias_grad", P(fine), ld, c, V, C.cast(db.data_ptr(), C.POINTER(C.c_float)))
+    size = fine.double().abs().sum(0)[:c] + 1
+    assert bool(((db[:c].double() - 1 - fine.double().sum(0)[:c]).abs() <= size * V * 2.0 ** -23).all()) and float(db[c]) == 1
