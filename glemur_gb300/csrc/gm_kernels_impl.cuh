@@ -802,9 +802,11 @@ __global__ void __launch_bounds__(256) k_stage(const __grid_constant__ StageArgs
     }
 }
 
-// Accept/reject and the dt rule, src/main.cu:321-383, on the device.
+// Accept/reject and the dt rule, src/main.cu:321-383, on the device.  The state is
+// read at once and written at once: field by field, each waited for the one before it.
 template <typename T>
-__device__ __forceinline__ void control_one(const KP<T>& p, DevState* st, double* log) {
+__device__ __forceinline__ void control_one(const KP<T>& p, DevState* state, double* log) {
+    DevState v = *state, *st = &v;
     if (st->done) return;
     if (st->status & (GM_ST_TIMEOUT | GM_ST_ALIGN)) {
         // a stage of this step gave up a bounded wait or failed its alignment
@@ -817,6 +819,7 @@ __device__ __forceinline__ void control_one(const KP<T>& p, DevState* st, double
         st->event = 0;
         st->done = 1;
         st->status |= GM_ST_DONE;
+        *state = v;
         return;
     }
     const double md = __longlong_as_double((long long)st->maxDeltaBits);
@@ -868,6 +871,7 @@ __device__ __forceinline__ void control_one(const KP<T>& p, DevState* st, double
         st->status |= GM_ST_EVENT;
     }
     if (st->done) st->status |= GM_ST_DONE;
+    *state = v;
 }
 
 template <typename T>
