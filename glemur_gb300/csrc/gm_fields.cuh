@@ -94,6 +94,8 @@ __device__ __forceinline__ void b_plain(const KP<T>& p, const GlobalX<T>& X, con
 template <typename T, bool OUT>
 __global__ void __launch_bounds__(field_threads<T>()) k_b_field(const __grid_constant__ StageArgs<T> a, int always) {
     const KP<T>& p = a.p;
+    after_previous();
+    let_next();
     if (!always && a.st->done) return;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const unsigned q = blockIdx.x * (unsigned)field_threads<T>() + threadIdx.x, N = (unsigned)p.N;
@@ -196,6 +198,8 @@ template <typename T, bool PRESS, bool INERTIA, bool JOUT, bool LAST>
 __global__ void __launch_bounds__(field_threads<T>()) k_stage_field(const __grid_constant__ StageArgs<T> a) {
     const KP<T>& p = a.p;
     DevState* st = a.st;
+    after_previous();
+    let_next();
     if (st->done) return;
     const int nx = p.nx, ny = p.ny, n = a.n, cur = st->cur;
     const unsigned q = blockIdx.x * (unsigned)field_threads<T>() + threadIdx.x;
@@ -433,6 +437,8 @@ __device__ __forceinline__ void cross_add(const T a[3], const T b[3], T c[3]) {
 template <typename T>
 __global__ void __launch_bounds__(field_threads<T>()) k_j_oct(const __grid_constant__ StageArgs<T> a, int always) {
     const KP<T>& p = a.p;
+    after_previous();
+    let_next();
     if (!always && a.st->done) return;
     const int nx = p.nx, ny = p.ny;
     const unsigned q = blockIdx.x * (unsigned)field_threads<T>() + threadIdx.x;
@@ -652,6 +658,8 @@ __device__ __noinline__ void j_quint_point(const KP<T>& p, const T* __restrict__
 template <typename T>
 __global__ void __launch_bounds__(field_threads<T>()) k_j_quint(const __grid_constant__ StageArgs<T> a, int always) {
     const KP<T>& p = a.p;
+    after_previous();
+    let_next();
     if (!always && a.st->done) return;
     const int nx = p.nx, ny = p.ny;
     const unsigned q = blockIdx.x * (unsigned)field_threads<T>() + threadIdx.x;
@@ -961,18 +969,14 @@ cudaError_t launch_b_field(const StageArgs<T>& a, int out, int always, cudaStrea
     const long long n = a.p.N + 2ll * ((long long)a.p.ny * a.p.nz + (long long)a.p.nx * a.p.nz + (long long)a.p.nx * a.p.ny);
     const int t = field_threads<T>();
     const unsigned nb = (unsigned)((n + t - 1) / t);
-    if (out) k_b_field<T, true><<<nb, t, 0, s>>>(a, always);
-    else k_b_field<T, false><<<nb, t, 0, s>>>(a, always);
-    return cudaGetLastError();
+    return launch_next(out ? k_b_field<T, true> : k_b_field<T, false>, nb, t, 0, s, a, always);
 }
 
 template <typename T>
 cudaError_t launch_j_own(const StageArgs<T>& a, int always, cudaStream_t s) {
     const int t = field_threads<T>();
     const unsigned nb = (unsigned)((a.p.N + t - 1) / t);
-    if (a.p.jOct) k_j_oct<T><<<nb, t, 0, s>>>(a, always);
-    else k_j_quint<T><<<nb, t, 0, s>>>(a, always);
-    return cudaGetLastError();
+    return launch_next(a.p.jOct ? k_j_oct<T> : k_j_quint<T>, nb, t, 0, s, a, always);
 }
 
 template <typename T>
@@ -980,19 +984,19 @@ cudaError_t launch_stage_field(const StageArgs<T>& a, int pressure, int jout, cu
     const int t = field_threads<T>();
     const unsigned nb = (unsigned)((a.p.N + t - 1) / t);
     auto by = [](int v, auto f) { v ? f(std::true_type()) : f(std::false_type()); };
-    bool known = true;
+    cudaError_t rc = cudaErrorInvalidValue;
     by(pressure, [&](auto P) {
         by(a.p.inertia, [&](auto I) {
             by(jout, [&](auto J) {
                 by(a.n == 5, [&](auto L) {
                     // FP32 frictional Stokes stages run in the tile kernel
-                    if constexpr (sizeof(T) == 4 && !I.value && !J.value) known = false;
-                    else k_stage_field<T, P.value, I.value, J.value, L.value><<<nb, t, 0, s>>>(a);
+                    if constexpr (sizeof(T) == 8 || I.value || J.value)
+                        rc = launch_next(k_stage_field<T, P.value, I.value, J.value, L.value>, nb, t, 0, s, a);
                 });
             });
         });
     });
-    return known ? cudaGetLastError() : cudaErrorInvalidValue;
+    return rc;
 }
 
 #define GMK_INSTANTIATE_FIELDS(T)                                                       \

@@ -32,6 +32,34 @@
 
 namespace gmk {
 
+// Programmatic dependent launch of the field passes and the controller of a step: each
+// is launched when every CTA of the one before it has started or ended, so its launch
+// runs during that kernel, and waits (after_previous, in every thread before anything
+// that a kernel writes or reads) until that one has completed and its writes are
+// visible.  A kernel completes after its own wait, so the order holds through the
+// chain.  32x32x64 in FP64 140 -> 136 us a step, 64x64x128 FP32 with inertia 296 ->
+// 291.  The tile kernel's stages are launched plainly: early CTAs wait in the slots
+// that the running ones' balance needs (97x75x133 line-tied 210 -> 245 us a step, and
+// 32x32x32 74 -> 76).
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
+
 constexpr int TX = 32;          // tile width in x = one warp
 constexpr int XRING = 5;        // planes of positions held in shared memory
 constexpr int BRING = 4;        // planes of B held in shared memory
