@@ -714,15 +714,12 @@ struct Impl : ImplBase {
     }
 
     int set_dt(double t, double dt, int timeIndex) override {
-        int rc = read_state();
-        if (rc) return rc;
-        h_st->t = gp.errMode == 0 ? (double)(T)t : t;
-        h_st->dt = gp.errMode == 0 ? (double)(T)dt : dt;
-        h_st->timeIndex = timeIndex;
-        h_st->done = !(h_st->dt > kp.dtMin);
+        // in stream order: reading the state, changing it and writing it back was two
+        // synchronisations (25 us of a 72 us step of 32x32x32)
+        const double d = gp.errMode == 0 ? (double)(T)dt : dt;
         ev_base = -1;
-        CUDA_TRY(cudaMemcpyAsync(st, h_st, sizeof(DevState), cudaMemcpyHostToDevice, stream));
-        CUDA_TRY(cudaStreamSynchronize(stream));
+        CUDA_TRY(gmk::launch_set_time<T>(st, gp.errMode == 0 ? (double)(T)t : t, d, timeIndex, !(d > kp.dtMin), stream));
+        launches++;
         return GM_OK;
     }
 

@@ -189,6 +189,8 @@ int stage_occupancy(int TY, int pressure, size_t smem);
 template <typename T>
 cudaError_t launch_control(const KP<T>& p, DevState* st, double* log, cudaStream_t s);
 template <typename T>
+cudaError_t launch_set_time(DevState* st, double t, double dt, int timeIndex, int done, cudaStream_t s);
+template <typename T>
 cudaError_t launch_finalize(const double* part, int nparts, double* out, cudaStream_t s);
 // ghosted AoS (reference layout) <-> padded SoA
 template <typename T>

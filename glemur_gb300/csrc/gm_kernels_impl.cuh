@@ -874,6 +874,14 @@ __device__ __forceinline__ void control_one(const KP<T>& p, DevState* state, dou
     *state = v;
 }
 
+// gm_set_dt on the device.
+static __global__ void k_set_time(DevState* st, double t, double dt, int timeIndex, int done) {
+    st->t = t;
+    st->dt = dt;
+    st->timeIndex = timeIndex;
+    st->done = done;
+}
+
 template <typename T>
 __global__ void k_control(const __grid_constant__ KP<T> p, DevState* st, double* log) {
     control_one<T>(p, st, log);
@@ -1222,6 +1230,12 @@ cudaError_t launch_control(const KP<T>& p, DevState* st, double* log, cudaStream
 }
 
 template <typename T>
+cudaError_t launch_set_time(DevState* st, double t, double dt, int timeIndex, int done, cudaStream_t s) {
+    k_set_time<<<1, 1, 0, s>>>(st, t, dt, timeIndex, done);
+    return cudaGetLastError();
+}
+
+template <typename T>
 cudaError_t launch_control_batch(const StageArgsTMA<T>* cases, int ncases, int* counters, cudaStream_t s) {
     const int n = ncases > 6 ? ncases : 6;
     k_control_batch<T><<<(n + 127) / 128, 128, 0, s>>>(cases, ncases, counters);
@@ -1316,6 +1330,7 @@ cudaError_t launch_eps_star(const KP<T>& p, const T* B, const T* J, const T* X, 
     template cudaError_t prepare_kernels<T>();                                                                    \
     template int stage_occupancy<T>(int, int, size_t);                                                            \
     template cudaError_t launch_control<T>(const KP<T>&, DevState*, double*, cudaStream_t);                       \
+    template cudaError_t launch_set_time<T>(DevState*, double, double, int, int, cudaStream_t);                    \
     template cudaError_t launch_control_batch<T>(const StageArgsTMA<T>*, int, int*, cudaStream_t);                \
     template cudaError_t launch_finalize<T>(const double*, int, double*, cudaStream_t);                           \
     template cudaError_t launch_unpack<T>(const KP<T>&, const T*, T*, cudaStream_t);                              \

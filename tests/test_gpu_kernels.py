@@ -194,3 +194,29 @@ def test_reductions_match_numpy_in_64_bits(shape, peri, scale, precision):
                 faces.append(D[tuple(ix)])
     assert r["minDetJac"] == min(v.min() for v in faces)
     g.close()
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+def test_set_time_in_stream_order(precision):
+    """Between steps in flight: the state is changed where the call stands, what it
+    does not name is kept, and a step size at the lower bound stops the steps."""
+    p, x, B0 = case((20, 18, 22), (1, 1, 0), precision)
+    g, h = Relaxation(p), Relaxation(p)
+    for q in (g, h):
+        q.upload(x, B0, 0.0, 1e-3)
+    for _ in range(3):
+        g.steps_async(1)
+        g.set_time(0.5, 2e-3, 7)
+    for _ in range(3):
+        h.steps_async(1)
+        n = h.state()["nAttempted"]
+        h.set_time(0.5, 2e-3, 7)
+        assert h.state()["nAttempted"] == n
+    np.testing.assert_array_equal(g.grid(), h.grid())
+    s, dt = g.state(), p.rnd(2e-3) if p.errMode == 0 else 2e-3      # errMode 0 keeps t and dt in REAL
+    assert (s["t"], s["dt"], s["timeIndex"]) == (0.5, dt, 7) and s["nAttempted"] == 3
+    g.set_time(0.5, p.dtMin)
+    g.steps_async(2)
+    assert g.state()["nAttempted"] == 3
+    for q in (g, h):
+        q.close()
