@@ -467,11 +467,8 @@ struct Impl : ImplBase {
         CUDA_TRY(cudaMemcpyAsync(outB, stage_buf, bytes, cudaMemcpyDeviceToDevice, stream));   // main.cu:195
         CUDA_TRY(cudaMemcpyAsync(stage_buf, xb, bytes, cudaMemcpyDefault, stream));
         T* bufs[4] = {X[0], X[1], XS[0], XS[1]};
-        for (T* b : bufs) {
-            CUDA_TRY(gmk::launch_unpack<T>(kp, stage_buf, b, stream));
-            CUDA_TRY(gmk::launch_images<T>(kp, b, stream));
-        }
-        launches += 10;
+        CUDA_TRY(gmk::launch_unpack_grid<T>(kp, stage_buf, bufs, stream));
+        launches += 3;
         if (kp.shear) {
             // the line-tied z ghost planes of the uploaded grid, with addDist
             CUDA_TRY(gmk::launch_shear_table<T>(kp, X[0], shear_tab, stream));

@@ -198,7 +198,7 @@ cudaError_t launch_unpack(const KP<T>& p, const T* aos, T* soa, cudaStream_t s);
 template <typename T>
 cudaError_t launch_pack(const KP<T>& p, const T* soa, T* aos, cudaStream_t s);
 template <typename T>
-cudaError_t launch_images(const KP<T>& p, T* soa, cudaStream_t s);
+cudaError_t launch_unpack_grid(const KP<T>& p, const T* aos, T* const grids[4], cudaStream_t s);
 template <typename T>
 cudaError_t launch_scale_b0(const KP<T>& p, const T* B0, T* B0s, cudaStream_t s);
 template <typename T>

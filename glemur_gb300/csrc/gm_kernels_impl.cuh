@@ -929,32 +929,42 @@ __global__ void k_unpack(const KP<T> p, const T* __restrict__ aos, T* __restrict
     }
 }
 
-// Depth-2 periodic images of the inner points (the depth-1 ghost layer keeps
-// the values the caller supplied, as the reference's first stage sees them).
+// The uploaded grid (ghosted AoS) into the four padded grids of a handle: every
+// ghosted point as supplied, and the depth-2 periodic images of the inner points (the
+// depth-1 ghost layer keeps the values the caller supplied, as the reference's first
+// stage sees them); other padded points are left.  One pass in place of an unpacking
+// and an imaging one per grid, each with two 64-bit divisions a point (256x256x512:
+// 2.0 ms; now 0.4).  Rows of x by threadIdx.y.
 template <typename T>
-__global__ void k_images(const KP<T> p, T* __restrict__ soa) {
-    const long long NP = (long long)(p.nx + 4) * (p.ny + 4) * (p.nz + 4);
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < NP; q += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(q % (p.nx + 4)) - 2;
-        const long long r = q / (p.nx + 4);
-        const int j = (int)(r % (p.ny + 4)) - 2;
-        const int k = (int)(r / (p.ny + 4)) - 2;
-        const bool xo = i < 0 || i >= p.nx, yo = j < 0 || j >= p.ny, zo = k < 0 || k >= p.nz;
-        if (!(xo || yo || zo)) continue;
-        if ((xo && !p.xPeri) || (yo && !p.yPeri) || (zo && !p.zPeri)) continue;
-        const bool depth2 = (i == -2 || i == p.nx + 1) || (j == -2 || j == p.ny + 1) || (k == -2 || k == p.nz + 1);
-        if (!depth2) continue;
-        const int wi = xo ? (i < 0 ? i + p.nx : i - p.nx) : i;
-        const int wj = yo ? (j < 0 ? j + p.ny : j - p.ny) : j;
-        const int wk = zo ? (k < 0 ? k + p.nz : k - p.nz) : k;
-        const long long gs = gidx(p.px, p.py, wi, wj, wk), gd = gidx(p.px, p.py, i, j, k);
-        T v0 = soa[gs], v1 = soa[p.cs + gs], v2 = soa[2 * p.cs + gs];
-        if (xo) v0 = i < 0 ? (v0 - p.Lx) - p.dx : (v0 + p.Lx) + p.dx;
-        if (yo) v1 = j < 0 ? (v1 - p.Ly) - p.dy : (v1 + p.Ly) + p.dy;
-        if (zo) v2 = k < 0 ? (v2 - p.Lz) - p.dz : (v2 + p.Lz) + p.dz;
-        soa[gd] = v0;
-        soa[p.cs + gd] = v1;
-        soa[2 * p.cs + gd] = v2;
+__global__ void __launch_bounds__(256) k_unpack_grid(const KP<T> p, const T* __restrict__ aos, T* __restrict__ s0,
+                                                     T* __restrict__ s1, T* __restrict__ s2, T* __restrict__ s3) {
+    const unsigned row = blockIdx.x * blockDim.y + threadIdx.y, rows = (unsigned)(p.ny + 4) * (unsigned)(p.nz + 4);
+    if (row >= rows) return;
+    const int k = (int)(row / (unsigned)(p.ny + 4)) - 2, j = (int)(row - (unsigned)(k + 2) * (p.ny + 4)) - 2;
+    const bool yo = j < 0 || j >= p.ny, zo = k < 0 || k >= p.nz, y2 = j == -2 || j == p.ny + 1, z2 = k == -2 || k == p.nz + 1;
+    for (int i = (int)threadIdx.x - 2; i < p.nx + 2; i += blockDim.x) {
+        const bool xo = i < 0 || i >= p.nx;
+        const bool depth2 = i == -2 || i == p.nx + 1 || y2 || z2;
+        int wi = i, wj = j, wk = k;
+        if (depth2) {
+            if ((xo && !p.xPeri) || (yo && !p.yPeri) || (zo && !p.zPeri)) continue;
+            if (xo) wi = i < 0 ? i + p.nx : i - p.nx;
+            if (yo) wj = j < 0 ? j + p.ny : j - p.ny;
+            if (zo) wk = k < 0 ? k + p.nz : k - p.nz;
+        }
+        const T* a = aos + 3 * ((wi + 1) + (long long)(p.nx + 2) * ((wj + 1) + (long long)(p.ny + 2) * (wk + 1)));
+        T v0 = a[0], v1 = a[1], v2 = a[2];
+        if (depth2) {
+            if (xo) v0 = i < 0 ? (v0 - p.Lx) - p.dx : (v0 + p.Lx) + p.dx;
+            if (yo) v1 = j < 0 ? (v1 - p.Ly) - p.dy : (v1 + p.Ly) + p.dy;
+            if (zo) v2 = k < 0 ? (v2 - p.Lz) - p.dz : (v2 + p.Lz) + p.dz;
+        }
+        const long long g = gidx(p.px, p.py, i, j, k);
+        for (T* s : {s0, s1, s2, s3}) {
+            s[g] = v0;
+            s[p.cs + g] = v1;
+            s[2 * p.cs + g] = v2;
+        }
     }
 }
 
@@ -1272,8 +1282,10 @@ cudaError_t launch_scale_b0(const KP<T>& p, const T* B0, T* B0s, cudaStream_t s)
 }
 
 template <typename T>
-cudaError_t launch_images(const KP<T>& p, T* soa, cudaStream_t s) {
-    k_images<T><<<nblk((long long)(p.nx + 4) * (p.ny + 4) * (p.nz + 4)), 256, 0, s>>>(p, soa);
+cudaError_t launch_unpack_grid(const KP<T>& p, const T* aos, T* const grids[4], cudaStream_t s) {
+    const unsigned rows = (unsigned)(p.ny + 4) * (unsigned)(p.nz + 4);
+    const dim3 block = p.nx > 60 ? dim3(128, 2) : dim3(32, 8);
+    k_unpack_grid<T><<<(rows + block.y - 1) / block.y, block, 0, s>>>(p, aos, grids[0], grids[1], grids[2], grids[3]);
     return cudaGetLastError();
 }
 
@@ -1335,7 +1347,7 @@ cudaError_t launch_eps_star(const KP<T>& p, const T* B, const T* J, const T* X, 
     template cudaError_t launch_finalize<T>(const double*, int, double*, cudaStream_t);                           \
     template cudaError_t launch_unpack<T>(const KP<T>&, const T*, T*, cudaStream_t);                              \
     template cudaError_t launch_pack<T>(const KP<T>&, const T*, T*, cudaStream_t);                                \
-    template cudaError_t launch_images<T>(const KP<T>&, T*, cudaStream_t);                                        \
+    template cudaError_t launch_unpack_grid<T>(const KP<T>&, const T*, T* const[4], cudaStream_t);               \
     template cudaError_t launch_scale_b0<T>(const KP<T>&, const T*, T*, cudaStream_t);                            \
     template cudaError_t launch_shear_table<T>(const KP<T>&, const T*, T*, cudaStream_t);                         \
     template cudaError_t launch_pack_k<T>(const KP<T>&, const T*, T*, cudaStream_t);                              \

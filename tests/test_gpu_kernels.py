@@ -197,6 +197,18 @@ def test_reductions_match_numpy_in_64_bits(shape, peri, scale, precision):
 
 
 @pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_uploaded_grids_are_the_callers(shape, precision):
+    """All four grids of a handle hold the uploaded points, ghosts included."""
+    p, x, B0 = case(shape, (1, 1, 0), precision)
+    g = Relaxation(p)
+    g.upload(x, B0, 0.0, 1e-3)
+    for which in (0, 1, 5, 6):
+        np.testing.assert_array_equal(g.x(which), x)
+    g.close()
+
+
+@pytest.mark.parametrize("precision", [32, 64])
 def test_set_time_in_stream_order(precision):
     """Between steps in flight: the state is changed where the call stands, what it
     does not name is kept, and a step size at the lower bound stops the steps."""
