@@ -508,7 +508,7 @@ struct Impl : ImplBase {
                 // reference's ghost values (current() before kk(), main.cu:272-281)
                 CUDA_TRY(gmk::launch_export_ghosts<T>(kp, outB, outD, stream));
                 CUDA_TRY(gmk::launch_j_own<T>(a, 0, stream));
-                launches += 1 + kp.xPeri + kp.yPeri + kp.zPeri;
+                launches += 1 + (kp.xPeri || kp.yPeri || kp.zPeri);
             }
             CUDA_TRY(gmk::launch_stage_field<T>(a, gp.pressure, own, stream));
             launches++;
@@ -528,7 +528,7 @@ struct Impl : ImplBase {
                 aj.jpass = 1;
                 CUDA_TRY(gmk::launch_stage<T>(aj, gmk::MODE_DIAG, gp.pressure, grid, block, smem_diag, stream));
                 CUDA_TRY(gmk::launch_export_ghosts<T>(kp, outB, outD, stream));
-                launches += 1 + kp.xPeri + kp.yPeri + kp.zPeri;
+                launches += 1 + (kp.xPeri || kp.yPeri || kp.zPeri);
                 if (kp.jOct || kp.jQuint || kp.jTri) {
                     CUDA_TRY(gmk::launch_j_own<T>(args(n), 0, stream));
                     launches++;
@@ -792,7 +792,7 @@ struct Impl : ImplBase {
         if ((rc = enqueue_diag())) return rc;
         // the exported arrays' periodic faces (setPeriFace)
         CUDA_TRY(gmk::launch_export_ghosts<T>(kp, outB, outD, stream));
-        launches += kp.xPeri + kp.yPeri + kp.zPeri;
+        launches += kp.xPeri || kp.yPeri || kp.zPeri;
         CUDA_TRY(gmk::launch_eps_star<T>(kp, outB, outJ, X[h_st->cur], eps_col, red + gmk::R_COUNT, stream));
         launches += 2;
         CUDA_TRY(cudaMemcpyAsync(h_red, red, (gmk::R_COUNT + 1) * sizeof(double), cudaMemcpyDeviceToHost, stream));
@@ -816,7 +816,7 @@ struct Impl : ImplBase {
         if (own) {
             CUDA_TRY(gmk::launch_export_ghosts<T>(kp, outB, outD, stream));
             CUDA_TRY(gmk::launch_j_own<T>(a, 1, stream));
-            launches += 1 + kp.xPeri + kp.yPeri + kp.zPeri;
+            launches += 1 + (kp.xPeri || kp.yPeri || kp.zPeri);
         }
         CUDA_TRY(gmk::launch_diag_field<T>(a, own, stream));
         CUDA_TRY(gmk::launch_finalize<T>(part, gmk::diag_blocks<T>(kp.N), red, stream));

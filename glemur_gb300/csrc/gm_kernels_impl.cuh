@@ -902,8 +902,9 @@ template <typename T>
 __global__ void __launch_bounds__(32 * R_COUNT) k_finalize(const double* __restrict__ part, int nparts, double* out) {
     const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double acc = r <= R_LAST_MAX ? 0.0 : r == R_MIN_CONVEX ? 1.0 : DBL_MAX;
+#pragma unroll 8
     for (int q = lane; q < nparts; q += 32) {
-        const double v = part[(long long)q * R_COUNT + r];
+        const double v = __ldg(part + (long long)q * R_COUNT + r);
         acc = r <= R_LAST_SUM ? acc + v : r <= R_LAST_MAX ? fmax(acc, v) : fmin(acc, v);
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -1065,27 +1066,38 @@ __global__ void k_unpack_k(const KP<T> p, const T* __restrict__ aos, T* __restri
     }
 }
 
-// Periodic ghost layers of the exported B (setPeriFace, boundaries.cu:450-488)
-// and of detJac, one face pair per launch in the order z, y, x.
+// The periodic ghost faces of the exported B and of detJac (setPeriFace's copies,
+// boundaries.cu:450-488, one face pair after the other in the order z, y, x): what they
+// come to is that a ghost point of a periodic direction takes the value of the point wrapped in all periodic
+// directions, which none of them writes, so one launch does all faces (a launch per
+// pair took 15 of the 180 us of a 48x48x96 FP64 octilateral stage).
 template <typename T>
-__global__ void k_export_peri(const KP<T> p, T* __restrict__ B, T* __restrict__ D, int face) {
-    const int nx2 = p.nx + 2, ny2 = p.ny + 2, nz2 = p.nz + 2;
-    const int n1 = face == 0 ? ny2 : nx2;
-    const int n2 = face == 2 ? ny2 : nz2;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < (long long)n1 * n2; q += (long long)gridDim.x * blockDim.x) {
-        const int a = (int)(q % n1), b = (int)(q / n1);
-        long long lo, hi, slo, shi;
-        auto G = [&](int i, int j, int k) { return (long long)i + (long long)nx2 * ((long long)j + (long long)ny2 * k); };
-        if (face == 2) { lo = G(a, b, 0); hi = G(a, b, p.nz + 1); slo = G(a, b, p.nz); shi = G(a, b, 1); }
-        else if (face == 1) { lo = G(a, 0, b); hi = G(a, p.ny + 1, b); slo = G(a, p.ny, b); shi = G(a, 1, b); }
-        else { lo = G(0, a, b); hi = G(p.nx + 1, a, b); slo = G(p.nx, a, b); shi = G(1, a, b); }
-        for (int l = 0; l < 3; l++) {
-            B[3 * lo + l] = B[3 * slo + l];
-            B[3 * hi + l] = B[3 * shi + l];
-        }
-        D[lo] = D[slo];
-        D[hi] = D[shi];
+__global__ void __launch_bounds__(256) k_export_peri(const __grid_constant__ KP<T> p, T* __restrict__ B, T* __restrict__ D) {
+    after_previous();
+    let_next();
+    const unsigned nx2 = p.nx + 2, ny2 = p.ny + 2, nz2 = p.nz + 2;
+    const unsigned fx = p.xPeri ? 2 * ny2 * nz2 : 0, fy = p.yPeri ? 2 * nx2 * nz2 : 0, fz = p.zPeri ? 2 * nx2 * ny2 : 0;
+    unsigned q = blockIdx.x * 256 + threadIdx.x;
+    if (q >= fx + fy + fz) return;
+    const int side = q & 1;
+    unsigned i, j, k;
+    if (q < fx) {
+        q >>= 1;
+        i = side ? nx2 - 1 : 0; k = q / ny2; j = q - k * ny2;
+    } else if ((q -= fx) < fy) {
+        q >>= 1;
+        j = side ? ny2 - 1 : 0; k = q / nx2; i = q - k * nx2;
+    } else {
+        q = (q - fy) >> 1;
+        k = side ? nz2 - 1 : 0; j = q / nx2; i = q - j * nx2;
     }
+    auto wrapped = [](unsigned v, unsigned n, int peri) { return !peri ? v : v == 0 ? n : v == n + 1 ? 1u : v; };
+    const unsigned si = wrapped(i, p.nx, p.xPeri), sj = wrapped(j, p.ny, p.yPeri), sk = wrapped(k, p.nz, p.zPeri);
+    const long long o = (long long)i + (long long)nx2 * ((long long)j + (long long)ny2 * k);
+    const long long from = (long long)si + (long long)nx2 * ((long long)sj + (long long)ny2 * sk);
+#pragma unroll
+    for (int l = 0; l < 3; l++) B[3 * o + l] = B[3 * from + l];
+    D[o] = D[from];
 }
 
 // Grid-quality fields at the inner points of a padded grid, inner layout:
@@ -1315,11 +1327,10 @@ cudaError_t launch_unpack_k(const KP<T>& p, const T* aos, T* k, cudaStream_t s) 
 
 template <typename T>
 cudaError_t launch_export_ghosts(const KP<T>& p, T* outB, T* outD, cudaStream_t s) {
-    const int nx2 = p.nx + 2, ny2 = p.ny + 2, nz2 = p.nz + 2;
-    if (p.zPeri) k_export_peri<T><<<nblk((long long)nx2 * ny2), 256, 0, s>>>(p, outB, outD, 2);
-    if (p.yPeri) k_export_peri<T><<<nblk((long long)nx2 * nz2), 256, 0, s>>>(p, outB, outD, 1);
-    if (p.xPeri) k_export_peri<T><<<nblk((long long)ny2 * nz2), 256, 0, s>>>(p, outB, outD, 0);
-    return cudaGetLastError();
+    const long long nx2 = p.nx + 2, ny2 = p.ny + 2, nz2 = p.nz + 2;
+    const long long n = 2 * ((p.xPeri ? ny2 * nz2 : 0) + (p.yPeri ? nx2 * nz2 : 0) + (p.zPeri ? nx2 * ny2 : 0));
+    if (n == 0) return cudaSuccess;
+    return launch_next(k_export_peri<T>, (unsigned)((n + 255) / 256), 256, 0, s, p, outB, outD);
 }
 
 template <typename T>

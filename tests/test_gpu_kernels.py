@@ -232,3 +232,23 @@ def test_set_time_in_stream_order(precision):
     assert g.state()["nAttempted"] == 3
     for q in (g, h):
         q.close()
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("peri", PERI + [(1, 1, 1)])
+@pytest.mark.parametrize("shape", [(3, 4, 5), (33, 13, 9)])
+def test_exported_ghosts_are_the_wrapped_points(shape, peri, precision):
+    """Faces, edges and corners: one face pair after the other in the order z, y, x."""
+    p, x, B0 = case(shape, peri, precision)
+    g = Relaxation(p)
+    g.upload(x, B0, 0.0, 1e-3)
+    g.refresh()
+    d = g.download()
+    g.close()
+    for f in (d["B"], d["detJac"]):
+        w = f.copy()
+        for axis, on in ((0, peri[2]), (1, peri[1]), (2, peri[0])):
+            if on:
+                v = np.moveaxis(w, axis, 0)
+                v[0], v[-1] = v[-2].copy(), v[1].copy()
+        np.testing.assert_array_equal(f, w)
