@@ -323,10 +323,29 @@ __global__ void __launch_bounds__(field_threads<T>()) k_stage_field(const __grid
 #pragma unroll
             for (int l = 0; l < 3; l++) km[5][l] = kn[l];
             if (plain && p.errMode != 0) {
+                // The FP64 sums matter only where they can raise the maximum of the
+                // launch so far: an FP32 estimate, off by at most 7 * 2^-24 of the sum of
+                // magnitudes, leaves most points out (the FP64 pipe was 41 of the 63 us
+                // of this stage at 64x64x128, which now takes 47).  NaN and infinities take
+                // the FP64 sums.
+                const float sofar = __double2float_rd(__longlong_as_double((long long)*(volatile unsigned long long*)&st->maxDeltaBits));
+                bool need = false;
 #pragma unroll
-                for (int l = 0; l < 3; l++)
+                for (int l = 0; l < 3; l++) {
+                    float est = 0, size = 0;
 #pragma unroll
-                    for (int m = 0; m < 6; m++) e[l] += p.cmc[m] * (double)km[m][l];
+                    for (int m = 0; m < 6; m++) {
+                        const float t = (float)p.cmcT[m] * (float)km[m][l];
+                        est += t;
+                        size += fabsf(t);
+                    }
+                    need |= !(fabsf(est) + (size * 0x1p-20f + 0x1p-140f) < sofar);
+                }
+                if (need)
+#pragma unroll
+                    for (int l = 0; l < 3; l++)
+#pragma unroll
+                        for (int m = 0; m < 6; m++) e[l] += p.cmc[m] * (double)km[m][l];
             }
             if (plain || p.errMode == 0) {
                 T xst[3];
