@@ -200,7 +200,7 @@ int main(int argc, char* argv[]) {
     printf("initial B: %s\n", p.bInit);
     if (p.inertia) printf("initial U: %s\n", p.uInit);
     if (p.pressure) printf("include pressure gradient with beta = %f\n", p.beta);
-    printf("tiles = 32 x 8 columns, one launch per Runge-Kutta stage, step loop on the device\n");
+    printf("tiles = 32 x 12 columns (32 x 4 on small grids), one launch per Runge-Kutta stage, step loop on the device\n");
     const int rc = precision == 32 ? run<float>(p, activeDevice) : run<double>(p, activeDevice);
     if (rc) return rc;
     printf("glemur terminated successfully\n");

@@ -381,7 +381,7 @@ struct Impl : ImplBase {
                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (r != CUDA_SUCCESS) return gm::fail(GM_ECUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
         }
-        // k_m over (nx, ny, nz, component), row pitch kpx: box 32 x 8 x 1 x 3, the tile
+        // k_m over (nx, ny, nz, component), row pitch kpx: box 32 x ty x 1 x 3, the tile
         // (rows start on 16-byte boundaries: kpx is a multiple of 8)
         cuuint64_t kdims[4] = {(cuuint64_t)kp.nx, (cuuint64_t)kp.ny, (cuuint64_t)kp.nz, 3};
         cuuint64_t kstrides[3] = {(cuuint64_t)kp.kpx * es, (cuuint64_t)kp.kpx * kp.ny * es, (cuuint64_t)kp.kcs * es};

@@ -88,7 +88,6 @@ struct ConvArgs {
     int nx, ny, nz, xper, yper;
     int Kc, Np;                              // padded input channels (multiple of 16), padded outputs
     int Nt;                                  // output channels per CTA (multiple of 16; blockIdx.y picks the slice)
-    int Kch;                                 // input channels per pipeline step (multiple of 16)
     int vec;                                 // out and mask rows start on 16 bytes: 8 channels an access
     int* status;
     int stall;                               // failure-detection test: wait on an mbarrier nothing arrives on
@@ -96,21 +95,9 @@ struct ConvArgs {
 
 __device__ __forceinline__ int wrap(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
 
-// Pipeline of the convolution: a step is one tap and one chunk of the input
-// channels, all of them up to 96 (one step per tap), else chunks of kConvKc
-// (so that the stages stay small enough for two CTAs per SM);
-// kConvStages steps of operands are in flight.
-constexpr int kConvKc = 64;
-constexpr int kConvStages = 4;
-
 // 16-byte asynchronous copy global -> shared (cp.async, L2 only), or 16 zero
 // bytes when !valid (source size 0: nothing is read from src).
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sm_addr(dst)), "l"(src),
-                 "r"(valid ? 16 : 0)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async16s(uint32_t dst, const void* src, bool valid) {
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
@@ -151,153 +138,12 @@ __device__ __forceinline__ void conv_store16(const ConvArgs& a, long long v, int
     }
 }
 
-// One CTA: 128 consecutive voxels x one slice of Nt output channels
-// (blockIdx.y; all Np when they fit), accumulated over the 27 taps.  The
-// operands of a step (the tap's A tile: 128 voxels x one chunk of input
-// channels at the tap's offset; and its B tile: the slice's weights for that
-// chunk) are copied straight into shared memory with cp.async, kConvStages
-// steps ahead, while one thread issues the tensor-core MMAs of the current
-// step; a stage is refilled once the MMAs that read it have committed.
-__global__ void __launch_bounds__(128) k_conv(const ConvArgs a) {
-    extern __shared__ __align__(128) unsigned char sm[];
-    constexpr int S = kConvStages;
-    const int Kc = a.Kc, KCH = a.Kch;
-    const int n0 = blockIdx.y * a.Nt;                 // first output channel of the slice
-    const int Np = min(a.Nt, a.Np - n0);              // channels of this slice (a multiple of 16)
-    const int aBytes = 128 * KCH * 2, bBytes = a.Nt * KCH * 2;
-    unsigned char* stA = sm;                          // S stages of A, then S stages of B
-    unsigned char* stB = sm + S * aBytes;
-    // mbarriers: one per stage (MMA commits) and one that nothing arrives on
-    // (the failure-detection test waits on it)
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + S * (aBytes + bBytes));
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + S + 1);
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const long long V = (long long)a.nx * a.ny * a.nz;
-    const long long v = (long long)blockIdx.x * 128 + tid;
-    const bool valid = v < V;
-    const int vi = valid ? (int)(v % a.nx) : 0;
-    const int vj = valid ? (int)((v / a.nx) % a.ny) : 0;
-    const int vk = valid ? (int)(v / ((long long)a.nx * a.ny)) : 0;
-    const int nk = (Kc + KCH - 1) / KCH;             // channel chunks per tap
-    const int T = 27 * nk;                           // steps
-    uint32_t ncols = 32;
-    while ((int)ncols < Np) ncols <<= 1;
-    if (tid == 0)
-        for (int q = 0; q <= S; q++) mbar_init_tc(&bars[q]);
-    if (warp == 0) tmem_alloc(tslot, ncols);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tbase = *tslot;
-    const uint32_t id = idesc_bf16(128, Np);
-
-    // the copies of step q into stage q % S
-    auto issue = [&](int q) {
-        const int st = q % S;
-        const int t = q / nk, kc0 = (q % nk) * KCH, kcw = min(KCH, Kc - kc0);
-        const int dk = t / 9 - 1, dj = (t / 3) % 3 - 1, di = t % 3 - 1;
-        // A: row tid = this thread's voxel at the tap's offset
-        int i = vi + di, j = vj + dj;
-        const int k = vk + dk;
-        bool in = valid && k >= 0 && k < a.nz && (a.xper || (i >= 0 && i < a.nx)) && (a.yper || (j >= 0 && j < a.ny));
-        i = wrap(i, a.nx);
-        j = wrap(j, a.ny);
-        const long long u = in ? (long long)i + (long long)a.nx * (j + (long long)a.ny * k) : 0;
-        unsigned char* dA = stA + st * aBytes;
-        for (int c = 0; c < kcw; c += 8) {
-            const int cc = kc0 + c;
-            const __nv_bfloat16* src = a.in1;
-            bool ok8 = in;
-            if (cc < a.c1) src = a.in1 + u * a.ld1 + cc;
-            else if (cc - a.c1 < a.c2) src = a.in2 + u * a.ld2 + (cc - a.c1);
-            else ok8 = false;
-            cp_async16(dA + kmajor_off(tid, c, KCH), ok8 ? src : a.in1, ok8);
-        }
-        // B: the slice's Np x kcw weights of the tap.  A thread copies the 8
-        // channels cc, cc + 64, ... (cc = 8 (tid / 16)) of rows tid % 16,
-        // tid % 16 + 16, ...: the 8 lanes of a shared-memory store phase write
-        // the 8 rows of one core matrix
-        const __nv_bfloat16* Wt = a.W + ((size_t)t * a.Np + n0) * Kc + kc0;
-        unsigned char* dB = stB + st * bBytes;
-        for (int cc = (tid >> 4) * 8; cc < kcw; cc += 64)
-            for (int r = tid & 15; r < Np; r += 16)
-                cp_async16(dB + kmajor_off(r, cc, KCH), Wt + (size_t)r * Kc + cc, true);
-    };
-
-    uint32_t ph[S];
-    bool pend[S];                    // a commit on bars[s] not yet waited for
-    for (int q = 0; q < S; q++) { ph[q] = 0; pend[q] = false; }
-    // failure-detection test: a bounded wait that runs out before any MMA
-    bool ok = a.stall ? mbar_wait_tc(&bars[S], 0, 1u << 10) : true;
-    if (__syncthreads_and(ok)) {
-        for (int q = 0; q < S - 1; q++) {
-            if (q < T) issue(q);
-            cp_async_commit();
-        }
-        for (int q = 0; q < T; q++) {
-            // refill the stage of step q + S - 1: the MMAs of step q - 1 read it
-            const int qn = q + S - 1;
-            if (qn < T) {
-                const int sn = qn % S;
-                if (pend[sn]) {
-                    if (!mbar_wait_tc(&bars[sn], ph[sn])) ok = false;
-                    ph[sn] ^= 1;
-                    pend[sn] = false;
-                }
-            }
-            // after a wait ran out no thread copies into a stage and no MMA is issued
-            if (!__syncthreads_and(ok)) {
-                ok = false;
-                break;
-            }
-            if (qn < T) issue(qn);
-            cp_async_commit();
-            cp_async_wait<S - 1>();                  // step q's copies have landed
-            fence_async_smem();
-            tc_fence_before();
-            __syncthreads();
-            tc_fence_after();
-            const int s = q % S;
-            if (tid == 0) {
-                const int kcw = min(KCH, Kc - (q % nk) * KCH);
-                for (int kk = 0; kk < kcw / 16; kk++) {
-                    const uint64_t ad = smem_desc(sm_addr(stA + s * aBytes) + kk * 256, 128, (uint32_t)KCH * 16);
-                    const uint64_t bd = smem_desc(sm_addr(stB + s * bBytes) + kk * 256, 128, (uint32_t)KCH * 16);
-                    mma_bf16(tbase, ad, bd, id, q > 0 || kk > 0);
-                }
-                mma_commit(&bars[s]);
-            }
-            pend[s] = true;
-        }
-    }
-    // the copies still in flight, and the commits not yet waited for: bounded
-    // waits before the accumulator is read or freed
-    cp_async_wait_all();
-    for (int q = 0; q < S; q++)
-        if (pend[q]) {
-            if (!mbar_wait_tc(&bars[q], ph[q])) ok = false;
-            ph[q] ^= 1;
-        }
-    ok = __syncthreads_and(ok);
-    tc_fence_after();
-    if (ok) {
-        for (int c0 = 0; c0 < Np; c0 += 16) {
-            float acc[16];
-            tmem_ld16(tbase + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, acc);
-            if (valid) conv_store16(a, v, n0 + c0, acc);
-        }
-    } else if (tid == 0) {
-        atomicExch(a.status, 1);
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) tmem_free(tbase, ncols);
-}
-
 // ---- convolution on resident input planes ---------------------------------------
 
-// The same convolution with every input plane copied once, the weights resident
-// and each MMA used for three taps.  A CTA takes items of 8 x 16 voxels and kz
+// Every input plane is copied once, the weights are resident and each MMA serves three
+// taps.  (Copying a tap's 128 voxels x K channels for every tap, 27 times the input,
+// took 375 us for 24 -> 24 channels at 64x64x128, with 3 % tensor activity; this takes
+// 38.)  A CTA takes items of 8 x 16 voxels and kz
 // output planes and marches along z; an input plane of the tile with its halo
 // (10 x 18 voxels) is copied into shared memory and all taps read it there.  In
 // the K-major no-swizzle layout a row of a core matrix is the 16 bytes of 8
@@ -311,12 +157,11 @@ __global__ void __launch_bounds__(128) k_conv(const ConvArgs a) {
 // accumulators of consecutive output planes lie in consecutive columns.  (An MMA
 // takes 46 clocks up to N = 48, 57 at N = 96, N / 2 from N = 128 on.)
 //
-// Warps 0-3 read finished accumulators and store, warps 4-7 copy planes, one
-// thread of warp 12 issues the MMAs; they meet in mbarriers only.  With the copies, MMAs and
-// stores of a step in one program order every step was a chain of about 9000
-// clocks around 2000 clocks of MMAs.
-//
-// The weights of the CTA's output channels (all 27 taps) are copied once.
+// Warps 0-3 read finished accumulators and store, warps 4-7 copy planes, warps 0-3 and
+// 8-11 the weights of the CTA's output channels (all 27 taps, once), one thread of warp
+// 12 issues the MMAs; they meet in mbarriers only.  With the copies, MMAs and stores of
+// a step in one program order every step was a chain of about 9000 clocks around 2000
+// clocks of MMAs.
 constexpr int kTileX = 8, kTileY = 16, kHaloX = kTileX + 2, kSlots = kHaloX * (kTileY + 2);
 constexpr int kMaxPlanes = 3, kMaxKz = 32;
 constexpr int kPlaneThreads = 416, kCopyThreads = 128;
@@ -426,7 +271,8 @@ __device__ __forceinline__ bool conv_copy_planes(const ConvArgs& a, int tx, int 
             }
             const int k = w.z0 + p - 1;
             const bool zin = k >= 0 && k < a.nz;
-            const __nv_bfloat16* src = a.in1 + (long long)a.nx * a.ny * (zin ? k : 0) * a.ld1 + 8 * gh;
+            const long long plane = (long long)a.nx * a.ny * (zin ? k : 0);
+            const __nv_bfloat16* src = a.in1 + plane * a.ld1 + 8 * gh;
             const uint32_t dst = stA + buf * planeBytes + gh * kGroupBytes;
 #pragma unroll
             for (int q = 0; q < 3; q++) {
@@ -434,9 +280,18 @@ __device__ __forceinline__ bool conv_copy_planes(const ConvArgs& a, int tx, int 
                 if (s >= kSlots) continue;
                 const bool in = zin && vx[q] >= 0;
                 const __nv_bfloat16* v = src + (long long)max(vx[q], 0) * a.ld1;
-                for (int g = 0; g < ng; g += 2) {
-                    const bool on = in && 8 * (g + gh) < a.c1;
-                    cp_async16s(dst + g * kGroupBytes + s * 16, on ? v + 8 * g : a.in1, on);
+                const uint32_t d = dst + s * 16;
+                if (a.c2 == 0) {
+                    for (int g = 0; g < ng; g += 2) {
+                        const bool on = in && 8 * (g + gh) < a.c1;
+                        cp_async16(d + g * kGroupBytes, on ? v + 8 * g : a.in1, on);
+                    }
+                } else {
+                    for (int g = 0; g < ng; g += 2) {
+                        const int c = 8 * (g + gh) - a.c1;
+                        const bool on = in && c < a.c2;
+                        cp_async16(d + g * kGroupBytes, !on ? a.in1 : c < 0 ? v + 8 * g : a.in2 + (plane + vx[q]) * a.ld2 + c, on);
+                    }
                 }
             }
             cp_async_commit();
@@ -906,7 +761,7 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const WgradArgs a) {
                             for (int g = gh; g < cs; g += 2) {
                                 const int c = c0 + 8 * g;
                                 const __nv_bfloat16* src = c < a.c1 ? a.in1 + v * a.ld1 + c : a.in2 + v * a.ld2 + (c - a.c1);
-                                cp_async16s(dst + p * planeBytes + g * kGroupBytes + s * 16, on && c < a.ci ? src : a.in1, on && c < a.ci);
+                                cp_async16(dst + p * planeBytes + g * kGroupBytes + s * 16, on && c < a.ci ? src : a.in1, on && c < a.ci);
                             }
                         }
                     }
@@ -921,7 +776,7 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const WgradArgs a) {
                             const long long v = in ? (long long)i + (long long)a.nx * (j + (long long)a.ny * (w.z0 + p)) : 0;
                             for (int g = gh; g < N / 8; g += 2) {
                                 const bool on = in && o0 + 8 * g < a.co;
-                                cp_async16s(dd + (p * (N / 8) + g) * kDoutGroup + s * 16, on ? a.dout + v * a.ldd + o0 + 8 * g : a.dout, on);
+                                cp_async16(dd + (p * (N / 8) + g) * kDoutGroup + s * 16, on ? a.dout + v * a.ldd + o0 + 8 * g : a.dout, on);
                             }
                         }
                     }
@@ -1349,7 +1204,7 @@ __global__ void k_wg_grid(const float* __restrict__ d, const T* __restrict__ xid
     }
 }
 
-// The launch of a convolution of one view: k_conv_planes with resident weights or
+// The launch of a convolution: k_conv_planes with resident weights or
 // k_conv_wide with streamed ones, the candidates (output slices, planes per item)
 // compared by an estimate in clocks.  An MMA with N columns takes
 // max(46, 32 + N / 4, N / 2) clocks; CTAs on an SM share the tensor core; resident
@@ -1484,16 +1339,6 @@ int gm_nn_conv(const void* in1, int ld1, int c1, const void* in2, int ld2, int c
     if (Kc % 16 || Kc < 16 || Kc > 256 || Np % 16 || Np < 16 || Np > 256 || c1 + (in2 ? c2 : 0) > Kc || co > Np ||
         c1 % 8)
         return gm::fail(GM_EPARAM, "gm_nn_conv: channel counts out of range");
-    // output channels per CTA: all of them when the operand stages fit the
-    // shared memory, else the widest multiple of 16 that fits (slices in
-    // blockIdx.y)
-    // input channels per pipeline step: all of them up to 96 (one step per
-    // tap), else kConvKc
-    const int Kch = Kc <= 96 ? Kc : gmnn::kConvKc;
-    auto conv_smem = [Kch](int nt) { return (size_t)gmnn::kConvStages * (128 + nt) * Kch * 2 + 64; };
-    int Nt = Np;
-    while (Nt > 16 && conv_smem(Nt) > 200 * 1024) Nt -= 16;
-    if (conv_smem(Nt) > 200 * 1024) return gm::fail(GM_EPARAM, "gm_nn_conv: channel counts out of range");
     int rc;
     if ((rc = check_view_align(in1, ld1, "gm_nn_conv in1")) || (rc = check_view_align(in2, ld2, "gm_nn_conv in2")))
         return rc;
@@ -1503,34 +1348,25 @@ int gm_nn_conv(const void* in1, int ld1, int c1, const void* in2, int ld2, int c
     a.W = (const __nv_bfloat16*)W; a.bias = bias;
     a.out = (__nv_bfloat16*)out; a.ldo = ldo; a.co = co;
     a.mask = (const __nv_bfloat16*)mask; a.ldm = ldm; a.relu = relu;
-    a.nx = nx; a.ny = ny; a.nz = nz; a.xper = xper; a.yper = yper; a.Kc = Kc; a.Np = Np; a.Nt = Nt; a.Kch = Kch; a.status = status;
+    a.nx = nx; a.ny = ny; a.nz = nz; a.xper = xper; a.yper = yper; a.Kc = Kc; a.Np = Np; a.status = status;
     a.stall = g_nn_stall;
     auto aligned = [](const void* q, int ld) { return q == nullptr || (!(reinterpret_cast<uintptr_t>(q) & 15) && ld % 8 == 0); };
     a.vec = aligned(out, ldo) && aligned(mask, ldm);
     gmnn::ConvPlan c;
-    if (!in2 && gmnn::choose_conv(a, &c)) {
-        a.Nt = c.Nt;
-        const int tx = (nx + gmnn::kTileX - 1) / gmnn::kTileX, ty = (ny + gmnn::kTileY - 1) / gmnn::kTileY;
-        cudaError_t e = c.wide ? cudaFuncSetAttribute(gmnn::k_conv_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)
-                               : cudaFuncSetAttribute(gmnn::k_conv_planes, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) return gm::fail(GM_ECUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-        if (c.wide)
-            gmnn::k_conv_wide<<<c.grid, gmnn::kWideThreads, c.smem, (cudaStream_t)stream>>>(
-                gmnn::ConvWideArgs{a, c.kz, tx, ty, (int)c.items, c.ncols, c.sets, c.planes, c.kch, c.stages});
-        else
-            gmnn::k_conv_planes<<<c.grid, gmnn::kPlaneThreads, c.smem, (cudaStream_t)stream>>>(
-                gmnn::ConvPlaneArgs{a, c.kz, tx, ty, (int)c.items, c.ncols, c.planes});
-        e = cudaGetLastError();
-        return e == cudaSuccess ? GM_OK : gm::fail(GM_ECUDA, std::string("convolution launch: ") + cudaGetErrorString(e));
-    }
-    const size_t smem = conv_smem(Nt);
-    cudaError_t e = cudaFuncSetAttribute(gmnn::k_conv, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (!gmnn::choose_conv(a, &c)) return gm::fail(GM_EPARAM, "gm_nn_conv: grid out of range");
+    a.Nt = c.Nt;
+    const int tx = (nx + gmnn::kTileX - 1) / gmnn::kTileX, ty = (ny + gmnn::kTileY - 1) / gmnn::kTileY;
+    cudaError_t e = c.wide ? cudaFuncSetAttribute(gmnn::k_conv_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)
+                           : cudaFuncSetAttribute(gmnn::k_conv_planes, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return gm::fail(GM_ECUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-    const long long V = (long long)nx * ny * nz;
-    const dim3 grid((unsigned)((V + 127) / 128), (unsigned)((Np + Nt - 1) / Nt));
-    gmnn::k_conv<<<grid, 128, smem, (cudaStream_t)stream>>>(a);
+    if (c.wide)
+        gmnn::k_conv_wide<<<c.grid, gmnn::kWideThreads, c.smem, (cudaStream_t)stream>>>(
+            gmnn::ConvWideArgs{a, c.kz, tx, ty, (int)c.items, c.ncols, c.sets, c.planes, c.kch, c.stages});
+    else
+        gmnn::k_conv_planes<<<c.grid, gmnn::kPlaneThreads, c.smem, (cudaStream_t)stream>>>(
+            gmnn::ConvPlaneArgs{a, c.kz, tx, ty, (int)c.items, c.ncols, c.planes});
     e = cudaGetLastError();
-    return e == cudaSuccess ? GM_OK : gm::fail(GM_ECUDA, std::string("k_conv: ") + cudaGetErrorString(e));
+    return e == cudaSuccess ? GM_OK : gm::fail(GM_ECUDA, std::string("convolution launch: ") + cudaGetErrorString(e));
 }
 
 int gm_nn_conv_wgrad(const void* dout, int ldd, int co, const void* in1, int ld1, int c1, const void* in2, int ld2,

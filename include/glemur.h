@@ -360,7 +360,7 @@ int gm_reduce_noalloc(const gm_params* p, const void* B, const void* J, const vo
 /* ---- many independent cases (no counterpart in the reference, which runs
  * one case per process) ------------------------------------------------------
  * Cases of uneven grid sizes advance together: each Runge-Kutta stage is ONE
- * persistent launch whose CTAs take 32 x 8 x 32 tiles of every case from a
+ * persistent launch whose CTAs take 32 x 12 x 32 tiles of every case from a
  * work counter, one launch runs every case's controller (src/main.cu:321-383
  * per case), and a step of all cases is one CUDA graph replay.  A case whose
  * controller has stopped (nCycle, dtMin, NaN) or that gm_batch_stop /
@@ -421,15 +421,15 @@ int gm_nn_tc_gemm_check(const void* A, const void* B, float* D, int N, int K, in
  *   of the views in1 (c1 channels, c1 a multiple of 8) and in2 (c2); W is
  *   BF16 [27][Np][Kc] (Kc >= c1 + c2 and Np >= co multiples of 16, <= 256).
  *   With W flipped in t and transposed it is the input gradient.  A CTA takes
- *   128 voxels and all Np outputs, or a slice of them when the two operand
- *   stages would not fit its shared memory. */
+ *   tiles of 8 x 16 voxels over several planes and all Np outputs or a slice of
+ *   them. */
 int gm_nn_conv(const void* in1, int ld1, int c1, const void* in2, int ld2, int c2, const void* W, const float* bias,
                void* out, int ldo, int co, const void* mask, int ldm, int relu, int nx, int ny, int nz, int xper,
                int yper, int Kc, int Np, int* status, void* stream);
 /* dW[t][o][i] += sum_v dout[v][o] in[v + off(t)][i] (FP32, i < ci <= c1 +
- * c2, o < co <= 256), on the tensor cores: one GEMM per chunk of vchunk voxels
- * (a multiple of 64; 0 lets the library choose) with the 27 taps' input
- * channels stacked as its rows, in tiles of 128.  dout is read up to co
+ * c2, o < co <= 256), on the tensor cores, a CTA taking at least vchunk voxels
+ * (a multiple of 64; 0 lets the library choose) in tiles of 8 x 16 over several
+ * planes, with the three z taps' input channels stacked as rows.  dout is read up to co
  * rounded up to 8 channels, the input views up to ci rounded up to 8; every
  * view starts on 16 bytes with a channel stride that is a multiple of 8. */
 int gm_nn_conv_wgrad(const void* dout, int ldd, int co, const void* in1, int ld1, int c1, const void* in2, int ld2,

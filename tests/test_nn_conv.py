@@ -7,7 +7,8 @@ import ctypes as C
 import numpy as np
 import pytest
 
-# nx, ny, nz, xper, yper, c1 (view), Kc, co, Np, relu, mask
+# nx, ny, nz, xper, yper, channels of the input (split: a second view from channel
+# c1 on), Kc, co, Np, relu, mask
 CASES = [
     (8, 16, 4, 1, 1, 16, 16, 16, 16, 1, 0),       # one tile
     (4, 4, 2, 1, 1, 8, 16, 3, 16, 0, 0),          # below a tile, head
@@ -22,6 +23,9 @@ CASES = [
     (8, 8, 4, 1, 1, 104, 112, 45, 48, 1, 0),
     (12, 6, 3, 1, 1, 200, 256, 256, 256, 1, 0),   # the largest channel counts
     (64, 48, 40, 1, 1, 24, 32, 24, 32, 1, 1),     # several items a CTA
+    (20, 17, 5, 1, 0, (48, 24), 80, 24, 32, 1, 0),     # two views, resident weights
+    (9, 8, 6, 1, 1, (24, 60), 96, 20, 32, 0, 1),
+    (16, 18, 4, 0, 1, (192, 48), 240, 48, 48, 1, 0),   # two views, streamed weights
 ]
 
 
@@ -49,7 +53,9 @@ def _reference(x, W, b, xper, yper):
 def test_conv(case):
     import torch
     from glemur_gb300 import _abi
-    nx, ny, nz, xper, yper, c1, Kc, co, Np, relu, mask = case
+    nx, ny, nz, xper, yper, chans, Kc, co, Np, relu, mask = case
+    n1, n2 = chans if isinstance(chans, tuple) else (chans, 0)
+    c1 = n1 + n2
     rng = np.random.default_rng(1)
     bf = lambda a: torch.tensor(a, dtype=torch.float32, device="cuda").to(torch.bfloat16)  # noqa: E731
     V = nx * ny * nz
@@ -61,9 +67,11 @@ def test_conv(case):
     m = bf(rng.normal(size=(V, lo)))
     st = torch.zeros(1, dtype=torch.int32, device="cuda")
     P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    l2 = (n2 + 7) // 8 * 8 + 8
+    x1, x2 = x[:, :n1].contiguous(), torch.nn.functional.pad(x[:, n1:], (0, l2 - n2), value=9.0)
     torch.cuda.synchronize()
     lib = _abi.load()
-    _abi.check(lib.gm_nn_conv(P(x), c1, c1, None, 0, 0, P(W), C.cast(b.data_ptr(), C.POINTER(C.c_float)), P(y), lo, co,
+    _abi.check(lib.gm_nn_conv(P(x1), n1, n1, P(x2) if n2 else None, l2, n2, P(W), C.cast(b.data_ptr(), C.POINTER(C.c_float)), P(y), lo, co,
                               P(m) if mask else None, lo if mask else 0, relu, nx, ny, nz, xper, yper, Kc, Np, P(st),
                               None), "gm_nn_conv")
     torch.cuda.synchronize()
