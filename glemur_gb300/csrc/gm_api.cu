@@ -334,12 +334,11 @@ struct Impl : ImplBase {
             if ((rc = init_tma(nsm))) return rc;
         }
         // Stages by the field kernels (gm_fields.cuh): FP64 frictional Stokes runs,
-        // the inertial equation and the currents with a kernel of their own.  Where
+        // the inertial equation and the currents other than Stokes.  Where
         // their B field does not fit the device's memory, the tile kernels stay.
         const bool stokes = strncmp(p->jMethod, "Stokes ", 7) == 0;
-        use_fields = p->stageKernel == 0 && !batched && !kp.jClassic && !kp.jxbAver &&
-                     (sizeof(T) == 8 || !stokes || kp.inertia);
-        if (use_fields && stokes && cudaMalloc((void**)&BF, 4 * (size_t)kp.cs * sizeof(T)) != cudaSuccess) {
+        use_fields = p->stageKernel == 0 && !batched && !kp.jxbAver && (sizeof(T) == 8 || !stokes || kp.inertia);
+        if (use_fields && (stokes || kp.jClassic) && cudaMalloc((void**)&BF, 4 * (size_t)kp.cs * sizeof(T)) != cudaSuccess) {
             cudaGetLastError();
             BF = nullptr;
             use_fields = false;
@@ -510,7 +509,7 @@ struct Impl : ImplBase {
                 CUDA_TRY(gmk::launch_j_own<T>(a, 0, stream));
                 launches += 1 + (kp.xPeri || kp.yPeri || kp.zPeri);
             }
-            CUDA_TRY(gmk::launch_stage_field<T>(a, gp.pressure, own, stream));
+            CUDA_TRY(gmk::launch_stage_field<T>(a, gp.pressure, own ? 1 : kp.jClassic ? 2 : 0, stream));
             launches++;
         } else if (use_tma) {
             gmk::StageArgsTMA<T> A;

@@ -10,9 +10,10 @@
 //     Here each B is formed once (34 operations) and the stage needs 57 more
 //     and its sums, lanes are full for any nx, and the points spread evenly over
 //     the SMs.  The second pass's reads hit L2 or hide behind the FP64 pipe.
-//   * the inertial equation, and the currents that come from a kernel of their
-//     own (Stokes4th, StokesQuint, StokesTri), in either precision: their stages
-//     ran in the general tile kernel, one CTA per SM, waiting for its loads.
+//   * the inertial equation, the Classic current, and the currents that come from a
+//     kernel of their own (Stokes4th, StokesQuint, StokesTri), in either precision:
+//     their stages ran in the general tile kernel, one CTA per SM, waiting for its
+//     loads.
 //   * gm_refresh and the convergence checks of a batch.
 //
 // In FP64 a point's arithmetic is that of the tile kernel (gm_stage_tma.cuh),
@@ -68,6 +69,22 @@ struct GlobalTile {
         return __ldg(X + l * p.cs + gidx(p.px, p.py, i, j, k));
     }
 };
+
+// As the general tile kernel's tile for j_classic: the positions, and 1/Delta from RF
+// (FP64: 1/det(a, b, c), so no division).
+template <typename T>
+struct ClassicTile {
+    const KP<T>& p;
+    const T *X, *RF;
+    __device__ __forceinline__ T x(int k, int l, int j, int i) const {
+        return __ldg(X + l * p.cs + gidx(p.px, p.py, i, j, k));
+    }
+};
+template <typename T>
+__device__ __forceinline__ T inv_delta(const ClassicTile<T>& t, int k, int j, int i) {
+    const T r = __ldg(t.RF + gidx(t.p.px, t.p.py, i, j, k));
+    return sizeof(T) == 4 ? rcp_rn(r) : vmul(r, t.p.vol8);
+}
 
 // B and Delta at an inner or image point: B_JacB0 (rungeKutta.cu:79-106), as
 // b_interior.
@@ -191,10 +208,11 @@ __device__ __forceinline__ void j_unscaled(const KP<T>& p, const T A[3][3], cons
 }
 
 // One RK stage from the B field: J, k_n and the next stage position (stage 5:
-// x_new and the error norm) at every inner point, as stage_tile.  JOUT: J and B
-// come from the exported arrays (a current with a kernel of its own).  INERTIA:
-// the velocity equation (rungeKutta.cu:195-212).
-template <typename T, bool PRESS, bool INERTIA, bool JOUT, bool LAST>
+// x_new and the error norm) at every inner point, as stage_tile.  JOUT:
+// 0 the Stokes current, 1 J and B come from the exported arrays (a current with a
+// kernel of its own), 2 the Classic current.  INERTIA: the velocity equation
+// (rungeKutta.cu:195-212).
+template <typename T, bool PRESS, bool INERTIA, int JOUT, bool LAST>
 __global__ void __launch_bounds__(field_threads<T>()) k_stage_field(const __grid_constant__ StageArgs<T> a) {
     const KP<T>& p = a.p;
     DevState* st = a.st;
@@ -214,8 +232,14 @@ __global__ void __launch_bounds__(field_threads<T>()) k_stage_field(const __grid
         const T dtT = (T)st->dt;
         T A[3][3], J[3], B[3], R = 0, D = 0, kn[3];
         const bool plain = kPlain<T>;
-        if (!plain && (!JOUT || PRESS)) diffs_v<T>(X, A);
-        if (!JOUT && plain) {
+        if (!plain && (JOUT == 0 || PRESS)) diffs_v<T>(X, A);
+        if (JOUT == 2) {
+            j_classic<T>(p, ClassicTile<T>{p, stage_input(a), a.RF}, a.B0, i, j, k, J);
+            R = __ldg(a.RF + g);
+#pragma unroll
+            for (int l = 0; l < 3; l++) B[l] = __ldg(a.BF + l * cs + g);
+            D = plain ? R : vmul(rcp_stage<T>(R), p.inv8);
+        } else if (JOUT == 0 && plain) {
             T xn[6][3], bn[6][3];
             const int px = p.px, pxy = p.px * p.py;
 #pragma unroll
@@ -231,7 +255,7 @@ __global__ void __launch_bounds__(field_threads<T>()) k_stage_field(const __grid
             }
             stokes<T>(xn, bn, J);
             D = __ldg(a.RF + g);
-        } else if (!JOUT) {
+        } else if (JOUT == 0) {
             j_unscaled(p, A, a.BF, g, J);
             R = __ldg(a.RF + g);
 #pragma unroll
@@ -252,7 +276,7 @@ __global__ void __launch_bounds__(field_threads<T>()) k_stage_field(const __grid
         T uc[3] = {0, 0, 0}, ku[3] = {0, 0, 0};
         if (!INERTIA) {
             T f = vmul(vmul(vmul(p.ex[i], p.ey[j]), dtT), p.ez[k]);
-            if (!JOUT && !plain) f = vmul(f, R);
+            if (JOUT == 0 && !plain) f = vmul(f, R);
 #pragma unroll
             for (int l = 0; l < 3; l++) {
                 kn[l] = vmul(kn[l], f);
@@ -263,7 +287,7 @@ __global__ void __launch_bounds__(field_threads<T>()) k_stage_field(const __grid
             const T* Un = n == 0 ? a.U[cur] : a.US[(n - 1) & 1];
             T f = vmul(dtT, D);
             const T w = vmul(f, p.nu);
-            if (!JOUT && !plain) f = vmul(f, R);
+            if (JOUT == 0 && !plain) f = vmul(f, R);
 #pragma unroll
             for (int l = 0; l < 3; l++) {
                 uc[l] = Un[l * KC + kl];
@@ -1006,12 +1030,12 @@ cudaError_t launch_stage_field(const StageArgs<T>& a, int pressure, int jout, cu
     cudaError_t rc = cudaErrorInvalidValue;
     by(pressure, [&](auto P) {
         by(a.p.inertia, [&](auto I) {
-            by(jout, [&](auto J) {
-                by(a.n == 5, [&](auto L) {
-                    // FP32 frictional Stokes stages run in the tile kernel
-                    if constexpr (sizeof(T) == 8 || I.value || J.value)
-                        rc = launch_next(k_stage_field<T, P.value, I.value, J.value, L.value>, nb, t, 0, s, a);
-                });
+            by(a.n == 5, [&](auto L) {
+                if (jout == 1) rc = launch_next(k_stage_field<T, P.value, I.value, 1, L.value>, nb, t, 0, s, a);
+                else if (jout == 2) rc = launch_next(k_stage_field<T, P.value, I.value, 2, L.value>, nb, t, 0, s, a);
+                // FP32 frictional Stokes stages run in the tile kernel
+                else if constexpr (sizeof(T) == 8 || I.value)
+                    rc = launch_next(k_stage_field<T, P.value, I.value, 0, L.value>, nb, t, 0, s, a);
             });
         });
     });

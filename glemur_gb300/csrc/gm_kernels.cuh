@@ -94,7 +94,7 @@ struct KP {
     T hdx1, hdy1, hdz1;      // dx1/2, dy1/2, dz1/2 (exact)
     T Lx, Ly, Lz, Ox, Oy, Oz;
     int xPeri, yPeri, zPeri, zUpdate, errMode, refDt;
-    int jClassic;            // jMethod = "Classic": the finite-difference current (generic kernel only)
+    int jClassic;            // jMethod = "Classic": the finite-difference current
     int jOct;                // jMethod = "Stokes4th": J from the octilateral pass (outJ; generic kernel only)
     int jQuint;              // jMethod = "StokesQuint": J from the quintilateral pass (outJ; generic kernel only)
     int jTri;                // jMethod = "StokesTri": J from the same pass in its triangle-only form

@@ -242,13 +242,17 @@ __device__ __forceinline__ void stokes(const T xn[6][3], const T bn[6][3], T J[3
 // and its face neighbours (the B ring, ghost values included) and B0 there
 // (global memory); B itself is not used.
 template <typename T, class TileT>
+__device__ __forceinline__ T inv_delta(const TileT& t, int k, int j, int i) {
+    return rcp_rn(t.b(k, 3, j, i));
+}
+template <typename T, class TileT>
 __device__ __forceinline__ void j_classic(const KP<T>& p, const TileT& t, const T* __restrict__ B0, int i, int j,
                                           int k, T Jv[3]) {
     T jac[3][3], jac1[3][3], dB0[3][3], dDet1[3], B0l[3];
 #define XV(di, dj, dk, l) t.x(k + (dk), l, j + (dj), i + (di))
 #define B0V(di, dj, dk, l) __ldg(&B0[(long long)(l) * p.cs + gidx(p.px, p.py, i + (di), j + (dj), k + (dk))])
-#define DV(di, dj, dk) t.b(k + (dk), 3, j + (dj), i + (di))
-    const T det1 = rcp_rn(DV(0, 0, 0));
+#define RV(di, dj, dk) inv_delta<T>(t, k + (dk), j + (dj), i + (di))
+    const T det1 = RV(0, 0, 0);
 #pragma unroll
     for (int l = 0; l < 3; l++) {
         jac[l][0] = (XV(1, 0, 0, l) - XV(-1, 0, 0, l)) * p.dx1 / 2;
@@ -268,9 +272,9 @@ __device__ __forceinline__ void j_classic(const KP<T>& p, const TileT& t, const 
     jac1[2][0] = (jac[1][0] * jac[2][1] - jac[1][1] * jac[2][0]) * det1;
     jac1[2][1] = (jac[0][1] * jac[2][0] - jac[0][0] * jac[2][1]) * det1;
     jac1[2][2] = (jac[0][0] * jac[1][1] - jac[0][1] * jac[1][0]) * det1;
-    dDet1[0] = (rcp_rn(DV(1, 0, 0)) - rcp_rn(DV(-1, 0, 0))) * p.dx1 / 2;
-    dDet1[1] = (rcp_rn(DV(0, 1, 0)) - rcp_rn(DV(0, -1, 0))) * p.dy1 / 2;
-    dDet1[2] = (rcp_rn(DV(0, 0, 1)) - rcp_rn(DV(0, 0, -1))) * p.dz1 / 2;
+    dDet1[0] = (RV(1, 0, 0) - RV(-1, 0, 0)) * p.dx1 / 2;
+    dDet1[1] = (RV(0, 1, 0) - RV(0, -1, 0)) * p.dy1 / 2;
+    dDet1[2] = (RV(0, 0, 1) - RV(0, 0, -1)) * p.dz1 / 2;
     Jv[0] = 0; Jv[1] = 0; Jv[2] = 0;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -306,7 +310,7 @@ __device__ __forceinline__ void j_classic(const KP<T>& p, const TileT& t, const 
     }
 #undef XV
 #undef B0V
-#undef DV
+#undef RV
 }
 
 // Pressure gradient grad(p) for p = p0(X)/Delta: gradPClassic,

@@ -84,17 +84,20 @@ def test_stage_matches_the_general_kernel(shape, peri, precision):
 
 
 @pytest.mark.parametrize("precision,form", [(p, f) for p in (32, 64) for f in
-                                            ("pressure", "inertia", "inertia_pressure", "Stokes4th", "StokesQuint")])
+                                            ("pressure", "inertia", "inertia_pressure", "Stokes4th", "StokesQuint",
+                                             "Classic", "Classic_pressure", "Classic_inertia")])
 @pytest.mark.parametrize("shape,peri", [((33, 13, 9), (1, 1, 0)), ((20, 24, 17), (0, 0, 0)), ((3, 40, 12), (0, 1, 1))])
 def test_options_match_the_general_kernel(shape, peri, precision, form):
-    """As above with the pressure gradient (second differences of the positions:
-    1e-3 in FP32, as in the large case's parity test), the velocity equation and
-    the currents with a kernel of their own."""
-    kw = dict(pressure="pressure" in form, inertia="inertia" in form, method=form if form.startswith("Stokes") else "Stokes")
+    """As above with the pressure gradient and the Classic current (second differences
+    of the positions: 1e-3 in FP32, as in the large case's parity test), the velocity
+    equation and the currents with a kernel of their own."""
+    method = "Classic" if form.startswith("Classic") else form if form.startswith("Stokes") else "Stokes"
+    kw = dict(pressure="pressure" in form, inertia="inertia" in form, method=method)
     a, _ = stages(*case(shape, peri, precision, **kw), 0)
     b, _ = stages(*case(shape, peri, precision, **kw), 1)
-    tol = 1e-12 if precision == 64 else (1e-3 if kw["pressure"] else 1e-5)
-    if precision == 64 and kw["pressure"]:
+    second = kw["pressure"] or method == "Classic"
+    tol = 1e-12 if precision == 64 else (1e-3 if second else 1e-5)
+    if precision == 64 and second:
         tol = 1e-10            # the same noise at FP64 rounding
     for name in a:
         assert relerr(a[name], b[name]) < tol, name
