@@ -531,18 +531,42 @@ __global__ void __launch_bounds__(kWideThreads) k_conv_wide(const ConvWideArgs b
         } else if (warp < 8) {
             ok = conv_copy_planes(a, b.tx, b.ty, b.items, b.kz, NA, sm_addr(stA), sh.full, sh.empty, warp & 3, lane);
         } else if (warp < 8 + 4 * kWideGroups) {
-            // weights: groups of four warps, a stage in turn
-            const int grp = (warp >> 2) - 2, wq = warp & 3;
+            // weights: groups of four warps, a stage in turn.  All stages have one shape, so
+            // a thread's at most eight 16-byte groups are worked out once (by the general
+            // row copy the instructions of the copies were the kernel's bound: 240 -> 48
+            // channels at 32x32x64 160 us, now 122)
+            const int grp = (warp >> 2) - 2, t = tid & 127;
+            uint32_t from[8], to[8];                   // ~0: none; rows beyond the channels are zero
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int e = t + 128 * q, r = e / LW.ng, g = e - r * LW.ng;
+                to[q] = r < Nt ? (uint32_t)(g * rs + r * 16) : ~0u;
+                from[q] = r < Nt && n0 + r < a.Np ? (uint32_t)(r * Kc + 8 * g) : ~0u;
+            }
+            const uint32_t st0 = sm_addr(stB);
             int tap = 0, c = 0, st = 0;
             uint32_t turn = 0, round = 0;              // stages so far, rounds of the ring
             for (int item = blockIdx.x; item < b.items && ok; item += gridDim.x)
                 for (int q = 0; q < 27 * nch && ok; q++, turn++) {
                     if (turn % kWideGroups == (uint32_t)grp) {
                         const __nv_bfloat16* W = a.W + ((size_t)tap * a.Np + n0) * Kc + c * KCH;
-                        ok = conv_copy_rows(LW, Nt, sm_addr(stB + st * stepBytes), rs, wq, lane,
-                                       [&](int r) { return n0 + r < a.Np ? W + (size_t)r * Kc : nullptr; },
-                                       [&] { return round == 0 || mbar_wait_tc(&sh.wempty[st], round - 1 & 1); });
-                        if (ok) mbar_arrive_tc(&sh.wfull[st]);
+                        uint4 v[8];
+#pragma unroll
+                        for (int e = 0; e < 8; e++) {
+                            v[e] = make_uint4(0, 0, 0, 0);
+                            if (from[e] != ~0u) v[e] = __ldg(reinterpret_cast<const uint4*>(W + from[e]));
+                        }
+                        // (the loads are out before the wait)
+                        ok = round == 0 || mbar_wait_tc(&sh.wempty[st], round - 1 & 1);
+                        if (!ok) break;
+#pragma unroll
+                        for (int e = 0; e < 8; e++)
+                            if (to[e] != ~0u)
+                                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(st0 + st * stepBytes + to[e]),
+                                             "r"(v[e].x), "r"(v[e].y), "r"(v[e].z), "r"(v[e].w)
+                                             : "memory");
+                        fence_async_smem();
+                        mbar_arrive_tc(&sh.wfull[st]);
                     }
                     if (++st == S) { st = 0; round++; }
                     if (++c == nch) { c = 0; if (++tap == 27) tap = 0; }
@@ -1212,7 +1236,7 @@ __global__ void k_wg_grid(const float* __restrict__ d, const T* __restrict__ xid
 // clocks more, and an item of k_conv_wide starts 4000 clocks late; a plane's barriers take about 700 clocks of one CTA that another
 // hides; starting and draining a CTA takes 5000.  Against all shapes that fit, the
 // choice was the fastest or within 10 % of it (64x64x128: 24 -> 24 channels 38 us,
-// 72 -> 24 75 us, 24 -> 72 81 us; 32x32x64: 240 -> 48 160 us with streamed weights,
+// 72 -> 24 75 us, 24 -> 72 81 us; 32x32x64: 240 -> 48 122 us with streamed weights,
 // the only form that fits; 16x16x32: 48 -> 192 19 us, 24 streamed).
 struct ConvPlan {
     bool wide;
