@@ -11,7 +11,7 @@ namespace gmk {
 
 // Reciprocal for the stage kernel, by Newton's iteration r <- r + r (1 - x r)
 // from the hardware's approximation: one step in FP32 (within ~1 ulp; FP32
-// parity is judged at 1e-5), two in FP64 (the approximation has about 20 bits;
+// parity is held to 1e-5), two in FP64 (the approximation has about 20 bits;
 // the last step's residual is exact to an FMA, so the result is the rounded
 // reciprocal but for rare ties).
 __device__ __forceinline__ float rcp_approx(float x) {

@@ -196,14 +196,11 @@ __device__ __forceinline__ ConvPlace conv_place(int item, int tx, int ty, int kz
 
 // rows x L.ng groups of weights to shared memory at dst (group stride gs) by four
 // warps, eight 16-byte loads of a thread in flight; src(r) is row r, or null for
-// zeros.  The first loads go out before acquire() waits for the buffer; false when
-// its wait ran out.
-template <class Src, class Acquire>
-__device__ __forceinline__ bool conv_copy_rows(const ConvLanes& L, int rows, uint32_t dst, int gs, int wq, int lane,
-                                               Src src, Acquire acquire) {
+// zeros.
+template <class Src>
+__device__ __forceinline__ void conv_copy_rows(const ConvLanes& L, int rows, uint32_t dst, int gs, int wq, int lane, Src src) {
     const int g0 = lane & (L.gl - 1), dr = 4 * L.sl;
     int r = wq * L.sl + lane / L.gl, g = g0;
-    bool first = true;
     do {
         uint4 v[8];
         uint32_t d[8];
@@ -221,10 +218,6 @@ __device__ __forceinline__ bool conv_copy_rows(const ConvLanes& L, int rows, uin
                 if (g - g0 >= L.ng) { g = g0; r += dr; }
             }
         }
-        if (first) {
-            first = false;
-            if (!acquire()) return false;
-        }
 #pragma unroll
         for (int q = 0; q < 8; q++)
             if (d[q])
@@ -233,7 +226,6 @@ __device__ __forceinline__ bool conv_copy_rows(const ConvLanes& L, int rows, uin
                              : "memory");
     } while (r < rows);
     fence_async_smem();
-    return true;
 }
 
 // The four warps that copy the planes of a CTA's items, in turn into NA buffers.  A
@@ -364,7 +356,7 @@ __global__ void __launch_bounds__(kPlaneThreads) k_conv_planes(const ConvPlaneAr
                 conv_copy_rows(L, 3 * Nt, sm_addr(stB + u * tapBytes), rs, warp & 3, lane, [&](int r) {
                     const int dk = r >= 2 * Nt ? 2 : r >= Nt ? 1 : 0, o = n0 + r - dk * Nt;
                     return o < a.Np ? a.W + ((size_t)((2 - dk) * 9 + u) * a.Np + o) * Kc : nullptr;
-                }, [] { return true; });
+                });
                 mbar_arrive_tc(&sh.wfull[u]);
             }
         if (warp < 4) {
