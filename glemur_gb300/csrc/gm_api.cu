@@ -823,6 +823,15 @@ struct Impl : ImplBase {
         return GM_OK;
     }
 
+    // What gm_refresh does beyond a check (enqueue_check, with no step since): the
+    // exported arrays' periodic faces and epsilon*.
+    int enqueue_finish() {
+        CUDA_TRY(gmk::launch_export_ghosts<T>(kp, outB, outD, stream));
+        CUDA_TRY(gmk::launch_eps_star<T>(kp, outB, outJ, X[h_st->cur], eps_col, red + gmk::R_COUNT, stream));
+        launches += 2 + (kp.xPeri || kp.yPeri || kp.zPeri);
+        return GM_OK;
+    }
+
     // The batched run's convergence check of this case, enqueued on `stream`
     // without waiting: the diagnostic pass and its reductions, then the
     // reductions and the controller state copied to the pinned host buffers.
@@ -1252,13 +1261,16 @@ struct Batch : BatchBase {
                 if (conv && !done && (rc = stop(c))) return rc;
                 if (conv || done) {
                     // a finished case's state and exported fields (with their
-                    // ghosts), as gm_batch_refresh leaves them
-                    if ((rc = im.refresh(nullptr))) return rc;
+                    // ghosts), as gm_batch_refresh leaves them: the check has
+                    // just computed them (a whole refresh per case was 3 ms of
+                    // the 28 of 24 small braids over six cycles)
+                    if ((rc = im.enqueue_finish())) return rc;
                     record(c, res, conv, sec);
                 } else {
                     still.push_back(c);
                 }
             }
+            if (still.size() < pending.size()) CUDA_TRY(cudaStreamSynchronize(stream));
             // As cases finish, the work list keeps only the running ones (no
             // CTA spends a claim on a stopped case), and where the depth the
             // run started with would leave fewer than two items per resident
