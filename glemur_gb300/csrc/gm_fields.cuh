@@ -861,13 +861,16 @@ struct DiagSumsF {
     }
 };
 
-constexpr int kDiagThreads = 256;
+constexpr int kDiagThreads = 128;
 
 // J (unless a current's own kernel has written it) and the reductions at the
 // current grid, from the exported B and Delta with their face ghosts as
 // k_b_field leaves them (diagnostics.cu:12-134).  One partial per CTA, in a fixed order.
+// FP32: dependent float-pair sums, so warps count more than registers (128x128x256:
+// 224 us at 16 warps an SM and 128 registers, 175 at 32 and 64, with some spills; at
+// 40 and 48 slower again).  FP64 does not care (its pipe is full).
 template <typename T, bool JOUT>
-__global__ void __launch_bounds__(kDiagThreads) k_diag_field(const __grid_constant__ StageArgs<T> a) {
+__global__ void __launch_bounds__(kDiagThreads, sizeof(T) == 4 ? 8 : 4) k_diag_field(const __grid_constant__ StageArgs<T> a) {
     const KP<T>& p = a.p;
     const int nx = p.nx, ny = p.ny, nz = p.nz, cur = a.st->cur;
     const long long nx2 = nx + 2, nxy2 = (long long)(nx + 2) * (ny + 2);
