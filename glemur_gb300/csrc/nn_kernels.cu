@@ -1421,9 +1421,10 @@ int gm_nn_conv_wgrad(const void* dout, int ldd, int co, const void* in1, int ld1
     // clocks, a block about 1000 more, its copies 1 clock per 7.5 bytes; vchunk asks for at least that many voxels a CTA.
     // Chains of lim voxels are those of four CTAs per SM with 128 of the stacked (tap,
     // channel) rows each; a chain is no longer (the truncation error no larger), and where
-    // the voxels are many no more than 3000 voxels shorter, so that the error is the same
-    // to 1e-5 of the gradient.
+    // the voxels are many no more than 3000 voxels (1500 of chains beyond 8000) shorter, so
+    // that the error is the same to 1e-5 of the gradient.
     const long long lim = std::max(512ll, V * ((27 * ng * 8 + 127) / 128) / (4 * nsm));
+    const long long shorter = lim > 8000 ? 1500 : 3000;
     const long long slices = (long long)a.cslices * nslices;
     double tbest = 0;
     long long gx = 1;
@@ -1431,7 +1432,7 @@ int gm_nn_conv_wgrad(const void* dout, int ldd, int co, const void* in1, int ld1
         if (gmnn::wgrad_smem(a.cs, kb, a.N) > 227 * 1024) break;
         const long long blocks = (long long)a.tx * a.ty * ((nz + kb - 1) / kb);
         long long g = std::max(1ll, std::min(blocks, nsm / slices));
-        if (lim > 3512) g = std::min(g, (V + lim - 3001) / (lim - 3000));
+        if (lim > 3512) g = std::min(g, (V + lim - shorter - 1) / (lim - shorter));
         if (vchunk > 0) g = std::min(g, (V + vchunk - 1) / vchunk);
         const double load = gmnn::wg_block_bytes(a.cs, kb, a.N) / 7.5;
         const double t = load + (double)((blocks + g - 1) / g) * (std::max(3300.0 * kb, load) + 1000);
