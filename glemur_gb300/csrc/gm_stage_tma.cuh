@@ -205,7 +205,17 @@ struct StageCtl {
     // warp reads behind the next barrier, so that all leave in the same iteration.
     int abort[2];
     int work;                    // batched launch: the current work item
+    int skip;                    // batched launch: the item's run is stopped (stage_stopped)
 };
+
+// Whether a tile has nothing to compute: a stopped run, or an earlier stage of this
+// step that gave up a wait or failed its alignment check.  Another CTA of the same
+// launch may set the status bits at any time, so one thread decides for its CTA, in
+// front of a barrier: warps that each read the word could part, and those that went
+// on would wait at the march's barrier (a fixed thread count) for the others forever.
+__device__ __forceinline__ int stage_stopped(const DevState* st) {
+    return st->done | (int)(st->status & (GM_ST_TIMEOUT | GM_ST_ALIGN));
+}
 
 // The start grid's own images, refreshed by stage 5 of the first attempted step
 // (a retry reads them; until then they are those the caller supplied).
@@ -305,7 +315,9 @@ __device__ __forceinline__ void grad_p2(const KP<T>& p, uint32_t xm, uint32_t x0
 // and the k planes of the next J phase.  `base` is the 128-byte aligned shared
 // buffer with initialised mbarriers; the mbarrier parities in its StageCtl
 // carry over to the next tile.  Returns false after a bounded wait ran out or
-// an alignment check failed (the status word says which).
+// an alignment check failed (the status word says which).  Every thread of the
+// CTA is here: whether the tile is computed at all has been settled for all of
+// them (stage_stopped).
 //
 // Stage 5 does not store x_6 = x_5 - sum b_5m k_m, the start of a rejected
 // step's retry (rungeKutta.cu:216-227): it is x_0 up to rounding, and X[cur]
@@ -329,9 +341,6 @@ __device__ __forceinline__ bool stage_tile(const StageArgsTMA<T>& A, int bx, int
     const StageArgs<T>& a = A.a;
     const KP<T>& p = a.p;
     DevState* st = a.st;
-    // a stopped run, or an earlier stage of this step that gave up a wait or
-    // failed its alignment check: nothing to compute
-    if (st->done || (st->status & (GM_ST_TIMEOUT | GM_ST_ALIGN))) return true;
 
     uint64_t* bars = reinterpret_cast<uint64_t*>(base + L::OFF_BAR);       // x | B0s | k
     T* s_wmax = reinterpret_cast<T*>(base + L::OFF_WMAX);
@@ -774,7 +783,7 @@ template <typename T, bool PRESS, int NS, int NW>
 __global__ void __launch_bounds__(stage_threads<NW>(), stage_ctas<T, NW>())
     k_stage_tma(const __grid_constant__ StageArgsTMA<T> A) {
     extern __shared__ __align__(128) unsigned char smraw[];
-    if (A.a.st->done || (A.a.st->status & (GM_ST_TIMEOUT | GM_ST_ALIGN))) return;
+    if (__syncthreads_or(threadIdx.x == 0 ? stage_stopped(A.a.st) : 0)) return;
     unsigned char* base = stage_smem_setup<T, PRESS, NS, NW>(smraw);
     stage_tile<T, PRESS, NS, NW>(A, blockIdx.x, blockIdx.y, blockIdx.z, base);
 }
@@ -790,13 +799,18 @@ __global__ void __launch_bounds__(stage_threads<STAGE_BATCH_NW>(), stage_ctas<T,
     using L = StageSmem<T, PRESS, NS, NW>;
     extern __shared__ __align__(128) unsigned char smraw[];
     unsigned char* base = stage_smem_setup<T, PRESS, NS, NW>(smraw);
-    int* s_w = &reinterpret_cast<StageCtl*>(base + L::OFF_CTL)->work;
+    StageCtl* ctl = reinterpret_cast<StageCtl*>(base + L::OFF_CTL);
     for (;;) {
-        if (threadIdx.x == 0) *s_w = atomicAdd(counter, 1);
+        if (threadIdx.x == 0) {
+            const int w = atomicAdd(counter, 1);
+            ctl->work = w;
+            ctl->skip = w < nwork && stage_stopped(cases[work[w].x].a.st);
+        }
         __syncthreads();
-        const int w = *s_w;
-        __syncthreads();   // s_w is rewritten only after every thread has read it
+        const int w = ctl->work, skip = ctl->skip;
+        __syncthreads();   // both are rewritten only after every thread has read them
         if (w >= nwork) break;
+        if (skip) continue;
         const int4 it = work[w];
         if (!stage_tile<T, PRESS, NS, NW>(cases[it.x], it.y, it.z, it.w, base)) break;
         __syncthreads();   // the next tile's copies overwrite slots this one read

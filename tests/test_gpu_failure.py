@@ -120,3 +120,24 @@ def test_convolution_wait_runs_out_and_is_reported():
     a = uo.forward(P, bf16(x))
     yg = y[:, :3].float().cpu().numpy().reshape(nz, ny, nx, 3)
     assert np.linalg.norm(yg - a["y"]) / np.linalg.norm(a["y"]) < 1.5e-2
+
+
+def test_waits_run_out_over_several_waves_of_blocks():
+    """More blocks than the device holds at once: the later ones start while the
+    earlier ones record their time-outs, and each of them either runs its own waits
+    out or leaves as a whole."""
+    p = configs.random_braid(3, shape=(128, 96, 64), precision=32)
+    B0, xb = configs.init_state(p)
+    lib = _abi.load()
+    g = Relaxation(p)
+    g.upload(xb, B0)
+    g.set_tile_z(4)
+    _abi.check(lib.gm_debug_stall(g.h, 1), "gm_debug_stall")
+    with pytest.raises(GlemurError, match="GM_ETIMEOUT"):
+        g.run(2)
+    s = g.state()
+    assert s["status"] & _abi.GM_ST_TIMEOUT and s["timeIndex"] == 0 and s["nAttempted"] == 1
+    _abi.check(lib.gm_debug_stall(g.h, 0), "gm_debug_stall")
+    g.upload(xb, B0)
+    assert g.run(2)["timeIndex"] == 2
+    g.close()
