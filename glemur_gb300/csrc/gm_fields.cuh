@@ -40,6 +40,22 @@ __device__ __forceinline__ const T* stage_input(const StageArgs<T>& a) {
     return a.n == 0 ? a.X[a.st->cur] : a.XS[(a.n - 1) & 1];
 }
 
+// A load of what a kernel of the step has written (positions, B and Delta, J, the
+// increments): these grids start while the one before still runs, and __ldg is for data
+// that no one writes while the grid is there.  An ordinary load, in its place behind
+// after_previous.  (Left to the compiler, the loads of k_b_field in FP64 came as they were
+// used: 32x32x64 133 -> 148 us a step.)  B0 and its scaled copy are the upload's.
+
+__device__ __forceinline__ float ld_step(const float* q) {
+    float r;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(r) : "l"(q));
+    return r;
+}
+__device__ __forceinline__ double ld_step(const double* q) {
+    double r;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(r) : "l"(q));
+    return r;
+}
 // Positions around the point at padded index g in global memory.
 template <typename T>
 struct GlobalX {
@@ -48,7 +64,7 @@ struct GlobalX {
     int px, pxy;
     long long cs;
     __device__ __forceinline__ T operator()(int l, int di, int dj, int dk) const {
-        return __ldg(x + l * cs + di + dj * px + dk * pxy);
+        return ld_step(x + l * cs + di + dj * px + dk * pxy);
     }
     __device__ __forceinline__ T s(int l) const { return __ldg(b0s + l * cs); }
 };
@@ -66,7 +82,7 @@ struct GlobalTile {
     const KP<T>& p;
     const T* X;
     __device__ __forceinline__ T x(int k, int l, int j, int i) const {
-        return __ldg(X + l * p.cs + gidx(p.px, p.py, i, j, k));
+        return ld_step(X + l * p.cs + gidx(p.px, p.py, i, j, k));
     }
 };
 
@@ -77,20 +93,20 @@ struct ClassicTile {
     const KP<T>& p;
     const T *X, *RF;
     __device__ __forceinline__ T x(int k, int l, int j, int i) const {
-        return __ldg(X + l * p.cs + gidx(p.px, p.py, i, j, k));
+        return ld_step(X + l * p.cs + gidx(p.px, p.py, i, j, k));
     }
 };
 template <typename T>
 __device__ __forceinline__ T inv_delta(const ClassicTile<T>& t, int k, int j, int i) {
-    const T r = __ldg(t.RF + gidx(t.p.px, t.p.py, i, j, k));
+    const T r = ld_step(t.RF + gidx(t.p.px, t.p.py, i, j, k));
     return sizeof(T) == 4 ? rcp_rn(r) : vmul(r, t.p.vol8);
 }
 
 // B and Delta at an inner or image point: B_JacB0 (rungeKutta.cu:79-106), as
 // b_interior.
 template <typename T>
-__device__ __forceinline__ void b_plain(const KP<T>& p, const GlobalX<T>& X, const T* __restrict__ B0, long long g, T B[3],
-                                        T* D) {
+__device__ __forceinline__ void b_plain(const KP<T>& p, const GlobalX<T>& X, const T* __restrict__ B0, long long g,
+                                        T B[3], T* D) {
     T jac[3][3];
 #pragma unroll
     for (int l = 0; l < 3; l++) {
@@ -185,14 +201,14 @@ __global__ void __launch_bounds__(field_threads<T>()) k_b_field(const __grid_con
 // J of the Stokes current at the point g, up to the factor 1/det(a, b, c) (see
 // stage_tile): a I1 + b I2 + c I0.
 template <typename T>
-__device__ __forceinline__ void j_unscaled(const KP<T>& p, const T A[3][3], const T* __restrict__ BF, long long g, T J[3]) {
+__device__ __forceinline__ void j_unscaled(const KP<T>& p, const T A[3][3], const T* BF, long long g, T J[3]) {
     const int px = p.px, pxy = p.px * p.py;
     T I0, I1, I2;
 #pragma unroll
     for (int l = 0; l < 3; l++) {
         const T* b = BF + l * p.cs + g;
-        const T dx = vsub(__ldg(b + 1), __ldg(b - 1)), dy = vsub(__ldg(b + px), __ldg(b - px)),
-                dz = vsub(__ldg(b + pxy), __ldg(b - pxy));
+        const T dx = vsub(ld_step(b + 1), ld_step(b - 1)), dy = vsub(ld_step(b + px), ld_step(b - px)),
+                dz = vsub(ld_step(b + pxy), ld_step(b - pxy));
         if (l == 0) {
             I0 = vfms(A[l][1], dx, vmul(A[l][0], dy));
             I1 = vfms(A[l][2], dy, vmul(A[l][1], dz));
@@ -235,9 +251,9 @@ __global__ void __launch_bounds__(field_threads<T>()) k_stage_field(const __grid
         if (!plain && (JOUT == 0 || PRESS)) diffs_v<T>(X, A);
         if (JOUT == 2) {
             j_classic<T>(p, ClassicTile<T>{p, stage_input(a), a.RF}, a.B0, i, j, k, J);
-            R = __ldg(a.RF + g);
+            R = ld_step(a.RF + g);
 #pragma unroll
-            for (int l = 0; l < 3; l++) B[l] = __ldg(a.BF + l * cs + g);
+            for (int l = 0; l < 3; l++) B[l] = ld_step(a.BF + l * cs + g);
             D = plain ? R : vmul(rcp_stage<T>(R), p.inv8);
         } else if (JOUT == 0 && plain) {
             T xn[6][3], bn[6][3];
@@ -245,27 +261,27 @@ __global__ void __launch_bounds__(field_threads<T>()) k_stage_field(const __grid
 #pragma unroll
             for (int l = 0; l < 3; l++) {
                 const T* b = a.BF + l * cs + g;
-                B[l] = __ldg(b);
+                B[l] = ld_step(b);
                 xn[0][l] = X(l, -1, 0, 0); xn[1][l] = X(l, 1, 0, 0);
                 xn[2][l] = X(l, 0, -1, 0); xn[3][l] = X(l, 0, 1, 0);
                 xn[4][l] = X(l, 0, 0, -1); xn[5][l] = X(l, 0, 0, 1);
-                bn[0][l] = __ldg(b - 1); bn[1][l] = __ldg(b + 1);
-                bn[2][l] = __ldg(b - px); bn[3][l] = __ldg(b + px);
-                bn[4][l] = __ldg(b - pxy); bn[5][l] = __ldg(b + pxy);
+                bn[0][l] = ld_step(b - 1); bn[1][l] = ld_step(b + 1);
+                bn[2][l] = ld_step(b - px); bn[3][l] = ld_step(b + px);
+                bn[4][l] = ld_step(b - pxy); bn[5][l] = ld_step(b + pxy);
             }
             stokes<T>(xn, bn, J);
-            D = __ldg(a.RF + g);
+            D = ld_step(a.RF + g);
         } else if (JOUT == 0) {
             j_unscaled(p, A, a.BF, g, J);
-            R = __ldg(a.RF + g);
+            R = ld_step(a.RF + g);
 #pragma unroll
-            for (int l = 0; l < 3; l++) B[l] = __ldg(a.BF + l * cs + g);
+            for (int l = 0; l < 3; l++) B[l] = ld_step(a.BF + l * cs + g);
             if (INERTIA) D = vmul(rcp_stage<T>(R), p.inv8);
         } else {
             const long long o = (long long)(i + 1) + (long long)(nx + 2) * ((long long)(j + 1) + (long long)(ny + 2) * (k + 1));
 #pragma unroll
-            for (int l = 0; l < 3; l++) { J[l] = a.outJ[3 * (long long)q + l]; B[l] = a.outB[3 * o + l]; }
-            D = a.outD[o];
+            for (int l = 0; l < 3; l++) { J[l] = ld_step(a.outJ + 3 * (long long)q + l); B[l] = ld_step(a.outB + 3 * o + l); }
+            D = ld_step(a.outD + o);
             if (PRESS && !plain) R = rcp_stage<T>(vmul(D, p.vol8));
         }
         if (plain) cross3(J, B, kn);
@@ -314,8 +330,16 @@ __global__ void __launch_bounds__(field_threads<T>()) k_stage_field(const __grid
                 const T w = p.db[n][m];
                 const T* Km = a.K[m] + kl;
 #pragma unroll
-                for (int l = 0; l < 3; l++) xa[l] = vfma(w, __ldg(Km + l * KC), xa[l]);
+                for (int l = 0; l < 3; l++) xa[l] = vfma(w, ld_step(Km + l * KC), xa[l]);
             }
+            // u_{n+1} = u_n + sum_{m<=n} (b[n+1][m] - b[n][m]) k_u,m
+            T ua[3] = {uc[0], uc[1], uc[2]};
+            if (INERTIA)
+                for (int m = 0; m < n; m++) {
+                    const T wm = p.db[n][m];
+#pragma unroll
+                    for (int l = 0; l < 3; l++) ua[l] = vfma(wm, ld_step(a.KU[m] + l * KC + kl), ua[l]);
+                }
             const T w = p.db[n][n];
 #pragma unroll
             for (int l = 0; l < 3; l++) {
@@ -323,13 +347,6 @@ __global__ void __launch_bounds__(field_threads<T>()) k_stage_field(const __grid
                 a.K[n][l * KC + kl] = kn[l];
             }
             if (INERTIA) {
-                // u_{n+1} = u_n + sum_{m<=n} (b[n+1][m] - b[n][m]) k_u,m
-                T ua[3] = {uc[0], uc[1], uc[2]};
-                for (int m = 0; m < n; m++) {
-                    const T wm = p.db[n][m];
-#pragma unroll
-                    for (int l = 0; l < 3; l++) ua[l] = vfma(wm, __ldg(a.KU[m] + l * KC + kl), ua[l]);
-                }
 #pragma unroll
                 for (int l = 0; l < 3; l++) {
                     a.KU[n][l * KC + kl] = ku[l];
@@ -343,7 +360,7 @@ __global__ void __launch_bounds__(field_threads<T>()) k_stage_field(const __grid
 #pragma unroll
             for (int m = 0; m < 5; m++)
 #pragma unroll
-                for (int l = 0; l < 3; l++) km[m][l] = __ldg(a.K[m] + l * KC + kl);
+                for (int l = 0; l < 3; l++) km[m][l] = ld_step(a.K[m] + l * KC + kl);
 #pragma unroll
             for (int l = 0; l < 3; l++) km[5][l] = kn[l];
             if (plain && p.errMode != 0) {
@@ -408,18 +425,20 @@ __global__ void __launch_bounds__(field_threads<T>()) k_stage_field(const __grid
             }
             if (INERTIA) {
                 // u_6 and u_new = u_6 + sum c k_u (rungeKutta.cu:311-322)
+                T kum[6][3];
+#pragma unroll
+                for (int m = 0; m < 5; m++)
+#pragma unroll
+                    for (int l = 0; l < 3; l++) kum[m][l] = ld_step(a.KU[m] + l * KC + kl);
 #pragma unroll
                 for (int l = 0; l < 3; l++) {
-                    T kum[6];
-#pragma unroll
-                    for (int m = 0; m < 5; m++) kum[m] = __ldg(a.KU[m] + l * KC + kl);
-                    kum[5] = ku[l];
+                    kum[5][l] = ku[l];
                     T u6 = uc[l];
 #pragma unroll
-                    for (int m = 0; m < 6; m++) u6 = vfma(p.db[5][m], kum[m], u6);
+                    for (int m = 0; m < 6; m++) u6 = vfma(p.db[5][m], kum[m][l], u6);
                     T un = u6;
 #pragma unroll
-                    for (int m = 0; m < 6; m++) un = vfma(p.c[m], kum[m], un);
+                    for (int m = 0; m < 6; m++) un = vfma(p.c[m], kum[m][l], un);
                     a.U[cur][l * KC + kl] = u6;
                     a.U[cur ^ 1][l * KC + kl] = un;
                 }
@@ -512,7 +531,7 @@ __global__ void __launch_bounds__(field_threads<T>()) k_j_oct(const __grid_const
 #pragma unroll
             for (int l = 0; l < 3; l++) {
                 chord[l] = vsub(x[(e + 1) & 7][l], x[(e + 7) & 7][l]);
-                s = vfma(__ldg(B + ru[e] * bs[u] + rv[e] * bs[v] + l), chord[l], s);
+                s = vfma(ld_step(B + ru[e] * bs[u] + rv[e] * bs[v] + l), chord[l], s);
             }
             if (!(e & 1)) {      // a corner
                 T edge[3];
@@ -561,8 +580,7 @@ __device__ __forceinline__ T quiet_nan() {
 }
 
 template <typename T>
-__device__ __noinline__ void j_quint_point(const KP<T>& p, const T* __restrict__ X, const T* __restrict__ Bg,
-                                           T* __restrict__ J, long long q, int i, int j, int k) {
+__device__ __noinline__ void j_quint_point(const KP<T>& p, const T* X, const T* Bg, T* J, long long q, int i, int j, int k) {
     const int ax[3][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}};
     const long long nx2 = p.nx + 2, ny2 = p.ny + 2;
     {
@@ -741,8 +759,8 @@ __global__ void __launch_bounds__(field_threads<T>()) k_j_quint(const __grid_con
     T I0, I1, I2;
 #pragma unroll
     for (int l = 0; l < 3; l++) {
-        const T dx = vsub(__ldg(B + o[0] + l), __ldg(B - o[0] + l)), dy = vsub(__ldg(B + o[1] + l), __ldg(B - o[1] + l)),
-                dz = vsub(__ldg(B + o[2] + l), __ldg(B - o[2] + l));
+        const T dx = vsub(ld_step(B + o[0] + l), ld_step(B - o[0] + l)), dy = vsub(ld_step(B + o[1] + l), ld_step(B - o[1] + l)),
+                dz = vsub(ld_step(B + o[2] + l), ld_step(B - o[2] + l));
         if (l == 0) {
             I0 = vfms(A[l][1], dx, vmul(A[l][0], dy));
             I1 = vfms(A[l][2], dy, vmul(A[l][1], dz));

@@ -32,11 +32,11 @@
 
 namespace gmk {
 
-// Programmatic dependent launch of the field passes and the controller of a step: each
-// is launched when every CTA of the one before it has started or ended, so its launch
-// runs during that kernel, and waits (after_previous, in every thread before anything
-// that a kernel writes or reads) until that one has completed and its writes are
-// visible.  A kernel completes after its own wait, so the order holds through the
+// Programmatic dependent launch of the field passes and the ghost faces of a step (the
+// controller is launched plainly): each is launched when every CTA of the one before it
+// has started or ended, so its launch runs during that kernel, and waits
+// (after_previous, in every thread before anything that a kernel writes or reads) until
+// that one has completed and its writes are visible.  A kernel completes after its own wait, so the order holds through the
 // chain.  32x32x64 in FP64 140 -> 136 us a step, 64x64x128 FP32 with inertia 296 ->
 // 291.  The tile kernel's stages are launched plainly: early CTAs wait in the slots
 // that the running ones' balance needs (97x75x133 line-tied 210 -> 245 us a step, and
