@@ -782,50 +782,37 @@ __global__ void __launch_bounds__(field_threads<T>()) k_j_quint(const __grid_con
 
 // ---- refresh: J and the reductions ---------------------------------------------
 
-// Unevaluated sums of two floats, about 46 bits.
-struct FF { float h, l; };
-__device__ __forceinline__ FF ff_quick(float a, float b) {
-    const float s = __fadd_rn(a, b);
-    return FF{s, __fsub_rn(b, __fsub_rn(s, a))};
-}
-__device__ __forceinline__ FF ff_two_sum(float a, float b) {
-    const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
-    return FF{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
-}
-__device__ __forceinline__ FF ff_prod(float a, float b) {
-    const float p = __fmul_rn(a, b);
-    return FF{p, __fmaf_rn(a, b, -p)};
-}
-__device__ __forceinline__ FF ff_add(FF a, FF b) {
-    const FF s = ff_two_sum(a.h, b.h);
-    return ff_quick(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
-}
-__device__ __forceinline__ FF ff_neg(FF a) { return FF{-a.h, -a.l}; }
-__device__ __forceinline__ FF ff_mul(FF a, FF b) {
-    const FF p = ff_prod(a.h, b.h);
-    return ff_quick(p.h, __fmaf_rn(a.h, b.l, __fmaf_rn(a.l, b.h, p.l)));
-}
-__device__ __forceinline__ FF ff_sqrt(FF a) {
-    if (!(a.h > 0.f)) return FF{0.f, 0.f};
-    const float y = __fsqrt_rn(a.h);
-    return ff_quick(y, __fmul_rn(__fadd_rn(__fmaf_rn(-y, y, a.h), a.l), __fdividef(0.5f, y)));
-}
-__device__ __forceinline__ FF ff_div(FF a, FF b) {
-    const float q = __fdividef(a.h, b.h);
-    const float r = __fadd_rn(__fmaf_rn(-q, b.h, a.h), __fmaf_rn(-q, b.l, a.l));
-    return ff_quick(q, __fdividef(r, b.h));
-}
-__device__ __forceinline__ double ff_double(FF a) { return (double)a.h + (double)a.l; }
+// 1 / sqrt(x) and sqrt(x) from an approximation y of the former: with t = x y and the
+// residual e = 1 - t y of its square, (1 - e)^(-1/2) = 1 + e/2 + 3 e^2/8 + ... (binomial series),
+// so x^(-1/2) = y (1 + w) and x^(1/2) = t (1 + w) with w = e (1/2 + 3 e/8).  The hardware's
+// approximation has about 20 bits; what is left out is of the order e^3 < 2^-57.
+struct InvSqrt {
+    double y, t, w;
+    __device__ __forceinline__ explicit InvSqrt(double x) {
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+        t = x * y;
+        const double e = fma(-t, y, 1.0);
+        w = e * fma(0.375, e, 0.5);
+    }
+    __device__ __forceinline__ double root() const { return fma(t, w, t); }
+    __device__ __forceinline__ double inverse() const { return fma(y, w, y); }
+};
 
-// The sums and maxima of one thread in the run precision's wider type: doubles,
-// and in FP32 pairs of floats.  Per point these are about 85 FP64 operations
-// (three square roots, a division); the FP64 pipe made them 570 of the 1190 us
-// of a 128x128x256 refresh in FP32.  B and J are floats there, so their pair
-// sums (46 bits) leave the results' error where B's and J's rounding puts it;
-// points outside the pairs' range take the double form.
+// x as a double, by integer operations; `plain` is cleared where x is subnormal or not finite.
+__device__ __forceinline__ double widen(float x, bool& plain) {
+    const unsigned b = __float_as_uint(x), t = b << 1;
+    plain &= t == 0 || t - 0x01000000u < 0xfe000000u;
+    const unsigned hi = (b & 0x80000000u) | (t ? ((b & 0x7fffffffu) >> 3) + 0x38000000u : 0u);
+    return __hiloint2double((int)hi, (int)(b << 29));
+}
+// x > 0, neither subnormal nor infinite nor NaN
+__device__ __forceinline__ bool normal(double x) { return (unsigned)__double2hiint(x) - 0x00100000u < 0x7fe00000u; }
+
+// The sums and maxima of one thread, in doubles.
 struct DiagSums {
     double s[5] = {0, 0, 0, 0, 0};       // |J x B|, |J||B|, their ratio, B^2 Delta, |B - e_z|^2
     double m[2] = {0, 0};                // |B|, |J|
+    double m2[2] = {0, 0};               // |B|^2, |J|^2 (the points of addf)
     __device__ __forceinline__ void add(const double B[3], const double J[3], double b2D) {
         const double bn = sqrt(B[0] * B[0] + B[1] * B[1] + B[2] * B[2]), jn = sqrt(J[0] * J[0] + J[1] * J[1] + J[2] * J[2]);
         const double cx = J[1] * B[2] - J[2] * B[1], cy = J[2] * B[0] - J[0] * B[2], cz = J[0] * B[1] - J[1] * B[0];
@@ -838,44 +825,40 @@ struct DiagSums {
         m[0] = fmax(m[0], bn);
         m[1] = fmax(m[1], jn);
     }
-};
-struct DiagSumsF {
-    DiagSums slow;
-    FF s[5] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}};
-    FF m[2] = {{0, 0}, {0, 0}};          // |B|^2, |J|^2
-    static __device__ __forceinline__ FF norm2(FF a, FF b, FF c) { return ff_add(ff_add(ff_mul(a, a), ff_mul(b, b)), ff_mul(c, c)); }
-    static __device__ __forceinline__ FF sq(float a, float b, float c) {
-        return ff_add(ff_add(ff_prod(a, a), ff_prod(b, b)), ff_prod(c, c));
-    }
-    static __device__ __forceinline__ FF cr(float a, float b, float c, float d) { return ff_add(ff_prod(a, b), ff_neg(ff_prod(c, d))); }
-    static __device__ __forceinline__ void maxf(FF& m, FF x) {
-        if (x.h > m.h || (x.h == m.h && x.l > m.l)) m = x;
-    }
-    // w: the boundary weight, a power of two
-    __device__ __forceinline__ void add(const float B[3], const float J[3], float b2, float D, float w) {
-        const float mj = fmaxf(fmaxf(fabsf(J[0]), fabsf(J[1])), fabsf(J[2])), mb = fmaxf(fmaxf(fabsf(B[0]), fabsf(B[1])), fabsf(B[2]));
-        if (!((mj == 0.f || (mj > 1e-10f && mj < 1e8f)) && mb > 1e-10f && mb < 1e8f)) {
-            const double Bd[3] = {B[0], B[1], B[2]}, Jd[3] = {J[0], J[1], J[2]};
-            slow.add(Bd, Jd, (double)b2 * (double)D * (double)w);
+    // B and J of an FP32 run: the squares of the components' products are far inside the
+    // range of doubles, so |J||B| is one square root, the maxima are those of the squares,
+    // and neither root nor quotient is an IEEE one: 34 FP64 operations a point against 85
+    // (an SM issues one FP64 warp instruction in 15 clocks; conversions and comparisons of
+    // doubles count too, so both are made of integer operations).  A 128x128x256 refresh
+    // takes 447 us with it, 684 with add() alone.  (Pairs of floats, 312 us, hold 46 bits of
+    // each term, and fewer where a square's lower half is subnormal.)  Where J, J x B or B
+    // is zero, or something is not finite, add()'s form.
+    __device__ __forceinline__ void addf(const float Bf[3], const float Jf[3], float b2, float Dw) {
+        bool plain = true;
+        const double B0 = widen(Bf[0], plain), B1 = widen(Bf[1], plain), B2 = widen(Bf[2], plain);
+        const double J0 = widen(Jf[0], plain), J1 = widen(Jf[1], plain), J2 = widen(Jf[2], plain);
+        const double b2w = widen(b2, plain), Dww = widen(Dw, plain);
+        const double bp = fma(B1, B1, B0 * B0), bb = fma(B2, B2, bp), z = B2 - 1.0;
+        const double jj = fma(J2, J2, fma(J1, J1, J0 * J0));
+        const double cx = fma(J1, B2, -(J2 * B1)), cy = fma(J2, B0, -(J0 * B2)), cz = fma(J0, B1, -(J1 * B0));
+        const double cc = fma(cz, cz, fma(cy, cy, cx * cx)), xx = jj * bb;
+        if (!(plain && normal(cc) && normal(xx))) {
+            const double Bd[3] = {Bf[0], Bf[1], Bf[2]}, Jd[3] = {Jf[0], Jf[1], Jf[2]};
+            add(Bd, Jd, (double)b2 * (double)Dw);
             return;
         }
-        const FF bb = sq(B[0], B[1], B[2]), jj = sq(J[0], J[1], J[2]);
-        const FF bn = ff_sqrt(bb), jn = ff_sqrt(jj), jb = ff_mul(jn, bn);
-        const FF cn = ff_sqrt(norm2(cr(J[1], B[2], J[2], B[1]), cr(J[2], B[0], J[0], B[2]), cr(J[0], B[1], J[1], B[0])));
-        s[0] = ff_add(s[0], cn);
-        s[1] = ff_add(s[1], jb);
-        if (jb.h > 0.f) s[2] = ff_add(s[2], ff_div(cn, jb));
-        const FF e = ff_prod(b2, D), z = ff_two_sum(B[2], -1.f);
-        s[3] = ff_add(s[3], FF{e.h * w, e.l * w});
-        s[4] = ff_add(s[4], ff_add(ff_add(ff_prod(B[0], B[0]), ff_prod(B[1], B[1])), ff_mul(z, z)));
-        maxf(m[0], bb);
-        maxf(m[1], jj);
+        const InvSqrt c(cc), x(xx);
+        const double cn = c.root();
+        s[0] += cn;
+        s[1] += x.root();
+        s[2] = fma(cn, x.inverse(), s[2]);
+        s[3] = fma(b2w, Dww, s[3]);
+        s[4] += fma(z, z, bp);
+        max_nn(m2[0], bb);
+        max_nn(m2[1], jj);
     }
-    __device__ __forceinline__ DiagSums total() const {
-        DiagSums t = slow;
-        for (int q = 0; q < 5; q++) t.s[q] += ff_double(s[q]);
-        for (int q = 0; q < 2; q++) t.m[q] = fmax(t.m[q], sqrt(ff_double(m[q])));
-        return t;
+    __device__ __forceinline__ void finish() {
+        for (int q = 0; q < 2; q++) m[q] = fmax(m[q], sqrt(m2[q]));
     }
 };
 
@@ -884,15 +867,14 @@ constexpr int kDiagThreads = 128;
 // J (unless a current's own kernel has written it) and the reductions at the
 // current grid, from the exported B and Delta with their face ghosts as
 // k_b_field leaves them (diagnostics.cu:12-134).  One partial per CTA, in a fixed order.
-// FP32: dependent float-pair sums, so warps count more than registers (128x128x256:
-// 224 us at 16 warps an SM and 128 registers, 175 at 32 and 64, with some spills; at
-// 40 and 48 slower again).  FP64 does not care (its pipe is full).
+// Both precisions fill the FP64 pipe (16 warps an SM and 128 registers; in FP32 a
+// 128x128x256 refresh takes 447 us so, 462 at 32 warps and 64 registers with some spills).
 template <typename T, bool JOUT>
-__global__ void __launch_bounds__(kDiagThreads, sizeof(T) == 4 ? 8 : 4) k_diag_field(const __grid_constant__ StageArgs<T> a) {
+__global__ void __launch_bounds__(kDiagThreads, 4) k_diag_field(const __grid_constant__ StageArgs<T> a) {
     const KP<T>& p = a.p;
     const int nx = p.nx, ny = p.ny, nz = p.nz, cur = a.st->cur;
     const long long nx2 = nx + 2, nxy2 = (long long)(nx + 2) * (ny + 2);
-    typename std::conditional<sizeof(T) == 4, DiagSumsF, DiagSums>::type sums;
+    DiagSums sums;
     double e2 = 0, u2 = 0, um = 0;
     T q1m = 0, wm = (T)(sizeof(T) == 4 ? FLT_MAX : DBL_MAX), dm = wm;
     bool convex = true;
@@ -933,7 +915,7 @@ __global__ void __launch_bounds__(kDiagThreads, sizeof(T) == 4 ? 8 : 4) k_diag_f
         q1m = fmax(q1m, sqrt(jxb[0] * jxb[0] + jxb[1] * jxb[1] + jxb[2] * jxb[2]) / b2);
         const int bound = (i == 0) + (j == 0) + (k == 0) + (i == nx - 1) + (j == ny - 1) + (k == nz - 1);
         const T w = (T)1 / (T)(1 << bound);
-        if constexpr (sizeof(T) == 4) sums.add(Bc, Jv, b2, D, w);
+        if constexpr (sizeof(T) == 4) sums.addf(Bc, Jv, b2, D * w);
         else sums.add(Bc, Jv, b2 * D * w);
         if (p.wantXbAn) {
             // distance to the analytically relaxed grid (maths.cu:332-377)
@@ -988,11 +970,9 @@ __global__ void __launch_bounds__(kDiagThreads, sizeof(T) == 4 ? 8 : 4) k_diag_f
             }
         wm = fmin(wm, wmin);
     }
-    DiagSums tot;
-    if constexpr (sizeof(T) == 4) tot = sums.total();
-    else tot = sums;
-    double v[R_COUNT] = {tot.s[0], tot.s[1], tot.s[2], tot.s[3], tot.s[4], e2, u2,
-                         (double)q1m, tot.m[0], tot.m[1], um, (double)dm, (double)wm, convex ? 1.0 : -1.0};
+    sums.finish();
+    double v[R_COUNT] = {sums.s[0], sums.s[1], sums.s[2], sums.s[3], sums.s[4], e2, u2,
+                         (double)q1m, sums.m[0], sums.m[1], um, (double)dm, (double)wm, convex ? 1.0 : -1.0};
     // fixed-order reduction: within the warps, then over them
     __shared__ double red[kDiagThreads / 32][R_COUNT];
 #pragma unroll

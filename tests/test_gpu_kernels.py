@@ -255,3 +255,32 @@ def test_exported_ghosts_are_the_wrapped_points(shape, peri, precision):
                 v = np.moveaxis(w, axis, 0)
                 v[0], v[-1] = v[-2].copy(), v[1].copy()
         np.testing.assert_array_equal(f, w)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("scale", [2.0 ** -33, 2.0 ** -30, 2.0 ** -24, 2.0 ** -20])
+def test_reductions_of_a_weak_current_keep_their_bits(scale, precision):
+    """J of 1e-10 to 1e-6 along a field that it turns by as little, so |J x B| is of the order
+    of J^2 and its square near the lower end of single precision.  A grid of exact
+    spacings, so J comes from B0 alone.  The terms are off by a few roundings of a double
+    and the sums by as many as the reduction tree is deep (12): 20 of 2^-53, and the
+    maxima, a root of a sum of three squares, by 1 ulp."""
+    p = configs.random_braid(1, shape=(17, 9, 25), precision=precision)
+    p.xPeri = p.yPeri = 0
+    p = configs.derive(p)
+    B0, x = configs.init_state(p)
+    B0[..., 0], B0[..., 1], B0[..., 2] = -scale * x[..., 1], scale * x[..., 0], 1
+    g = Relaxation(p)
+    g.upload(x, B0)
+    r = g.refresh()
+    f = g.download()
+    g.close()
+    B, J = (a.astype(np.longdouble) for a in (inner(f["B"]), f["J"]))
+    jn, bn = np.sqrt((J * J).sum(-1)), np.sqrt((B * B).sum(-1))
+    cn = np.sqrt((np.cross(J, B) ** 2).sum(-1))
+    assert 1e-10 < float(jn.max()) < 1e-5 and float(cn.max()) < 10 * float(jn.max()) ** 2
+    want = dict(residual=cn.sum() / (jn * bn).sum(), residualPw=(cn / (jn * bn)).mean())
+    for k, v in want.items():
+        assert abs(r[k] / v - 1) < 20 * 2.0 ** -53, (k, r[k], v)
+    for k, v in dict(BMax=bn.max(), JMax=jn.max()).items():
+        assert abs(r[k] / v - 1) <= 2.0 ** -52, (k, r[k], v)
