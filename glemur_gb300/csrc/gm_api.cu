@@ -501,7 +501,7 @@ struct Impl : ImplBase {
         if (use_fields && !stall_on) {
             const StageArgs<T> a = args(n);
             const bool own = kp.jOct || kp.jQuint || kp.jTri;
-            CUDA_TRY(gmk::launch_b_field<T>(a, own, 0, stream));
+            CUDA_TRY(gmk::launch_b_field<T>(a, own ? gmk::B_OUT : gmk::B_FIELD, 0, stream));
             if (own) {
                 // these currents read B at the edge neighbours too, with the
                 // reference's ghost values (current() before kk(), main.cu:272-281)
@@ -811,7 +811,7 @@ struct Impl : ImplBase {
             return GM_OK;
         }
         const bool own = kp.jOct || kp.jQuint || kp.jTri;
-        CUDA_TRY(gmk::launch_b_field<T>(a, 1, 1, stream));
+        CUDA_TRY(gmk::launch_b_field<T>(a, gmk::B_EXPORT, 1, stream));
         if (own) {
             CUDA_TRY(gmk::launch_export_ghosts<T>(kp, outB, outD, stream));
             CUDA_TRY(gmk::launch_j_own<T>(a, 1, stream));

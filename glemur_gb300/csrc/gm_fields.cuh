@@ -17,7 +17,8 @@
 //   * gm_refresh and the convergence checks of a batch.
 //
 // In FP64 a point's arithmetic is that of the tile kernel (gm_stage_tma.cuh),
-// operation by operation, so results do not depend on which of the two ran.  In
+// operation by operation, so results do not depend on which of the two ran (the B and
+// Delta that gm_refresh exports are the general tile kernel's).  In
 // FP32 B, J and the velocity's increments keep the formulas of the general tile
 // kernel (`kPlain`): J is a difference quotient of B, and its rounding (1e-5 of
 // |J| on 128x128x256) enters the velocity and the exported J at first order, so
@@ -123,8 +124,11 @@ __device__ __forceinline__ void b_plain(const KP<T>& p, const GlobalX<T>& X, con
 
 // B at the inner points and on the faces next to them (line-tied: updateBbound's
 // formula; periodic: at the image points).  OUT: B and Delta into the exported
-// arrays; else B and 1/det(a, b, c) (FP32: Delta) into the padded fields BF, RF.
-template <typename T, bool OUT>
+// arrays; else B and 1/det(a, b, c) (FP32: Delta) into the padded fields BF, RF.  PLAIN:
+// by the general tile kernel's formulas, for FP32 and for what gm_refresh exports: the
+// folded constants of the other form are one more rounding each (FP64 braids: B off by
+// 2.2e-16 of its norm against 1.8e-16, Delta by 2.0e-16 against 1.7e-16).
+template <typename T, bool OUT, bool PLAIN>
 __global__ void __launch_bounds__(field_threads<T>()) k_b_field(const __grid_constant__ StageArgs<T> a, int always) {
     const KP<T>& p = a.p;
     after_previous();
@@ -164,7 +168,7 @@ __global__ void __launch_bounds__(field_threads<T>()) k_b_field(const __grid_con
     const GlobalX<T> X = at_point(p, stage_input(a), a.B0s, g);
     const bool tied = (face == 0 && !p.xPeri) || (face == 1 && !p.yPeri) || (face == 2 && !p.zPeri);
     T B[3], r, D;
-    if (kPlain<T>) {
+    if (PLAIN) {
         const GlobalTile<T> t{p, stage_input(a)};
         if (tied && face == 0) b_face<T>(p, t, a.B0, 0, i, j, k, B, &D);
         else if (tied && face == 1) b_face<T>(p, t, a.B0, 1, i, j, k, B, &D);
@@ -1013,7 +1017,10 @@ cudaError_t launch_b_field(const StageArgs<T>& a, int out, int always, cudaStrea
     const long long n = a.p.N + 2ll * ((long long)a.p.ny * a.p.nz + (long long)a.p.nx * a.p.nz + (long long)a.p.nx * a.p.ny);
     const int t = field_threads<T>();
     const unsigned nb = (unsigned)((n + t - 1) / t);
-    return launch_next(out ? k_b_field<T, true> : k_b_field<T, false>, nb, t, 0, s, a, always);
+    auto kern = out == B_EXPORT ? k_b_field<T, true, true>
+                : out == B_OUT  ? k_b_field<T, true, kPlain<T>>
+                                : k_b_field<T, false, kPlain<T>>;
+    return launch_next(kern, nb, t, 0, s, a, always);
 }
 
 template <typename T>

@@ -164,7 +164,9 @@ struct StageArgs {
 };
 
 // Host-side launchers (explicitly instantiated for float and double).
-// field kernels (gm_fields.cuh)
+// field kernels (gm_fields.cuh).  B goes into the field that the stage kernel reads, into
+// the exported arrays for a current's own kernel, or there as gm_refresh exports it
+enum { B_FIELD = 0, B_OUT = 1, B_EXPORT = 2 };
 template <typename T>
 cudaError_t launch_b_field(const StageArgs<T>& a, int out, int always, cudaStream_t s);
 template <typename T>
