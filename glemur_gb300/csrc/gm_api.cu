@@ -333,19 +333,25 @@ struct Impl : ImplBase {
         if (use_tma) {
             if ((rc = init_tma(nsm))) return rc;
         }
-        // Stages by the field kernels (gm_fields.cuh): FP64 frictional Stokes runs,
-        // the inertial equation and the currents other than Stokes.  Where
-        // their B field does not fit the device's memory, the tile kernels stay.
-        const bool stokes = strncmp(p->jMethod, "Stokes ", 7) == 0;
-        use_fields = p->stageKernel == 0 && !batched && !kp.jxbAver && (sizeof(T) == 8 || !stokes || kp.inertia);
-        if (use_fields && (stokes || kp.jClassic) && cudaMalloc((void**)&BF, 4 * (size_t)kp.cs * sizeof(T)) != cudaSuccess) {
-            cudaGetLastError();
-            BF = nullptr;
-            use_fields = false;
-        }
         const int np = std::max(nparts, gmk::diag_blocks<T>(kp.N));
         if ((rc = alloc((void**)&part, (size_t)np * gmk::R_COUNT * sizeof(double)))) return rc;
         if ((rc = alloc((void**)&red, (gmk::R_COUNT + 1) * sizeof(double)))) return rc;   // + eps*
+        // Stages by the field kernels (gm_fields.cuh): FP64 frictional Stokes runs,
+        // the inertial equation and the currents other than Stokes.  Their B field
+        // is taken last, and only where it leaves room for what the driver allocates
+        // when kernels and graphs are first used; else the tile kernels stay.
+        const bool stokes = strncmp(p->jMethod, "Stokes ", 7) == 0;
+        use_fields = p->stageKernel == 0 && !batched && !kp.jxbAver && (sizeof(T) == 8 || !stokes || kp.inertia);
+        if (use_fields && (stokes || kp.jClassic)) {
+            const size_t bytes = 4 * (size_t)kp.cs * sizeof(T), spare = (size_t)64 << 20;
+            size_t avail = 0, total = 0;
+            CUDA_TRY(cudaMemGetInfo(&avail, &total));
+            if (avail < bytes + spare || cudaMalloc((void**)&BF, bytes) != cudaSuccess) {
+                cudaGetLastError();
+                BF = nullptr;
+                use_fields = false;
+            }
+        }
         CUDA_TRY(cudaStreamSynchronize(stream));
         return GM_OK;
     }
