@@ -600,8 +600,11 @@ struct Impl : ImplBase {
     int autotune(int trials, int* tz_out, double* ms_out) override {
         if (!uploaded) return gm::fail(GM_ENOTREADY, "gm_autotune before gm_upload");
         if (trials < 1) return gm::fail(GM_EPARAM, "gm_autotune: trials must be >= 1");
-        if (!use_tma) {   // the generic kernel's tile is chosen by its own model
-            if (tz_out) *tz_out = TZ;
+        if (!use_tma || use_fields) {
+            // nothing to time: the generic kernel's tile is chosen by its own model, and
+            // the field passes have no tiles (nine depths of the same passes took 9 x 3
+            // rounds of an executable's start in FP64, and kept one by chance)
+            if (tz_out) *tz_out = use_tma ? TZ2 : TZ;
             if (ms_out) *ms_out = 0;
             return GM_OK;
         }
@@ -666,6 +669,7 @@ struct Impl : ImplBase {
         if (!use_tma) return gm::fail(GM_EPARAM, "gm_set_tile_z: the run does not use the TMA stage kernel");
         if (tz < 1 || tz > kp.nz) return gm::fail(GM_EPARAM, "gm_set_tile_z: depth must be 1..nz");
         set_tile(tz);
+        if (use_fields && !stall_on) return GM_OK;      // the captured step has no tiles
         if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
         if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
         return GM_OK;

@@ -282,13 +282,17 @@ int gm_grid_fields(gm_handle* h, void* cellVol, void* convexity, void* wedgeMin)
  * one) with CUDA events on the handle's stream, keeps the fastest and
  * recaptures the step graph.  Stages 0..4 write only the stage buffers, so
  * the state a run starts from is unchanged; results do not depend on the
- * depth.  Call after gm_upload; *tz and *ms (mean time of stages 0..4) may be
- * NULL.  No counterpart in the reference (its block shape is fixed,
+ * depth.  Runs whose stages have no such depth (FP64 runs by the field passes, the
+ * inertial equation, the currents other than Stokes) time nothing: *tz is the
+ * depth chosen at creation and *ms 0.  Call after gm_upload; *tz and *ms (mean
+ * time of stages 0..4) may be NULL.  No counterpart in the reference (its block shape is fixed,
  * src/main.cu:130-137). */
 int gm_autotune(gm_handle* h, int trials, int* tz, double* ms);
-/* Set the stage kernel's z-chunk depth directly (1..nz; the TMA stage kernel
- * only), e.g. to repeat a depth gm_autotune chose; the step graph is
- * recaptured.  No counterpart in the reference. */
+/* Set the TMA stage kernel's z-chunk depth directly (1..nz), e.g. to repeat a depth
+ * gm_autotune chose; the step graph is recaptured.  FP64 runs by the field passes
+ * take it too, as a depth that gm_autotune returned, but have no tiles: it applies
+ * where the tile kernel runs in their place.  Refused for runs the tile kernel
+ * cannot do.  No counterpart in the reference. */
 int gm_set_tile_z(gm_handle* h, int tz);
 /* Failure-detection test hook (no counterpart in the reference, which has no
  * bounded waits).  While `on` is non-zero, the TMA stage kernel's copy

@@ -8,7 +8,7 @@ import pytest
 import cases  # noqa: F401  (tests/golden on the path)
 import make_folded
 from conftest import ROOT, inner, relerr
-from glemur_gb300 import BatchRelaxation, Relaxation, _abi, configs
+from glemur_gb300 import BatchRelaxation, GlemurError, Relaxation, _abi, configs
 
 pytestmark = pytest.mark.gpu
 
@@ -311,3 +311,43 @@ def test_exported_b_and_delta_are_as_exact_as_the_plain_formula(shape):
     off = lambda a, e: float(np.linalg.norm((a - e).astype(np.float64).ravel()) / np.linalg.norm(e.astype(np.float64).ravel()))  # noqa: E731
     assert off(inner(f["B"]), Bx) < 1.15 * off(B, Bx)
     assert off(inner(f["detJac"]), Dx) < 1.15 * off(D, Dx)
+
+
+def test_runs_without_tiles_have_nothing_to_tune():
+    """FP64 runs by the field passes: the autotuner launches nothing and returns the depth
+    chosen at creation, which can be set again (and any other within 1..nz) without
+    changing the run; a tile run is timed, and a run the tile kernel cannot do
+    refuses a depth."""
+    p, x, B0 = case((20, 18, 22), (1, 1, 0), 64)
+    grids = []
+    for tune in (False, True):
+        g = Relaxation(p)
+        g.upload(x, B0, 0.0, 1e-3)
+        if tune:
+            n = g.launches
+            r = g.autotune(2)
+            assert g.launches == n and r["ms_stages_0_4"] == 0 and 1 <= r["tz"] <= p.nz
+            g.steps_async(1)
+            for tz in (r["tz"], 1, p.nz):
+                g.set_tile_z(tz)
+            for tz in (0, p.nz + 1):
+                with pytest.raises(GlemurError):
+                    g.set_tile_z(tz)
+            g.steps_async(2)
+        else:
+            g.steps_async(3)
+        grids.append(g.grid())
+        g.close()
+    np.testing.assert_array_equal(*grids)
+    p, x, B0 = case((20, 18, 22), (1, 1, 0), 32)
+    g = Relaxation(p)
+    g.upload(x, B0, 0.0, 1e-3)
+    n = g.launches
+    assert g.autotune(2)["ms_stages_0_4"] > 0 and g.launches > n
+    g.close()
+    p, x, B0 = case((20, 18, 22), (1, 1, 0), 32, inertia=True)
+    g = Relaxation(p)
+    g.upload(x, B0, 0.0, 1e-3)
+    with pytest.raises(GlemurError):
+        g.set_tile_z(4)
+    g.close()
