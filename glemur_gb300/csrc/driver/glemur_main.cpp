@@ -200,7 +200,13 @@ int main(int argc, char* argv[]) {
     printf("initial B: %s\n", p.bInit);
     if (p.inertia) printf("initial U: %s\n", p.uInit);
     if (p.pressure) printf("include pressure gradient with beta = %f\n", p.beta);
-    printf("tiles = 32 x 12 columns (32 x 4 on small grids), one launch per Runge-Kutta stage, step loop on the device\n");
+    // which of the stage kernels runs (gm_api.cu, Impl::init)
+    if (p.jxbAver)
+        printf("stages: the general tile kernel behind a pass for J, step loop on the device\n");
+    else if (precision == 32 && starts(p.jMethod, "Stokes ") && !p.inertia)
+        printf("stages: tiles of 32 x 12 columns (32 x 4 on small grids), one launch each, step loop on the device\n");
+    else
+        printf("stages: passes over all points for B and then the increment, step loop on the device\n");
     const int rc = precision == 32 ? run<float>(p, activeDevice) : run<double>(p, activeDevice);
     if (rc) return rc;
     printf("glemur terminated successfully\n");

@@ -220,3 +220,23 @@ def test_inertia_run_directory_and_restart(tmp_path):
     np.testing.assert_array_equal(sa.points, sc.points)
     np.testing.assert_array_equal(sa.point_data["ufield"], sc.point_data["ufield"])
     np.testing.assert_array_equal(sa.point_data["bfield"], sc.point_data["bfield"])
+
+
+@pytest.mark.parametrize("precision,inertia,says", [(32, False, "tiles of 32 x 12"), (64, False, "passes over all points"),
+                                                    (32, True, "passes over all points")])
+def test_the_stages_that_run_are_the_ones_named(tmp_path, precision, inertia, says):
+    """Three accepted steps.  The line on standard output against the launches of a step of
+    the same run: 7 by tiles (six stages and the controller), 13 by the two passes."""
+    d = tmp_path / "run"
+    make_run(d, 3, inertia=inertia)
+    out = run_exe(d, precision)
+    lines = [ln for ln in out.splitlines() if ln.startswith("stages: ")]
+    assert len(lines) == 1 and says in lines[0]
+    p = read_params(d, precision)
+    g = Relaxation(p)
+    B0, xb = configs.init_state(p)
+    g.upload(xb, B0)
+    n = g.launches
+    g.steps_async(1)
+    assert g.launches - n == (7 if "tiles" in says else 13)
+    g.close()
