@@ -640,7 +640,7 @@ __global__ void __launch_bounds__(kWideThreads) k_conv_wide(const ConvWideArgs b
 // bytes) against as many of the upstream gradient, [8-channel group][voxel][16 bytes].
 // Accumulators stay in tensor memory over a chain of blocks and are then added to dW.
 // (The tensor core's sums are truncated: the error grows with the products in a
-// chain, 3e-6 of the gradient at 3500 voxels.)  Slices of 5 groups (120 rows) take
+// chain, 3e-6 of the gradient at 3500 voxels; kWgChain bounds it.)  Slices of 5 groups (120 rows) take
 // fewer MMAs, but the copies bound them, as their planes leave room for two a block
 // (72 -> 24 channels at 64x64x128: 195 us).
 //
@@ -651,6 +651,7 @@ __global__ void __launch_bounds__(kWideThreads) k_conv_wide(const ConvWideArgs b
 // 8-11 the upstream gradient, one thread of warp 12 issues the MMAs; an accumulator's
 // next chain starts when it has been read.
 constexpr int kWgKb = 6, kWgGroups = 3, kWgN = 48, kWgThreads = 416;
+constexpr long long kWgChain = 22528;
 constexpr int kDoutGroup = 128 * 16;           // one plane of 8 output channels
 
 struct WgradArgs {
@@ -1419,11 +1420,14 @@ int gm_nn_conv_wgrad(const void* dout, int ldd, int co, const void* in1, int ld1
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     // planes per block and CTAs along the blocks: one wave; a plane's MMAs take 3300
     // clocks, a block about 1000 more, its copies 1 clock per 7.5 bytes; vchunk asks for at least that many voxels a CTA.
-    // Chains of lim voxels are those of four CTAs per SM with 128 of the stacked (tap,
-    // channel) rows each; a chain is no longer (the truncation error no larger), and where
-    // the voxels are many no more than 3000 voxels (1500 of chains beyond 8000) shorter, so
-    // that the error is the same to 1e-5 of the gradient.
-    const long long lim = std::max(512ll, V * ((27 * ng * 8 + 127) / 128) / (4 * nsm));
+    // Chains of lim voxels are those of 608 CTAs (four on each of 152 SMs) with 128 of the
+    // stacked (tap, channel) rows each; a chain is no longer (the truncation error no
+    // larger), and where the voxels are many no more than 3000 voxels (1500 of chains
+    // beyond 8000) shorter, so that the error is the same to 1e-5 of the gradient.  No chain
+    // is longer than kWgChain, so that on larger grids the error stops growing with them
+    // (72 -> 24 channels at 128x128x256: 110,080 voxels, 1.5e-4 of the gradient and 1355 us
+    // without it, 2.6e-5 and 1167 with it).
+    const long long lim = std::min(gmnn::kWgChain, std::max(512ll, V * ((27 * ng * 8 + 127) / 128) / 608));
     const long long shorter = lim > 8000 ? 1500 : 3000;
     const long long slices = (long long)a.cslices * nslices;
     double tbest = 0;

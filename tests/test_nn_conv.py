@@ -191,3 +191,60 @@ def test_elementwise_passes(c, ld):
     run("gm_nn_bias_grad", P(fine), ld, c, V, C.cast(db.data_ptr(), C.POINTER(C.c_float)))
     size = fine.double().abs().sum(0)[:c] + 1
     assert bool(((db[:c].double() - 1 - fine.double().sum(0)[:c]).abs() <= size * V * 2.0 ** -23).all()) and float(db[c]) == 1
+
+
+def _wgrad(x, d, n, ci, co, xper, yper, chunk):
+    """The kernel's gradient of [V, >= ci] inputs and [V, >= co] upstream gradients, and the
+    same sums in FP64 by torch."""
+    import torch
+    from glemur_gb300 import _abi
+    nx, ny, nz = n
+    dW = torch.zeros(27, co, ci, device="cuda")
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    P = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    torch.cuda.synchronize()
+    _abi.check(_abi.load().gm_nn_conv_wgrad(P(d), d.shape[1], co, P(x), x.shape[1], x.shape[1], None, 0, 0,
+                                            C.cast(dW.data_ptr(), C.POINTER(C.c_float)), ci, nx, ny, nz, xper, yper, chunk,
+                                            P(st), None), "gm_nn_conv_wgrad")
+    torch.cuda.synchronize()
+    assert int(st[0]) == 0
+    v = torch.zeros(nz + 2, ny + 2, nx + 2, ci, device="cuda", dtype=torch.float64)
+    v[1:-1, 1:-1, 1:-1] = x[:, :ci].double().view(nz, ny, nx, ci)
+    if xper:
+        v[:, :, 0], v[:, :, -1] = v[:, :, -2].clone(), v[:, :, 1].clone()
+    if yper:
+        v[:, 0], v[:, -1] = v[:, -2].clone(), v[:, 1].clone()
+    g = d[:, :co].double()
+    ref = torch.stack([g.T @ v[t // 9:t // 9 + nz, t // 3 % 3:t // 3 % 3 + ny, t % 3:t % 3 + nx].reshape(-1, ci) for t in range(27)])
+    return dW.double(), ref
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,ci,co,xper,yper,chunk", [((64, 64, 128), 72, 24, 1, 1, 0), ((64, 64, 128), 3, 24, 1, 1, 0),
+                                                     ((60, 50, 75), 24, 20, 0, 1, 65536), ((32, 32, 64), 100, 70, 1, 0, 0),
+                                                     ((70, 41, 90), 16, 3, 1, 1, 131072), ((80, 80, 280), 20, 8, 1, 1, 896000)])
+def test_conv_wgrad_of_whole_numbers_is_exact(n, ci, co, xper, yper, chunk):
+    """Operands -3 .. 3: every partial sum is a whole number below 2^24 (9 x 1,792,000), so a
+    lost or doubled tile, plane or chain shows as itself.  Several blocks a chain and
+    several chains a block of threads."""
+    import torch
+    V = n[0] * n[1] * n[2]
+    g = torch.Generator(device="cuda").manual_seed(4)
+    whole = lambda c: torch.randint(-3, 4, (V, (c + 7) // 8 * 8), device="cuda", generator=g).to(torch.bfloat16)  # noqa: E731
+    got, ref = _wgrad(whole(ci), whole(co), n, ci, co, xper, yper, chunk)
+    assert torch.equal(got, ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,ci,co", [((64, 64, 128), 72, 24), ((128, 128, 256), 72, 24)])
+def test_conv_wgrad_error_is_bounded_on_any_grid(n, ci, co):
+    """Sums of one sign mostly.  A chain of at most 22,528 voxels is 1408 truncated additions;
+    each takes half of 2^-23 of the sum on average, which is half its final value on
+    average: 1408 x 2^-23 / 4 = 4.2e-5 of the gradient."""
+    import torch
+    V = n[0] * n[1] * n[2]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(V, (ci + 7) // 8 * 8, device="cuda", generator=g).relu().to(torch.bfloat16)
+    d = (torch.randn(V, (co + 7) // 8 * 8, device="cuda", generator=g) + 0.3).to(torch.bfloat16)
+    got, ref = _wgrad(x, d, n, ci, co, 1, 1, 0)
+    assert float((got - ref).norm() / ref.norm()) < 1408 * 2.0 ** -23 / 4
