@@ -1356,6 +1356,7 @@ int gm_nn_conv(const void* in1, int ld1, int c1, const void* in2, int ld2, int c
     if (Kc % 16 || Kc < 16 || Kc > 256 || Np % 16 || Np < 16 || Np > 256 || c1 + (in2 ? c2 : 0) > Kc || co > Np ||
         c1 % 8)
         return gm::fail(GM_EPARAM, "gm_nn_conv: channel counts out of range");
+    if (nx < 1 || ny < 1 || nz < 1) return gm::fail(GM_EPARAM, "gm_nn_conv: grid out of range");
     int rc;
     if ((rc = check_view_align(in1, ld1, "gm_nn_conv in1")) || (rc = check_view_align(in2, ld2, "gm_nn_conv in2")))
         return rc;

@@ -233,3 +233,14 @@ def test_executable_without_a_gpu_stops_before_any_output(tmp_path):
     assert r.returncode != 0
     assert "could not locate CUDA devices" in r.stdout or "no CUDA compatible devices" in r.stdout
     assert list(tmp_path.iterdir()) == []
+
+
+@pytest.mark.parametrize("n", [(0, 8, 8), (8, 0, 8), (8, 8, 0), (-8, 8, 8), (8, -40, 8), (8, 8, -1)])
+def test_convolutions_refuse_an_empty_grid(n):
+    """Before anything is launched: as a grid of no blocks is refused by the runtime."""
+    lib = _abi.load()
+    p = C.c_void_p(1 << 12)                 # not read: the sizes are looked at first
+    f = C.cast(p, C.POINTER(C.c_float))
+    assert lib.gm_nn_conv(p, 16, 16, None, 0, 0, p, None, p, 16, 16, None, 0, 0, *n, 1, 1, 16, 16, p, None) == -1
+    assert "grid" in lib.gm_last_error().decode()
+    assert lib.gm_nn_conv_wgrad(p, 16, 16, p, 16, 16, None, 0, 0, f, 16, *n, 1, 1, 0, p, None) == -1
