@@ -35,7 +35,7 @@
 namespace gmk {
 
 constexpr int HX2 = TX + 4;              // row pitch of position, B0s and B planes: the tile + 2-point halo
-constexpr unsigned kWaitLimit = 1u << 22;
+constexpr unsigned kWaitLimit = 1u << 20;      // polls: about 1.3 s
 
 // Tile of NW warps: 32 x 2 NW columns.
 template <int NW>

@@ -297,7 +297,7 @@ int gm_set_tile_z(gm_handle* h, int tz);
 /* Failure-detection test hook (no counterpart in the reference, which has no
  * bounded waits).  While `on` is non-zero, the TMA stage kernel's copy
  * producer withholds the copies of each tile's first position planes, so
- * every CTA's bounded wait for them (2^22 polls each) runs out: the CTA
+ * every CTA's bounded wait for them (2^20 polls each) runs out: the CTA
  * records GM_ST_TIMEOUT in the status word, waits (bounded) for the copies
  * it did issue and returns; the step is neither accepted nor used to adapt
  * dt, and the run stops with GM_ETIMEOUT.  No copy is left in flight and no

@@ -125,7 +125,9 @@ def test_convolution_wait_runs_out_and_is_reported():
 def test_waits_run_out_over_several_waves_of_blocks():
     """More blocks than the device holds at once: the later ones start while the
     earlier ones record their time-outs, and each of them either runs its own waits
-    out or leaves as a whole."""
+    out or leaves as a whole.  A block gives up some six waits of about a second in turn
+    (four for planes, two for copies that may be in flight)."""
+    import time
     p = configs.random_braid(3, shape=(128, 96, 64), precision=32)
     B0, xb = configs.init_state(p)
     lib = _abi.load()
@@ -133,8 +135,10 @@ def test_waits_run_out_over_several_waves_of_blocks():
     g.upload(xb, B0)
     g.set_tile_z(4)
     _abi.check(lib.gm_debug_stall(g.h, 1), "gm_debug_stall")
+    began = time.monotonic()
     with pytest.raises(GlemurError, match="GM_ETIMEOUT"):
         g.run(2)
+    assert time.monotonic() - began < 16
     s = g.state()
     assert s["status"] & _abi.GM_ST_TIMEOUT and s["timeIndex"] == 0 and s["nAttempted"] == 1
     _abi.check(lib.gm_debug_stall(g.h, 0), "gm_debug_stall")
