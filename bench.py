@@ -234,19 +234,20 @@ class NvmlClocks:
                 "reasons": reasons, "samples": len(self.samples), "sampler": "nvml, ~1 ms"}
 
 
-def traffic_per_launch(p):
-    """DRAM bytes per stage launch from the committed ncu summary, if any."""
+def traffic_per_launch(p, kernel=""):
+    """DRAM bytes per stage launch from the committed ncu summary, if any: of the pair
+    kernel (kernel="_pairs"), or of the one-point kernel before it."""
     f = ROOT / "profiles" / "stage_kernel_traffic.json"
     if not f.exists():
         return None, None
     d = json.loads(f.read_text())
-    key = f"{p.nx}x{p.ny}x{p.nz}_fp{p.precision}" + ("_pressure" if p.pressure else "")
+    key = f"{p.nx}x{p.ny}x{p.nz}_fp{p.precision}" + ("_pressure" if p.pressure else "") + kernel
     e = d.get(key)
     if e:
         return float(e["bytes_per_launch"]), e.get("source")
     # a per-point figure measured on a smaller grid of the same kernel scales
     # with the inner points (the traffic is streaming: each plane once)
-    e = d.get(f"per_point_fp{p.precision}" + ("_pressure" if p.pressure else ""))
+    e = d.get(f"per_point_fp{p.precision}" + ("_pressure" if p.pressure else "") + kernel)
     if not e:
         return None, None
     n = p.nx * p.ny * p.nz
@@ -502,7 +503,7 @@ def run_gpu(args):
     alg_bytes = BYTES_PER_CELL_STAGE[p.precision] * N
     achieved = alg_bytes / (launch_ms / 1e3) / 1e9
     peak, peak_kind = peaks()
-    traffic, traffic_src = traffic_per_launch(p)
+    traffic, traffic_src = traffic_per_launch(p, "_pairs")
 
     # --- end to end through the C-ABI with host buffers ------------------------
     xb_h = torch.from_numpy(xb).pin_memory()

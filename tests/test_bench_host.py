@@ -106,3 +106,18 @@ def test_reference_arm_loads_no_product_library():
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600, cwd=bench.ROOT)
     assert r.returncode == 0, r.stderr[-2000:]
     assert "CLEAN" in r.stdout and "NO_PACKAGE" in r.stdout, r.stdout[-500:]
+
+
+def test_the_bench_line_reports_the_pair_kernels_traffic():
+    """The figures of the kernel that runs, from the tables of its captures (sums over the
+    six stages, MB); the one-point kernel's stay beside them."""
+    reads, writes = (115.1, 169.1, 224.3, 278.6, 333.0, 383.6), (65.5, 74.9, 80.6, 84.0, 86.6, 46.5)
+    t, src = bench.traffic_per_launch(configs.braid6(128, 128, 256, precision=32), "_pairs")
+    assert abs(t - (sum(reads) + sum(writes)) / 6 * 1e6) < 1e3 and "pair kernel" in src
+    table = (bench.ROOT / "profiles" / "k_stage_tma_braid6_128x128x256.md").read_text()
+    assert all(f"| {r} (" in table and f"| {w} (" in table for r, w in zip(reads, writes))
+    t, src = bench.traffic_per_launch(configs.braid6_large(256, 256, 512, precision=32), "_pairs")
+    per_point = (120.1 + 175.5 + 228.3 + 279.5 + 330.2 + 380.4 + 63.3 + 72.6 + 77.3 + 80.9 + 84.2 + 44.9) / 6e-6 / (128 * 128 * 256)
+    assert abs(t / (256 * 256 * 512) - per_point) < 0.01 and "pair kernel" in src
+    import inspect
+    assert 'traffic_per_launch(p, "_pairs")' in inspect.getsource(bench)
