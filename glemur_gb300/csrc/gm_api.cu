@@ -327,8 +327,8 @@ struct Impl : ImplBase {
         smem_diag = gmk::stage_smem_bytes<T>(TY, gmk::MODE_DIAG, p->pressure);
         nparts = (int)(grid.x * grid.y * grid.z);
         // the TMA kernel computes the Stokes current of the frictional
-        // equation only; the other currents, the inertial equation and the
-        // averaged Lorentz force run in the generic kernel
+        // equation only; the other currents and the inertial equation run in the
+        // field kernels, the averaged Lorentz force in the generic kernel
         use_tma = p->stageKernel == 0 && strncmp(p->jMethod, "Stokes ", 7) == 0 && !p->inertia && !p->jxbAver;
         if (use_tma) {
             if ((rc = init_tma(nsm))) return rc;

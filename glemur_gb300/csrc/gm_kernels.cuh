@@ -59,7 +59,6 @@ inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, unsigned threads
     return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 
-
 constexpr int TX = 32;          // tile width in x = one warp
 constexpr int XRING = 5;        // planes of positions held in shared memory
 constexpr int BRING = 4;        // planes of B held in shared memory
@@ -95,10 +94,10 @@ struct KP {
     T Lx, Ly, Lz, Ox, Oy, Oz;
     int xPeri, yPeri, zPeri, zUpdate, errMode, refDt;
     int jClassic;            // jMethod = "Classic": the finite-difference current
-    int jOct;                // jMethod = "Stokes4th": J from the octilateral pass (outJ; generic kernel only)
-    int jQuint;              // jMethod = "StokesQuint": J from the quintilateral pass (outJ; generic kernel only)
+    int jOct;                // jMethod = "Stokes4th": J from the octilateral pass (outJ)
+    int jQuint;              // jMethod = "StokesQuint": J from the quintilateral pass (outJ)
     int jTri;                // jMethod = "StokesTri": J from the same pass in its triangle-only form
-    int inertia;             // the velocity equation (generic kernel only)
+    int inertia;             // the velocity equation
     T nu;                    // velocity damping
     int jxbAver;             // neighbour-averaged Lorentz force (generic kernel only)
     T jxbW;                  // its weight

@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(kPlaneThreads) k_conv_planes(const ConvPlaneAr
 // ---- convolution with many input channels -------------------------------------------
 
 // The same with the weights streamed, for layers whose weights do not fit the
-// shared memory: for each tap (along z first, k_conv's order) and chunk of
+// shared memory: for each tap (along z first) and chunk of
 // input channels a stage of Nt x kch weights, used for the kz output planes of
 // the item; the planes in a ring of at least kz + 1 buffers with all channels.
 // Warps 0-3 store, 4-7 copy planes, the next copy weights (the latency of

@@ -314,8 +314,8 @@ int gm_download_k(gm_handle* h, int m, void* k);
 
 /* Grid buffers of the last step in the reference layout (ghosted AoS):
  * which = 0..4: stage position x_{which+1} written by stage `which`
- * (the xb_tmp of src/rungeKutta.cu:234); 5: x_6, the start grid of a
- * rejected retry; 6: x_new of the combine (src/rungeKutta.cu:345). */
+ * (the xb_tmp of src/rungeKutta.cu:234); 5: the start grid of a
+ * rejected retry (x_6, which is x_0 up to rounding: the grid the step began with); 6: x_new of the combine (src/rungeKutta.cu:345). */
 int gm_download_x(gm_handle* h, int which, void* xb);
 
 /* Velocity of an inertia run (inertia = T), inner points, AoS 3*nx*ny*nz in
