@@ -834,7 +834,7 @@ struct DiagSums {
     // and neither root nor quotient is an IEEE one: 34 FP64 operations a point against 85
     // (an SM issues one FP64 warp instruction in 15 clocks; conversions and comparisons of
     // doubles count too, so both are made of integer operations).  A 128x128x256 refresh
-    // takes 447 us with it, 684 with add() alone.  (Pairs of floats, 312 us, hold 46 bits of
+    // takes 425 us with it, about 660 with add() alone.  (Pairs of floats, 312 us, hold 46 bits of
     // each term, and fewer where a square's lower half is subnormal.)  Where J, J x B or B
     // is zero, or something is not finite, add()'s form.
     __device__ __forceinline__ void addf(const float Bf[3], const float Jf[3], float b2, float Dw) {
@@ -871,8 +871,10 @@ constexpr int kDiagThreads = 128;
 // J (unless a current's own kernel has written it) and the reductions at the
 // current grid, from the exported B and Delta with their face ghosts as
 // k_b_field leaves them (diagnostics.cu:12-134).  One partial per CTA, in a fixed order.
-// Both precisions fill the FP64 pipe (16 warps an SM and 128 registers; in FP32 a
-// 128x128x256 refresh takes 447 us so, 462 at 32 warps and 64 registers with some spills).
+// Both precisions fill the FP64 pipe (FP32: 86 % active, 40 instructions a point) at 16
+// warps an SM and 128 registers, in one wave of CTAs: a CTA's own reduction is another 70 of
+// its threads' FP64 instructions (128x128x256 in FP32, the refresh: 425 us; two waves 447,
+// 32 warps and 64 registers with some spills 462).
 template <typename T, bool JOUT>
 __global__ void __launch_bounds__(kDiagThreads, 4) k_diag_field(const __grid_constant__ StageArgs<T> a) {
     const KP<T>& p = a.p;

@@ -170,7 +170,7 @@ template <typename T>
 cudaError_t launch_b_field(const StageArgs<T>& a, int out, int always, cudaStream_t s);
 template <typename T>
 cudaError_t launch_diag_field(const StageArgs<T>& a, int jout, cudaStream_t s);
-constexpr int kMaxDiagBlocks = 152 * 8;
+constexpr int kMaxDiagBlocks = 152 * 4;      // the CTAs that k_diag_field is built for (four an SM)
 template <typename T>
 int diag_blocks(long long N);
 template <typename T>
