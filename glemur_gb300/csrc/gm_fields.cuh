@@ -809,8 +809,9 @@ __device__ __forceinline__ double widen(float x, bool& plain) {
     const unsigned hi = (b & 0x80000000u) | (t ? ((b & 0x7fffffffu) >> 3) + 0x38000000u : 0u);
     return __hiloint2double((int)hi, (int)(b << 29));
 }
-// x > 0, neither subnormal nor infinite nor NaN
-__device__ __forceinline__ bool normal(double x) { return (unsigned)__double2hiint(x) - 0x00100000u < 0x7fe00000u; }
+// +0, or x > 0 and neither subnormal nor infinite nor NaN
+__device__ __forceinline__ bool is_zero(double x) { return (__double2hiint(x) | __double2loint(x)) == 0; }
+__device__ __forceinline__ bool in_range(double x) { return (unsigned)__double2hiint(x) - 0x00100000u < 0x7fe00000u || is_zero(x); }
 
 // The sums and maxima of one thread, in doubles.
 struct DiagSums {
@@ -834,9 +835,9 @@ struct DiagSums {
     // and neither root nor quotient is an IEEE one: 34 FP64 operations a point against 85
     // (an SM issues one FP64 warp instruction in 15 clocks; conversions and comparisons of
     // doubles count too, so both are made of integer operations).  A 128x128x256 refresh
-    // takes 425 us with it, about 660 with add() alone.  (Pairs of floats, 312 us, hold 46 bits of
-    // each term, and fewer where a square's lower half is subnormal.)  Where J, J x B or B
-    // is zero, or something is not finite, add()'s form.
+    // takes 425 us with it, about 660 with add() alone.  (Pairs of floats, 312 us, hold 46
+    // bits of each term, and fewer where a square's lower half is subnormal.)  Where
+    // something is subnormal or not finite, add()'s form.
     __device__ __forceinline__ void addf(const float Bf[3], const float Jf[3], float b2, float Dw) {
         bool plain = true;
         const double B0 = widen(Bf[0], plain), B1 = widen(Bf[1], plain), B2 = widen(Bf[2], plain);
@@ -846,16 +847,16 @@ struct DiagSums {
         const double jj = fma(J2, J2, fma(J1, J1, J0 * J0));
         const double cx = fma(J1, B2, -(J2 * B1)), cy = fma(J2, B0, -(J0 * B2)), cz = fma(J0, B1, -(J1 * B0));
         const double cc = fma(cz, cz, fma(cy, cy, cx * cx)), xx = jj * bb;
-        if (!(plain && normal(cc) && normal(xx))) {
+        if (!(plain && in_range(cc) && in_range(xx))) {
             const double Bd[3] = {Bf[0], Bf[1], Bf[2]}, Jd[3] = {Jf[0], Jf[1], Jf[2]};
             add(Bd, Jd, (double)b2 * (double)Dw);
             return;
         }
         const InvSqrt c(cc), x(xx);
-        const double cn = c.root();
+        const double cn = is_zero(cc) ? 0.0 : c.root();
         s[0] += cn;
-        s[1] += x.root();
-        s[2] = fma(cn, x.inverse(), s[2]);
+        s[1] += is_zero(xx) ? 0.0 : x.root();
+        s[2] = fma(cn, is_zero(xx) ? 0.0 : x.inverse(), s[2]);
         s[3] = fma(b2w, Dww, s[3]);
         s[4] += fma(z, z, bp);
         max_nn(m2[0], bb);

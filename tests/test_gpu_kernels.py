@@ -351,3 +351,46 @@ def test_runs_without_tiles_have_nothing_to_tune():
     with pytest.raises(GlemurError):
         g.set_tile_z(4)
     g.close()
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("what", ["no_current", "aligned", "tiny_field", "not_a_number", "infinite"])
+def test_reductions_of_zeros_and_what_is_not_finite(what, precision):
+    """On a grid of exact spacings: a current of zero, one along the field, a field whose
+    squares underflow in FP32, and a point that is not finite: sums as numpy's on the
+    downloaded fields (NaN where theirs is), maxima that leave NaN out."""
+    p = configs.random_braid(1, shape=(17, 9, 25), precision=precision)
+    p.xPeri = p.yPeri = 0
+    p = configs.derive(p)
+    B0, x = configs.init_state(p)
+    B0[...] = (0, 0, 1)
+    if what == "aligned":
+        B0[..., 0], B0[..., 1] = -0.25 * x[..., 1], 0.25 * x[..., 0]
+        B0[..., 2] = 0
+    if what == "tiny_field":
+        B0 *= 2.0 ** -70
+        B0[..., 0] = 2.0 ** -72 * np.sin(x[..., 1])
+    if what in ("not_a_number", "infinite"):
+        B0[12, 5, 8, 1] = np.nan if what == "not_a_number" else np.inf
+    g = Relaxation(p)
+    g.upload(x, B0)
+    r = g.refresh()
+    f = g.download()
+    g.close()
+    B, J = (a.astype(np.float64) for a in (inner(f["B"]), f["J"]))
+    with np.errstate(all="ignore"):
+        jn, bn = np.sqrt((J * J).sum(-1)), np.sqrt((B * B).sum(-1))
+        cn = np.sqrt((np.cross(J, B) ** 2).sum(-1))
+        both = jn * bn
+        pw = np.where(both > 0, cn / both, 0)
+        want = dict(residual=cn.sum() / both.sum() if both.sum() > 0 or np.isnan(both.sum()) else 0.0, residualPw=pw.mean(),
+                    BMax=np.nanmax(bn), JMax=np.nanmax(jn))
+    if what == "no_current":
+        assert want["JMax"] == 0
+    for k, v in want.items():
+        if np.isfinite(v):
+            assert abs(r[k] - v) <= 1e-13 * abs(v), (k, r[k], v)
+        elif k in ("BMax", "JMax"):
+            assert r[k] == v, (k, r[k], v)
+        else:
+            assert not np.isfinite(r[k]) or (k == "residual" and r[k] == 0), (k, r[k], v)
