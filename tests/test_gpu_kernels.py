@@ -394,3 +394,37 @@ def test_reductions_of_zeros_and_what_is_not_finite(what, precision):
             assert r[k] == v, (k, r[k], v)
         else:
             assert not np.isfinite(r[k]) or (k == "residual" and r[k] == 0), (k, r[k], v)
+
+
+@pytest.mark.parametrize("name", ["braid_f64", "tied_f64", "zperi_f64", "shear_f64", "centershift_tied_f64", "oct_tied_f64", "braid_f32",
+                                  "shear_f32"])
+def test_refresh_matches_the_oracle_on_every_face(name):
+    """What gm_refresh exports, the ghost faces with it: periodic, line-tied, and line-tied on
+    an initially distorted grid."""
+    from oracle.pyoracle import Oracle
+    p = cases.make(name)
+    B0, x = configs.init_state(p)
+    d = np.array([p.dx, p.dy, p.dz])
+    x[1:-1, 1:-1, 1:-1] += (0.2 * np.random.default_rng(3).uniform(-1, 1, size=inner(x).shape) * d).astype(x.dtype)
+    for axis, peri, L in ((2, p.xPeri, p.Lx + p.dx), (1, p.yPeri, p.Ly + p.dy), (0, p.zPeri, p.Lz + p.dz)):
+        if peri:                         # the ghosts of a periodic face are the images
+            v = np.moveaxis(x, axis, 0)
+            v[0], v[-1] = v[-2], v[1]
+            v[0, ..., 2 - axis] -= x.dtype.type(L)
+            v[-1, ..., 2 - axis] += x.dtype.type(L)
+    g, o = Relaxation(p), Oracle(p, B0, x)
+    g.upload(x, B0)
+    g.refresh()
+    o.refresh()
+    f, w = g.download(), o.get()
+    g.close()
+    o.close()
+    tol = 1e-12 if p.precision == 64 else 1e-5
+    assert relerr(inner(f["B"]), inner(w["B"])) < tol and relerr(f["J"], w["J"]) < 50 * tol
+    assert relerr(inner(f["detJac"]), inner(w["detJac"])) < tol
+    for axis, peri in ((0, p.zPeri), (1, p.yPeri), (2, p.xPeri)):
+        for side in (0, -1):
+            ix = [slice(1, -1)] * 3
+            ix[axis] = side
+            for k in ("B", "detJac"):
+                assert relerr(f[k][tuple(ix)], w[k][tuple(ix)]) < tol, (axis, side, k)
